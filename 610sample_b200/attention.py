@@ -13,6 +13,11 @@ first backward is itself differentiable; its ``backward`` is the double backward
 treated as functions of Q, K, V, hence ``None`` for the saved O and L.  Third
 order is not supported.
 
+``flash_attention_v7`` itself runs the same two functions from their C++ form in the
+extension (``attention_cuda.flash_attention``), which the autograd engine executes
+without the interpreter; the Python classes are the reference-facing surface for
+code that applies them directly.
+
 Additive extension: ``mask_mode`` (0 = reference mask, 1 = no mask) as a trailing
 keyword of ``flash_attention_v7``.
 
@@ -90,4 +95,8 @@ def flash_attention_v7(Q, K, V, window_size, chunk_id, mask_mode=0):
     ``N_q == N_kv == N, window_size >= N, chunk_id == 0``.
     Returns O: (B, H, N_q, D).
     """
+    fused = getattr(_attention_cuda, "flash_attention", None)
+    if fused is not None:
+        return fused(Q, K, V, window_size, chunk_id, mask_mode)
+    # a module with the reference's three functions only (an older build, a test's stand-in)
     return FlashAttentionV7.apply(Q, K, V, window_size, chunk_id, mask_mode)
