@@ -15,8 +15,10 @@
 #include <torch/extension.h>
 #include <torch/csrc/autograd/custom_function.h>
 #include <ATen/cuda/CUDAContext.h>
+#include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAGuard.h>
 
+#include <atomic>
 #include <cstdio>
 #include <mutex>
 #include <vector>
@@ -41,6 +43,13 @@ torch::Tensor dense(const torch::Tensor& t) {
   if (reinterpret_cast<uintptr_t>(c.data_ptr()) % 16 != 0) c = c.clone();
   return c;
 }
+
+// New tensors of a contiguous shape on t's device, straight from the caching allocator: the
+// dispatcher's factory functions take twice as long, and a call makes three to five tensors.
+torch::Tensor fresh(at::IntArrayRef sizes, at::ScalarType type, const torch::Tensor& t) {
+  return at::detail::empty_cuda(sizes, type, t.device(), c10::nullopt);
+}
+torch::Tensor fresh_like(const torch::Tensor& t) { return fresh(t.sizes(), t.scalar_type(), t); }
 
 void check_qkv(const torch::Tensor& Q, const torch::Tensor& K, const torch::Tensor& V) {
   TORCH_CHECK(Q.is_cuda(), "Q must be a CUDA tensor");
@@ -87,15 +96,19 @@ void check_rc(int rc, const char* what) {
 // first call that starts after it, and the good path costs one read of host memory.
 uint32_t* status_mirror(int device) {
   static torch::Tensor words[64];
+  static std::atomic<uint32_t*> known[64];
   static std::mutex mu;
   TORCH_CHECK(device >= 0 && device < 64, "device index out of range");
+  if (uint32_t* w = known[device].load(std::memory_order_acquire)) return w;
   std::lock_guard<std::mutex> lock(mu);
   if (!words[device].defined()) {
     words[device] = torch::zeros({1}, torch::dtype(torch::kInt32).pinned_memory(true));
     check_rc(attn_b200_set_status_mirror(reinterpret_cast<uint32_t*>(words[device].data_ptr<int32_t>())),
              "attn_b200_set_status_mirror");
   }
-  return reinterpret_cast<uint32_t*>(words[device].data_ptr<int32_t>());
+  uint32_t* w = reinterpret_cast<uint32_t*>(words[device].data_ptr<int32_t>());
+  known[device].store(w, std::memory_order_release);
+  return w;
 }
 
 void raise_if_earlier_call_timed_out(int device) {
@@ -119,8 +132,8 @@ std::vector<torch::Tensor> v7_forward_cuda(torch::Tensor Q, torch::Tensor K, tor
   raise_if_earlier_call_timed_out(Q.device().index());
   Q = dense(Q); K = dense(K); V = dense(V);
   attn_shape_t s = make_shape(Q, K, window_size, chunk_id, mask_mode, impl);
-  auto O = torch::empty_like(Q);
-  auto L = torch::empty({Q.size(0), Q.size(1), Q.size(2)}, Q.options().dtype(torch::kFloat32));
+  auto O = fresh_like(Q);
+  auto L = fresh({Q.size(0), Q.size(1), Q.size(2)}, at::kFloat, Q);
   check_rc(attn_b200_forward(&s, Q.data_ptr(), K.data_ptr(), V.data_ptr(), O.data_ptr(), L.data_ptr<float>(),
                              at::cuda::getCurrentCUDAStream().stream()),
            "v7_forward");
@@ -139,11 +152,10 @@ std::vector<torch::Tensor> v7_backward_cuda(torch::Tensor dO, torch::Tensor Q, t
   raise_if_earlier_call_timed_out(Q.device().index());
   dO = dense(dO); Q = dense(Q); K = dense(K); V = dense(V); O = dense(O); L = L.contiguous();
   attn_shape_t s = make_shape(Q, K, window_size, chunk_id, mask_mode, impl);
-  auto dQ = torch::empty_like(Q);
-  auto dK = torch::empty_like(K);
-  auto dV = torch::empty_like(V);
-  auto scratch = torch::empty({(int64_t)(attn_b200_backward_scratch_bytes(&s) / sizeof(float)) + 4},
-                              Q.options().dtype(torch::kFloat32));
+  auto dQ = fresh_like(Q);
+  auto dK = fresh_like(K);
+  auto dV = fresh_like(V);
+  auto scratch = fresh({(int64_t)(attn_b200_backward_scratch_bytes(&s) / sizeof(float)) + 4}, at::kFloat, Q);
   check_rc(attn_b200_backward(&s, dO.data_ptr(), Q.data_ptr(), K.data_ptr(), V.data_ptr(), O.data_ptr(),
                               L.data_ptr<float>(), dQ.data_ptr(), dK.data_ptr(), dV.data_ptr(),
                               scratch.data_ptr<float>(), at::cuda::getCurrentCUDAStream().stream()),
@@ -167,12 +179,11 @@ std::vector<torch::Tensor> v7_double_backward_cuda(torch::Tensor g_dQ, torch::Te
   g_dQ = dense(g_dQ); g_dK = dense(g_dK); g_dV = dense(g_dV);
   dO = dense(dO); Q = dense(Q); K = dense(K); V = dense(V); L = L.contiguous();
   attn_shape_t s = make_shape(Q, K, window_size, chunk_id, mask_mode, impl);
-  auto g_dO = torch::empty_like(Q);
-  auto g_Q = torch::empty_like(Q);
-  auto g_K = torch::empty_like(K);
-  auto g_V = torch::empty_like(V);
-  auto scratch = torch::empty({(int64_t)(attn_b200_double_backward_scratch_bytes(&s) / sizeof(float)) + 4},
-                              Q.options().dtype(torch::kFloat32));
+  auto g_dO = fresh_like(Q);
+  auto g_Q = fresh_like(Q);
+  auto g_K = fresh_like(K);
+  auto g_V = fresh_like(V);
+  auto scratch = fresh({(int64_t)(attn_b200_double_backward_scratch_bytes(&s) / sizeof(float)) + 4}, at::kFloat, Q);
   check_like(O, Q, "O");
   O = dense(O);
   check_rc(attn_b200_double_backward(&s, g_dQ.data_ptr(), g_dK.data_ptr(), g_dV.data_ptr(), dO.data_ptr(),
@@ -277,7 +288,7 @@ torch::Tensor qk_norm_rope_cuda(torch::Tensor x, c10::optional<torch::Tensor> we
     TORCH_CHECK(weight->is_cuda() && weight->numel() == x.size(2), "weight must be a CUDA tensor [d]");
     w = weight->to(x.scalar_type()).contiguous();
   }
-  auto out = torch::empty({1, x.size(1), x.size(0), x.size(2)}, x.options());
+  auto out = fresh({1, x.size(1), x.size(0), x.size(2)}, x.scalar_type(), x);
   check_rc(attn_b200_qk_norm_rope(x.data_ptr(), w.defined() ? w.data_ptr() : nullptr, freqs.data_ptr<float>(), out.data_ptr(),
                                   (int32_t)x.size(0), (int32_t)x.size(1), (int32_t)x.size(2), pos0, norm_from, (float)eps,
                                   dtype_code(x), at::cuda::getCurrentCUDAStream().stream()),

@@ -4,6 +4,7 @@
 #include "attn_launch.h"
 #include "tc_primitives.cuh"
 
+#include <atomic>
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
@@ -29,23 +30,28 @@ int fail(int code, const char* fmt, ...) {
 __device__ attn::tc::StatusBlock g_status_block = {0u, 0u, nullptr};
 
 constexpr int kMaxDevices = 64;
-unsigned int* g_status_ptr[kMaxDevices] = {nullptr};
-std::mutex g_status_mutex;
+std::atomic<unsigned int*> g_status_ptr[kMaxDevices];
+
+// `dev` is the current device; two threads that find the slot empty store the same address
+int status_pointer(int dev, unsigned int** out) {
+  if (dev < 0 || dev >= kMaxDevices) return fail(ATTN_EINVAL, "device index %d out of range", dev);
+  unsigned int* known = g_status_ptr[dev].load(std::memory_order_acquire);
+  if (known == nullptr) {
+    void* p = nullptr;
+    cudaError_t e = cudaGetSymbolAddress(&p, g_status_block);
+    if (e != cudaSuccess) return fail(ATTN_ECUDA, "cudaGetSymbolAddress: %s", cudaGetErrorString(e));
+    known = static_cast<unsigned int*>(p);
+    g_status_ptr[dev].store(known, std::memory_order_release);
+  }
+  *out = known;
+  return ATTN_OK;
+}
 
 int status_pointer(unsigned int** out) {
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return fail(ATTN_ECUDA, "cudaGetDevice: %s", cudaGetErrorString(e));
-  if (dev < 0 || dev >= kMaxDevices) return fail(ATTN_EINVAL, "device index %d out of range", dev);
-  std::lock_guard<std::mutex> lock(g_status_mutex);
-  if (g_status_ptr[dev] == nullptr) {
-    void* p = nullptr;
-    e = cudaGetSymbolAddress(&p, g_status_block);
-    if (e != cudaSuccess) return fail(ATTN_ECUDA, "cudaGetSymbolAddress: %s", cudaGetErrorString(e));
-    g_status_ptr[dev] = static_cast<unsigned int*>(p);
-  }
-  *out = g_status_ptr[dev];
-  return ATTN_OK;
+  return status_pointer(dev, out);
 }
 
 int check_shape(const attn_shape_t* s) {
@@ -80,6 +86,7 @@ attn::Geometry make_geometry(const attn_shape_t* s) {
   g.window = s->window_size > (1 << 30) ? (1 << 30) : s->window_size;
   g.mask_mode = s->mask_mode;
   g.head_group = 1;
+  g.beside = 0;
   g.scale = 1.0f / sqrtf((float)s->D);
   g.scale_log2e = g.scale * attn::kLog2e;
   return g;
@@ -125,18 +132,20 @@ int run(int op, const attn_shape_t* s, attn::Tensors& t, void* stream, int phase
   // driver call and fails with "invalid context" on a thread that has made no runtime
   // call yet (e.g. a freshly started autograd worker thread).  cudaSetDevice on the current
   // device does that and, unlike a null cudaFree, is legal while a stream is being captured.
-  {
-    int dev = 0;
-    cudaError_t e0 = cudaGetDevice(&dev);
-    if (e0 == cudaSuccess) e0 = cudaSetDevice(dev);
-    if (e0 != cudaSuccess) return fail(ATTN_ECUDA, "binding the device context: %s", cudaGetErrorString(e0));
+  // Once per thread and device.
+  static thread_local int bound_device = -1;
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess && dev != bound_device) {
+    e = cudaSetDevice(dev);
+    if (e == cudaSuccess) bound_device = dev;
   }
-  int rc = status_pointer(&t.status);
+  if (e != cudaSuccess) return fail(ATTN_ECUDA, "binding the device context: %s", cudaGetErrorString(e));
+  int rc = status_pointer(dev, &t.status);
   if (rc != ATTN_OK) return rc;
   const bool use_tc = s->impl == ATTN_IMPL_TENSOR ||
                       (s->impl == ATTN_IMPL_AUTO && attn::tc_supported(s->dtype, s->D));
   cudaStream_t cs = static_cast<cudaStream_t>(stream);
-  cudaError_t e;
   if (use_tc) {
     const char* why = nullptr;
     e = attn::launch_tc(op, s->dtype, g, t, cs, &tl_launches, &why, phases);
@@ -302,8 +311,8 @@ int attn_b200_double_backward_static(const attn_shape_t* shape, const void* g_dQ
     t.dot3 = scratch + 2 * (size_t)rows;
   }
   // the common tail of every entry point (context binding, empty problems, kernel-family
-  // dispatch); SERIAL keeps every launch on the caller's stream, so no helper stream is created
-  return run(attn::OP_DOUBLE_BACKWARD, shape, t, stream, attn::HVP_PHASE_ALL | attn::HVP_PHASE_SERIAL);
+  // dispatch)
+  return run(attn::OP_DOUBLE_BACKWARD, shape, t, stream);
 }
 
 int attn_b200_last_launch_count(void) { return tl_launches; }

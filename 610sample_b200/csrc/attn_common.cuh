@@ -34,6 +34,9 @@ struct Geometry {
   // tile, heavy tiles first, over all heads of the group.  Large groups balance the SMs (longest
   // work first), small groups keep the streamed tensors of the heads in flight inside the L2.
   int head_group;
+  // 1: this launch shares the GPU with its predecessor in the stream, whose results it does not
+  // read (dQ beside dK/dV, g_Q beside g_K/g_V); see tc_common.cuh
+  int beside;
   float scale;       // 1/sqrt(D)
   float scale_log2e; // scale * log2(e)
 };

@@ -32,6 +32,8 @@ template <> __device__ __forceinline__ float2 widen_pair<__half>(uint32_t w) {
 template <typename T, int G>
 __global__ void __launch_bounds__(256)
 rowdot_kernel(const T* __restrict__ a, const T* __restrict__ b, float* __restrict__ out, long long rows, int D) {
+  pdl_wait();
+  pdl_trigger();
   const int sub = threadIdx.x % G;
   const long long r0 = ((long long)blockIdx.x * (256 / G) + threadIdx.x / G) * kRowdotRows;
   const bool lane_on = sub * 8 < D;
@@ -66,10 +68,8 @@ static cudaError_t launch_rowdot(const T* a, const T* b, float* out, long long r
   const long long rows_per_cta = (long long)(256 / G) * kRowdotRows;
   const long long ctas = (rows + rows_per_cta - 1) / rows_per_cta;
   if (ctas > 0x7fffffffLL) return cudaErrorInvalidValue;
-  if (G == 4) rowdot_kernel<T, 4><<<(unsigned)ctas, 256, 0, s>>>(a, b, out, rows, D);
-  else if (G == 8) rowdot_kernel<T, 8><<<(unsigned)ctas, 256, 0, s>>>(a, b, out, rows, D);
-  else rowdot_kernel<T, 16><<<(unsigned)ctas, 256, 0, s>>>(a, b, out, rows, D);
-  return cudaGetLastError();
+  auto kern = G == 4 ? rowdot_kernel<T, 4> : G == 8 ? rowdot_kernel<T, 8> : rowdot_kernel<T, 16>;
+  return launch_pdl(kern, (unsigned)ctas, 256, 0, s, a, b, out, rows, D);
 }
 
 // ---------------------------------------------------------------------------
@@ -238,38 +238,30 @@ static bool encode_map(CUtensorMap* map, const void* ptr, int is_bf16, long long
   return r == CUDA_SUCCESS;
 }
 
-bool encode_all_maps(TmaMaps* maps, int op, const Geometry& g, const Tensors& t, int is_bf16, const char** err) {
-  memset(maps, 0, sizeof(*maps));
-  const void* ptrs[T_COUNT] = {t.Q, t.K, t.V, t.dO, t.g_dQ, t.g_dK, t.g_dV};
-  const int rows[T_COUNT] = {g.N_q, g.N_kv, g.N_kv, g.N_q, g.N_q, g.N_kv, g.N_kv};
-  for (int i = 0; i < T_COUNT; ++i) {
-    const void* p = ptrs[i] ? ptrs[i] : t.Q;   // unused maps still need a valid encoding
-    const int r = ptrs[i] ? rows[i] : g.N_q;
-    if (!encode_map(&maps->m[i], p, is_bf16, g.BH, r, g.D)) {
-      *err = tl_encode_error;
-      return false;
-    }
-  }
-  // outputs of this operation, stored by TMA in boxes of 64 columns x 128 rows
+// The maps an operation uses; the others are left alone.
+bool encode_maps(TmaMaps* maps, int op, const Geometry& g, const Tensors& t, int is_bf16, const char** err) {
+  const void* ins[T_COUNT] = {t.Q, t.K, t.V, t.dO, t.g_dQ, t.g_dK, t.g_dV};
+  const int in_rows[T_COUNT] = {g.N_q, g.N_kv, g.N_kv, g.N_q, g.N_q, g.N_kv, g.N_kv};
+  const int n_in = op == OP_FORWARD ? 3 : op == OP_BACKWARD ? 4 : T_COUNT;
+  // outputs, stored by TMA in boxes of 64 columns x 128 rows
   void* outs[TO_COUNT] = {nullptr, nullptr, nullptr, nullptr};
   int out_rows[TO_COUNT] = {g.N_q, g.N_q, g.N_kv, g.N_kv};
+  int n_out = TO_COUNT;
   if (op == OP_FORWARD) {
     outs[TO_O] = t.out_O;
+    n_out = 1;
   } else if (op == OP_BACKWARD) {
     outs[TO_dQ] = t.out_dQ; outs[TO_dK] = t.out_dK; outs[TO_dV] = t.out_dV;
     out_rows[TO_dK] = g.N_kv; out_rows[TO_dV] = g.N_kv;
+    n_out = 3;
   } else {
     outs[TO_gdO] = t.out_g_dO; outs[TO_gQ] = t.out_g_Q; outs[TO_gK] = t.out_g_K; outs[TO_gV] = t.out_g_V;
   }
-  for (int i = 0; i < TO_COUNT; ++i) {
-    void* p = outs[i] ? outs[i] : const_cast<void*>(t.Q);
-    const int r = outs[i] ? out_rows[i] : g.N_q;
-    if (!encode_map(&maps->out[i], p, is_bf16, g.BH, r, g.D, 128)) {
-      *err = tl_encode_error;
-      return false;
-    }
-  }
-  return true;
+  bool ok = true;
+  for (int i = 0; i < n_in && ok; ++i) ok = encode_map(&maps->m[i], ins[i], is_bf16, g.BH, in_rows[i], g.D);
+  for (int i = 0; i < n_out && ok; ++i) ok = encode_map(&maps->out[i], outs[i], is_bf16, g.BH, out_rows[i], g.D, 128);
+  if (!ok) *err = tl_encode_error;
+  return ok;
 }
 
 cudaError_t launch_hvp_col(int D, int is_bf16, const TmaMaps& maps, const Geometry& g, const Tensors& t,
@@ -281,71 +273,11 @@ cudaError_t launch_fwd_bwd(int kind, int D, int is_bf16, const TmaMaps& maps, co
                            cudaStream_t s);
 cudaError_t launch_fwd(int D, int is_bf16, const TmaMaps& maps, const Geometry& g, const Tensors& t, cudaStream_t s);
 
-// Kernels of one operation that do not depend on one another (g_Q and g_K/g_V of the double
-// backward; dQ and dK/dV of the backward) run side by side: the second is launched on a helper
-// stream of the device between an event fork and an event join on the caller's stream, so the
-// SMs that one kernel's last CTAs leave idle take CTAs of the other.  One helper stream and two
-// events per device, created on first use and shared by every caller stream and host thread (the
-// mutex covers one fork ... join enqueue).  A stream that is being captured is never forked: a
-// capture would pull the shared helper stream into the graph until the capture ends, long after
-// the mutex is released, and an eager call of another thread in that window would either
-// invalidate the capture or be merged into it.  Under capture, and whenever the helper cannot be
-// had, both launches stay on the caller's stream.
-struct Helper {
-  cudaStream_t stream = nullptr;
-  cudaEvent_t fork = nullptr, join = nullptr;
-  bool tried = false;
-  std::mutex in_use;   // host threads share the events: one fork ... join sequence at a time
-};
-
-static Helper* helper_for_current_device() {
-  static Helper helpers[64];
-  static std::mutex mu;
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
-  std::lock_guard<std::mutex> lock(mu);
-  Helper& h = helpers[dev];
-  if (!h.tried) {
-    h.tried = true;
-    if (cudaStreamCreateWithFlags(&h.stream, cudaStreamNonBlocking) != cudaSuccess ||
-        cudaEventCreateWithFlags(&h.fork, cudaEventDisableTiming) != cudaSuccess ||
-        cudaEventCreateWithFlags(&h.join, cudaEventDisableTiming) != cudaSuccess) {
-      (void)cudaGetLastError();
-      h.stream = nullptr;
-    }
-  }
-  return h.stream != nullptr ? &h : nullptr;
-}
-
-// first(s) and second(helper stream) between fork and join; serial on s without a helper
-template <typename F1, typename F2>
-static cudaError_t run_side_by_side(cudaStream_t s, bool allow_helper, F1 first, F2 second) {
-  if (allow_helper) {
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(s, &cap) != cudaSuccess) {   // e.g. the legacy stream while another stream captures
-      (void)cudaGetLastError();
-      allow_helper = false;
-    } else if (cap != cudaStreamCaptureStatusNone) {
-      allow_helper = false;
-    }
-  }
-  Helper* h = allow_helper ? helper_for_current_device() : nullptr;
-  if (h == nullptr) {
-    cudaError_t e = first(s);
-    return e == cudaSuccess ? second(s) : e;
-  }
-  std::lock_guard<std::mutex> lock(h->in_use);
-  if (cudaEventRecord(h->fork, s) != cudaSuccess || cudaStreamWaitEvent(h->stream, h->fork, 0) != cudaSuccess) {
-    (void)cudaGetLastError();
-    cudaError_t e = first(s);
-    return e == cudaSuccess ? second(s) : e;
-  }
-  cudaError_t e1 = first(s);
-  cudaError_t e2 = second(h->stream);
-  // the join is made even after a failed launch, so that the helper stream never outlives the call
-  cudaError_t ej = cudaEventRecord(h->join, h->stream);
-  if (ej == cudaSuccess) ej = cudaStreamWaitEvent(s, h->join, 0);
-  return e1 != cudaSuccess ? e1 : e2 != cudaSuccess ? e2 : ej;
+// dQ beside dK/dV and g_Q beside g_K/g_V: the kernel with the longer CTAs first, the other one on
+// the SMs its last CTAs leave idle (tc_common.cuh)
+static Geometry beside(Geometry g) {
+  g.beside = 1;
+  return g;
 }
 
 template <typename T>
@@ -362,23 +294,14 @@ static cudaError_t launch_op(int op, const TmaMaps& maps, const Geometry& g, con
     if (rows > 0) {
       e = launch_rowdot<T>((const T*)t.dO, (const T*)t.O, t.Dv, rows, g.D, s);
     }
-    if (e == cudaSuccess)
-      e = run_side_by_side(s, true,
-                           [&](cudaStream_t q) { return launch_fwd_bwd(2, D, bf, maps, g, t, q); },     // dQ
-                           [&](cudaStream_t q) { return launch_fwd_bwd(3, D, bf, maps, g, t, q); });    // dK, dV
+    if (e == cudaSuccess) e = launch_fwd_bwd(3, D, bf, maps, g, t, s);                // dK, dV
+    if (e == cudaSuccess) e = launch_fwd_bwd(2, D, bf, maps, beside(g), t, s);        // dQ
     *n = 3;
   } else {
     if (phases & HVP_PHASE_PRE) { e = launch_hvp_row(0, D, bf, maps, g, t, s); ++*n; }                        // scalars + g_dO
     const bool row = (phases & HVP_PHASE_ROW) != 0, col = (phases & HVP_PHASE_COL) != 0;
-    if (e == cudaSuccess && row && col) {
-      e = run_side_by_side(s, (phases & HVP_PHASE_SERIAL) == 0,
-                           [&](cudaStream_t q) { return launch_hvp_col(D, bf, maps, g, t, q); },        // g_K, g_V
-                           [&](cudaStream_t q) { return launch_hvp_row(1, D, bf, maps, g, t, q); });    // g_Q
-      *n += 2;
-    } else {
-      if (e == cudaSuccess && row) { e = launch_hvp_row(1, D, bf, maps, g, t, s); ++*n; }  // g_Q
-      if (e == cudaSuccess && col) { e = launch_hvp_col(D, bf, maps, g, t, s); ++*n; }     // g_K, g_V
-    }
+    if (e == cudaSuccess && col) { e = launch_hvp_col(D, bf, maps, g, t, s); ++*n; }                          // g_K, g_V
+    if (e == cudaSuccess && row) { e = launch_hvp_row(1, D, bf, maps, col ? beside(g) : g, t, s); ++*n; }     // g_Q
   }
   return e;
 }
@@ -395,7 +318,7 @@ cudaError_t launch_tc(int op, int dtype, const Geometry& g, const Tensors& t, cu
   *err = nullptr;
   TmaMaps maps;
   const int bf = dtype == 1;
-  if (!encode_all_maps(&maps, op, g, t, bf, err)) return cudaErrorInvalidValue;
+  if (!encode_maps(&maps, op, g, t, bf, err)) return cudaErrorInvalidValue;
   return bf ? launch_op<__nv_bfloat16>(op, maps, g, t, s, launches, phases)
             : launch_op<__half>(op, maps, g, t, s, launches, phases);
 }

@@ -137,7 +137,14 @@ fb_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Tensors 
   auto bar_rb_full = [&](int b) { return smem_u32(&ctl->rb_full[b]); };
   auto bar_op_full = [&](int b) { return smem_u32(&ctl->op_full[b]); };
 
-  if (threadIdx.x == 0) {
+  // one barrier round of set-up: the producer initialises the mbarriers and, once the kernels this
+  // one depends on are complete, requests the stationary tiles and the first streamed tile (their
+  // latency is the longest item of the prologue); meanwhile an issuing warp allocates tensor memory
+  if (warp == kProducerWarp && lane == 0) {
+    for (int x = 0; x < 2; ++x) {
+      tma_prefetch_desc(&maps.m[CF::stat_tensor(x)]);
+      tma_prefetch_desc(&maps.m[CF::stream_tensor(x)]);
+    }
     mbar_init(bar_staging_full, 1);
     mbar_init(bar_stat_ready, kMathWarps);
     for (int s = 0; s < CF::kStages; ++s) {
@@ -154,12 +161,38 @@ fb_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Tensors 
     }
     mbar_init(bar_acc_done, 1);
     ctl->abort_flag = 0u;
-    ctl->tmem_base = 0u;
     fence_barrier_init();
     fence_proxy_async_smem();
   }
-  __syncthreads();
+  // the streamed tile `it` into its stage
+  auto request_tile = [&](int it) {
+    const int st = it % CF::kStages;
+    mbar_arrive_expect_tx(bar_stream_full(st), CF::kStageBytes);
+    const uint32_t stage = strm_base + st * CF::kStageBytes;
+#pragma unroll
+    for (int s = 0; s < CF::kNStream; ++s)
+#pragma unroll
+      for (int a = 0; a < kAtoms; ++a)
+        tma_load_3d(stage + CF::stream_off(s, a), &maps.m[CF::stream_tensor(s)], a * 64, (t_begin + it) * BN, bh,
+                    bar_stream_full(st));
+  };
   if (warp == kFbMmaWarp) tmem_alloc(smem_u32(&ctl->tmem_base), kTmemCols);
+  pdl_begin(g);
+  if (warp == kProducerWarp && lane == 0) {
+    pdl_trigger();
+    if (n_iter > 0) {
+      mbar_arrive_expect_tx(bar_staging_full, CF::kStagingBytes);
+#pragma unroll
+      for (int x = 0; x < CF::kNStat; ++x)
+#pragma unroll
+        for (int a = 0; a < kAtoms; ++a)
+#pragma unroll
+          for (int h = 0; h < 2; ++h)
+            tma_load_3d(staging + (x * kAtoms + a) * kAtomBytesStat + h * kAtomBytesStrm,
+                        &maps.m[CF::stat_tensor(x)], a * 64, r0 + h * 64, bh, bar_staging_full);
+      request_tile(0);
+    }
+  }
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
@@ -171,29 +204,11 @@ fb_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Tensors 
   // =========================================================================
   if (warp == kProducerWarp) {
     if (lane == 0 && n_iter > 0) {
-      for (int i = 0; i < T_COUNT; ++i) tma_prefetch_desc(&maps.m[i]);
-      mbar_arrive_expect_tx(bar_staging_full, CF::kStagingBytes);
-#pragma unroll
-      for (int x = 0; x < CF::kNStat; ++x)
-#pragma unroll
-        for (int a = 0; a < kAtoms; ++a)
-#pragma unroll
-          for (int h = 0; h < 2; ++h)
-            tma_load_3d(staging + (x * kAtoms + a) * kAtomBytesStat + h * kAtomBytesStrm,
-                        &maps.m[CF::stat_tensor(x)], a * 64, r0 + h * 64, bh, bar_staging_full);
       bool ok = true;
-      for (int it = 0; it < n_iter; ++it) {
-        const int st = it % CF::kStages;
-        ok = mbar_wait(bar_stream_empty(st), ((it / CF::kStages) & 1) ^ 1, abort_flag, t.status, wait_code(KCODE, 1));
+      for (int it = 1; it < n_iter; ++it) {     // tile 0 was requested above
+        ok = mbar_wait(bar_stream_empty(it % CF::kStages), ((it / CF::kStages) & 1) ^ 1, abort_flag, t.status, wait_code(KCODE, 1));
         if (!ok) break;
-        mbar_arrive_expect_tx(bar_stream_full(st), CF::kStageBytes);
-        const uint32_t stage = strm_base + st * CF::kStageBytes;
-#pragma unroll
-        for (int s = 0; s < CF::kNStream; ++s)
-#pragma unroll
-          for (int a = 0; a < kAtoms; ++a)
-            tma_load_3d(stage + CF::stream_off(s, a), &maps.m[CF::stream_tensor(s)], a * 64,
-                        (t_begin + it) * BN, bh, bar_stream_full(st));
+        request_tile(it);
       }
       if (!ok) {   // give copies already in flight a bounded chance to land before the CTA exits
         const long long t0 = clock64();
@@ -620,6 +635,7 @@ fb_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Tensors 
     tc_fence_after_sync();
     tmem_dealloc(tmem_base, kTmemCols);
   }
+  pdl_end(g);
 }
 
 template <int KIND, int D, typename T>
@@ -635,10 +651,9 @@ static cudaError_t launch_fb(const TmaMaps& maps, const Geometry& g_in, const Te
   // tensor-memory allocation never waits for a co-resident CTA
   const size_t smem = CF::kSmemBytes < 122880u ? 122880u : CF::kSmemBytes;
   auto kern = fb_kernel<KIND, D, T>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return e;
-  kern<<<(unsigned)ctas, kFbThreads, smem, s>>>(maps, g, t);
-  return cudaGetLastError();
+  static std::atomic<unsigned long long> smem_set{0};
+  cudaError_t e = set_smem_once(kern, smem, smem_set);
+  return e != cudaSuccess ? e : launch_pdl(kern, (unsigned)ctas, kFbThreads, smem, s, maps, g, t);
 }
 
 template <int D, typename T>

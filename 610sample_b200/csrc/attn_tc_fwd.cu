@@ -114,7 +114,13 @@ fwd_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Tensors
   auto bar_p_full = [&](int b) { return smem_u32(&ctl->p_full[b]); };
   auto bar_pv_done = [&](int b) { return smem_u32(&ctl->pv_done[b]); };
 
-  if (threadIdx.x == 0) {
+  // one barrier round of set-up: the producer initialises the mbarriers and, once the kernels this
+  // one depends on are complete, requests Q and the first K tile (their latency is the longest item
+  // of the prologue); meanwhile an issuing warp allocates tensor memory
+  if (warp == kProducerWarp && lane == 0) {
+    tma_prefetch_desc(&maps.m[T_Q]);
+    tma_prefetch_desc(&maps.m[T_K]);
+    tma_prefetch_desc(&maps.m[T_V]);
     mbar_init(bar_staging_full, 1);
     mbar_init(bar_q_ready, kMathWarps);
     for (int s = 0; s < CF::kStages; ++s)
@@ -129,11 +135,9 @@ fwd_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Tensors
     }
     mbar_init(bar_acc_done, 1);
     ctl->abort_flag = 0u;
-    ctl->tmem_base = 0u;
     fence_barrier_init();
     fence_proxy_async_smem();
   }
-  __syncthreads();
 
   // one half of the stage of tile `it`: K (h = 0) or V (h = 1)
   auto request_half = [&](int it, int h) {
@@ -145,19 +149,20 @@ fwd_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Tensors
       tma_load_3d(stage + CF::stream_off(h, a), &maps.m[h == 0 ? T_K : T_V], a * 64, (t_begin + it) * BN, bh,
                   bar_stream_full(h, st));
   };
-  // Q and the first K tile are requested before the tensor-memory allocation and the second
-  // barrier: their latency is the longest item of the prologue
-  if (warp == kProducerWarp && lane == 0 && n_iter > 0) {
-    tma_prefetch_desc(&maps.m[T_Q]); tma_prefetch_desc(&maps.m[T_K]); tma_prefetch_desc(&maps.m[T_V]);
-    mbar_arrive_expect_tx(bar_staging_full, CF::kStagingBytes);
-#pragma unroll
-    for (int a = 0; a < kAtoms; ++a)
-#pragma unroll
-      for (int h = 0; h < 2; ++h)
-        tma_load_3d(staging + a * kAtomBytesStat + h * kAtomBytesStrm, &maps.m[T_Q], a * 64, r0 + h * 64, bh, bar_staging_full);
-    request_half(0, 0);
-  }
   if (warp == kFwdSWarp) tmem_alloc(smem_u32(&ctl->tmem_base), kTmemCols);
+  pdl_begin(g);
+  if (warp == kProducerWarp && lane == 0) {
+    pdl_trigger();
+    if (n_iter > 0) {
+      mbar_arrive_expect_tx(bar_staging_full, CF::kStagingBytes);
+#pragma unroll
+      for (int a = 0; a < kAtoms; ++a)
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+          tma_load_3d(staging + a * kAtomBytesStat + h * kAtomBytesStrm, &maps.m[T_Q], a * 64, r0 + h * 64, bh, bar_staging_full);
+      request_half(0, 0);
+    }
+  }
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
@@ -448,6 +453,7 @@ fwd_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Tensors
     tc_fence_after_sync();
     tmem_dealloc(tmem_base, kTmemCols);
   }
+  pdl_end(g);
 }
 
 template <int D, typename T>
@@ -462,10 +468,9 @@ static cudaError_t launch_fwd_one(const TmaMaps& maps, const Geometry& g_in, con
   // tensor-memory allocation never waits for a co-resident CTA
   const size_t smem = CF::kSmemBytes < 122880u ? 122880u : CF::kSmemBytes;
   auto kern = fwd_kernel<D, T>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return e;
-  kern<<<(unsigned)ctas, kFwdThreads, smem, s>>>(maps, g, t);
-  return cudaGetLastError();
+  static std::atomic<unsigned long long> smem_set{0};
+  cudaError_t e = set_smem_once(kern, smem, smem_set);
+  return e != cudaSuccess ? e : launch_pdl(kern, (unsigned)ctas, kFwdThreads, smem, s, maps, g, t);
 }
 
 // forward: O and L in one launch

@@ -129,7 +129,11 @@ hvp_col_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Ten
   auto bar_stream_full_do = [&](int s) { return smem_u32(&ctl->stream_full_do[s]); };
   auto bar_stream_empty = [&](int s) { return smem_u32(&ctl->stream_empty[s]); };
 
-  if (threadIdx.x == 0) {
+  // one barrier round of set-up: the producer initialises the mbarriers and, once the kernels this
+  // one depends on are complete, requests the stationary tiles and the first streamed tile (their
+  // latency is the longest item of the prologue); meanwhile an issuing warp allocates tensor memory
+  if (warp == kProducerWarp && lane == 0) {
+    for (int i = 0; i < T_COUNT; ++i) tma_prefetch_desc(&maps.m[i]);
     mbar_init(bar_stat_full, 1);
     for (int s = 0; s < CF::kStages; ++s) {
       mbar_init(bar_stream_full(s), 1);
@@ -144,13 +148,12 @@ hvp_col_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Ten
     mbar_init(bar_op_half, kMathWarps);
     mbar_init(bar_acc_done, 1);
     ctl->abort_flag = 0u;
-    ctl->tmem_base = 0u;
     fence_barrier_init();
     fence_proxy_async_smem();
   }
-  __syncthreads();
-  // the stationary tiles and the first streamed tile are requested before the tensor-memory
-  // allocation and the second barrier: their latency is the longest item of the prologue
+  if (warp == kColMmaWarp) tmem_alloc(smem_u32(&ctl->tmem_base), kTmemCols);
+  pdl_begin(g);
+  if (warp == kProducerWarp && lane == 0) pdl_trigger();
   if (warp == kProducerWarp && lane == 0 && n_iter > 0) {
     mbar_arrive_expect_tx(bar_stat_full, CF::kStatBytes);
     mbar_arrive_expect_tx(bar_stream_full(0), 2 * kAtoms * kAtomBytesStrm);
@@ -173,7 +176,6 @@ hvp_col_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Ten
       }
     }
   }
-  if (warp == kColMmaWarp) tmem_alloc(smem_u32(&ctl->tmem_base), kTmemCols);
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
@@ -552,6 +554,7 @@ hvp_col_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Ten
     tc_fence_after_sync();
     tmem_dealloc(tmem_base, kTmemCols);
   }
+  pdl_end(g);
 }
 
 template <int D, typename T>
@@ -566,10 +569,9 @@ static cudaError_t launch_col(const TmaMaps& maps, const Geometry& g_in, const T
   // tensor-memory allocation never waits for a co-resident CTA
   const size_t smem = CF::kSmemBytes < 122880u ? 122880u : CF::kSmemBytes;
   auto kern = hvp_col_kernel<D, T>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return e;
-  kern<<<(unsigned)ctas, kColThreads, smem, s>>>(maps, g, t);
-  return cudaGetLastError();
+  static std::atomic<unsigned long long> smem_set{0};
+  cudaError_t e = set_smem_once(kern, smem, smem_set);
+  return e != cudaSuccess ? e : launch_pdl(kern, (unsigned)ctas, kColThreads, smem, s, maps, g, t);
 }
 
 cudaError_t launch_hvp_col(int D, int is_bf16, const TmaMaps& maps, const Geometry& g, const Tensors& t,

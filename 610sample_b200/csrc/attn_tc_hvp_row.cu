@@ -154,7 +154,11 @@ hvp_row_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Ten
   auto bar_stream_full = [&](int h, int s) { return smem_u32(&ctl->stream_full[h][s]); };
   auto bar_stream_empty = [&](int h, int s) { return smem_u32(&ctl->stream_empty[h][s]); };
 
-  if (threadIdx.x == 0) {
+  // one barrier round of set-up: the producer initialises the mbarriers and, once the kernels this
+  // one depends on are complete, requests the stationary tiles and the first streamed tile (their
+  // latency is the longest item of the prologue); meanwhile an issuing warp allocates tensor memory
+  if (warp == kProducerWarp && lane == 0) {
+    for (int i = 0; i < T_COUNT; ++i) tma_prefetch_desc(&maps.m[i]);
     mbar_init(bar_stat_full, 1);
     mbar_init(bar_staging_full, 1);
     mbar_init(bar_stat_tmem_ready, kMathWarps);
@@ -174,13 +178,12 @@ hvp_row_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Ten
     mbar_init(bar_rb_issued(0), 1);
     mbar_init(bar_rb_issued(1), 1);
     ctl->abort_flag = 0u;
-    ctl->tmem_base = 0u;
     fence_barrier_init();
     fence_proxy_async_smem();
   }
-  __syncthreads();
-  // the stationary tiles and the first streamed tile are requested before the tensor-memory
-  // allocation and the second barrier: their latency is the longest item of the prologue
+  if (warp == kRowMmaWarp) tmem_alloc(smem_u32(&ctl->tmem_base), kTmemCols);
+  pdl_begin(g);
+  if (warp == kProducerWarp && lane == 0) pdl_trigger();
   if (warp == kProducerWarp && lane == 0 && n_iter > 0) {
     mbar_arrive_expect_tx(bar_staging_full, CF::kStageBytes);
 #pragma unroll
@@ -207,7 +210,6 @@ hvp_row_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Ten
         tma_load_3d(stat_base + a * kAtomBytesStat + h * kAtomBytesStrm, &maps.m[T_gQ], a * 64, r0 + h * 64, bh,
                     bar_stat_full);
   }
-  if (warp == kRowMmaWarp) tmem_alloc(smem_u32(&ctl->tmem_base), kTmemCols);
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
@@ -629,6 +631,7 @@ hvp_row_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Ten
     tc_fence_after_sync();
     tmem_dealloc(tmem_base, kTmemCols);
   }
+  pdl_end(g);
 }
 
 template <int MODE, int D, typename T>
@@ -643,10 +646,9 @@ static cudaError_t launch_row(const TmaMaps& maps, const Geometry& g_in, const T
   // tensor-memory allocation never waits for a co-resident CTA
   const size_t smem = CF::kSmemBytes < 122880u ? 122880u : CF::kSmemBytes;
   auto kern = hvp_row_kernel<MODE, D, T>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return e;
-  kern<<<(unsigned)ctas, kRowThreads, smem, s>>>(maps, g, t);
-  return cudaGetLastError();
+  static std::atomic<unsigned long long> smem_set{0};
+  cudaError_t e = set_smem_once(kern, smem, smem_set);
+  return e != cudaSuccess ? e : launch_pdl(kern, (unsigned)ctas, kRowThreads, smem, s, maps, g, t);
 }
 
 // mode 0: per-row scalars + g_dO;  mode 1: g_Q

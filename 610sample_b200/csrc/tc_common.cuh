@@ -5,6 +5,8 @@
 #include "attn_common.cuh"
 #include "tc_primitives.cuh"
 
+#include <atomic>
+
 namespace attn {
 namespace tc {
 
@@ -21,6 +23,49 @@ constexpr uint32_t kAtomBytesStrm = BN * 128;   // [ 64 rows][64 halves],  8 KB
 // 20, the self-test 0x6f); the values are documented with the C ABI and do not change.
 enum Kind { HVP_PRE = 4, HVP_ROW = 5, HVP_COL = 6 };
 enum TensorId { T_Q = 0, T_K, T_V, T_dO, T_gQ, T_gK, T_gV, T_COUNT };
+
+// Launches and the order between them.  Every tensor-core kernel is launched with programmatic
+// stream serialization: its CTAs may become resident while the predecessor in the stream still
+// runs, set up their barriers and tensor memory, and wait (pdl_wait) before the first access to
+// global memory.  Each CTA triggers its successor right after that wait.  A kernel that only has to
+// come after the predecessor of its predecessor (Geometry::beside) skips the wait at its start: it
+// is launched when every CTA of the predecessor has passed ITS wait, so everything before the
+// predecessor is complete, and its CTAs take the SMs the predecessor's last CTAs leave idle.  Its
+// last CTA waits at its end instead, so that this kernel never completes before its predecessor
+// and whatever follows in the stream may rely on both.  A second stream with an event fork and join does the same for 4 us more
+// of host time and a launch latency on either side, and cannot be used under stream capture.
+__device__ __forceinline__ void pdl_begin(const Geometry& g) { if (!g.beside) pdl_wait(); }
+__device__ __forceinline__ void pdl_end(const Geometry& g) {
+  if (g.beside && blockIdx.x + 1 == gridDim.x && threadIdx.x == 0) pdl_wait();
+}
+
+// Opt-in to `smem` bytes of dynamic shared memory, once per kernel and device (`done`: one bit per device).
+template <typename Kern>
+inline cudaError_t set_smem_once(Kern kern, size_t smem, std::atomic<unsigned long long>& done) {
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  const unsigned long long bit = 1ull << (dev & 63);
+  if (done.load(std::memory_order_acquire) & bit) return cudaSuccess;
+  e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e == cudaSuccess) done.fetch_or(bit, std::memory_order_release);
+  return e;
+}
+
+template <typename... P, typename... A>
+inline cudaError_t launch_pdl(void (*kern)(P...), unsigned ctas, unsigned threads, size_t smem, cudaStream_t s, const A&... args) {
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(ctas);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+}
 
 // Output tensors by operation: forward {O}; backward {dQ, dK, dV}; double backward
 // {g_dO, g_Q, g_K, g_V}.  Output maps have a box of 64 columns x 128 rows.

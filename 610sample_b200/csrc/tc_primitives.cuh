@@ -102,6 +102,12 @@ __device__ __forceinline__ void named_barrier_sync(uint32_t id, uint32_t threads
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
 }
 
+// Programmatic dependent launch.  pdl_wait returns once every kernel this launch depends on has
+// completed and its writes are visible (at once when there is none); pdl_trigger allows the next
+// kernel of the stream to be launched when every CTA of this one has issued it or exited.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // ---------------------------------------------------------------------------
 // TMA: 3-D tiled load, global -> shared, completion on an mbarrier.
 // The innermost coordinate x is always a multiple of 64 half-precision elements
