@@ -296,9 +296,154 @@ torch::Tensor qk_norm_rope_cuda(torch::Tensor x, c10::optional<torch::Tensor> we
   return out;
 }
 
+namespace {
+
+// The differentiable form: the forward and the first backward run the fused kernels; the second
+// backward differentiates the formulas below with the autograd engine.
+struct PrepArgs { int pos0; double eps; int norm_from; };
+
+// "No weight" is an empty tensor between the autograd functions, which take defined tensors only.
+torch::Tensor weight_or_none(const torch::Tensor& w) { return w.numel() > 0 ? w : torch::Tensor(); }
+
+// The same computation out of ordinary operations, with the kernel's rounding points.
+torch::Tensor qk_norm_rope_formula(const torch::Tensor& x, const torch::Tensor& weight, const torch::Tensor& freqs, const PrepArgs& a) {
+  const int64_t n_tok = x.size(0), H = x.size(1), d = x.size(2);
+  torch::Tensor y = x;
+  if (weight.defined()) {
+    const torch::Tensor xf = x.to(torch::kFloat);
+    torch::Tensor normed = (xf * torch::rsqrt(xf.pow(2).mean({-1}, true) + a.eps)).to(x.scalar_type()) * weight.to(x.scalar_type());
+    if (a.norm_from > 0) {
+      const torch::Tensor keep = (torch::arange(n_tok, x.options().dtype(torch::kLong)) < a.norm_from).view({n_tok, 1, 1});
+      normed = torch::where(keep, x, normed);
+    }
+    y = normed;
+  }
+  const torch::Tensor f = freqs.slice(0, a.pos0, a.pos0 + n_tok).unsqueeze(1);
+  const torch::Tensor pair = y.to(torch::kFloat).reshape({n_tok, H, d / 2, 2});
+  const torch::Tensor u = pair.select(-1, 0), v = pair.select(-1, 1), c = f.select(-1, 0), s = f.select(-1, 1);
+  return torch::stack({u * c - v * s, u * s + v * c}, -1).reshape({n_tok, H, d}).to(x.scalar_type()).permute({1, 0, 2}).unsqueeze(0);
+}
+
+// {gx, gw}; gw is undefined without a weight or when it is not wanted
+variable_list qk_norm_rope_backward(const torch::Tensor& g_in, const torch::Tensor& x_in, const torch::Tensor& weight,
+                                    const torch::Tensor& freqs_in, const PrepArgs& a, bool want_gw) {
+  const int64_t n_tok = x_in.size(0), H = x_in.size(1), d = x_in.size(2);
+  if (d % 8 != 0 || x_in.numel() == 0) {      // no 16-byte accesses at these widths: the kernels do not take them
+    at::AutoGradMode on(true);
+    variable_list wrt{x_in.detach().requires_grad_(true)};
+    if (weight.defined()) wrt.push_back(weight.detach().requires_grad_(true));
+    const torch::Tensor y = qk_norm_rope_formula(wrt[0], weight.defined() ? wrt[1] : weight, freqs_in, a);
+    variable_list r = torch::autograd::grad({y}, wrt, {g_in});
+    r.resize(2);
+    return r;
+  }
+  c10::cuda::CUDAGuard guard(x_in.device());
+  const torch::Tensor x = dense(x_in), g = dense(g_in), freqs = dense(freqs_in);
+  torch::Tensor w, gw, scratch;
+  if (weight.defined()) w = dense(weight.to(x.scalar_type()));
+  torch::Tensor gx = fresh_like(x);
+  want_gw = want_gw && w.defined();
+  if (want_gw) {
+    gw = fresh(weight.sizes(), x.scalar_type(), x);
+    scratch = fresh({(int64_t)(attn_b200_qk_norm_rope_backward_scratch_bytes((int32_t)n_tok, (int32_t)H, (int32_t)d) / sizeof(float))},
+                    at::kFloat, x);
+  }
+  check_rc(attn_b200_qk_norm_rope_backward(x.data_ptr(), w.defined() ? w.data_ptr() : nullptr, freqs.data_ptr<float>(), g.data_ptr(),
+                                           gx.data_ptr(), want_gw ? gw.data_ptr() : nullptr, want_gw ? scratch.data_ptr<float>() : nullptr,
+                                           (int32_t)n_tok, (int32_t)H, (int32_t)d, a.pos0, a.norm_from, (float)a.eps, dtype_code(x),
+                                           at::cuda::getCurrentCUDAStream().stream()),
+           "qk_norm_rope_backward");
+  if (want_gw && weight.scalar_type() != gw.scalar_type()) gw = gw.to(weight.scalar_type());
+  return {gx, gw};
+}
+
+void save_prep(AutogradContext* ctx, int64_t pos0, double eps, int64_t norm_from) {
+  ctx->set_materialize_grads(false);
+  ctx->saved_data["pos0"] = pos0;
+  ctx->saved_data["eps"] = eps;
+  ctx->saved_data["norm_from"] = norm_from;
+}
+PrepArgs saved_prep(AutogradContext* ctx) {
+  return {(int)ctx->saved_data["pos0"].toInt(), ctx->saved_data["eps"].toDouble(), (int)ctx->saved_data["norm_from"].toInt()};
+}
+
+struct QKNormRopeBackward : public torch::autograd::Function<QKNormRopeBackward> {
+  static variable_list forward(AutogradContext* ctx, const torch::Tensor& g, const torch::Tensor& x, const torch::Tensor& weight,
+                               const torch::Tensor& freqs, int64_t pos0, double eps, int64_t norm_from) {
+    save_prep(ctx, pos0, eps, norm_from);
+    ctx->save_for_backward({g, x, weight, freqs});
+    variable_list r = qk_norm_rope_backward(g, x, weight_or_none(weight), freqs, {(int)pos0, eps, (int)norm_from}, true);
+    if (weight.numel() == 0) r.resize(1);
+    return r;
+  }
+
+  static variable_list backward(AutogradContext* ctx, variable_list tangents) {
+    variable_list out(7);      // g, x, weight, freqs, pos0, eps, norm_from
+    const variable_list s = ctx->get_saved_variables();
+    const PrepArgs a = saved_prep(ctx);
+    const bool keep_graph = at::GradMode::is_enabled();
+    at::AutoGradMode on(true);
+    // aliases of the inputs, so that the derivatives are partial ones even where the inputs depend on
+    // one another (g often depends on x); connected to them when a third derivative may be asked for
+    auto alias = [&](const torch::Tensor& t) {
+      return keep_graph && t.requires_grad() ? t.view_as(t) : t.detach().requires_grad_(true);
+    };
+    const torch::Tensor g = alias(s[0]), x = alias(s[1]);
+    variable_list first_wrt{x}, wrt{g, x};
+    torch::Tensor w;
+    if (s[2].numel() > 0) {
+      w = alias(s[2]);
+      first_wrt.push_back(w);
+      wrt.push_back(w);
+    }
+    const variable_list first = torch::autograd::grad({qk_norm_rope_formula(x, w, s[3], a)}, first_wrt, {g}, true, true);
+    variable_list of, with;
+    for (size_t i = 0; i < first.size(); ++i)
+      if (tangents[i].defined()) { of.push_back(first[i]); with.push_back(tangents[i]); }
+    if (of.empty()) return out;
+    const variable_list r = torch::autograd::grad(of, wrt, with, true, keep_graph, true);
+    for (size_t i = 0; i < r.size(); ++i) out[i] = r[i];
+    return out;
+  }
+};
+
+struct QKNormRope : public torch::autograd::Function<QKNormRope> {
+  static torch::Tensor forward(AutogradContext* ctx, const torch::Tensor& x, const torch::Tensor& weight, const torch::Tensor& freqs,
+                               int64_t pos0, double eps, int64_t norm_from) {
+    save_prep(ctx, pos0, eps, norm_from);
+    ctx->save_for_backward({x, weight, freqs});
+    return qk_norm_rope_cuda(x, weight_or_none(weight), freqs, (int)pos0, eps, (int)norm_from);
+  }
+
+  static variable_list backward(AutogradContext* ctx, variable_list g) {
+    variable_list out(6);      // x, weight, freqs, pos0, eps, norm_from
+    if (!g[0].defined()) return out;
+    const variable_list s = ctx->get_saved_variables();
+    const PrepArgs a = saved_prep(ctx);
+    variable_list r = at::GradMode::is_enabled()
+                          ? QKNormRopeBackward::apply(g[0], s[0], s[1], s[2], (int64_t)a.pos0, a.eps, (int64_t)a.norm_from)
+                          : qk_norm_rope_backward(g[0], s[0], weight_or_none(s[1]), s[2], a, ctx->needs_input_grad(1));
+    for (size_t i = 0; i < r.size(); ++i) out[i] = r[i];
+    return out;
+  }
+};
+
+}  // namespace
+
+torch::Tensor qk_norm_rope_diff(const torch::Tensor& x, c10::optional<torch::Tensor> weight, const torch::Tensor& freqs, int pos0,
+                                double eps, int norm_from) {
+  const bool has_weight = weight.has_value() && weight->defined();
+  if (!at::GradMode::is_enabled() || !(x.requires_grad() || (has_weight && weight->requires_grad())))
+    return qk_norm_rope_cuda(x, weight, freqs, pos0, eps, norm_from);
+  return QKNormRope::apply(x, has_weight ? *weight : fresh({0}, x.scalar_type(), x), freqs, (int64_t)pos0, eps, (int64_t)norm_from);
+}
+
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("qk_norm_rope", &qk_norm_rope_cuda, "fused RMS norm + rotary embedding + [n_tok,H,d] -> [1,H,n_tok,d]",
         py::arg("x"), py::arg("weight"), py::arg("freqs"), py::arg("pos0") = 0, py::arg("eps") = 1e-6, py::arg("norm_from") = 0);
+  m.def("qk_norm_rope_diff", &qk_norm_rope_diff, "qk_norm_rope, twice differentiable",
+        py::arg("x"), py::arg("weight"), py::arg("freqs"), py::arg("pos0") = 0, py::arg("eps") = 1e-6, py::arg("norm_from") = 0,
+        py::call_guard<py::gil_scoped_release>());
   m.def("flash_attention", &flash_attention, "Rectangular sliding-window flash attention, twice differentiable -> O",
         py::arg("Q"), py::arg("K"), py::arg("V"), py::arg("window_size"), py::arg("chunk_id"), py::arg("mask_mode") = 0,
         py::call_guard<py::gil_scoped_release>());

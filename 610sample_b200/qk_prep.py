@@ -7,9 +7,9 @@ The reference does these steps as separate eager operations (`RMSNorm.forward`,
 e2e/ttt_pytorch/model.py:76-84, 96-116, 182-184, used at :260-263 and :309-316).  This is an
 additive entry point: the reference surface (`attention.py`) does not depend on it.
 
-`qk_norm_rope` is differentiable to second order, as test-time training needs: the forward
-runs the fused kernel; the backward re-evaluates the same formulas with ordinary PyTorch
-operations on the saved inputs, under the caller's grad mode, so its own derivative exists.
+`qk_norm_rope` is differentiable to second order, as test-time training needs
+(`attention_cuda.qk_norm_rope_diff`): the forward and the first backward run fused kernels; the
+second backward differentiates the same formulas written as ordinary operations.
 """
 import torch
 
@@ -47,34 +47,8 @@ def qk_norm_rope_torch(x, weight, freqs, pos0=0, eps=1e-6, norm_from=0):
     return out.permute(1, 0, 2).unsqueeze(0)
 
 
-class _QKNormRope(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, x, weight, freqs, pos0, eps, norm_from):
-        ctx.save_for_backward(x, weight if weight is not None else x.new_empty(0), freqs)
-        ctx.has_weight = weight is not None
-        ctx.args = (pos0, eps, norm_from)
-        return _attention_cuda.qk_norm_rope(x, weight, freqs, pos0, eps, norm_from)
-
-    @staticmethod
-    def backward(ctx, g):
-        x, weight, freqs = ctx.saved_tensors
-        weight = weight if ctx.has_weight else None
-        pos0, eps, norm_from = ctx.args
-        with torch.enable_grad():
-            xs = x if x.requires_grad else x.detach().requires_grad_(True)
-            ws = None
-            if weight is not None:
-                ws = weight if weight.requires_grad else weight.detach().requires_grad_(True)
-            y = qk_norm_rope_torch(xs, ws, freqs, pos0, eps, norm_from)
-            wrt = [xs] + ([ws] if ws is not None else [])
-            grads = torch.autograd.grad(y, wrt, g, create_graph=torch.is_grad_enabled(), allow_unused=True)
-        gx = grads[0]
-        gw = grads[1] if ws is not None else None
-        return gx, gw, None, None, None, None
-
-
 def qk_norm_rope(x, weight, freqs, pos0=0, eps=1e-6, norm_from=0):
     """x: [n_tok, H, d] (fp16 / bf16 / fp32, CUDA); weight: [d] or None; freqs: `rope_table(...)`.
     Rows below `norm_from` are only rotated (keys taken from a cache are stored normalised).
     Returns [1, H, n_tok, d], ready for `flash_attention_v7`."""
-    return _QKNormRope.apply(x, weight, freqs, pos0, eps, norm_from)
+    return _attention_cuda.qk_norm_rope_diff(x, weight, freqs, pos0, eps, norm_from)

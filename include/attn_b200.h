@@ -161,6 +161,15 @@ int attn_b200_qk_norm_rope(const void* x, const void* weight, const float* freqs
                            int32_t n_tok, int32_t H, int32_t d, int32_t pos0, int32_t norm_from,
                            float eps, int32_t dtype, void* stream);
 
+/* Gradients of attn_b200_qk_norm_rope: g [H, n_tok, d] is the gradient of its output; gx [n_tok, H, d]
+ * and gw [d] (null: not wanted; needs a weight and `scratch` of the size given by the function
+ * below) receive those of x and of the weight, in the element type of x.  d a multiple of 8, at most
+ * 128, every tensor of x's element type 16-byte aligned, at least one token and one head. */
+size_t attn_b200_qk_norm_rope_backward_scratch_bytes(int32_t n_tok, int32_t H, int32_t d);
+int attn_b200_qk_norm_rope_backward(const void* x, const void* weight, const float* freqs, const void* g, void* gx,
+                                    void* gw, float* scratch, int32_t n_tok, int32_t H, int32_t d, int32_t pos0,
+                                    int32_t norm_from, float eps, int32_t dtype, void* stream);
+
 /* Number of kernels the last successful call of the calling thread launched. */
 int attn_b200_last_launch_count(void);
 

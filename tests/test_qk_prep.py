@@ -116,3 +116,43 @@ def test_wrapper_is_differentiable_to_second_order_and_feeds_attention(prep):
     O = flash_attention_v7(Q, Q.detach(), Q.detach(), n, 0)
     g, = torch.autograd.grad(O.float().sum(), [xq])
     assert g.shape == xq.shape and torch.isfinite(g.float()).all() and float(g.float().abs().max()) > 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("n,H,D,norm_from,weighted", [
+    (1, 1, 8, 0, True),          # one row, one lane of the group at work
+    (33, 5, 64, 10, True),       # one token beyond a CTA's 32, one head beyond a group of four
+    (17, 4, 128, 0, True),       # one token beyond the 16 of a wide head
+    (64, 12, 80, 64, True),      # nothing is normalised: the weight's gradient is zero
+    (40, 3, 96, 0, False),       # rotation only
+    (9473, 8, 64, 0, True),      # 594 tasks: two more than the CTAs, so two CTAs walk on
+    (65, 2, 20, 5, True),        # a width without 16-byte accesses
+])
+def test_backward_kernel_matches_autograd_of_the_formulas(prep, n, H, D, norm_from, weighted, dtype):
+    torch.manual_seed(n + D)
+    x = torch.randn(n, H, D, device="cuda").to(dtype).requires_grad_(True)
+    w = (1 + 0.1 * torch.randn(D, device="cuda")).to(dtype).requires_grad_(True) if weighted else None
+    g = torch.randn(1, H, n, D, device="cuda").to(dtype)
+    table = prep.rope_table(D, n + 3, device="cuda")
+    wrt = [x, w] if weighted else [x]
+    got = torch.autograd.grad(prep.qk_norm_rope(x, w, table, pos0=3, norm_from=norm_from), wrt, g)
+    again = torch.autograd.grad(prep.qk_norm_rope(x, w, table, pos0=3, norm_from=norm_from), wrt, g, create_graph=True)
+    x64 = x.detach().double().requires_grad_(True)
+    w64 = w.detach().double().requires_grad_(True) if weighted else None
+    # qk_norm_rope_torch works in fp32 inside: the formulas in fp64 instead
+    y = x64
+    if weighted:
+        y = x64 * torch.rsqrt(x64.pow(2).mean(-1, keepdim=True) + 1e-6) * w64
+        y = torch.where((torch.arange(n, device="cuda") < norm_from).view(n, 1, 1), x64, y)
+    f = table[3:3 + n].double().unsqueeze(1)
+    p = y.reshape(n, H, D // 2, 2)
+    y = torch.stack([p[..., 0] * f[..., 0] - p[..., 1] * f[..., 1], p[..., 0] * f[..., 1] + p[..., 1] * f[..., 0]], -1)
+    want = torch.autograd.grad(y.reshape(n, H, D).permute(1, 0, 2).unsqueeze(0), [x64, w64] if weighted else [x64], g.double())
+    # results and the normalised factor are rounded to the type once each (unit roundoff u = 2^-9, 2^-12): 4 u of the
+    # largest value; fp32 sums of up to n * H terms in a tree of 32-term chains: 1e-5
+    tol = {torch.bfloat16: 2 ** -7, torch.float16: 2 ** -10, torch.float32: 1e-5}[dtype]
+    for a, b, c in zip(got, again, want):
+        assert a.dtype == dtype and a.shape == c.shape
+        assert torch.equal(a, b.detach())
+        assert float((a.double() - c).abs().max()) <= tol * float(c.abs().max()), (n, H, D)
