@@ -1,484 +1,570 @@
-// fp32 SIMT kernels for attention forward / backward / double-backward.
+// fp32 CUDA-core kernels for attention forward / backward / double backward.
 //
-// This family serves float32 inputs (where results must agree with an fp64
-// oracle to 1e-4) and half-precision inputs whose head dimension has no
-// tensor-core kernel.  All arithmetic is fp32 on CUDA cores; inputs are widened
-// when a tile is staged in shared memory.  Nothing here materialises more than
-// a 32 x 32 score tile per CTA.
+// This family serves float32 inputs (where results must agree with an fp64 oracle to 1e-4) and, when
+// asked for, half-precision inputs.  All arithmetic is fp32 on CUDA cores; inputs are widened when a
+// tile is staged in shared memory.  Nothing here materialises more than a 32 x 64 score tile per CTA.
 //
-// Tiling: a CTA of 256 threads owns 32 "stationary" rows of one (batch, head)
-// -- query rows in the row kernels, key rows in the column kernels -- and streams
-// 32-row tiles of the other axis.  Thread (ty, tx), ty = tid/16, tx = tid%16,
-// holds score elements (ty + 16a, tx + 16b) and output elements
-// (ty + 16a, tx + 16c).  Every output element is produced by exactly one thread
-// in a fixed order, so results are bitwise reproducible.
+// A CTA of 256 threads owns 32 STATIONARY rows of one (batch, head) -- query rows in the row kinds,
+// key rows in the column kinds -- and streams 64-row tiles of the other axis:
+//
+//   kind      stationary        streamed          produces
+//   FWD       Q                 K, V              O, L (online softmax)
+//   BWD_ROW   Q, dO             K, V              dQ = s dS K
+//   BWD_COL   K, V              Q, dO             dV = P^T dO, dK = s dS^T Q
+//   HVP_PRE   Q, dO, g_dQ       K, V, g_dK, g_dV  Dv, dot2, dot3;  g_dO = P g_dV + (P o gdS) V - dot2 o O
+//   HVP_ROW   Q, dO, g_dQ       K, V, g_dK, g_dV  g_Q = s (dS g_dK + g_S K)
+//   HVP_COL   K, V, g_dK, g_dV  Q, dO, g_dQ       g_K = s (dS^T g_dQ + g_S^T Q), g_V = g_dp^T dO
+//
+// Bound by the FMA pipe and, next to it, by shared-memory reads.  A warp is 4 x 8 threads and a
+// thread holds 2 x 4 scores of every score matrix of the kind, so that each float4 it reads serves
+// several products (HVP: 22 reads for 160 multiply-adds; every read of a warp touches at most eight
+// rows, one pass through the banks) and the packed f32x2 multiply-adds run along the head dimension
+// without a move.  Rows are stored without padding where D is a multiple of 32, their 16-byte chunks
+// XOR-swizzled by the row, which lets two CTAs of every kind share an SM at D <= 64: one computes
+// while the other loads.
+// Small problems: with fewer than two CTAs per SM the streamed tiles of a stationary tile are dealt
+// out to a CLUSTER of 2 to 8 CTAs (split_for), whose partial sums are added through distributed
+// shared memory in a fixed order; results are bitwise reproducible either way.
+// B2 H4 N256 D64 causal, forward + backward + double backward on an idle B200: 447 us with 32 x 32
+// tiles, 2 x 2 scores per thread and no split (64 CTAs).
 #include "attn_common.cuh"
 #include "attn_launch.h"
+#include "tc_common.cuh"
+
+#include <cooperative_groups.h>
 
 namespace attn {
 namespace simt {
 
+namespace cg = cooperative_groups;
+
 constexpr int TS = 32;        // stationary rows per CTA
-constexpr int TT = 32;        // streamed rows per iteration
-constexpr int NT = 256;       // threads per CTA
-constexpr int OPLD = 33;      // leading dimension of an operand tile
-constexpr int MAXC = 8;       // output columns per thread = D/16 <= 8
+constexpr int TT = 64;        // streamed rows per iteration
+constexpr int NT = 256;       // threads per CTA: 4 x 2 warps over the 32 x 64 score tile
+constexpr int kMaxSplit = 8;  // CTAs per cluster (the portable maximum)
 
-enum Kind { K_FWD = 0, K_BWD_ROW, K_BWD_COL, K_HVP_ROW, K_HVP_COL };
+enum Kind { K_FWD = 0, K_BWD_ROW, K_BWD_COL, K_HVP_PRE, K_HVP_ROW, K_HVP_COL };
 
-// Stage rows [row0, row0+32) of a [n_rows, D] matrix as fp32, zero beyond n_rows.
-template <typename T>
-__device__ __forceinline__ void stage_tile(float* dst, int ldd, const T* src, int row0, int n_rows,
-                                           int D) {
-  const int per_row = D >> 1;
-  for (int idx = threadIdx.x; idx < 32 * per_row; idx += NT) {
-    const int r = idx / per_row, c = (idx - r * per_row) << 1;
-    float v0 = 0.f, v1 = 0.f;
-    const int gr = row0 + r;
-    if (gr >= 0 && gr < n_rows) {
-      const T* p = src + (size_t)gr * D + c;
-      v0 = Elem<T>::to_float(p[0]);
-      v1 = Elem<T>::to_float(p[1]);
-    }
-    dst[r * ldd + c] = v0;
-    dst[r * ldd + c + 1] = v1;
+template <int KIND> struct Spec {
+  static constexpr bool kCol = KIND == K_BWD_COL || KIND == K_HVP_COL;
+  static constexpr bool kHvp = KIND >= K_HVP_PRE;
+  static constexpr int kNStat = KIND == K_FWD ? 1 : !kHvp ? 2 : kCol ? 4 : 3;
+  static constexpr int kNStream = !kHvp ? 2 : kCol ? 3 : 4;
+  static constexpr int kNAcc = KIND == K_FWD ? 1 : kHvp ? 4 : 2;       // S, dP | S, gdS, dP, gPdV
+  static constexpr int kNOp = KIND == K_FWD || KIND == K_BWD_ROW ? 1 : KIND == K_HVP_COL ? 3 : 2;
+  static constexpr int kNOut = kCol ? 2 : 1;
+};
+
+// Tile layout: row r at r * pitch floats; with D a multiple of 32 the pitch is D and the float4
+// chunks of a row are XORed with r % 8, otherwise the pitch is D + 4.
+struct Layout {
+  int pitch, mask;
+  __host__ __device__ __forceinline__ explicit Layout(int D) : pitch(D % 32 == 0 ? D : D + 4), mask(D % 32 == 0 ? 7 : 0) {}
+  __device__ __forceinline__ int at(int row, int chunk) const { return row * pitch + ((chunk ^ (row & mask)) << 2); }
+};
+__device__ __forceinline__ int op_at(int row, int col) { return row * TT + ((((col >> 2) ^ (row & 7)) << 2) | (col & 3)); }
+
+__device__ __forceinline__ void cp_async16(float* dst, const void* src, bool in) {
+  const unsigned bytes = in ? 16u : 0u;       // 0: the destination is filled with zeros
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(tc::smem_u32(dst)), "l"(src), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+// Four consecutive elements of a half-precision row, widened.
+template <typename T> __device__ __forceinline__ float4 widen4(const T* p) {
+  const uint2 w = *reinterpret_cast<const uint2*>(p);
+  const float2 a = tc::Pack<T>::unpack(w.x), b = tc::Pack<T>::unpack(w.y);
+  return make_float4(a.x, a.y, b.x, b.y);
+}
+
+// Stage `rows` rows from row0 of a [n_rows, D] matrix as fp32, zero beyond n_rows.  DC * 16 threads
+// share a row.  float goes by cp.async (complete after cp_async_wait_all and a barrier).
+template <int DC, typename T>
+__device__ __forceinline__ void stage_tile(float* dst, const Layout& lay, const T* src, int row0, int rows, int n_rows, int D) {
+  constexpr int kLanes = 16 * DC;
+  const int chunk = threadIdx.x % kLanes;
+  if (chunk * 4 >= D) return;
+  for (int r = threadIdx.x / kLanes; r < rows; r += NT / kLanes) {
+    const bool in = row0 + r < n_rows;
+    const T* p = src + (size_t)(in ? row0 + r : 0) * D + chunk * 4;
+    float* q = dst + lay.at(r, chunk);
+    if constexpr (sizeof(T) == 4) cp_async16(q, p, in);
+    else *reinterpret_cast<float4*>(q) = in ? widen4<T>(p) : make_float4(0.f, 0.f, 0.f, 0.f);
   }
 }
 
-// acc[a][b] += <A[ty+16a, :], B[tx+16b, :]>
-__device__ __forceinline__ void score_fma(const float* A, const float* Bm, int D, int ldd, int ty,
-                                          int tx, float acc[2][2]) {
-  const float4* a0 = reinterpret_cast<const float4*>(A + ty * ldd);
-  const float4* a1 = reinterpret_cast<const float4*>(A + (ty + 16) * ldd);
-  const float4* b0 = reinterpret_cast<const float4*>(Bm + tx * ldd);
-  const float4* b1 = reinterpret_cast<const float4*>(Bm + (tx + 16) * ldd);
-  for (int k = 0; k < (D >> 2); ++k) {
-    const float4 x0 = a0[k], x1 = a1[k], y0 = b0[k], y1 = b1[k];
-    acc[0][0] += x0.x * y0.x + x0.y * y0.y + x0.z * y0.z + x0.w * y0.w;
-    acc[0][1] += x0.x * y1.x + x0.y * y1.y + x0.z * y1.z + x0.w * y1.w;
-    acc[1][0] += x1.x * y0.x + x1.y * y0.y + x1.z * y0.z + x1.w * y0.w;
-    acc[1][1] += x1.x * y1.x + x1.y * y1.y + x1.z * y1.z + x1.w * y1.w;
-  }
+__device__ __forceinline__ void mac(float2& acc, const float4& x, const float4& y) {
+  acc = __ffma2_rn(make_float2(x.x, x.y), make_float2(y.x, y.y), acc);
+  acc = __ffma2_rn(make_float2(x.z, x.w), make_float2(y.z, y.w), acc);
 }
 
-// out[a][c] += sum_j Op[ty+16a, j] * Z[j, tx+16c]
-__device__ __forceinline__ void out_fma(const float* Op, const float* Z, int ncol, int ldd, int ty,
-                                        int tx, float out[2][MAXC]) {
-  for (int j = 0; j < TT; ++j) {
-    const float o0 = Op[ty * OPLD + j], o1 = Op[(ty + 16) * OPLD + j];
+// The raw score matrices of a kind for this thread's 2 x 4 elements.
+template <int KIND>
+__device__ __forceinline__ void scores(float* const (&stat)[4], float* const (&strm)[4], const Layout& lay, int D,
+                                       int row0, int col0, float (&out)[Spec<KIND>::kNAcc][2][4]) {
+  using SP = Spec<KIND>;
+  constexpr int kScored = KIND == K_FWD ? 1 : SP::kNStream;     // the forward's V takes no part in the scores
+  float2 acc[SP::kNAcc][2][4];
 #pragma unroll
-    for (int c = 0; c < MAXC; ++c) {
-      if (c < ncol) {
-        const float z = Z[j * ldd + tx + 16 * c];
-        out[0][c] = fmaf(o0, z, out[0][c]);
-        out[1][c] = fmaf(o1, z, out[1][c]);
+  for (int m = 0; m < SP::kNAcc; ++m)
+#pragma unroll
+    for (int a = 0; a < 2; ++a)
+#pragma unroll
+      for (int b = 0; b < 4; ++b) acc[m][a][b] = make_float2(0.f, 0.f);
+#pragma unroll 2
+  for (int k = 0; k < (D >> 2); ++k) {
+    float4 x[SP::kNStat][2];
+#pragma unroll
+    for (int i = 0; i < SP::kNStat; ++i)
+#pragma unroll
+      for (int a = 0; a < 2; ++a) x[i][a] = *reinterpret_cast<const float4*>(stat[i] + lay.at(row0 + 4 * a, k));
+#pragma unroll
+    for (int b = 0; b < 4; ++b) {
+      float4 y[kScored];
+#pragma unroll
+      for (int i = 0; i < kScored; ++i) y[i] = *reinterpret_cast<const float4*>(strm[i] + lay.at(col0 + 8 * b, k));
+#pragma unroll
+      for (int a = 0; a < 2; ++a) {
+        mac(acc[0][a][b], x[0][a], y[0]);                       // Q K^T               | K Q^T
+        if constexpr (SP::kNAcc == 2) mac(acc[1][a][b], x[1][a], y[1]);      // dO V^T  | V dO^T
+        if constexpr (SP::kHvp) {
+          mac(acc[1][a][b], x[2][a], y[0]);                     // g_dQ K^T            | g_dK Q^T
+          mac(acc[1][a][b], x[0][a], y[2]);                     // + Q g_dK^T          | + K g_dQ^T
+          mac(acc[2][a][b], x[1][a], y[1]);                     // dO V^T              | V dO^T
+          if constexpr (SP::kCol) mac(acc[3][a][b], x[3][a], y[1]);          //         | g_dV dO^T
+          else mac(acc[3][a][b], x[1][a], y[3]);                // dO g_dV^T
+        }
       }
     }
   }
+#pragma unroll
+  for (int m = 0; m < SP::kNAcc; ++m)
+#pragma unroll
+    for (int a = 0; a < 2; ++a)
+#pragma unroll
+      for (int b = 0; b < 4; ++b) out[m][a][b] = acc[m][a][b].x + acc[m][a][b].y;
 }
 
-__device__ __forceinline__ float half_warp_sum(float v) {
+// out[a][c] += sum_j Op[row0 + 4a, j] * Z[j, chunk c of this thread]
+template <int DC>
+__device__ __forceinline__ void out_fma(const float* op, const float* Z, const Layout& lay, int row0, int chunk0, int chunks,
+                                        float2 (&out)[2][DC][2]) {
+#pragma unroll 2
+  for (int j = 0; j < TT; j += 4) {
+    float o[2][4];
 #pragma unroll
-  for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
-}
-__device__ __forceinline__ float half_warp_max(float v) {
-#pragma unroll
-  for (int o = 8; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
-  return v;
-}
-
-template <typename T>
-__device__ __forceinline__ void store_rows(T* dst, int row0, int n_rows, int D, int ncol, int ty,
-                                           int tx, const float out[2][MAXC], float mul) {
-#pragma unroll
-  for (int a = 0; a < 2; ++a) {
-    const int r = row0 + ty + 16 * a;
-    if (r < n_rows) {
-#pragma unroll
-      for (int c = 0; c < MAXC; ++c)
-        if (c < ncol) dst[(size_t)r * D + tx + 16 * c] = Elem<T>::from_float(out[a][c] * mul);
+    for (int a = 0; a < 2; ++a) {
+      const float4 v = *reinterpret_cast<const float4*>(op + op_at(row0 + 4 * a, j));
+      o[a][0] = v.x; o[a][1] = v.y; o[a][2] = v.z; o[a][3] = v.w;
     }
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+#pragma unroll
+      for (int c = 0; c < DC; ++c) {
+        if (chunk0 + 16 * c < chunks) {
+          const float4 z = *reinterpret_cast<const float4*>(Z + lay.at(j + u, chunk0 + 16 * c));
+#pragma unroll
+          for (int a = 0; a < 2; ++a) {
+            const float2 oo = make_float2(o[a][u], o[a][u]);
+            out[a][c][0] = __ffma2_rn(oo, make_float2(z.x, z.y), out[a][c][0]);
+            out[a][c][1] = __ffma2_rn(oo, make_float2(z.z, z.w), out[a][c][1]);
+          }
+        }
+      }
   }
 }
 
-// One kernel per Kind.  Row kinds: stationary = query rows.  Column kinds:
-// stationary = key rows and the score tile is held transposed.
-template <int KIND, typename T>
-__global__ void __launch_bounds__(NT) attn_simt_kernel(const Geometry g, const Tensors t) {
+// sum over the eight threads of a warp that share a row
+__device__ __forceinline__ float row_sum(float v) {
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+__device__ __forceinline__ float row_max(float v) {
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
+  return v;
+}
+
+template <typename T> __device__ __forceinline__ void store4(T* p, const float4& v) {
+  *reinterpret_cast<uint2*>(p) = make_uint2(tc::Pack<T>::pack(v.x, v.y), tc::Pack<T>::pack(v.z, v.w));
+}
+template <> __device__ __forceinline__ void store4<float>(float* p, const float4& v) { *reinterpret_cast<float4*>(p) = v; }
+template <typename T> __device__ __forceinline__ float4 load4(const T* p) { return widen4<T>(p); }
+template <> __device__ __forceinline__ float4 load4<float>(const float* p) { return *reinterpret_cast<const float4*>(p); }
+
+// shared memory in floats
+template <int KIND>
+__host__ __device__ constexpr int smem_floats(int D) {
+  const int pitch = D % 32 == 0 ? D : D + 4;
+  return (Spec<KIND>::kNStat * TS + Spec<KIND>::kNStream * TT) * pitch + Spec<KIND>::kNOp * TS * TT + 4 * TT;
+}
+
+// DC: 1 for D <= 64, 2 up to 128.
+template <int KIND, int DC, typename T>
+__global__ void __launch_bounds__(NT, DC == 1 ? 2 : 1) attn_simt_kernel(const Geometry g, const Tensors t, const int split) {
+  using SP = Spec<KIND>;
   extern __shared__ __align__(16) float smem[];
-  constexpr bool kCol = (KIND == K_BWD_COL || KIND == K_HVP_COL);
-  constexpr int kNStat = (KIND == K_FWD) ? 1 : (KIND == K_BWD_ROW) ? 2 : (KIND == K_BWD_COL) ? 2
-                         : (KIND == K_HVP_ROW) ? 3 : 4;
-  constexpr int kNStream = (KIND == K_FWD) ? 2 : (KIND == K_BWD_ROW) ? 2 : (KIND == K_BWD_COL) ? 2
-                           : (KIND == K_HVP_ROW) ? 4 : 3;
-  constexpr int kNOp = (KIND == K_FWD) ? 1 : (KIND == K_BWD_ROW) ? 1 : (KIND == K_BWD_COL) ? 2
-                       : (KIND == K_HVP_ROW) ? 4 : 3;
-  const int D = g.D, ldd = D + 4, ncol = D >> 4;
-  const int n_stat = kCol ? g.N_kv : g.N_q;
+  const int D = g.D;
+  const Layout lay(D);
+  const int n_stat = SP::kCol ? g.N_kv : g.N_q, n_strm = SP::kCol ? g.N_q : g.N_kv;
   const int tiles = (n_stat + TS - 1) / TS;
-  const int bh = blockIdx.x / tiles;
-  const int r0 = (blockIdx.x - bh * tiles) * TS;
-  const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
+  const int unit = blockIdx.x / split, part = blockIdx.x - unit * split;
+  const int bh = unit % g.BH, rank = unit / g.BH;
+  const int tile = (SP::kCol || g.mask_mode != 0) ? rank : tiles - 1 - rank;     // heavy tiles first
+  const int r0 = tile * TS;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int ty = lane >> 3, tx = lane & 7, wcol = warp & 1;
+  const int row0 = (warp >> 1) * 8 + ty;              // this thread's rows: row0, row0 + 4
+  const int col0 = wcol * 32 + tx;                    // its score columns: col0 + 8 b
+  const int chunk0 = wcol * 8 + tx, chunks = D >> 2;  // its output float4s: chunk0 + 16 c
 
   float* stat[4];
   float* strm[4];
-  float* op[4];
+  float* op[3];
   float* p = smem;
-  for (int i = 0; i < kNStat; ++i) { stat[i] = p; p += TS * ldd; }
-  for (int i = 0; i < kNStream; ++i) { strm[i] = p; p += TT * ldd; }
-  for (int i = 0; i < kNOp; ++i) { op[i] = p; p += TS * OPLD; }
-  float* sL2 = p;  p += 32;   // per query row of the current tile (stationary or streamed)
-  float* sDv = p;  p += 32;
-  float* sD2 = p;  p += 32;
-  float* sD3 = p;  p += 32;
+  for (int i = 0; i < 4; ++i) { stat[i] = p; if (i < SP::kNStat) p += TS * lay.pitch; }
+  float* const strm_base = p;
+  for (int i = 0; i < 4; ++i) { strm[i] = p; if (i < SP::kNStream) p += TT * lay.pitch; }
+  for (int i = 0; i < 3; ++i) { op[i] = p; if (i < SP::kNOp) p += TS * TT; }
+  float* const aux = p;                               // [4][64]: scalars of the streamed queries, or row exchange
 
-  const size_t q_off = (size_t)bh * g.N_q * D, kv_off = (size_t)bh * g.N_kv * D;
-  const T* Q = (const T*)t.Q + q_off;
-  const T* K = (const T*)t.K + kv_off;
-  const T* V = (const T*)t.V + kv_off;
-  const T* dO = t.dO ? (const T*)t.dO + q_off : nullptr;
-  const T* gQ = t.g_dQ ? (const T*)t.g_dQ + q_off : nullptr;
-  const T* gK = t.g_dK ? (const T*)t.g_dK + kv_off : nullptr;
-  const T* gV = t.g_dV ? (const T*)t.g_dV + kv_off : nullptr;
-  const size_t row_off = (size_t)bh * g.N_q;
+  const size_t q_off = (size_t)bh * g.N_q * D, kv_off = (size_t)bh * g.N_kv * D, row_off = (size_t)bh * g.N_q;
+  const T* const Q = (const T*)t.Q + q_off;
+  const T* const K = (const T*)t.K + kv_off;
+  const T* const V = (const T*)t.V + kv_off;
+  const T* const dO = (const T*)t.dO + q_off;
+  const T* const O = (const T*)t.O + q_off;
+  const T* const gQ = (const T*)t.g_dQ + q_off;
+  const T* const gK = (const T*)t.g_dK + kv_off;
+  const T* const gV = (const T*)t.g_dV + kv_off;
+  const T* const stat_src[4] = {SP::kCol ? K : Q, SP::kCol ? V : dO, SP::kCol ? gK : gQ, gV};
+  const T* const strm_src[4] = {SP::kCol ? Q : K, SP::kCol ? dO : V, SP::kCol ? gQ : gK, gV};
 
-  // ---- stationary tiles -----------------------------------------------------
-  if constexpr (KIND == K_FWD) {
-    stage_tile<T>(stat[0], ldd, Q, r0, g.N_q, D);
-  } else if constexpr (KIND == K_BWD_ROW) {
-    stage_tile<T>(stat[0], ldd, Q, r0, g.N_q, D);
-    stage_tile<T>(stat[1], ldd, dO, r0, g.N_q, D);
-  } else if constexpr (KIND == K_BWD_COL) {
-    stage_tile<T>(stat[0], ldd, K, r0, g.N_kv, D);
-    stage_tile<T>(stat[1], ldd, V, r0, g.N_kv, D);
-  } else if constexpr (KIND == K_HVP_ROW) {
-    stage_tile<T>(stat[0], ldd, Q, r0, g.N_q, D);
-    stage_tile<T>(stat[1], ldd, dO, r0, g.N_q, D);
-    stage_tile<T>(stat[2], ldd, gQ, r0, g.N_q, D);
-  } else {
-    stage_tile<T>(stat[0], ldd, K, r0, g.N_kv, D);
-    stage_tile<T>(stat[1], ldd, V, r0, g.N_kv, D);
-    stage_tile<T>(stat[2], ldd, gK, r0, g.N_kv, D);
-    stage_tile<T>(stat[3], ldd, gV, r0, g.N_kv, D);
-  }
-
-  // ---- range of streamed tiles ---------------------------------------------
   int lo, hi;
-  if constexpr (kCol) query_range_for_keys(g, r0, r0 + TS, lo, hi);
+  if constexpr (SP::kCol) query_range_for_keys(g, r0, r0 + TS, lo, hi);
   else key_range_for_queries(g, r0, r0 + TS, lo, hi);
-  const int t_begin = lo / TT, t_end = (hi + TT - 1) / TT;
+  const int t_end = hi > lo ? (hi + TT - 1) / TT : 0;
+  const int t_first = lo / TT + part;
 
-  float out0[2][MAXC], out1[2][MAXC];
-#pragma unroll
-  for (int a = 0; a < 2; ++a)
-#pragma unroll
-    for (int c = 0; c < MAXC; ++c) out0[a][c] = out1[a][c] = 0.f;
+  tc::pdl_begin(g);
+  tc::pdl_trigger();
 
-  // ======================= forward =========================================
-  if constexpr (KIND == K_FWD) {
-    // pass 1: log-sum-exp per row, in the log2 domain
-    float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};
-    for (int tt = t_begin; tt < t_end; ++tt) {
+#pragma unroll
+  for (int i = 0; i < SP::kNStat; ++i) stage_tile<DC, T>(stat[i], lay, stat_src[i], r0, TS, n_stat, D);
+
+  // ---- scalars of this thread's two rows (row kinds)
+  float L2[2] = {0.f, 0.f}, Dv[2] = {0.f, 0.f}, d2[2] = {0.f, 0.f}, d3[2] = {0.f, 0.f};
+  if constexpr (!SP::kCol && KIND != K_FWD) {
+#pragma unroll
+    for (int a = 0; a < 2; ++a) {
+      const int r = r0 + row0 + 4 * a;
+      const bool in = r < g.N_q;
+      L2[a] = in ? t.L[row_off + r] * kLog2e : INFINITY;
+      if constexpr (KIND == K_HVP_ROW) {
+        if (in) { Dv[a] = t.Dv[row_off + r]; d2[a] = t.dot2[row_off + r]; d3[a] = t.dot3[row_off + r]; }
+      }
+      if constexpr (KIND == K_BWD_ROW) {      // D_i = sum_d dO * O from the stored (rounded) O
+        float s = 0.f;
+        if (in)
+          for (int c = tx; c < chunks; c += 8) {
+            const float4 x = load4(dO + (size_t)r * D + 4 * c), y = load4(O + (size_t)r * D + 4 * c);
+            s += x.x * y.x + x.y * y.y + x.z * y.z + x.w * y.w;
+          }
+        Dv[a] = row_sum(s);
+      }
+    }
+  }
+  float m_run[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.f, 0.f};                       // FWD
+  float aD[2] = {0.f, 0.f}, a2[2] = {0.f, 0.f}, aA[2] = {0.f, 0.f}, aE[2] = {0.f, 0.f};   // HVP_PRE
+  float2 out[SP::kNOut][2][DC][2];
+#pragma unroll
+  for (int o = 0; o < SP::kNOut; ++o)
+#pragma unroll
+    for (int a = 0; a < 2; ++a)
+#pragma unroll
+      for (int c = 0; c < DC; ++c) out[o][a][c][0] = out[o][a][c][1] = make_float2(0.f, 0.f);
+
+  for (int tt = t_first; tt < t_end; tt += split) {
+    const int s0 = tt * TT;
+    __syncthreads();                                  // the previous tile has been used
+#pragma unroll
+    for (int i = 0; i < SP::kNStream; ++i) stage_tile<DC, T>(strm[i], lay, strm_src[i], s0, TT, n_strm, D);
+    if constexpr (SP::kCol) {                         // [L2 | Dv | dot2 | dot3] of the streamed queries
+      if constexpr (SP::kHvp) {
+        const int which = tid >> 6, r = s0 + (tid & 63);
+        const float* src = which == 0 ? t.L : which == 1 ? t.Dv : which == 2 ? t.dot2 : t.dot3;
+        const float v = r < g.N_q ? src[row_off + r] : 0.f;
+        aux[tid] = which == 0 ? (r < g.N_q ? v * kLog2e : INFINITY) : v;
+      } else {
+        const int r = s0 + (tid >> 2);                // four threads per query
+        float s = 0.f;
+        if (r < g.N_q)
+          for (int c = tid & 3; c < chunks; c += 4) {
+            const float4 x = load4(dO + (size_t)r * D + 4 * c), y = load4(O + (size_t)r * D + 4 * c);
+            s += x.x * y.x + x.y * y.y + x.z * y.z + x.w * y.w;
+          }
+        s += __shfl_xor_sync(0xffffffffu, s, 2);
+        s += __shfl_xor_sync(0xffffffffu, s, 1);
+        if ((tid & 3) == 0) {
+          aux[tid >> 2] = r < g.N_q ? t.L[row_off + r] * kLog2e : INFINITY;
+          aux[TT + (tid >> 2)] = s;
+        }
+      }
+    }
+    cp_async_wait_all();
+    __syncthreads();
+    float s[SP::kNAcc][2][4];
+    scores<KIND>(stat, strm, lay, D, row0, col0, s);
+    const bool full = SP::kCol ? tile_fully_visible(g, s0, s0 + TT, r0, r0 + TS) : tile_fully_visible(g, r0, r0 + TS, s0, s0 + TT);
+    auto sees = [&](int a, int b) {
+      const int i = r0 + row0 + 4 * a, j = s0 + col0 + 8 * b;
+      return full || (SP::kCol ? visible(g, j, i) : visible(g, i, j));
+    };
+
+    if constexpr (KIND == K_FWD) {
+      // running maximum of a row: over this warp's 32 columns, then over the two warps of the row
+#pragma unroll
+      for (int a = 0; a < 2; ++a) {
+        float mx = -INFINITY;
+#pragma unroll
+        for (int b = 0; b < 4; ++b) {
+          s[0][a][b] = sees(a, b) ? s[0][a][b] * g.scale_log2e : -INFINITY;
+          mx = fmaxf(mx, s[0][a][b]);
+        }
+        mx = row_max(mx);
+        if (tx == 0) aux[wcol * TS + row0 + 4 * a] = mx;
+      }
       __syncthreads();
-      stage_tile<T>(strm[0], ldd, K, tt * TT, g.N_kv, D);
-      __syncthreads();
-      float s[2][2] = {{0.f, 0.f}, {0.f, 0.f}};
-      score_fma(stat[0], strm[0], D, ldd, ty, tx, s);
+#pragma unroll
+      for (int a = 0; a < 2; ++a) {
+        const float m_new = fmaxf(m_run[a], fmaxf(aux[row0 + 4 * a], aux[TS + row0 + 4 * a]));
+        const float f = m_new == -INFINITY ? 1.f : exp2f(m_run[a] - m_new);
+        m_run[a] = m_new;
+        l_run[a] *= f;
+#pragma unroll
+        for (int c = 0; c < DC; ++c)
+#pragma unroll
+          for (int h = 0; h < 2; ++h) out[0][a][c][h] = make_float2(out[0][a][c][h].x * f, out[0][a][c][h].y * f);
+#pragma unroll
+        for (int b = 0; b < 4; ++b) {
+          const float pr = m_new == -INFINITY ? 0.f : exp2f(s[0][a][b] - m_new);
+          l_run[a] += pr;
+          op[0][op_at(row0 + 4 * a, col0 + 8 * b)] = pr;
+        }
+      }
+    } else {
 #pragma unroll
       for (int a = 0; a < 2; ++a)
 #pragma unroll
-        for (int b = 0; b < 2; ++b) {
-          if (visible(g, r0 + ty + 16 * a, tt * TT + tx + 16 * b)) {
-            const float x = s[a][b] * g.scale_log2e;
-            const float mn = fmaxf(m[a], x);
-            l[a] = l[a] * exp2f(m[a] - mn) + exp2f(x - mn);
-            m[a] = mn;
+        for (int b = 0; b < 4; ++b) {
+          const int col = col0 + 8 * b, at = op_at(row0 + 4 * a, col);
+          RowStats rs;
+          if constexpr (SP::kCol) rs = RowStats{aux[col], aux[TT + col], SP::kHvp ? aux[2 * TT + col] : 0.f, SP::kHvp ? aux[3 * TT + col] : 0.f};
+          else rs = RowStats{L2[a], Dv[a], d2[a], d3[a]};
+          const float pr = prob(s[0][a][b], g.scale_log2e, rs.L2, sees(a, b));
+          if constexpr (KIND == K_BWD_ROW) {
+            op[0][at] = pr * (s[1][a][b] - rs.Dv);
+          } else if constexpr (KIND == K_BWD_COL) {
+            op[0][at] = pr;
+            op[1][at] = pr * (s[1][a][b] - rs.Dv);
+          } else if constexpr (KIND == K_HVP_PRE) {
+            const float pg = pr * (s[1][a][b] * g.scale);
+            aD[a] = fmaf(pr, s[2][a][b], aD[a]);
+            a2[a] += pg;
+            aA[a] = fmaf(pg, s[2][a][b], aA[a]);
+            aE[a] = fmaf(pr, s[3][a][b], aE[a]);
+            op[0][at] = pr;
+            op[1][at] = pg;
+          } else {
+            const HvpTerms h = hvp_terms(pr, s[2][a][b], s[1][a][b], s[3][a][b], g.scale, rs);
+            op[0][at] = h.dS;
+            op[1][at] = h.g_S;
+            if constexpr (KIND == K_HVP_COL) op[2][at] = h.g_dp;
           }
         }
     }
+    __syncthreads();
+    auto add = [&](int o, int which, int z) { out_fma<DC>(op[which], strm[z], lay, row0, chunk0, chunks, out[o]); };
+    if constexpr (KIND == K_FWD) add(0, 0, 1);                                   // O += P V
+    else if constexpr (KIND == K_BWD_ROW) add(0, 0, 0);                          // dQ += dS K
+    else if constexpr (KIND == K_BWD_COL) { add(0, 0, 1); add(1, 1, 0); }        // dV += P^T dO; dK += dS^T Q
+    else if constexpr (KIND == K_HVP_PRE) { add(0, 0, 3); add(0, 1, 1); }        // g_dO' += P g_dV + (P o gdS) V
+    else if constexpr (KIND == K_HVP_ROW) { add(0, 0, 2); add(0, 1, 0); }        // g_Q += dS g_dK + g_S K
+    else { add(0, 0, 2); add(0, 1, 0); add(1, 2, 1); }                           // g_K += dS^T g_dQ + g_S^T Q; g_V += g_dp^T dO
+  }
+  cp_async_wait_all();                                // a CTA without tiles has its stationary loads in flight
+  __syncthreads();
+
+  // ---- results.  Row scalars of the two column halves (and of the other CTAs of the cluster) and
+  // the output tiles are combined in the order of the halves and ranks.
+  cg::cluster_group cluster = cg::this_cluster();
+  float* const partial = strm_base;                   // [kNOut][TS][D] of this CTA, when the cluster has several
+  float* const sums = op[0];                          // [2 halves][4][TS] row sums
+  if constexpr (KIND == K_FWD || KIND == K_HVP_PRE) {
 #pragma unroll
     for (int a = 0; a < 2; ++a) {
-      const float mt = half_warp_max(m[a]);
-      const float lt = half_warp_sum(mt == -INFINITY ? 0.f : l[a] * exp2f(m[a] - mt));
-      const float L2 = (lt > 0.f) ? mt + log2f(lt) : -INFINITY;
-      const int r = r0 + ty + 16 * a;
+      const float v0 = KIND == K_FWD ? m_run[a] : row_sum(aD[a]);
+      const float v1 = row_sum(KIND == K_FWD ? l_run[a] : a2[a]);
+      const float v2 = row_sum(aA[a]), v3 = row_sum(aE[a]);
       if (tx == 0) {
-        sL2[ty + 16 * a] = (r < g.N_q) ? L2 : INFINITY;
-        if (r < g.N_q) t.out_L[row_off + r] = L2 * kLn2;
+        float* q = sums + wcol * 4 * TS + row0 + 4 * a;
+        q[0] = v0; q[TS] = v1; q[2 * TS] = v2; q[3 * TS] = v3;
       }
     }
-    // pass 2: O = P V
-    for (int tt = t_begin; tt < t_end; ++tt) {
-      __syncthreads();
-      stage_tile<T>(strm[0], ldd, K, tt * TT, g.N_kv, D);
-      stage_tile<T>(strm[1], ldd, V, tt * TT, g.N_kv, D);
-      __syncthreads();
-      float s[2][2] = {{0.f, 0.f}, {0.f, 0.f}};
-      score_fma(stat[0], strm[0], D, ldd, ty, tx, s);
+  }
+  if (split > 1) {
+#pragma unroll
+    for (int o = 0; o < SP::kNOut; ++o)
 #pragma unroll
       for (int a = 0; a < 2; ++a)
 #pragma unroll
-        for (int b = 0; b < 2; ++b) {
-          const int i = ty + 16 * a, j = tx + 16 * b;
-          op[0][i * OPLD + j] = prob(s[a][b], g.scale_log2e, sL2[i], visible(g, r0 + i, tt * TT + j));
-        }
-      __syncthreads();
-      out_fma(op[0], strm[1], ncol, ldd, ty, tx, out0);
-    }
-    store_rows<T>((T*)t.out_O + q_off, r0, g.N_q, D, ncol, ty, tx, out0, 1.f);
-    return;
-  }
-
-  // ======================= first backward, row side ========================
-  if constexpr (KIND == K_BWD_ROW) {
-    // D_i = sum_d dO * O from the stored (rounded) O; kept for the column kernel
+        for (int c = 0; c < DC; ++c)
+          if (chunk0 + 16 * c < chunks)
+            reinterpret_cast<float4*>(partial)[(o * TS + row0 + 4 * a) * chunks + chunk0 + 16 * c] =
+                make_float4(out[o][a][c][0].x, out[o][a][c][0].y, out[o][a][c][1].x, out[o][a][c][1].y);
+    cluster.sync();
+  } else {
     __syncthreads();
-    {
-      const T* O = (const T*)t.O + q_off;
-#pragma unroll
-      for (int a = 0; a < 2; ++a) {
-        const int i = ty + 16 * a, r = r0 + i;
-        float acc = 0.f;
-        if (r < g.N_q)
-          for (int d = tx; d < D; d += 16) acc += stat[1][i * ldd + d] * Elem<T>::to_float(O[(size_t)r * D + d]);
-        acc = half_warp_sum(acc);
-        if (tx == 0) {
-          sDv[i] = acc;
-          sL2[i] = (r < g.N_q) ? t.L[row_off + r] * kLog2e : INFINITY;
-          if (r < g.N_q) t.Dv[row_off + r] = acc;
-        }
-      }
-    }
-    for (int tt = t_begin; tt < t_end; ++tt) {
-      __syncthreads();
-      stage_tile<T>(strm[0], ldd, K, tt * TT, g.N_kv, D);
-      stage_tile<T>(strm[1], ldd, V, tt * TT, g.N_kv, D);
-      __syncthreads();
-      float s[2][2] = {{0.f, 0.f}, {0.f, 0.f}}, dp[2][2] = {{0.f, 0.f}, {0.f, 0.f}};
-      score_fma(stat[0], strm[0], D, ldd, ty, tx, s);
-      score_fma(stat[1], strm[1], D, ldd, ty, tx, dp);
-#pragma unroll
-      for (int a = 0; a < 2; ++a)
-#pragma unroll
-        for (int b = 0; b < 2; ++b) {
-          const int i = ty + 16 * a, j = tx + 16 * b;
-          const float pr = prob(s[a][b], g.scale_log2e, sL2[i], visible(g, r0 + i, tt * TT + j));
-          op[0][i * OPLD + j] = pr * (dp[a][b] - sDv[i]);
-        }
-      __syncthreads();
-      out_fma(op[0], strm[0], ncol, ldd, ty, tx, out0);
-    }
-    store_rows<T>((T*)t.out_dQ + q_off, r0, g.N_q, D, ncol, ty, tx, out0, g.scale);
-    return;
   }
-
-  // ======================= first backward, column side =====================
-  if constexpr (KIND == K_BWD_COL) {
-    for (int tt = t_begin; tt < t_end; ++tt) {
-      __syncthreads();
-      stage_tile<T>(strm[0], ldd, Q, tt * TT, g.N_q, D);
-      stage_tile<T>(strm[1], ldd, dO, tt * TT, g.N_q, D);
-      if (tid < 32) {
-        const int r = tt * TT + tid;
-        sL2[tid] = (r < g.N_q) ? t.L[row_off + r] * kLog2e : INFINITY;
-        sDv[tid] = (r < g.N_q) ? t.Dv[row_off + r] : 0.f;
-      }
-      __syncthreads();
-      float s[2][2] = {{0.f, 0.f}, {0.f, 0.f}}, dp[2][2] = {{0.f, 0.f}, {0.f, 0.f}};
-      score_fma(stat[0], strm[0], D, ldd, ty, tx, s);    // S^T  = K Q^T
-      score_fma(stat[1], strm[1], D, ldd, ty, tx, dp);   // dP^T = V dO^T
-#pragma unroll
-      for (int a = 0; a < 2; ++a)
-#pragma unroll
-        for (int b = 0; b < 2; ++b) {
-          const int jk = ty + 16 * a, iq = tx + 16 * b;
-          const float pr = prob(s[a][b], g.scale_log2e, sL2[iq], visible(g, tt * TT + iq, r0 + jk));
-          op[0][jk * OPLD + iq] = pr;
-          op[1][jk * OPLD + iq] = pr * (dp[a][b] - sDv[iq]);
-        }
-      __syncthreads();
-      out_fma(op[0], strm[1], ncol, ldd, ty, tx, out0);   // dV += P^T dO
-      out_fma(op[1], strm[0], ncol, ldd, ty, tx, out1);   // dK += dS^T Q
+  // what a row's scalars are after all parts: fwd (max, sum) and the factor of part q; pre (Dv, dot2, dot3)
+  auto row_part = [&](int q, int which, int half, int r) {
+    const float* base = split > 1 ? cluster.map_shared_rank(sums, q) : sums;
+    return base[half * 4 * TS + which * TS + r];
+  };
+  auto fwd_max = [&](int r) {
+    float m = -INFINITY;
+    for (int q = 0; q < split; ++q) m = fmaxf(m, row_part(q, 0, 0, r));      // both halves hold the same maximum
+    return m;
+  };
+  auto factor = [&](int q, int r, float m) {
+    const float mq = row_part(q, 0, 0, r);
+    return mq == -INFINITY ? 0.f : exp2f(mq - m);
+  };
+  auto row_total = [&](int which, int r) {
+    float v = 0.f;
+    for (int q = 0; q < split; ++q) v += row_part(q, which, 0, r) + row_part(q, which, 1, r);
+    return v;
+  };
+  if (tid < TS && part == 0 && r0 + tid < g.N_q) {
+    if constexpr (KIND == K_FWD) {
+      const float m = fwd_max(tid);
+      float l = 0.f;
+      for (int q = 0; q < split; ++q) l += (row_part(q, 1, 0, tid) + row_part(q, 1, 1, tid)) * factor(q, tid, m);
+      t.out_L[row_off + r0 + tid] = l > 0.f ? (m + log2f(l)) * kLn2 : -INFINITY;
+    } else if constexpr (KIND == K_HVP_PRE) {
+      const float D_ = row_total(0, tid), d2_ = row_total(1, tid), A = row_total(2, tid), E = row_total(3, tid);
+      t.Dv[row_off + r0 + tid] = D_;
+      t.dot2[row_off + r0 + tid] = d2_;
+      t.dot3[row_off + r0 + tid] = A - 2.f * D_ * d2_ + E;
     }
-    store_rows<T>((T*)t.out_dV + kv_off, r0, g.N_kv, D, ncol, ty, tx, out0, 1.f);
-    store_rows<T>((T*)t.out_dK + kv_off, r0, g.N_kv, D, ncol, ty, tx, out1, g.scale);
-    return;
   }
-
-  // ======================= double backward, row side =======================
-  if constexpr (KIND == K_HVP_ROW) {
-    __syncthreads();
-    if (tid < 32) {
-      const int r = r0 + tid;
-      sL2[tid] = (r < g.N_q) ? t.L[row_off + r] * kLog2e : INFINITY;
+  // one float4 of output o, row r (within the tile), given its sum over the parts
+  auto finish = [&](int o, int r, int chunk, float4 v) {
+    if (r0 + r >= n_stat) return;
+    const size_t at = (size_t)(r0 + r) * D + 4 * chunk;
+    float mul = 1.f;
+    if constexpr (KIND == K_BWD_ROW || KIND == K_HVP_ROW) mul = g.scale;
+    if constexpr (KIND == K_BWD_COL) mul = o == 1 ? g.scale : 1.f;
+    if constexpr (KIND == K_HVP_COL) mul = o == 0 ? g.scale : 1.f;
+    if constexpr (KIND == K_FWD) {
+      const float m = fwd_max(r);
+      float l = 0.f;
+      for (int q = 0; q < split; ++q) l += (row_part(q, 1, 0, r) + row_part(q, 1, 1, r)) * factor(q, r, m);
+      mul = l > 0.f ? 1.f / l : 0.f;
     }
-    // pass 1: Dv, dot2, dot3 per row
-    float aD[2] = {0.f, 0.f}, a2[2] = {0.f, 0.f}, aA[2] = {0.f, 0.f}, aE[2] = {0.f, 0.f};
-    for (int tt = t_begin; tt < t_end; ++tt) {
-      __syncthreads();
-      stage_tile<T>(strm[0], ldd, K, tt * TT, g.N_kv, D);
-      stage_tile<T>(strm[1], ldd, V, tt * TT, g.N_kv, D);
-      stage_tile<T>(strm[2], ldd, gK, tt * TT, g.N_kv, D);
-      stage_tile<T>(strm[3], ldd, gV, tt * TT, g.N_kv, D);
-      __syncthreads();
-      float s[2][2] = {{0.f, 0.f}, {0.f, 0.f}}, dp[2][2] = {{0.f, 0.f}, {0.f, 0.f}};
-      float gs[2][2] = {{0.f, 0.f}, {0.f, 0.f}}, gp[2][2] = {{0.f, 0.f}, {0.f, 0.f}};
-      score_fma(stat[0], strm[0], D, ldd, ty, tx, s);    // Q K^T
-      score_fma(stat[1], strm[1], D, ldd, ty, tx, dp);   // dO V^T
-      score_fma(stat[2], strm[0], D, ldd, ty, tx, gs);   // g_dQ K^T
-      score_fma(stat[0], strm[2], D, ldd, ty, tx, gs);   // + Q g_dK^T
-      score_fma(stat[1], strm[3], D, ldd, ty, tx, gp);   // dO g_dV^T
-#pragma unroll
-      for (int a = 0; a < 2; ++a)
-#pragma unroll
-        for (int b = 0; b < 2; ++b) {
-          const int i = ty + 16 * a, j = tx + 16 * b;
-          const float pr = prob(s[a][b], g.scale_log2e, sL2[i], visible(g, r0 + i, tt * TT + j));
-          const float gds = gs[a][b] * g.scale;
-          aD[a] = fmaf(pr, dp[a][b], aD[a]);
-          a2[a] = fmaf(pr, gds, a2[a]);
-          aA[a] = fmaf(pr * gds, dp[a][b], aA[a]);
-          aE[a] = fmaf(pr, gp[a][b], aE[a]);
-        }
+    v = make_float4(v.x * mul, v.y * mul, v.z * mul, v.w * mul);
+    if constexpr (KIND == K_HVP_PRE) {
+      const float4 of = load4(O + at);
+      const float dd = row_total(1, r);
+      v.x = fmaf(-dd, of.x, v.x); v.y = fmaf(-dd, of.y, v.y); v.z = fmaf(-dd, of.z, v.z); v.w = fmaf(-dd, of.w, v.w);
     }
-    __syncthreads();
-#pragma unroll
-    for (int a = 0; a < 2; ++a) {
-      const float Dv = half_warp_sum(aD[a]), d2 = half_warp_sum(a2[a]);
-      const float A = half_warp_sum(aA[a]), E = half_warp_sum(aE[a]);
-      const float d3 = A - 2.f * Dv * d2 + E;
-      const int i = ty + 16 * a, r = r0 + i;
-      if (tx == 0) {
-        sDv[i] = Dv; sD2[i] = d2; sD3[i] = d3;
-        if (r < g.N_q) { t.Dv[row_off + r] = Dv; t.dot2[row_off + r] = d2; t.dot3[row_off + r] = d3; }
+    T* dst;
+    if constexpr (KIND == K_FWD) dst = (T*)t.out_O + q_off;
+    else if constexpr (KIND == K_BWD_ROW) dst = (T*)t.out_dQ + q_off;
+    else if constexpr (KIND == K_BWD_COL) dst = (T*)(o == 0 ? t.out_dV : t.out_dK) + kv_off;
+    else if constexpr (KIND == K_HVP_PRE) dst = (T*)t.out_g_dO + q_off;
+    else if constexpr (KIND == K_HVP_ROW) dst = (T*)t.out_g_Q + q_off;
+    else dst = (T*)(o == 0 ? t.out_g_K : t.out_g_V) + kv_off;
+    store4<T>(dst + at, v);
+  };
+  if (split > 1) {
+    // each CTA of the cluster finishes its share of the float4s, adding the parts in rank order
+    const int total = SP::kNOut * TS * chunks;
+    for (int i = part * NT + tid; i < total; i += split * NT) {
+      const int row = i / chunks, chunk = i - row * chunks, r = row % TS;
+      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+      float m = 0.f;
+      if constexpr (KIND == K_FWD) m = fwd_max(r);
+      for (int q = 0; q < split; ++q) {
+        const float4 x = reinterpret_cast<const float4*>(cluster.map_shared_rank(partial, q))[i];
+        const float f = KIND == K_FWD ? factor(q, r, m) : 1.f;
+        v.x = fmaf(x.x, f, v.x); v.y = fmaf(x.y, f, v.y); v.z = fmaf(x.z, f, v.z); v.w = fmaf(x.w, f, v.w);
       }
+      finish(row / TS, r, chunk, v);
     }
-    // pass 2: g_Q and g_dO
-    for (int tt = t_begin; tt < t_end; ++tt) {
-      __syncthreads();
-      stage_tile<T>(strm[0], ldd, K, tt * TT, g.N_kv, D);
-      stage_tile<T>(strm[1], ldd, V, tt * TT, g.N_kv, D);
-      stage_tile<T>(strm[2], ldd, gK, tt * TT, g.N_kv, D);
-      stage_tile<T>(strm[3], ldd, gV, tt * TT, g.N_kv, D);
-      __syncthreads();
-      float s[2][2] = {{0.f, 0.f}, {0.f, 0.f}}, dp[2][2] = {{0.f, 0.f}, {0.f, 0.f}};
-      float gs[2][2] = {{0.f, 0.f}, {0.f, 0.f}}, gp[2][2] = {{0.f, 0.f}, {0.f, 0.f}};
-      score_fma(stat[0], strm[0], D, ldd, ty, tx, s);
-      score_fma(stat[1], strm[1], D, ldd, ty, tx, dp);
-      score_fma(stat[2], strm[0], D, ldd, ty, tx, gs);
-      score_fma(stat[0], strm[2], D, ldd, ty, tx, gs);
-      score_fma(stat[1], strm[3], D, ldd, ty, tx, gp);
+    cluster.sync();                                   // nobody leaves while its shared memory is being read
+  } else {
+#pragma unroll
+    for (int o = 0; o < SP::kNOut; ++o)
 #pragma unroll
       for (int a = 0; a < 2; ++a)
 #pragma unroll
-        for (int b = 0; b < 2; ++b) {
-          const int i = ty + 16 * a, j = tx + 16 * b;
-          const float pr = prob(s[a][b], g.scale_log2e, sL2[i], visible(g, r0 + i, tt * TT + j));
-          const RowStats rs{sL2[i], sDv[i], sD2[i], sD3[i]};
-          const HvpTerms h = hvp_terms(pr, dp[a][b], gs[a][b], gp[a][b], g.scale, rs);
-          op[0][i * OPLD + j] = h.dS;
-          op[1][i * OPLD + j] = h.g_S;
-          op[2][i * OPLD + j] = h.p;
-          op[3][i * OPLD + j] = h.g_dp;
-        }
-      __syncthreads();
-      out_fma(op[0], strm[2], ncol, ldd, ty, tx, out0);   // g_Q  += dS g_dK
-      out_fma(op[1], strm[0], ncol, ldd, ty, tx, out0);   //       + g_S K
-      out_fma(op[2], strm[3], ncol, ldd, ty, tx, out1);   // g_dO += P g_dV
-      out_fma(op[3], strm[1], ncol, ldd, ty, tx, out1);   //       + g_dp V
-    }
-    store_rows<T>((T*)t.out_g_Q + q_off, r0, g.N_q, D, ncol, ty, tx, out0, g.scale);
-    store_rows<T>((T*)t.out_g_dO + q_off, r0, g.N_q, D, ncol, ty, tx, out1, 1.f);
-    return;
+        for (int c = 0; c < DC; ++c)
+          if (chunk0 + 16 * c < chunks)
+            finish(o, row0 + 4 * a, chunk0 + 16 * c,
+                   make_float4(out[o][a][c][0].x, out[o][a][c][0].y, out[o][a][c][1].x, out[o][a][c][1].y));
   }
-
-  // ======================= double backward, column side ====================
-  if constexpr (KIND == K_HVP_COL) {
-    for (int tt = t_begin; tt < t_end; ++tt) {
-      __syncthreads();
-      stage_tile<T>(strm[0], ldd, Q, tt * TT, g.N_q, D);
-      stage_tile<T>(strm[1], ldd, dO, tt * TT, g.N_q, D);
-      stage_tile<T>(strm[2], ldd, gQ, tt * TT, g.N_q, D);
-      if (tid < 32) {
-        const int r = tt * TT + tid;
-        const bool in = r < g.N_q;
-        sL2[tid] = in ? t.L[row_off + r] * kLog2e : INFINITY;
-        sDv[tid] = in ? t.Dv[row_off + r] : 0.f;
-        sD2[tid] = in ? t.dot2[row_off + r] : 0.f;
-        sD3[tid] = in ? t.dot3[row_off + r] : 0.f;
-      }
-      __syncthreads();
-      float s[2][2] = {{0.f, 0.f}, {0.f, 0.f}}, dp[2][2] = {{0.f, 0.f}, {0.f, 0.f}};
-      float gs[2][2] = {{0.f, 0.f}, {0.f, 0.f}}, gp[2][2] = {{0.f, 0.f}, {0.f, 0.f}};
-      score_fma(stat[0], strm[0], D, ldd, ty, tx, s);    // K Q^T
-      score_fma(stat[1], strm[1], D, ldd, ty, tx, dp);   // V dO^T
-      score_fma(stat[0], strm[2], D, ldd, ty, tx, gs);   // K g_dQ^T
-      score_fma(stat[2], strm[0], D, ldd, ty, tx, gs);   // + g_dK Q^T
-      score_fma(stat[3], strm[1], D, ldd, ty, tx, gp);   // g_dV dO^T
-#pragma unroll
-      for (int a = 0; a < 2; ++a)
-#pragma unroll
-        for (int b = 0; b < 2; ++b) {
-          const int jk = ty + 16 * a, iq = tx + 16 * b;
-          const float pr = prob(s[a][b], g.scale_log2e, sL2[iq], visible(g, tt * TT + iq, r0 + jk));
-          const RowStats rs{sL2[iq], sDv[iq], sD2[iq], sD3[iq]};
-          const HvpTerms h = hvp_terms(pr, dp[a][b], gs[a][b], gp[a][b], g.scale, rs);
-          op[0][jk * OPLD + iq] = h.dS;
-          op[1][jk * OPLD + iq] = h.g_S;
-          op[2][jk * OPLD + iq] = h.g_dp;
-        }
-      __syncthreads();
-      out_fma(op[0], strm[2], ncol, ldd, ty, tx, out0);   // g_K += dS^T g_dQ
-      out_fma(op[1], strm[0], ncol, ldd, ty, tx, out0);   //      + g_S^T Q
-      out_fma(op[2], strm[1], ncol, ldd, ty, tx, out1);   // g_V += g_dp^T dO
-    }
-    store_rows<T>((T*)t.out_g_K + kv_off, r0, g.N_kv, D, ncol, ty, tx, out0, g.scale);
-    store_rows<T>((T*)t.out_g_V + kv_off, r0, g.N_kv, D, ncol, ty, tx, out1, 1.f);
-    return;
-  }
+  tc::pdl_end(g);
 }
 
-template <int KIND>
-static size_t smem_bytes(int D) {
-  constexpr int nStat = (KIND == K_FWD) ? 1 : (KIND == K_BWD_ROW) ? 2 : (KIND == K_BWD_COL) ? 2
-                        : (KIND == K_HVP_ROW) ? 3 : 4;
-  constexpr int nStream = (KIND == K_FWD) ? 2 : (KIND == K_BWD_ROW) ? 2 : (KIND == K_BWD_COL) ? 2
-                          : (KIND == K_HVP_ROW) ? 4 : 3;
-  constexpr int nOp = (KIND == K_FWD) ? 1 : (KIND == K_BWD_ROW) ? 1 : (KIND == K_BWD_COL) ? 2
-                      : (KIND == K_HVP_ROW) ? 4 : 3;
-  return sizeof(float) * ((size_t)(nStat + nStream) * 32 * (D + 4) + (size_t)nOp * 32 * OPLD + 128);
+// CTAs per stationary tile: enough for two CTAs on each of 148 SMs, but no more than there are
+// streamed tiles for a stationary one.
+static int split_for(const Geometry& g, long long units, int n_strm) {
+  const int most = g.mask_mode == 0 && g.window < n_strm ? g.window + TS : n_strm;
+  int c = 1;
+  while (c < kMaxSplit && units * c * 2 <= 2 * 148 && 2 * c <= (most + TT - 1) / TT) c *= 2;
+  return c;
+}
+
+template <int KIND, int DC, typename T>
+static cudaError_t launch_dc(const Geometry& g, const Tensors& t, cudaStream_t stream) {
+  const int n_stat = Spec<KIND>::kCol ? g.N_kv : g.N_q;
+  const long long units = (long long)g.BH * ((n_stat + TS - 1) / TS);
+  if (units <= 0) return cudaSuccess;
+  if (units * kMaxSplit > 0x7fffffffLL) return cudaErrorInvalidValue;
+  const int split = split_for(g, units, Spec<KIND>::kCol ? g.N_q : g.N_kv);
+  const size_t smem = sizeof(float) * smem_floats<KIND>(g.D);
+  auto kern = attn_simt_kernel<KIND, DC, T>;
+  static std::atomic<unsigned long long> smem_set{0};
+  // the size at the variant's largest D, so that one setting serves every call
+  const cudaError_t e = tc::set_smem_once(kern, sizeof(float) * smem_floats<KIND>(64 * DC), smem_set);
+  if (e != cudaSuccess) return e;
+  return tc::launch_pdl_cluster(kern, (unsigned)(units * split), NT, smem, (unsigned)split, stream, g, t, split);
 }
 
 template <int KIND, typename T>
 static cudaError_t launch_one(const Geometry& g, const Tensors& t, cudaStream_t stream) {
-  constexpr bool kCol = (KIND == K_BWD_COL || KIND == K_HVP_COL);
-  const int n_stat = kCol ? g.N_kv : g.N_q;
-  const long long ctas = (long long)g.BH * ((n_stat + TS - 1) / TS);
-  if (ctas <= 0) return cudaSuccess;
-  if (ctas > 0x7fffffffLL) return cudaErrorInvalidValue;
-  const size_t smem = smem_bytes<KIND>(g.D);
-  auto kern = attn_simt_kernel<KIND, T>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return e;
-  kern<<<(unsigned)ctas, NT, smem, stream>>>(g, t);
-  return cudaGetLastError();
+  return g.D <= 64 ? launch_dc<KIND, 1, T>(g, t, stream) : launch_dc<KIND, 2, T>(g, t, stream);
 }
 
 template <typename T>
 static cudaError_t dispatch(int op, const Geometry& g, const Tensors& t, cudaStream_t s, int* n, int phases) {
   cudaError_t e = cudaSuccess;
   *n = 0;
+  Geometry beside = g;      // behind the kernel in front of it in the stream, without waiting for it
+  beside.beside = 1;
   if (op == OP_FORWARD) {
     e = launch_one<K_FWD, T>(g, t, s); *n = 1;
   } else if (op == OP_BACKWARD) {
-    e = launch_one<K_BWD_ROW, T>(g, t, s);
-    if (e == cudaSuccess) e = launch_one<K_BWD_COL, T>(g, t, s);
+    e = launch_one<K_BWD_COL, T>(g, t, s);
+    if (e == cudaSuccess) e = launch_one<K_BWD_ROW, T>(beside, t, s);
     *n = 2;
   } else {
-    // the row kernel computes the per-row scalars itself (its first pass)
-    if (phases & (HVP_PHASE_PRE | HVP_PHASE_ROW)) { e = launch_one<K_HVP_ROW, T>(g, t, s); ++*n; }
-    if (e == cudaSuccess && (phases & HVP_PHASE_COL)) { e = launch_one<K_HVP_COL, T>(g, t, s); ++*n; }
+    const bool row = (phases & HVP_PHASE_ROW) != 0, col = (phases & HVP_PHASE_COL) != 0;
+    if (phases & HVP_PHASE_PRE) { e = launch_one<K_HVP_PRE, T>(g, t, s); ++*n; }
+    if (e == cudaSuccess && col) { e = launch_one<K_HVP_COL, T>(g, t, s); ++*n; }
+    if (e == cudaSuccess && row) { e = launch_one<K_HVP_ROW, T>(col ? beside : g, t, s); ++*n; }
   }
   return e;
 }

@@ -53,18 +53,26 @@ inline cudaError_t set_smem_once(Kern kern, size_t smem, std::atomic<unsigned lo
 }
 
 template <typename... P, typename... A>
-inline cudaError_t launch_pdl(void (*kern)(P...), unsigned ctas, unsigned threads, size_t smem, cudaStream_t s, const A&... args) {
-  cudaLaunchAttribute attr;
-  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr.val.programmaticStreamSerializationAllowed = 1;
+inline cudaError_t launch_pdl_cluster(void (*kern)(P...), unsigned ctas, unsigned threads, size_t smem, unsigned cluster,
+                                      cudaStream_t s, const A&... args) {
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = cluster;
+  attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(ctas);
   cfg.blockDim = dim3(threads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
-  cfg.attrs = &attr;
-  cfg.numAttrs = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = cluster > 1 ? 2 : 1;
   return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+}
+template <typename... P, typename... A>
+inline cudaError_t launch_pdl(void (*kern)(P...), unsigned ctas, unsigned threads, size_t smem, cudaStream_t s, const A&... args) {
+  return launch_pdl_cluster(kern, ctas, threads, smem, 1, s, args...);
 }
 
 // Output tensors by operation: forward {O}; backward {dQ, dK, dV}; double backward
