@@ -4,7 +4,7 @@
 // asked for, half-precision inputs.  All arithmetic is fp32 on CUDA cores; inputs are widened when a
 // tile is staged in shared memory.  Nothing here materialises more than a 32 x 64 score tile per CTA.
 //
-// A CTA of 256 threads owns 32 STATIONARY rows of one (batch, head) -- query rows in the row kinds,
+// A CTA owns 32 STATIONARY rows of one (batch, head) -- query rows in the row kinds,
 // key rows in the column kinds -- and streams 64-row tiles of the other axis:
 //
 //   kind      stationary        streamed          produces
@@ -15,13 +15,16 @@
 //   HVP_ROW   Q, dO, g_dQ       K, V, g_dK, g_dV  g_Q = s (dS g_dK + g_S K)
 //   HVP_COL   K, V, g_dK, g_dV  Q, dO, g_dQ       g_K = s (dS^T g_dQ + g_S^T Q), g_V = g_dp^T dO
 //
-// Bound by the FMA pipe and, next to it, by shared-memory reads.  A warp is 4 x 8 threads and a
-// thread holds 2 x 4 scores of every score matrix of the kind, so that each float4 it reads serves
-// several products (HVP: 22 reads for 160 multiply-adds; every read of a warp touches at most eight
-// rows, one pass through the banks) and the packed f32x2 multiply-adds run along the head dimension
-// without a move.  Rows are stored without padding where D is a multiple of 32, their 16-byte chunks
-// XOR-swizzled by the row, which lets two CTAs of every kind share an SM at D <= 64: one computes
-// while the other loads.
+// Bound by shared-memory reads: a float4 read of a warp takes four clocks of the SM's 128 bytes per
+// clock whether its lanes broadcast or not, so a thread has to do 16 multiply-adds per float4 before
+// the FMA pipe is the limit.  A warp is 4 x 8 threads and, at D <= 64, a thread holds 4 x 4 scores
+// of every score matrix of the kind, so that each float4 it reads serves several products (HVP: 28
+// reads for 320 multiply-adds).  Above, where one CTA fills the shared memory of an SM, a thread
+// holds 2 x 4 (22 for 160; 45 % of the FMA rate with the read path at 80 %): twice the warps hide
+// the latencies that eat what 4 x 4 saves (2.60 against 3.37 ms at B2 H8 N1024 D128).  The packed
+// f32x2 multiply-adds run along the head dimension without a move.  Rows are stored without padding
+// where D is a multiple of 32, their 16-byte chunks XOR-swizzled by the row, which lets two CTAs of
+// every kind share an SM at D <= 64: one computes while the other loads.
 // Small problems: with fewer than two CTAs per SM the streamed tiles of a stationary tile are dealt
 // out to a CLUSTER of 2 to 8 CTAs (split_for), whose partial sums are added through distributed
 // shared memory in a fixed order; results are bitwise reproducible either way.
@@ -40,7 +43,11 @@ namespace cg = cooperative_groups;
 
 constexpr int TS = 32;        // stationary rows per CTA
 constexpr int TT = 64;        // streamed rows per iteration
-constexpr int NT = 256;       // threads per CTA: 4 x 2 warps over the 32 x 64 score tile
+constexpr int CB = 4;         // score columns per thread, 8 apart
+// By tile width (DC = 1: D <= 64, 2: D <= 128): score rows per thread, 4 apart, and threads per CTA,
+// (8 / RA) x 2 warps over the 32 x 64 score tile.
+__host__ __device__ constexpr int rows_of(int DC) { return DC == 1 ? 4 : 2; }
+__host__ __device__ constexpr int threads_of(int DC) { return DC == 1 ? 128 : 256; }
 constexpr int kMaxSplit = 8;  // CTAs per cluster (the portable maximum)
 
 enum Kind { K_FWD = 0, K_BWD_ROW, K_BWD_COL, K_HVP_PRE, K_HVP_ROW, K_HVP_COL };
@@ -81,7 +88,7 @@ template <typename T> __device__ __forceinline__ float4 widen4(const T* p) {
 // share a row.  float goes by cp.async (complete after cp_async_wait_all and a barrier).
 template <int DC, typename T>
 __device__ __forceinline__ void stage_tile(float* dst, const Layout& lay, const T* src, int row0, int rows, int n_rows, int D) {
-  constexpr int kLanes = 16 * DC;
+  constexpr int kLanes = 16 * DC, NT = threads_of(DC);
   const int chunk = threadIdx.x % kLanes;
   if (chunk * 4 >= D) return;
   for (int r = threadIdx.x / kLanes; r < rows; r += NT / kLanes) {
@@ -99,32 +106,32 @@ __device__ __forceinline__ void mac(float2& acc, const float4& x, const float4& 
 }
 
 // The raw score matrices of a kind for this thread's 2 x 4 elements.
-template <int KIND>
+template <int KIND, int RA>
 __device__ __forceinline__ void scores(float* const (&stat)[4], float* const (&strm)[4], const Layout& lay, int D,
-                                       int row0, int col0, float (&out)[Spec<KIND>::kNAcc][2][4]) {
+                                       int row0, int col0, float (&out)[Spec<KIND>::kNAcc][RA][CB]) {
   using SP = Spec<KIND>;
   constexpr int kScored = KIND == K_FWD ? 1 : SP::kNStream;     // the forward's V takes no part in the scores
-  float2 acc[SP::kNAcc][2][4];
+  float2 acc[SP::kNAcc][RA][CB];
 #pragma unroll
   for (int m = 0; m < SP::kNAcc; ++m)
 #pragma unroll
-    for (int a = 0; a < 2; ++a)
+    for (int a = 0; a < RA; ++a)
 #pragma unroll
-      for (int b = 0; b < 4; ++b) acc[m][a][b] = make_float2(0.f, 0.f);
+      for (int b = 0; b < CB; ++b) acc[m][a][b] = make_float2(0.f, 0.f);
 #pragma unroll 2
   for (int k = 0; k < (D >> 2); ++k) {
-    float4 x[SP::kNStat][2];
+    float4 x[SP::kNStat][RA];
 #pragma unroll
     for (int i = 0; i < SP::kNStat; ++i)
 #pragma unroll
-      for (int a = 0; a < 2; ++a) x[i][a] = *reinterpret_cast<const float4*>(stat[i] + lay.at(row0 + 4 * a, k));
+      for (int a = 0; a < RA; ++a) x[i][a] = *reinterpret_cast<const float4*>(stat[i] + lay.at(row0 + 4 * a, k));
 #pragma unroll
-    for (int b = 0; b < 4; ++b) {
+    for (int b = 0; b < CB; ++b) {
       float4 y[kScored];
 #pragma unroll
       for (int i = 0; i < kScored; ++i) y[i] = *reinterpret_cast<const float4*>(strm[i] + lay.at(col0 + 8 * b, k));
 #pragma unroll
-      for (int a = 0; a < 2; ++a) {
+      for (int a = 0; a < RA; ++a) {
         mac(acc[0][a][b], x[0][a], y[0]);                       // Q K^T               | K Q^T
         if constexpr (SP::kNAcc == 2) mac(acc[1][a][b], x[1][a], y[1]);      // dO V^T  | V dO^T
         if constexpr (SP::kHvp) {
@@ -140,20 +147,20 @@ __device__ __forceinline__ void scores(float* const (&stat)[4], float* const (&s
 #pragma unroll
   for (int m = 0; m < SP::kNAcc; ++m)
 #pragma unroll
-    for (int a = 0; a < 2; ++a)
+    for (int a = 0; a < RA; ++a)
 #pragma unroll
-      for (int b = 0; b < 4; ++b) out[m][a][b] = acc[m][a][b].x + acc[m][a][b].y;
+      for (int b = 0; b < CB; ++b) out[m][a][b] = acc[m][a][b].x + acc[m][a][b].y;
 }
 
 // out[a][c] += sum_j Op[row0 + 4a, j] * Z[j, chunk c of this thread]
-template <int DC>
+template <int DC, int RA>
 __device__ __forceinline__ void out_fma(const float* op, const float* Z, const Layout& lay, int row0, int chunk0, int chunks,
-                                        float2 (&out)[2][DC][2]) {
+                                        float2 (&out)[RA][DC][2]) {
 #pragma unroll 2
   for (int j = 0; j < TT; j += 4) {
-    float o[2][4];
+    float o[RA][4];
 #pragma unroll
-    for (int a = 0; a < 2; ++a) {
+    for (int a = 0; a < RA; ++a) {
       const float4 v = *reinterpret_cast<const float4*>(op + op_at(row0 + 4 * a, j));
       o[a][0] = v.x; o[a][1] = v.y; o[a][2] = v.z; o[a][3] = v.w;
     }
@@ -164,7 +171,7 @@ __device__ __forceinline__ void out_fma(const float* op, const float* Z, const L
         if (chunk0 + 16 * c < chunks) {
           const float4 z = *reinterpret_cast<const float4*>(Z + lay.at(j + u, chunk0 + 16 * c));
 #pragma unroll
-          for (int a = 0; a < 2; ++a) {
+          for (int a = 0; a < RA; ++a) {
             const float2 oo = make_float2(o[a][u], o[a][u]);
             out[a][c][0] = __ffma2_rn(oo, make_float2(z.x, z.y), out[a][c][0]);
             out[a][c][1] = __ffma2_rn(oo, make_float2(z.z, z.w), out[a][c][1]);
@@ -202,8 +209,9 @@ __host__ __device__ constexpr int smem_floats(int D) {
 
 // DC: 1 for D <= 64, 2 up to 128.
 template <int KIND, int DC, typename T>
-__global__ void __launch_bounds__(NT, DC == 1 ? 2 : 1) attn_simt_kernel(const Geometry g, const Tensors t, const int split) {
+__global__ void __launch_bounds__(threads_of(DC), DC == 1 ? 2 : 1) attn_simt_kernel(const Geometry g, const Tensors t, const int split) {
   using SP = Spec<KIND>;
+  constexpr int RA = rows_of(DC), NT = threads_of(DC);
   extern __shared__ __align__(16) float smem[];
   const int D = g.D;
   const Layout lay(D);
@@ -215,7 +223,7 @@ __global__ void __launch_bounds__(NT, DC == 1 ? 2 : 1) attn_simt_kernel(const Ge
   const int r0 = tile * TS;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int ty = lane >> 3, tx = lane & 7, wcol = warp & 1;
-  const int row0 = (warp >> 1) * 8 + ty;              // this thread's rows: row0, row0 + 4
+  const int row0 = (warp >> 1) * 4 * RA + ty;         // this thread's rows: row0 + 4 a
   const int col0 = wcol * 32 + tx;                    // its score columns: col0 + 8 b
   const int chunk0 = wcol * 8 + tx, chunks = D >> 2;  // its output float4s: chunk0 + 16 c
 
@@ -253,11 +261,11 @@ __global__ void __launch_bounds__(NT, DC == 1 ? 2 : 1) attn_simt_kernel(const Ge
 #pragma unroll
   for (int i = 0; i < SP::kNStat; ++i) stage_tile<DC, T>(stat[i], lay, stat_src[i], r0, TS, n_stat, D);
 
-  // ---- scalars of this thread's two rows (row kinds)
-  float L2[2] = {0.f, 0.f}, Dv[2] = {0.f, 0.f}, d2[2] = {0.f, 0.f}, d3[2] = {0.f, 0.f};
+  // ---- scalars of this thread's rows (row kinds)
+  float L2[RA] = {}, Dv[RA] = {}, d2[RA] = {}, d3[RA] = {};
   if constexpr (!SP::kCol && KIND != K_FWD) {
 #pragma unroll
-    for (int a = 0; a < 2; ++a) {
+    for (int a = 0; a < RA; ++a) {
       const int r = r0 + row0 + 4 * a;
       const bool in = r < g.N_q;
       L2[a] = in ? t.L[row_off + r] * kLog2e : INFINITY;
@@ -275,13 +283,15 @@ __global__ void __launch_bounds__(NT, DC == 1 ? 2 : 1) attn_simt_kernel(const Ge
       }
     }
   }
-  float m_run[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.f, 0.f};                       // FWD
-  float aD[2] = {0.f, 0.f}, a2[2] = {0.f, 0.f}, aA[2] = {0.f, 0.f}, aE[2] = {0.f, 0.f};   // HVP_PRE
-  float2 out[SP::kNOut][2][DC][2];
+  float m_run[RA], l_run[RA] = {};                           // FWD
+  float aD[RA] = {}, a2[RA] = {}, aA[RA] = {}, aE[RA] = {};   // HVP_PRE
+#pragma unroll
+  for (int a = 0; a < RA; ++a) m_run[a] = -INFINITY;
+  float2 out[SP::kNOut][RA][DC][2];
 #pragma unroll
   for (int o = 0; o < SP::kNOut; ++o)
 #pragma unroll
-    for (int a = 0; a < 2; ++a)
+    for (int a = 0; a < RA; ++a)
 #pragma unroll
       for (int c = 0; c < DC; ++c) out[o][a][c][0] = out[o][a][c][1] = make_float2(0.f, 0.f);
 
@@ -292,30 +302,34 @@ __global__ void __launch_bounds__(NT, DC == 1 ? 2 : 1) attn_simt_kernel(const Ge
     for (int i = 0; i < SP::kNStream; ++i) stage_tile<DC, T>(strm[i], lay, strm_src[i], s0, TT, n_strm, D);
     if constexpr (SP::kCol) {                         // [L2 | Dv | dot2 | dot3] of the streamed queries
       if constexpr (SP::kHvp) {
-        const int which = tid >> 6, r = s0 + (tid & 63);
-        const float* src = which == 0 ? t.L : which == 1 ? t.Dv : which == 2 ? t.dot2 : t.dot3;
-        const float v = r < g.N_q ? src[row_off + r] : 0.f;
-        aux[tid] = which == 0 ? (r < g.N_q ? v * kLog2e : INFINITY) : v;
+#pragma unroll
+        for (int i = tid; i < 4 * TT; i += NT) {
+          const int r = s0 + (i & 63), which = i >> 6;
+          const float* src = which == 0 ? t.L : which == 1 ? t.Dv : which == 2 ? t.dot2 : t.dot3;
+          const float v = r < g.N_q ? src[row_off + r] : 0.f;
+          aux[i] = which == 0 ? (r < g.N_q ? v * kLog2e : INFINITY) : v;
+        }
       } else {
-        const int r = s0 + (tid >> 2);                // four threads per query
+        constexpr int TQ = NT / TT;                   // threads per query
+        const int r = s0 + tid / TQ;
         float s = 0.f;
         if (r < g.N_q)
-          for (int c = tid & 3; c < chunks; c += 4) {
+          for (int c = tid % TQ; c < chunks; c += TQ) {
             const float4 x = load4(dO + (size_t)r * D + 4 * c), y = load4(O + (size_t)r * D + 4 * c);
             s += x.x * y.x + x.y * y.y + x.z * y.z + x.w * y.w;
           }
-        s += __shfl_xor_sync(0xffffffffu, s, 2);
-        s += __shfl_xor_sync(0xffffffffu, s, 1);
-        if ((tid & 3) == 0) {
-          aux[tid >> 2] = r < g.N_q ? t.L[row_off + r] * kLog2e : INFINITY;
-          aux[TT + (tid >> 2)] = s;
+#pragma unroll
+        for (int o = TQ / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        if (tid % TQ == 0) {
+          aux[tid / TQ] = r < g.N_q ? t.L[row_off + r] * kLog2e : INFINITY;
+          aux[TT + tid / TQ] = s;
         }
       }
     }
     cp_async_wait_all();
     __syncthreads();
-    float s[SP::kNAcc][2][4];
-    scores<KIND>(stat, strm, lay, D, row0, col0, s);
+    float s[SP::kNAcc][RA][CB];
+    scores<KIND, RA>(stat, strm, lay, D, row0, col0, s);
     const bool full = SP::kCol ? tile_fully_visible(g, s0, s0 + TT, r0, r0 + TS) : tile_fully_visible(g, r0, r0 + TS, s0, s0 + TT);
     auto sees = [&](int a, int b) {
       const int i = r0 + row0 + 4 * a, j = s0 + col0 + 8 * b;
@@ -325,10 +339,10 @@ __global__ void __launch_bounds__(NT, DC == 1 ? 2 : 1) attn_simt_kernel(const Ge
     if constexpr (KIND == K_FWD) {
       // running maximum of a row: over this warp's 32 columns, then over the two warps of the row
 #pragma unroll
-      for (int a = 0; a < 2; ++a) {
+      for (int a = 0; a < RA; ++a) {
         float mx = -INFINITY;
 #pragma unroll
-        for (int b = 0; b < 4; ++b) {
+        for (int b = 0; b < CB; ++b) {
           s[0][a][b] = sees(a, b) ? s[0][a][b] * g.scale_log2e : -INFINITY;
           mx = fmaxf(mx, s[0][a][b]);
         }
@@ -337,7 +351,7 @@ __global__ void __launch_bounds__(NT, DC == 1 ? 2 : 1) attn_simt_kernel(const Ge
       }
       __syncthreads();
 #pragma unroll
-      for (int a = 0; a < 2; ++a) {
+      for (int a = 0; a < RA; ++a) {
         const float m_new = fmaxf(m_run[a], fmaxf(aux[row0 + 4 * a], aux[TS + row0 + 4 * a]));
         const float f = m_new == -INFINITY ? 1.f : exp2f(m_run[a] - m_new);
         m_run[a] = m_new;
@@ -347,7 +361,7 @@ __global__ void __launch_bounds__(NT, DC == 1 ? 2 : 1) attn_simt_kernel(const Ge
 #pragma unroll
           for (int h = 0; h < 2; ++h) out[0][a][c][h] = make_float2(out[0][a][c][h].x * f, out[0][a][c][h].y * f);
 #pragma unroll
-        for (int b = 0; b < 4; ++b) {
+        for (int b = 0; b < CB; ++b) {
           const float pr = m_new == -INFINITY ? 0.f : exp2f(s[0][a][b] - m_new);
           l_run[a] += pr;
           op[0][op_at(row0 + 4 * a, col0 + 8 * b)] = pr;
@@ -355,9 +369,9 @@ __global__ void __launch_bounds__(NT, DC == 1 ? 2 : 1) attn_simt_kernel(const Ge
       }
     } else {
 #pragma unroll
-      for (int a = 0; a < 2; ++a)
+      for (int a = 0; a < RA; ++a)
 #pragma unroll
-        for (int b = 0; b < 4; ++b) {
+        for (int b = 0; b < CB; ++b) {
           const int col = col0 + 8 * b, at = op_at(row0 + 4 * a, col);
           RowStats rs;
           if constexpr (SP::kCol) rs = RowStats{aux[col], aux[TT + col], SP::kHvp ? aux[2 * TT + col] : 0.f, SP::kHvp ? aux[3 * TT + col] : 0.f};
@@ -385,7 +399,7 @@ __global__ void __launch_bounds__(NT, DC == 1 ? 2 : 1) attn_simt_kernel(const Ge
         }
     }
     __syncthreads();
-    auto add = [&](int o, int which, int z) { out_fma<DC>(op[which], strm[z], lay, row0, chunk0, chunks, out[o]); };
+    auto add = [&](int o, int which, int z) { out_fma<DC, RA>(op[which], strm[z], lay, row0, chunk0, chunks, out[o]); };
     if constexpr (KIND == K_FWD) add(0, 0, 1);                                   // O += P V
     else if constexpr (KIND == K_BWD_ROW) add(0, 0, 0);                          // dQ += dS K
     else if constexpr (KIND == K_BWD_COL) { add(0, 0, 1); add(1, 1, 0); }        // dV += P^T dO; dK += dS^T Q
@@ -403,7 +417,7 @@ __global__ void __launch_bounds__(NT, DC == 1 ? 2 : 1) attn_simt_kernel(const Ge
   float* const sums = op[0];                          // [2 halves][4][TS] row sums
   if constexpr (KIND == K_FWD || KIND == K_HVP_PRE) {
 #pragma unroll
-    for (int a = 0; a < 2; ++a) {
+    for (int a = 0; a < RA; ++a) {
       const float v0 = KIND == K_FWD ? m_run[a] : row_sum(aD[a]);
       const float v1 = row_sum(KIND == K_FWD ? l_run[a] : a2[a]);
       const float v2 = row_sum(aA[a]), v3 = row_sum(aE[a]);
@@ -417,7 +431,7 @@ __global__ void __launch_bounds__(NT, DC == 1 ? 2 : 1) attn_simt_kernel(const Ge
 #pragma unroll
     for (int o = 0; o < SP::kNOut; ++o)
 #pragma unroll
-      for (int a = 0; a < 2; ++a)
+      for (int a = 0; a < RA; ++a)
 #pragma unroll
         for (int c = 0; c < DC; ++c)
           if (chunk0 + 16 * c < chunks)
@@ -508,7 +522,7 @@ __global__ void __launch_bounds__(NT, DC == 1 ? 2 : 1) attn_simt_kernel(const Ge
 #pragma unroll
     for (int o = 0; o < SP::kNOut; ++o)
 #pragma unroll
-      for (int a = 0; a < 2; ++a)
+      for (int a = 0; a < RA; ++a)
 #pragma unroll
         for (int c = 0; c < DC; ++c)
           if (chunk0 + 16 * c < chunks)
@@ -540,7 +554,7 @@ static cudaError_t launch_dc(const Geometry& g, const Tensors& t, cudaStream_t s
   // the size at the variant's largest D, so that one setting serves every call
   const cudaError_t e = tc::set_smem_once(kern, sizeof(float) * smem_floats<KIND>(64 * DC), smem_set);
   if (e != cudaSuccess) return e;
-  return tc::launch_pdl_cluster(kern, (unsigned)(units * split), NT, smem, (unsigned)split, stream, g, t, split);
+  return tc::launch_pdl_cluster(kern, (unsigned)(units * split), threads_of(DC), smem, (unsigned)split, stream, g, t, split);
 }
 
 template <int KIND, typename T>

@@ -1,0 +1,39 @@
+"""fp32 kernels at the edges of their tiles and at every size of the cluster split: 32 stationary and
+64 streamed rows per tile, 1 / 2 / 4 / 8 CTAs per stationary tile, both tile widths, head dimensions
+with and without the swizzled layout."""
+import importlib
+
+import pytest
+import torch
+
+import attention_oracle as orc
+
+pytestmark = pytest.mark.gpu
+tcapi = importlib.import_module("610sample_b200.torch_capi")
+
+
+@pytest.mark.parametrize("B,H,N_q,N_kv,D,window,chunk,mask", [
+    (1, 1, 32, 64, 64, 64, 0, 1),        # exactly one tile
+    (1, 1, 33, 65, 48, 40, 1, 0),        # one row more on both axes; pitch with padding
+    (1, 2, 31, 129, 128, 1000, 0, 0),    # split 2, last part nearly empty
+    (1, 1, 95, 250, 80, 250, 2, 0),      # split 4
+    (1, 2, 64, 520, 64, 520, 3, 0),      # split 8; keys in front of the sequence in no window
+    (2, 1, 64, 520, 16, 70, 9, 0),       # a window shorter than the keys: parts without a visible key
+    (2, 8, 600, 600, 64, 600, 0, 0),     # no split
+    (1, 3, 40, 1, 96, 1, 0, 1),          # one key
+])
+def test_fp32_kernels_match_the_oracle(B, H, N_q, N_kv, D, window, chunk, mask):
+    inp = orc.make_inputs(B, H, N_q, N_kv, D, seed=N_q + D, dtype=torch.float32)
+    ref = orc.closed_form_all(*(inp[n] for n in orc.INPUT_NAMES), window_size=window, chunk_id=chunk, mask_mode=mask)
+    g = {n: t.cuda() for n, t in inp.items()}
+    runs = []
+    for _ in range(2):
+        O, L = tcapi.forward(g["Q"], g["K"], g["V"], window, chunk, mask)
+        b = tcapi.backward(g["dO"], g["Q"], g["K"], g["V"], O, L, window, chunk, mask)
+        h = tcapi.double_backward(g["g_dQ"], g["g_dK"], g["g_dV"], g["dO"], g["Q"], g["K"], g["V"], O, L, window, chunk, mask)
+        runs.append((O,) + tuple(b) + tuple(h))
+    for got, again, n in zip(*runs, ("O", "dQ", "dK", "dV", "g_dO", "g_Q", "g_K", "g_V")):
+        assert torch.equal(got, again), n
+        r = ref[n].double()
+        # the family's stated tolerance: 1e-4 of the largest value (fp32 sums of at most N * D terms)
+        assert float((got.double().cpu() - r).abs().max()) <= 1e-4 * max(1.0, float(r.abs().max())), n
