@@ -10,10 +10,15 @@
 // its OWN running maximum m, running sum l and O accumulator, i.e. the keys are split in two
 // interleaved streams that never have to agree on a maximum while the loop runs; the epilogue
 // merges them: O = (O_0 2^(m_0 - m) + O_1 2^(m_1 - m)) / (l_0 2^(m_0 - m) + l_1 2^(m_1 - m)).
-// Rescaling is lazy: m only moves when a tile's maximum exceeds it by more than kTau (in log2
-// units), so P <= 2^kTau, and the O row is then multiplied in tensor memory by 2^(m_old - m_new)
+// Rescaling is lazy: m only moves when a tile's maximum exceeds it by more than tau (in log2
+// units), so P <= 2^tau, and the O row is then multiplied in tensor memory by 2^(m_old - m_new)
 // (a read-modify-write of the row by its owner thread, after the group's previous P V product has
-// completed).  With inputs of ordinary scale that happens in the first tile or two of a row only.
+// completed).  tau is as large as P's type allows: P has the same relative precision whatever its
+// exponent, in bf16 up to far beyond any sum that occurs, so 24 (O and l stay below 2^24 N |V|); in
+// f16 15, one below the largest exponent.  With peaked rows (scores of standard deviation 4) a
+// threshold of 8 made every row of a warp rescale once or twice at tiles of its own, each time
+// stalling the warp for about a tile: 2.20 against 1.85 ms at H32 N16384 D128, Q and K of twice unit
+// variance; 24 is beyond what a row's first tile leaves to come.
 // Tensor memory (512 columns): three score buffers S0, S1, S2 [0,192), Q [192,192+D/2),
 // O_0 [256,256+D), O_1 [256+D, 256+2D).  P is written (two halves per 32-bit column) over the
 // first 32 columns of the score buffer it was computed from and read from there as the A operand
@@ -33,7 +38,7 @@ constexpr int kFwdPvWarp = 10;      // issues O += P V
 constexpr int kFwdThreads = 352;    // 8 math warps, TMA producer, two MMA issuers
 constexpr int kFwdMaxStages = 8;
 constexpr int kFwdSBufs = 3;
-constexpr float kTau = 8.f;         // log2 units: P <= 256
+template <typename T> constexpr float kTau = Pack<T>::kIsBf16 ? 24.f : 15.f;     // log2 units
 constexpr int KFWD = 20;            // kernel id inside device status codes
 
 struct FwdControl {
@@ -341,8 +346,8 @@ fwd_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Tensors
         for (int e = 0; e < 8; ++e) mx8[e] = fmaxf(mx8[e], fmaxf(__uint_as_float(s_[c][e]), __uint_as_float(s_[c][8 + e])));
       const float mx = fmaxf(fmaxf(fmaxf(mx8[0], mx8[1]), fmaxf(mx8[2], mx8[3])), fmaxf(fmaxf(mx8[4], mx8[5]), fmaxf(mx8[6], mx8[7]))) *
                        g.scale_log2e;
-      // lazy rescale: the reference moves only when this tile exceeds it by more than kTau
-      const bool grow = mx > m_ref + kTau || (m_ref == -INFINITY && mx > -INFINITY);
+      // lazy rescale: the reference moves only when this tile exceeds it by more than kTau<T>
+      const bool grow = mx > m_ref + kTau<T> || (m_ref == -INFINITY && mx > -INFINITY);
       if (__any_sync(0xffffffffu, grow)) {
         const float m_new = grow ? mx : m_ref;
         const float f = (m_ref == -INFINITY) ? 0.f : ex2(m_ref - m_new);   // 1 for the rows that do not move
