@@ -273,11 +273,26 @@ cudaError_t launch_fwd_bwd(int kind, int D, int is_bf16, const TmaMaps& maps, co
                            cudaStream_t s);
 cudaError_t launch_fwd(int D, int is_bf16, const TmaMaps& maps, const Geometry& g, const Tensors& t, cudaStream_t s);
 
-// dQ beside dK/dV and g_Q beside g_K/g_V: the kernel with the longer CTAs first, the other one on
-// the SMs its last CTAs leave idle (tc_common.cuh)
-static Geometry beside(Geometry g) {
-  g.beside = 1;
-  return g;
+// dQ beside dK/dV and g_Q beside g_K/g_V: one kernel first, the other one on the SMs its last CTAs
+// leave idle (tc_common.cuh).  The kernel with the longer CTAs goes first, so that the tail is made
+// of short ones: the row kernel where a query sees more keys than a key is seen by queries (chunks of
+// 1024 queries against a window of 8192: 128 tiles per row CTA, 16 per column CTA; backward 410 ->
+// 392 us at H32 D80), else the column kernel, whose tile costs more.
+static bool row_side_first(const Geometry& g) {
+  if (g.mask_mode != 0) return g.N_kv > g.N_q;
+  return (g.window < g.N_kv ? g.window : g.N_kv) > (g.window < g.N_q ? g.window : g.N_q);
+}
+
+template <typename Row, typename Col>
+static cudaError_t side_by_side(const Geometry& g, Row row, Col col) {
+  Geometry second = g;
+  second.beside = 1;
+  if (row_side_first(g)) {
+    const cudaError_t e = row(g);
+    return e == cudaSuccess ? col(second) : e;
+  }
+  const cudaError_t e = col(g);
+  return e == cudaSuccess ? row(second) : e;
 }
 
 template <typename T>
@@ -294,14 +309,18 @@ static cudaError_t launch_op(int op, const TmaMaps& maps, const Geometry& g, con
     if (rows > 0) {
       e = launch_rowdot<T>((const T*)t.dO, (const T*)t.O, t.Dv, rows, g.D, s);
     }
-    if (e == cudaSuccess) e = launch_fwd_bwd(3, D, bf, maps, g, t, s);                // dK, dV
-    if (e == cudaSuccess) e = launch_fwd_bwd(2, D, bf, maps, beside(g), t, s);        // dQ
+    if (e == cudaSuccess)
+      e = side_by_side(g, [&](const Geometry& q) { return launch_fwd_bwd(2, D, bf, maps, q, t, s); },      // dQ
+                       [&](const Geometry& q) { return launch_fwd_bwd(3, D, bf, maps, q, t, s); });       // dK, dV
     *n = 3;
   } else {
     if (phases & HVP_PHASE_PRE) { e = launch_hvp_row(0, D, bf, maps, g, t, s); ++*n; }                        // scalars + g_dO
     const bool row = (phases & HVP_PHASE_ROW) != 0, col = (phases & HVP_PHASE_COL) != 0;
-    if (e == cudaSuccess && col) { e = launch_hvp_col(D, bf, maps, g, t, s); ++*n; }                          // g_K, g_V
-    if (e == cudaSuccess && row) { e = launch_hvp_row(1, D, bf, maps, col ? beside(g) : g, t, s); ++*n; }     // g_Q
+    auto g_q = [&](const Geometry& q) { ++*n; return launch_hvp_row(1, D, bf, maps, q, t, s); };          // g_Q
+    auto g_kv = [&](const Geometry& q) { ++*n; return launch_hvp_col(D, bf, maps, q, t, s); };            // g_K, g_V
+    if (e == cudaSuccess && row && col) e = side_by_side(g, g_q, g_kv);
+    else if (e == cudaSuccess && row) e = g_q(g);
+    else if (e == cudaSuccess && col) e = g_kv(g);
   }
   return e;
 }
