@@ -127,6 +127,18 @@ fb_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Tensors 
   else key_range_for_queries(g, r0, r0 + BM, lo, hi);
   const int t_begin = lo / BN;
   const int n_iter = (hi > lo) ? ((hi + BN - 1) / BN - t_begin) : 0;
+  if (n_iter == 0) {       // nothing to visit
+    pdl_begin(g);
+    pdl_trigger();
+    if constexpr (CF::kCol) {
+      zero_rows(t.out_dK, bh, r0, g.N_kv, g.D);
+      zero_rows(t.out_dV, bh, r0, g.N_kv, g.D);
+    } else {
+      zero_rows(t.out_dQ, bh, r0, g.N_q, g.D);
+    }
+    pdl_end(g);
+    return;
+  }
 
   const uint32_t bar_staging_full = smem_u32(&ctl->staging_full), bar_stat_ready = smem_u32(&ctl->stat_ready);
   const uint32_t bar_acc_done = smem_u32(&ctl->acc_done);

@@ -110,6 +110,14 @@ fwd_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Tensors
   key_range_for_queries(g, r0, r0 + BM, lo, hi);
   const int t_begin = lo / BN;
   const int n_iter = (hi > lo) ? ((hi + BN - 1) / BN - t_begin) : 0;
+  if (n_iter == 0) {       // nothing to visit
+    pdl_begin(g);
+    pdl_trigger();
+    zero_rows(t.out_O, bh, r0, g.N_q, g.D);
+    if (threadIdx.x < BM && r0 + threadIdx.x < g.N_q) t.out_L[(size_t)bh * g.N_q + r0 + threadIdx.x] = -INFINITY;
+    pdl_end(g);
+    return;
+  }
 
   const uint32_t bar_staging_full = smem_u32(&ctl->staging_full), bar_q_ready = smem_u32(&ctl->q_ready);
   const uint32_t bar_acc_done = smem_u32(&ctl->acc_done);

@@ -119,6 +119,14 @@ hvp_col_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Ten
   query_range_for_keys(g, r0, r0 + BM, lo, hi);
   const int t_begin = lo / BN;
   const int n_iter = (hi > lo) ? ((hi + BN - 1) / BN - t_begin) : 0;
+  if (n_iter == 0) {       // nothing to visit
+    pdl_begin(g);
+    pdl_trigger();
+    zero_rows(t.out_g_K, bh, r0, g.N_kv, g.D);
+    zero_rows(t.out_g_V, bh, r0, g.N_kv, g.D);
+    pdl_end(g);
+    return;
+  }
 
   const uint32_t bar_stat_full = smem_u32(&ctl->stat_full);
   const uint32_t bar_ra_full = smem_u32(&ctl->ra_full), bar_ra_free = smem_u32(&ctl->ra_free);

@@ -141,6 +141,20 @@ hvp_row_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Ten
   key_range_for_queries(g, r0, r0 + BM, lo, hi);
   const int t_begin = lo / BN;
   const int n_iter = (hi > lo) ? ((hi + BN - 1) / BN - t_begin) : 0;
+  if (n_iter == 0) {       // nothing to visit
+    pdl_begin(g);
+    pdl_trigger();
+    zero_rows(MODE == ROW_PREDO ? t.out_g_dO : t.out_g_Q, bh, r0, g.N_q, g.D);
+    if constexpr (MODE == ROW_PREDO) {
+      const int r = r0 + threadIdx.x;
+      if (threadIdx.x < BM && r < g.N_q) {
+        const size_t at = (size_t)bh * g.N_q + r;
+        t.Dv[at] = t.dot2[at] = t.dot3[at] = 0.f;
+      }
+    }
+    pdl_end(g);
+    return;
+  }
 
   const uint32_t bar_stat_full = smem_u32(&ctl->stat_full);
   const uint32_t bar_staging_full = smem_u32(&ctl->staging_full);

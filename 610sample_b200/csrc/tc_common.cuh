@@ -134,6 +134,17 @@ __device__ __forceinline__ void store_op16(uint32_t tile, int row, int col0, con
 }
 
 
+// Zeros in rows [row0, row0 + BM) of plane `plane` of a [planes][n_rows][D] half-precision tensor: the
+// result of a CTA that has no tile to visit (keys in front of the sequence in a chunk's window,
+// queries without a visible key).  It needs no barriers, tensor memory or loads.  At H12, the fourth
+// chunk of 1024 queries, 9216 keys, D64, 480 of 864 column CTAs are of this kind: backward 85 -> 78,
+// double backward 171 -> 165 us.
+__device__ __forceinline__ void zero_rows(void* out, int plane, int row0, int n_rows, int D) {
+  const int rows = min(BM, n_rows - row0);
+  uint4* p = reinterpret_cast<uint4*>(static_cast<uint16_t*>(out) + ((size_t)plane * n_rows + row0) * D);
+  for (int i = threadIdx.x; i < rows * D / 8; i += blockDim.x) p[i] = make_uint4(0u, 0u, 0u, 0u);
+}
+
 // Epilogue of the tensor-core kernels.  The 256 math threads have written a [128 rows][cols]
 // half-precision result tile to shared memory at `tile`, one 128-byte-swizzled 16 KB atom per 64
 // columns (store_op16).  All of them call this; `leader` (one thread) then writes the tile to
