@@ -87,6 +87,7 @@ attn::Geometry make_geometry(const attn_shape_t* s) {
   g.mask_mode = s->mask_mode;
   g.head_group = 1;
   g.beside = 0;
+  g.split = 1;
   g.scale = 1.0f / sqrtf((float)s->D);
   g.scale_log2e = g.scale * attn::kLog2e;
   return g;

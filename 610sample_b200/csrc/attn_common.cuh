@@ -37,6 +37,8 @@ struct Geometry {
   // 1: this launch shares the GPU with its predecessor in the stream, whose results it does not
   // read (dQ beside dK/dV, g_Q beside g_K/g_V); see tc_common.cuh
   int beside;
+  // CTAs (one cluster) that share the streamed tiles of a stationary tile
+  int split;
   float scale;       // 1/sqrt(D)
   float scale_log2e; // scale * log2(e)
 };
@@ -133,11 +135,11 @@ template <> struct Elem<__nv_bfloat16> {
 };
 
 // Pointer bundle shared by every launcher.  Unused members stay null.
-// blockIdx -> (head, rank of the tile within the head) under the grouped order
-__device__ __forceinline__ void cta_to_head_and_rank(const Geometry& g, int tiles, int& bh, int& rank) {
+// number of the stationary tile -> (head, rank of the tile within the head) under the grouped order
+__device__ __forceinline__ void tile_to_head_and_rank(const Geometry& g, unsigned unit, int tiles, int& bh, int& rank) {
   const int per_group = g.head_group * tiles;
-  const int grp = (int)(blockIdx.x / (unsigned)per_group);
-  const int rem = (int)(blockIdx.x - (unsigned)(grp * per_group));
+  const int grp = (int)(unit / (unsigned)per_group);
+  const int rem = (int)(unit - (unsigned)(grp * per_group));
   const int first = grp * g.head_group;
   const int gsize = min(g.head_group, g.BH - first);
   rank = rem / gsize;

@@ -73,6 +73,7 @@ struct FbCfg {
   static constexpr int kFit = (int)((kMaxSmem - 1024 - kStagingBytes - kAuxBytes) / kStageBytes);
   static constexpr int kStages = kFit < kFbMaxStages ? kFit : kFbMaxStages;
   static_assert(kStages >= 3, "too few stream stages");
+  static_assert(kStages * kStageBytes >= kNOut * BM * D * 4, "the partial results of a split tile lie over the stages");
   static constexpr uint32_t kContentBytes = kStagingBytes + kStages * kStageBytes + kAuxBytes;
   static constexpr uint32_t kSmemBytes = kContentBytes + 1024;
   // tensor-memory columns
@@ -88,7 +89,7 @@ struct FbCfg {
   __host__ __device__ static constexpr int stream_tensor(int s) { return kCol ? (s == 0 ? T_Q : T_dO) : (s == 0 ? T_K : T_V); }
 };
 
-template <int KIND, int D, typename T>
+template <int KIND, int D, typename T, bool SPLIT>
 __global__ void __launch_bounds__(kFbThreads, 1)
 fb_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Tensors t) {
   using CF = FbCfg<KIND, D>;
@@ -112,33 +113,39 @@ fb_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Tensors 
   const uint32_t strm_base = staging + CF::kStagingBytes;
   const uint32_t aux_off = CF::kStagingBytes + CF::kStages * CF::kStageBytes;
   FbControl* ctl = reinterpret_cast<FbControl*>(smem_gen + aux_off);
+  float* partial = reinterpret_cast<float*>(smem_gen + CF::kStagingBytes);     // over the stream stages, once every product is done
   float* aux_f = reinterpret_cast<float*>(smem_gen + aux_off + 512);   // 512 floats
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int n_stat = CF::kCol ? g.N_kv : g.N_q;
   const int tiles = (n_stat + BM - 1) / BM;
+  const unsigned split = SPLIT ? (unsigned)g.split : 1u;      // CTAs that share this tile: a cluster (tc_common.cuh)
+  const int part = SPLIT ? (int)(blockIdx.x % split) : 0;
   int bh, rank;
-  cta_to_head_and_rank(g, tiles, bh, rank);
+  tile_to_head_and_rank(g, blockIdx.x / split, tiles, bh, rank);
   const int tile = (CF::kCol || g.mask_mode != 0) ? rank : (tiles - 1 - rank);   // heavy tiles first
   const int r0 = tile * BM;
 
   int lo, hi;
   if (CF::kCol) query_range_for_keys(g, r0, r0 + BM, lo, hi);
   else key_range_for_queries(g, r0, r0 + BM, lo, hi);
-  const int t_begin = lo / BN;
-  const int n_iter = (hi > lo) ? ((hi + BN - 1) / BN - t_begin) : 0;
+  int t_begin = lo / BN;
+  int n_iter = (hi > lo) ? ((hi + BN - 1) / BN - t_begin) : 0;
   if (n_iter == 0) {       // nothing to visit
     pdl_begin(g);
     pdl_trigger();
-    if constexpr (CF::kCol) {
-      zero_rows(t.out_dK, bh, r0, g.N_kv, g.D);
-      zero_rows(t.out_dV, bh, r0, g.N_kv, g.D);
-    } else {
-      zero_rows(t.out_dQ, bh, r0, g.N_q, g.D);
+    if (part == 0) {
+      if constexpr (CF::kCol) {
+        zero_rows(t.out_dK, bh, r0, g.N_kv, g.D);
+        zero_rows(t.out_dV, bh, r0, g.N_kv, g.D);
+      } else {
+        zero_rows(t.out_dQ, bh, r0, g.N_q, g.D);
+      }
     }
     pdl_end(g);
     return;
   }
+  if constexpr (SPLIT) take_share((int)split, part, t_begin, n_iter);      // may be none
 
   const uint32_t bar_staging_full = smem_u32(&ctl->staging_full), bar_stat_ready = smem_u32(&ctl->stat_ready);
   const uint32_t bar_acc_done = smem_u32(&ctl->acc_done);
@@ -620,16 +627,23 @@ fb_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Tensors 
         for (int ch = 0; ch < kChunks; ++ch) {
           const int col = half * kColsPerHalf + ch * 16;
           if (col >= g.D) break;   // padding columns (uniform over the warp)
-          uint32_t w[8];
+          if constexpr (SPLIT) {
+            float f[16];
 #pragma unroll
-          for (int e = 0; e < 8; ++e)
-            w[e] = Pack<T>::pack(__uint_as_float(v[ch][2 * e]) * mul, __uint_as_float(v[ch][2 * e + 1]) * mul);
-          store_op16(tile + (uint32_t)(col >> 6) * kAtomBytesStat, row, col & 63, w);
+            for (int e = 0; e < 16; ++e) f[e] = __uint_as_float(v[ch][e]) * mul;
+            store_partial16<D>(partial + o * BM * D, row, col, f);
+          } else {
+            uint32_t w[8];
+#pragma unroll
+            for (int e = 0; e < 8; ++e)
+              w[e] = Pack<T>::pack(__uint_as_float(v[ch][2 * e]) * mul, __uint_as_float(v[ch][2 * e + 1]) * mul);
+            store_op16(tile + (uint32_t)(col >> 6) * kAtomBytesStat, row, col & 63, w);
+          }
         }
       }
       fence_proxy_async_smem();
       named_barrier_sync(2, kMathWarps * 32);
-      if (threadIdx.x == 0) {
+      if (!SPLIT && threadIdx.x == 0) {
         for (int o = 0; o < CF::kNOut; ++o) {
           const int id = (KIND == FB_BWD_ROW) ? TO_dQ : (o == 0 ? TO_dV : TO_dK);
           for (int a = 0; a * 64 < g.D; ++a)
@@ -641,6 +655,17 @@ fb_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Tensors 
     }
   }
 
+  if constexpr (SPLIT) {
+    cluster_barrier();
+    if (warp < kMathWarps) {
+      T* const outs[2] = {(T*)(CF::kCol ? t.out_dV : t.out_dQ), (T*)t.out_dK};
+#pragma unroll
+      for (int o = 0; o < CF::kNOut; ++o)
+        reduce_parts<D, T>(partial + o * BM * D, (int)split, part, outs[o] + ((size_t)bh * n_stat + r0) * g.D, min(BM, n_stat - r0), g.D,
+                           [](int, int) { return 1.f; }, [](int, int, float4&) {});
+    }
+    cluster_barrier();      // nobody leaves while its shared memory is being read
+  }
   tc_fence_before_sync();
   __syncthreads();
   if (warp == kFbMmaWarp) {
@@ -654,18 +679,11 @@ template <int KIND, int D, typename T>
 static cudaError_t launch_fb(const TmaMaps& maps, const Geometry& g_in, const Tensors& t, cudaStream_t s) {
   using CF = FbCfg<KIND, D>;
   Geometry g = g_in;
-  const int n_stat = CF::kCol ? g.N_kv : g.N_q;
-  const long long ctas = (long long)g.BH * ((n_stat + BM - 1) / BM);
-  if (ctas <= 0) return cudaSuccess;
-  if (ctas > 0x7fffffffLL) return cudaErrorInvalidValue;
-  g.head_group = pick_head_group(ctas, g.BH, 2ll * (KIND == FB_BWD_COL ? g.N_q : g.N_kv) * g.D * 2);
-  // more than half of an SM's shared memory: one CTA per SM, so the 512-column
-  // tensor-memory allocation never waits for a co-resident CTA
-  const size_t smem = CF::kSmemBytes < 122880u ? 122880u : CF::kSmemBytes;
-  auto kern = fb_kernel<KIND, D, T>;
-  static std::atomic<unsigned long long> smem_set{0};
-  cudaError_t e = set_smem_once(kern, smem, smem_set);
-  return e != cudaSuccess ? e : launch_pdl(kern, (unsigned)ctas, kFbThreads, smem, s, maps, g, t);
+  const long long ctas = (long long)g.BH * (((CF::kCol ? g.N_kv : g.N_q) + BM - 1) / BM);
+  g.head_group = pick_head_group(ctas, g.BH, 2ll * (CF::kCol ? g.N_q : g.N_kv) * g.D * 2);
+  static TileKernelState state;
+  return launch_tiles(fb_kernel<KIND, D, T, false>, fb_kernel<KIND, D, T, true>, maps, g, t, s, CF::kCol, kFbThreads, CF::kSmemBytes,
+                      CF::kCol ? 1700.f : 1150.f, CF::kCol ? 1150.f : 1700.f, state);
 }
 
 template <int D, typename T>

@@ -66,6 +66,7 @@ struct FwdCfg {
   static constexpr int kFit = (int)((kMaxSmem - 1024 - kStagingBytes - kAuxBytes) / kStageBytes);
   static constexpr int kStages = kFit < kFwdMaxStages ? kFit : kFwdMaxStages;
   static_assert(kStages >= 4, "too few stream stages");
+  static_assert(kStages * kStageBytes >= BM * D * 4 && kStagingBytes >= (2 + kMaxSplit) * BM * 4, "room for a split tile's results");
   static constexpr uint32_t kContentBytes = kStagingBytes + kStages * kStageBytes + kAuxBytes;
   static constexpr uint32_t kSmemBytes = kContentBytes + 1024;
   static constexpr int kS = 0, kQT = 192, kO = 256;       // O of group w at kO + w * D
@@ -75,7 +76,7 @@ struct FwdCfg {
   }
 };
 
-template <int D, typename T>
+template <int D, typename T, bool SPLIT>
 __global__ void __launch_bounds__(kFwdThreads, 1)
 fwd_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Tensors t) {
   using CF = FwdCfg<D>;
@@ -98,26 +99,36 @@ fwd_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Tensors
   const uint32_t aux_off = CF::kStagingBytes + CF::kStages * CF::kStageBytes;
   FwdControl* ctl = reinterpret_cast<FwdControl*>(smem_gen + aux_off);
   float* ml = reinterpret_cast<float*>(smem_gen + aux_off + 512);   // [2 groups][m | l][128]
+  // a split tile: this part's unnormalised O over the stream stages, its (m, l) and the factors of
+  // the parts over the staging buffer
+  float* partial = reinterpret_cast<float*>(smem_gen + CF::kStagingBytes);
+  float* part_ml = reinterpret_cast<float*>(smem_gen);        // [m | l][128]
+  float* part_f = part_ml + 2 * BM;                           // [parts][128]
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int tiles = (g.N_q + BM - 1) / BM;
+  const unsigned split = SPLIT ? (unsigned)g.split : 1u;      // CTAs that share this tile: a cluster (tc_common.cuh)
+  const int part = SPLIT ? (int)(blockIdx.x % split) : 0;
   int bh, rank;
-  cta_to_head_and_rank(g, tiles, bh, rank);
+  tile_to_head_and_rank(g, blockIdx.x / split, tiles, bh, rank);
   const int tile = (g.mask_mode != 0) ? rank : (tiles - 1 - rank);   // heavy tiles first
   const int r0 = tile * BM;
 
   int lo, hi;
   key_range_for_queries(g, r0, r0 + BM, lo, hi);
-  const int t_begin = lo / BN;
-  const int n_iter = (hi > lo) ? ((hi + BN - 1) / BN - t_begin) : 0;
+  int t_begin = lo / BN;
+  int n_iter = (hi > lo) ? ((hi + BN - 1) / BN - t_begin) : 0;
   if (n_iter == 0) {       // nothing to visit
     pdl_begin(g);
     pdl_trigger();
-    zero_rows(t.out_O, bh, r0, g.N_q, g.D);
-    if (threadIdx.x < BM && r0 + threadIdx.x < g.N_q) t.out_L[(size_t)bh * g.N_q + r0 + threadIdx.x] = -INFINITY;
+    if (part == 0) {
+      zero_rows(t.out_O, bh, r0, g.N_q, g.D);
+      if (threadIdx.x < BM && r0 + threadIdx.x < g.N_q) t.out_L[(size_t)bh * g.N_q + r0 + threadIdx.x] = -INFINITY;
+    }
     pdl_end(g);
     return;
   }
+  if constexpr (SPLIT) take_share((int)split, part, t_begin, n_iter);      // may be none
 
   const uint32_t bar_staging_full = smem_u32(&ctl->staging_full), bar_q_ready = smem_u32(&ctl->q_ready);
   const uint32_t bar_acc_done = smem_u32(&ctl->acc_done);
@@ -423,8 +434,11 @@ fwd_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Tensors
       f_ot = (m_o > -INFINITY) ? ex2(m_o - m_all) : 0.f;
       l_all = l_sum * f_me + l_o * f_ot;
     }
-    const float inv = l_all > 0.f ? 1.f / l_all : 0.f;
-    if (grp == 0 && gidx < g.N_q) t.out_L[row_off + gidx] = (l_all > 0.f) ? (m_all + log2f(l_all)) * kLn2 : -INFINITY;
+    // a split tile is normalised where the parts meet
+    const float inv = l_all > 0.f ? (SPLIT ? 1.f : 1.f / l_all) : 0.f;
+    if constexpr (SPLIT) {
+      if (grp == 0) { part_ml[row] = m_all; part_ml[BM + row] = l_all; }
+    } else if (grp == 0 && gidx < g.N_q) t.out_L[row_off + gidx] = (l_all > 0.f) ? (m_all + log2f(l_all)) * kLn2 : -INFINITY;
 
     if (n_iter > 0 && ok) ok = mbar_wait(bar_acc_done, 0, abort_flag, t.status, wait_code(KFWD, 9));
     ok = __all_sync(0xffffffffu, ok);
@@ -445,6 +459,7 @@ fwd_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Tensors
         tmem_ld_wait(b_);
       }
       uint32_t w[8];
+      float f[16];
 #pragma unroll
       for (int e = 0; e < 8; ++e) {
         float v0 = 0.f, v1 = 0.f;
@@ -453,11 +468,40 @@ fwd_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Tensors
           if (use1) { v0 = fmaf(__uint_as_float(b_[2 * e]), f1, v0); v1 = fmaf(__uint_as_float(b_[2 * e + 1]), f1, v1); }
         }
         w[e] = Pack<T>::pack(v0, v1);
+        f[2 * e] = v0; f[2 * e + 1] = v1;
       }
-      if (gidx < g.N_q) store_op16(staging + (uint32_t)(col >> 6) * kAtomBytesStat, row, col & 63, w);
+      if constexpr (SPLIT) store_partial16<D>(partial, row, col, f);
+      else if (gidx < g.N_q) store_op16(staging + (uint32_t)(col >> 6) * kAtomBytesStat, row, col & 63, w);
     }
     // the O tile leaves through the staging buffer (Q has been in tensor memory since the prologue)
-    store_tile_tma(&maps.out[TO_O], staging, g.D, r0, bh, threadIdx.x == 0);
+    store_tile_tma(&maps.out[TO_O], staging, g.D, r0, bh, !SPLIT && threadIdx.x == 0);
+  }
+
+  if constexpr (SPLIT) {
+    cluster_barrier();
+    if (warp < kMathWarps) {
+      // per row: the parts' maxima and sums, then the factor of every part
+      if (threadIdx.x < BM) {
+        cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+        float m = -INFINITY, l = 0.f;
+        for (int q = 0; q < (int)split; ++q) m = fmaxf(m, cluster.map_shared_rank(part_ml, q)[threadIdx.x]);
+        for (int q = 0; q < (int)split; ++q) {
+          const float* theirs = cluster.map_shared_rank(part_ml, q);
+          const float mq = theirs[threadIdx.x];
+          const float f = mq > -INFINITY ? ex2(mq - m) : 0.f;
+          part_f[q * BM + threadIdx.x] = f;
+          l = fmaf(theirs[BM + threadIdx.x], f, l);
+        }
+        const float inv = l > 0.f ? 1.f / l : 0.f;
+        for (int q = 0; q < (int)split; ++q) part_f[q * BM + threadIdx.x] *= inv;
+        if (part == 0 && r0 + threadIdx.x < g.N_q)
+          t.out_L[(size_t)bh * g.N_q + r0 + threadIdx.x] = l > 0.f ? (m + log2f(l)) * kLn2 : -INFINITY;
+      }
+      named_barrier_sync(1, kMathThreads);
+      reduce_parts<D, T>(partial, (int)split, part, (T*)t.out_O + ((size_t)bh * g.N_q + r0) * g.D, min(BM, g.N_q - r0), g.D,
+                         [&](int q, int row) { return part_f[q * BM + row]; }, [](int, int, float4&) {});
+    }
+    cluster_barrier();      // nobody leaves while its shared memory is being read
   }
 
   tc_fence_before_sync();
@@ -473,17 +517,9 @@ template <int D, typename T>
 static cudaError_t launch_fwd_one(const TmaMaps& maps, const Geometry& g_in, const Tensors& t, cudaStream_t s) {
   using CF = FwdCfg<D>;
   Geometry g = g_in;
-  const long long ctas = (long long)g.BH * ((g.N_q + BM - 1) / BM);
-  if (ctas <= 0) return cudaSuccess;
-  if (ctas > 0x7fffffffLL) return cudaErrorInvalidValue;
-  g.head_group = pick_head_group(ctas, g.BH, 2ll * g.N_kv * g.D * 2);   // K, V
-  // more than half of an SM's shared memory: one CTA per SM, so the 512-column
-  // tensor-memory allocation never waits for a co-resident CTA
-  const size_t smem = CF::kSmemBytes < 122880u ? 122880u : CF::kSmemBytes;
-  auto kern = fwd_kernel<D, T>;
-  static std::atomic<unsigned long long> smem_set{0};
-  cudaError_t e = set_smem_once(kern, smem, smem_set);
-  return e != cudaSuccess ? e : launch_pdl(kern, (unsigned)ctas, kFwdThreads, smem, s, maps, g, t);
+  g.head_group = pick_head_group((long long)g.BH * ((g.N_q + BM - 1) / BM), g.BH, 2ll * g.N_kv * g.D * 2);   // K, V
+  static TileKernelState state;
+  return launch_tiles(fwd_kernel<D, T, false>, fwd_kernel<D, T, true>, maps, g, t, s, false, kFwdThreads, CF::kSmemBytes, 850.f, 0.f, state);
 }
 
 // forward: O and L in one launch

@@ -67,6 +67,7 @@ struct ColCfg {
   static constexpr uint32_t kContentBytes = kStatBytes + kStages * kStageBytes + kAuxBytes;
   static constexpr uint32_t kMaxSmem = 232448;
   static_assert(kContentBytes + 768 <= kMaxSmem, "shared memory over-subscribed");
+  static_assert(kStatBytes >= 2 * BM * D * 4, "the partial results of a split tile lie over the stationary operands");
   static constexpr uint32_t kSmemBytes = (kContentBytes + 1024 <= kMaxSmem) ? kContentBytes + 1024 : kMaxSmem;
   static constexpr int kRA = 0, kRB = 128, kOut0 = 256, kOut1 = 256 + D;
   static_assert(kOut1 + D <= kTmemCols, "tensor memory over-subscribed");
@@ -83,7 +84,7 @@ struct ColCfg {
   __host__ __device__ static constexpr int stream_tensor(int slot) { return slot == 0 ? T_Q : slot == 1 ? T_gQ : T_dO; }
 };
 
-template <int D, typename T>
+template <int D, typename T, bool SPLIT>
 __global__ void __launch_bounds__(kColThreads, 1)
 hvp_col_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Tensors t) {
   using CF = ColCfg<D>;
@@ -107,26 +108,32 @@ hvp_col_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Ten
   const uint32_t strm_base = stat_base + CF::kStatBytes;
   const uint32_t aux_off = CF::kStatBytes + CF::kStages * CF::kStageBytes;
   ColControl* ctl = reinterpret_cast<ColControl*>(smem_gen + aux_off);
+  float* partial = reinterpret_cast<float*>(smem_gen);      // a split tile's results over the stationary operands, once every product is done
   float* col_stats = reinterpret_cast<float*>(smem_gen + aux_off + 256);   // [2][4][64]
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int tiles = (g.N_kv + BM - 1) / BM;
+  const unsigned split = SPLIT ? (unsigned)g.split : 1u;      // CTAs that share this tile: a cluster (tc_common.cuh)
+  const int part = SPLIT ? (int)(blockIdx.x % split) : 0;
   int bh, tile;   // early key tiles are the heavy ones
-  cta_to_head_and_rank(g, tiles, bh, tile);
+  tile_to_head_and_rank(g, blockIdx.x / split, tiles, bh, tile);
   const int r0 = tile * BM;
 
   int lo, hi;
   query_range_for_keys(g, r0, r0 + BM, lo, hi);
-  const int t_begin = lo / BN;
-  const int n_iter = (hi > lo) ? ((hi + BN - 1) / BN - t_begin) : 0;
+  int t_begin = lo / BN;
+  int n_iter = (hi > lo) ? ((hi + BN - 1) / BN - t_begin) : 0;
   if (n_iter == 0) {       // nothing to visit
     pdl_begin(g);
     pdl_trigger();
-    zero_rows(t.out_g_K, bh, r0, g.N_kv, g.D);
-    zero_rows(t.out_g_V, bh, r0, g.N_kv, g.D);
+    if (part == 0) {
+      zero_rows(t.out_g_K, bh, r0, g.N_kv, g.D);
+      zero_rows(t.out_g_V, bh, r0, g.N_kv, g.D);
+    }
     pdl_end(g);
     return;
   }
+  if constexpr (SPLIT) take_share((int)split, part, t_begin, n_iter);      // may be none
 
   const uint32_t bar_stat_full = smem_u32(&ctl->stat_full);
   const uint32_t bar_ra_full = smem_u32(&ctl->ra_full), bar_ra_free = smem_u32(&ctl->ra_free);
@@ -537,16 +544,23 @@ hvp_col_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Ten
       for (int ch = 0; ch < kChunks; ++ch) {
         const int col = half * kColsPerHalf + ch * 16;
         if (col >= g.D) break;   // padding columns (uniform over the warp)
-        uint32_t w[8];
+        if constexpr (SPLIT) {
+          float f[16];
 #pragma unroll
-        for (int e = 0; e < 8; ++e)
-          w[e] = Pack<T>::pack(__uint_as_float(v[ch][2 * e]) * mul, __uint_as_float(v[ch][2 * e + 1]) * mul);
-        store_op16(tile + (uint32_t)(col >> 6) * kAtomBytesStat, row, col & 63, w);
+          for (int e = 0; e < 16; ++e) f[e] = __uint_as_float(v[ch][e]) * mul;
+          store_partial16<D>(partial + o * BM * D, row, col, f);
+        } else {
+          uint32_t w[8];
+#pragma unroll
+          for (int e = 0; e < 8; ++e)
+            w[e] = Pack<T>::pack(__uint_as_float(v[ch][2 * e]) * mul, __uint_as_float(v[ch][2 * e + 1]) * mul);
+          store_op16(tile + (uint32_t)(col >> 6) * kAtomBytesStat, row, col & 63, w);
+        }
       }
     }
     fence_proxy_async_smem();
     named_barrier_sync(2, kMathWarps * 32);
-    if (threadIdx.x == 0) {
+    if (!SPLIT && threadIdx.x == 0) {
       for (int o = 0; o < 2; ++o)
         for (int a = 0; a * 64 < g.D; ++a)
           tma_store_3d(&maps.out[o == 0 ? TO_gK : TO_gV], stat_base + (uint32_t)(o * kAtoms + a) * kAtomBytesStat,
@@ -556,6 +570,17 @@ hvp_col_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Ten
     }
   }
 
+  if constexpr (SPLIT) {
+    cluster_barrier();
+    if (warp < kMathWarps) {
+      const size_t at = ((size_t)bh * g.N_kv + r0) * g.D;
+#pragma unroll
+      for (int o = 0; o < 2; ++o)
+        reduce_parts<D, T>(partial + o * BM * D, (int)split, part, (T*)(o == 0 ? t.out_g_K : t.out_g_V) + at, min(BM, g.N_kv - r0), g.D,
+                           [](int, int) { return 1.f; }, [](int, int, float4&) {});
+    }
+    cluster_barrier();      // nobody leaves while its shared memory is being read
+  }
   tc_fence_before_sync();
   __syncthreads();
   if (warp == kColMmaWarp) {
@@ -569,17 +594,9 @@ template <int D, typename T>
 static cudaError_t launch_col(const TmaMaps& maps, const Geometry& g_in, const Tensors& t, cudaStream_t s) {
   using CF = ColCfg<D>;
   Geometry g = g_in;
-  const long long ctas = (long long)g.BH * ((g.N_kv + BM - 1) / BM);
-  if (ctas <= 0) return cudaSuccess;
-  if (ctas > 0x7fffffffLL) return cudaErrorInvalidValue;
-  g.head_group = pick_head_group(ctas, g.BH, 3ll * g.N_q * g.D * 2);   // Q, g_dQ, dO
-  // more than half of an SM's shared memory: one CTA per SM, so the 512-column
-  // tensor-memory allocation never waits for a co-resident CTA
-  const size_t smem = CF::kSmemBytes < 122880u ? 122880u : CF::kSmemBytes;
-  auto kern = hvp_col_kernel<D, T>;
-  static std::atomic<unsigned long long> smem_set{0};
-  cudaError_t e = set_smem_once(kern, smem, smem_set);
-  return e != cudaSuccess ? e : launch_pdl(kern, (unsigned)ctas, kColThreads, smem, s, maps, g, t);
+  g.head_group = pick_head_group((long long)g.BH * ((g.N_kv + BM - 1) / BM), g.BH, 3ll * g.N_q * g.D * 2);   // Q, g_dQ, dO
+  static TileKernelState state;
+  return launch_tiles(hvp_col_kernel<D, T, false>, hvp_col_kernel<D, T, true>, maps, g, t, s, true, kColThreads, CF::kSmemBytes, 2700.f, 2000.f, state);
 }
 
 cudaError_t launch_hvp_col(int D, int is_bf16, const TmaMaps& maps, const Geometry& g, const Tensors& t,

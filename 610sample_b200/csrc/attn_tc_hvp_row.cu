@@ -84,6 +84,7 @@ struct RowCfg {
   static constexpr uint32_t kContentBytes = kStatBytes + kStages * kStageBytes + kAuxBytes;
   static constexpr uint32_t kMaxSmem = 232448;
   static_assert(kContentBytes <= kMaxSmem, "shared memory over-subscribed");
+  static_assert(kStages * kStageBytes >= BM * D * 4 && kStatBytes >= 13 * BM * 4, "room for a split tile's results");
   static constexpr uint32_t kSmemBytes = (kContentBytes + 1024 <= kMaxSmem) ? kContentBytes + 1024 : kMaxSmem;
   // At D = 64 the accumulator and the stationary operands take half the columns, which leaves
   // room for a second RB region: the RB products then run a tile ahead of the outputs instead of
@@ -101,7 +102,7 @@ struct RowCfg {
   }
 };
 
-template <int MODE, int D, typename T>
+template <int MODE, int D, typename T, bool SPLIT>
 __global__ void __launch_bounds__(kRowThreads, 1)
 hvp_row_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Tensors t) {
   using CF = RowCfg<D>;
@@ -129,32 +130,42 @@ hvp_row_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Ten
   // [2 halves][4][128] floats of row sums, exchanged after the last product has read the
   // g_dQ tile: its shared memory is reused
   float* row_sums = reinterpret_cast<float*>(smem_gen);
+  // a split tile: this part's four sums per row and the total dot2 behind them, its result tile over
+  // the stream stages
+  float* part_sums = row_sums + 2 * 4 * BM;       // [4][128]
+  float* part_dot2 = part_sums + 4 * BM;
+  float* partial = reinterpret_cast<float*>(smem_gen + CF::kStatBytes);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int tiles = (g.N_q + BM - 1) / BM;
+  const unsigned split = SPLIT ? (unsigned)g.split : 1u;      // CTAs that share this tile: a cluster (tc_common.cuh)
+  const int part = SPLIT ? (int)(blockIdx.x % split) : 0;
   int bh, rank;
-  cta_to_head_and_rank(g, tiles, bh, rank);
+  tile_to_head_and_rank(g, blockIdx.x / split, tiles, bh, rank);
   const int tile = (g.mask_mode != 0) ? rank : (tiles - 1 - rank);   // heavy tiles first
   const int r0 = tile * BM;
 
   int lo, hi;
   key_range_for_queries(g, r0, r0 + BM, lo, hi);
-  const int t_begin = lo / BN;
-  const int n_iter = (hi > lo) ? ((hi + BN - 1) / BN - t_begin) : 0;
+  int t_begin = lo / BN;
+  int n_iter = (hi > lo) ? ((hi + BN - 1) / BN - t_begin) : 0;
   if (n_iter == 0) {       // nothing to visit
     pdl_begin(g);
     pdl_trigger();
-    zero_rows(MODE == ROW_PREDO ? t.out_g_dO : t.out_g_Q, bh, r0, g.N_q, g.D);
-    if constexpr (MODE == ROW_PREDO) {
-      const int r = r0 + threadIdx.x;
-      if (threadIdx.x < BM && r < g.N_q) {
-        const size_t at = (size_t)bh * g.N_q + r;
-        t.Dv[at] = t.dot2[at] = t.dot3[at] = 0.f;
+    if (part == 0) {
+      zero_rows(MODE == ROW_PREDO ? t.out_g_dO : t.out_g_Q, bh, r0, g.N_q, g.D);
+      if constexpr (MODE == ROW_PREDO) {
+        const int r = r0 + threadIdx.x;
+        if (threadIdx.x < BM && r < g.N_q) {
+          const size_t at = (size_t)bh * g.N_q + r;
+          t.Dv[at] = t.dot2[at] = t.dot3[at] = 0.f;
+        }
       }
     }
     pdl_end(g);
     return;
   }
+  if constexpr (SPLIT) take_share((int)split, part, t_begin, n_iter);      // may be none
 
   const uint32_t bar_stat_full = smem_u32(&ctl->stat_full);
   const uint32_t bar_staging_full = smem_u32(&ctl->staging_full);
@@ -570,7 +581,9 @@ hvp_row_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Ten
       const float Dv = sD + other[row], d2 = s2 + other[128 + row];
       const float A = sA + other[256 + row], E = sE + other[384 + row];
       dot2_row = d2;
-      if (half == 0 && gidx < g.N_q) {
+      if constexpr (SPLIT) {
+        if (half == 0) { part_sums[row] = Dv; part_sums[BM + row] = d2; part_sums[2 * BM + row] = A; part_sums[3 * BM + row] = E; }
+      } else if (half == 0 && gidx < g.N_q) {
         t.Dv[row_off + gidx] = Dv;
         t.dot2[row_off + gidx] = d2;
         t.dot3[row_off + gidx] = A - 2.f * Dv * d2 + E;
@@ -587,7 +600,7 @@ hvp_row_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Ten
     if constexpr (MODE == ROW_PREDO) {
 #pragma unroll
       for (int ch = 0; ch < kChunks; ++ch) {
-        const bool in = gidx < g.N_q && half * kColsPerHalf + ch * 16 < g.D;
+        const bool in = !SPLIT && gidx < g.N_q && half * kColsPerHalf + ch * 16 < g.D;
         const uint4* orow = reinterpret_cast<const uint4*>((const T*)t.O + elem0 + ch * 16);
         o_[2 * ch] = in ? __ldg(orow) : make_uint4(0u, 0u, 0u, 0u);
         o_[2 * ch + 1] = in ? __ldg(orow + 1) : make_uint4(0u, 0u, 0u, 0u);
@@ -628,15 +641,57 @@ hvp_row_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Ten
             f[2 * e + 1] = fmaf(-dot2_row, of.y, f[2 * e + 1]);
           }
         }
-        uint32_t w[8];
-#pragma unroll
-        for (int e = 0; e < 8; ++e) w[e] = Pack<T>::pack(f[2 * e], f[2 * e + 1]);
         const int col = half * kColsPerHalf + ch * 16;
-        store_op16(strm_base + (uint32_t)(col >> 6) * kAtomBytesStat, row, col & 63, w);
+        if constexpr (SPLIT) {      // O was not fetched: dot2 is not known yet
+          store_partial16<D>(partial, row, col, f);
+        } else {
+          uint32_t w[8];
+#pragma unroll
+          for (int e = 0; e < 8; ++e) w[e] = Pack<T>::pack(f[2 * e], f[2 * e + 1]);
+          store_op16(strm_base + (uint32_t)(col >> 6) * kAtomBytesStat, row, col & 63, w);
+        }
       }
     }
     // the result tile goes out through the first stream stage (every product has completed)
-    store_tile_tma(&maps.out[MODE == ROW_PREDO ? TO_gdO : TO_gQ], strm_base, g.D, r0, bh, threadIdx.x == 0);
+    store_tile_tma(&maps.out[MODE == ROW_PREDO ? TO_gdO : TO_gQ], strm_base, g.D, r0, bh, !SPLIT && threadIdx.x == 0);
+  }
+
+  if constexpr (SPLIT) {
+    cluster_barrier();
+    if (warp < kMathWarps) {
+      if constexpr (MODE == ROW_PREDO) {
+        if (threadIdx.x < BM) {
+          cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+          float sum[4] = {0.f, 0.f, 0.f, 0.f};
+          for (int q = 0; q < (int)split; ++q) {
+            const float* theirs = cluster.map_shared_rank(part_sums, q);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) sum[i] += theirs[i * BM + threadIdx.x];
+          }
+          part_dot2[threadIdx.x] = sum[1];
+          if (part == 0 && r0 + threadIdx.x < g.N_q) {
+            const size_t at = (size_t)bh * g.N_q + r0 + threadIdx.x;
+            t.Dv[at] = sum[0];
+            t.dot2[at] = sum[1];
+            t.dot3[at] = sum[2] - 2.f * sum[0] * sum[1] + sum[3];
+          }
+        }
+        named_barrier_sync(1, kMathThreads);
+      }
+      const size_t at = ((size_t)bh * g.N_q + r0) * g.D;
+      const T* O_rows = (const T*)t.O + at;
+      reduce_parts<D, T>(partial, (int)split, part, (T*)(MODE == ROW_PREDO ? t.out_g_dO : t.out_g_Q) + at, min(BM, g.N_q - r0), g.D,
+                         [](int, int) { return 1.f; },
+                         [&](int row, int col, float4& v) {
+                           if constexpr (MODE == ROW_PREDO) {
+                             const uint2 w = __ldg(reinterpret_cast<const uint2*>(O_rows + (size_t)row * g.D + col));
+                             const float2 a = Pack<T>::unpack(w.x), b = Pack<T>::unpack(w.y);
+                             const float d = -part_dot2[row];
+                             v.x = fmaf(d, a.x, v.x); v.y = fmaf(d, a.y, v.y); v.z = fmaf(d, b.x, v.z); v.w = fmaf(d, b.y, v.w);
+                           }
+                         });
+    }
+    cluster_barrier();      // nobody leaves while its shared memory is being read
   }
 
   tc_fence_before_sync();
@@ -652,17 +707,10 @@ template <int MODE, int D, typename T>
 static cudaError_t launch_row(const TmaMaps& maps, const Geometry& g_in, const Tensors& t, cudaStream_t s) {
   using CF = RowCfg<D>;
   Geometry g = g_in;
-  const long long ctas = (long long)g.BH * ((g.N_q + BM - 1) / BM);
-  if (ctas <= 0) return cudaSuccess;
-  if (ctas > 0x7fffffffLL) return cudaErrorInvalidValue;
-  g.head_group = pick_head_group(ctas, g.BH, 4ll * g.N_kv * g.D * 2);   // K, g_dK, V, g_dV
-  // more than half of an SM's shared memory: one CTA per SM, so the 512-column
-  // tensor-memory allocation never waits for a co-resident CTA
-  const size_t smem = CF::kSmemBytes < 122880u ? 122880u : CF::kSmemBytes;
-  auto kern = hvp_row_kernel<MODE, D, T>;
-  static std::atomic<unsigned long long> smem_set{0};
-  cudaError_t e = set_smem_once(kern, smem, smem_set);
-  return e != cudaSuccess ? e : launch_pdl(kern, (unsigned)ctas, kRowThreads, smem, s, maps, g, t);
+  g.head_group = pick_head_group((long long)g.BH * ((g.N_q + BM - 1) / BM), g.BH, 4ll * g.N_kv * g.D * 2);   // K, g_dK, V, g_dV
+  static TileKernelState state;
+  return launch_tiles(hvp_row_kernel<MODE, D, T, false>, hvp_row_kernel<MODE, D, T, true>, maps, g, t, s, false, kRowThreads, CF::kSmemBytes,
+                      2000.f, MODE == ROW_Q ? 2700.f : 0.f, state);
 }
 
 // mode 0: per-row scalars + g_dO;  mode 1: g_Q

@@ -6,6 +6,7 @@
 #include "tc_primitives.cuh"
 
 #include <atomic>
+#include <cooperative_groups.h>
 
 namespace attn {
 namespace tc {
@@ -23,6 +24,34 @@ constexpr uint32_t kAtomBytesStrm = BN * 128;   // [ 64 rows][64 halves],  8 KB
 // 20, the self-test 0x6f); the values are documented with the C ABI and do not change.
 enum Kind { HVP_PRE = 4, HVP_ROW = 5, HVP_COL = 6 };
 enum TensorId { T_Q = 0, T_K, T_V, T_dO, T_gQ, T_gK, T_gV, T_COUNT };
+
+// Output tensors by operation: forward {O}; backward {dQ, dK, dV}; double backward
+// {g_dO, g_Q, g_K, g_V}.  Output maps have a box of 64 columns x 128 rows.
+enum OutId { TO_O = 0, TO_dQ = 0, TO_dK = 1, TO_dV = 2, TO_gdO = 0, TO_gQ = 1, TO_gK = 2, TO_gV = 3, TO_COUNT = 4 };
+
+struct TmaMaps { CUtensorMap m[T_COUNT]; CUtensorMap out[TO_COUNT]; };
+
+template <typename T> struct Pack;
+template <> struct Pack<__nv_bfloat16> {
+  static constexpr int kIsBf16 = 1;
+  static __device__ __forceinline__ uint32_t pack(float lo, float hi) {
+    __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
+    return *reinterpret_cast<uint32_t*>(&v);
+  }
+  static __device__ __forceinline__ float2 unpack(uint32_t w) {
+    return __bfloat1622float2(*reinterpret_cast<__nv_bfloat162*>(&w));
+  }
+};
+template <> struct Pack<__half> {
+  static constexpr int kIsBf16 = 0;
+  static __device__ __forceinline__ uint32_t pack(float lo, float hi) {
+    __half2 v = __floats2half2_rn(lo, hi);
+    return *reinterpret_cast<uint32_t*>(&v);
+  }
+  static __device__ __forceinline__ float2 unpack(uint32_t w) {
+    return __half22float2(*reinterpret_cast<__half2*>(&w));
+  }
+};
 
 // Launches and the order between them.  Every tensor-core kernel is launched with programmatic
 // stream serialization: its CTAs may become resident while the predecessor in the stream still
@@ -75,11 +104,162 @@ inline cudaError_t launch_pdl(void (*kern)(P...), unsigned ctas, unsigned thread
   return launch_pdl_cluster(kern, ctas, threads, smem, 1, s, args...);
 }
 
-// Output tensors by operation: forward {O}; backward {dQ, dK, dV}; double backward
-// {g_dO, g_Q, g_K, g_V}.  Output maps have a box of 64 columns x 128 rows.
-enum OutId { TO_O = 0, TO_dQ = 0, TO_dK = 1, TO_dV = 2, TO_gdO = 0, TO_gQ = 1, TO_gK = 2, TO_gV = 3, TO_COUNT = 4 };
+// ---- Splitting the streamed tiles of a stationary tile over a cluster --------------------------
+// Problems with few stationary tiles (small batches, short chunks against a long window) leave SMs
+// idle.  There the streamed tiles of a stationary tile are dealt out, in contiguous shares, to the
+// CTAs of a cluster; each leaves its fp32 result in its own shared memory, and all of them add the
+// parts through distributed shared memory, in rank order (so results are reproducible), each for its
+// share of the elements.  The kernels have the split as a template parameter: with the shared form's
+// epilogue in the common kernel, every launch paid a few per cent for it.
 
-struct TmaMaps { CUtensorMap m[T_COUNT]; CUtensorMap out[TO_COUNT]; };
+// this CTA's share of the n tiles from t0
+__device__ __forceinline__ void take_share(int split, int part, int& t0, int& n) {
+  const int first = n * part / split, last = n * (part + 1) / split;
+  t0 += first;
+  n = last - first;
+}
+
+// fp32 result tile [BM][DT] in shared memory, 16-byte chunks XORed with row % 8: a thread writes its row
+template <int DT>
+__device__ __forceinline__ int partial_at(int row, int chunk) { return row * DT + ((chunk ^ (row & 7)) << 2); }
+
+template <int DT>
+__device__ __forceinline__ void store_partial16(float* partial, int row, int col, const float (&f)[16]) {
+#pragma unroll
+  for (int q = 0; q < 4; ++q)
+    *reinterpret_cast<float4*>(partial + partial_at<DT>(row, (col >> 2) + q)) = make_float4(f[4 * q], f[4 * q + 1], f[4 * q + 2], f[4 * q + 3]);
+}
+
+// Every thread of the cluster: the shared memory written before is readable by all its CTAs.
+__device__ __forceinline__ void cluster_barrier() { cooperative_groups::this_cluster().sync(); }
+
+// The math threads of every CTA: rows [0, rows) of the sum over the parts, weight(part, row) times
+// each, post(row, column, float4) applied to it, to dst (row pitch D).
+template <int DT, typename T, typename Weight, typename Post>
+__device__ __forceinline__ void reduce_parts(float* partial, int split, int part, T* dst, int rows, int D, Weight weight, Post post) {
+  cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+  const int chunks = D >> 2;
+  for (int i = part * kMathThreads + (int)threadIdx.x; i < rows * chunks; i += split * kMathThreads) {
+    const int row = i / chunks, chunk = i - row * chunks;
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int q = 0; q < split; ++q) {
+      const float4 x = *reinterpret_cast<const float4*>(cluster.map_shared_rank(partial, q) + partial_at<DT>(row, chunk));
+      const float w = weight(q, row);
+      v.x = fmaf(x.x, w, v.x); v.y = fmaf(x.y, w, v.y); v.z = fmaf(x.z, w, v.z); v.w = fmaf(x.w, w, v.w);
+    }
+    post(row, 4 * chunk, v);
+    *reinterpret_cast<uint2*>(dst + (size_t)row * D + 4 * chunk) = make_uint2(Pack<T>::pack(v.x, v.y), Pack<T>::pack(v.z, v.w));
+  }
+}
+
+// Host: how many CTAs share a stationary tile.  A CTA costs kCtaClocks besides `tile_clocks` for each
+// tile it visits (prologue, pipeline fill, epilogue), and split_clocks more when it shares a tile (two
+// cluster barriers, the sum).  Only splits whose clusters all fit the GPU at a time are considered (a
+// second wave of clusters starts late: 36 against 29 us for 96 tiles in pairs, 148 CTAs fitting),
+// and only where the time of the longest CTA falls by a tenth; with another kernel beside this one, whose
+// CTAs take the SMs left over, where the longer of the two falls by a quarter.
+// Measured at B1 H8 D128, 256 queries against 4352 keys (16 tiles of 66): forward 34 -> 17 us with six
+// parts, backward 44 -> 31, double backward 160 -> 64 us; B1 H8 N512 D64 (32 tiles of 8): no split,
+// 10.5 us, with two 10.4.
+constexpr float kCtaClocks = 12000.f;
+constexpr int kMaxSplit = 8;
+constexpr int kSms = 148;
+inline float split_clocks(int D) { return 3000.f + 45.f * D; }
+
+// a kernel's stationary tiles, the most streamed tiles one of them visits, clocks per tile
+struct SplitLoad { float units, longest, tile_clocks; };
+
+template <typename Slots>
+inline int pick_split(const SplitLoad& w, const SplitLoad* other, int D, Slots slots) {
+  int best = 1;
+  float least = 0.f;
+  for (int c = 1; c <= kMaxSplit && (c == 1 || (c <= w.longest && w.units * c <= kSms)); ++c) {
+    if (c > 1 && w.units * c > slots(c)) continue;
+    float t = w.longest / c * w.tile_clocks + kCtaClocks + (c > 1 ? split_clocks(D) : 0.f);
+    if (other != nullptr) {
+      const float left = kSms - w.units * c > 1.f ? kSms - w.units * c : 1.f;
+      const float theirs = (float)(int)(other->units / left + 0.999f) * (other->longest * other->tile_clocks + kCtaClocks);
+      if (theirs > t) t = theirs;
+    }
+    if (c == 1 || t < (best > 1 ? 1.f : other != nullptr ? 0.75f : 0.9f) * least) { best = c; least = t; }
+  }
+  return best;
+}
+
+inline SplitLoad stream_load(const Geometry& g, bool col, float tile_clocks) {
+  const int n = col ? g.N_kv : g.N_q, tiles = (n + BM - 1) / BM;
+  int most = 0;
+  for (int i = 0; i < tiles; ++i) {
+    int lo, hi;
+    if (col) query_range_for_keys(g, i * BM, (i + 1) * BM, lo, hi);
+    else key_range_for_queries(g, i * BM, (i + 1) * BM, lo, hi);
+    const int k = hi > lo ? (hi + BN - 1) / BN - lo / BN : 0;
+    if (k > most) most = k;
+  }
+  return {(float)g.BH * tiles, (float)most, tile_clocks};
+}
+
+// What a kernel's launches keep: the devices its shared-memory opt-in has been made on, and the CTAs
+// that run at a time in clusters of each size.
+struct TileKernelState {
+  std::atomic<unsigned long long> smem_set{0}, smem_set_split{0};
+  std::atomic<int> slots[kMaxSplit + 1] = {};
+};
+
+// CTAs of `kern` that run at a time in clusters of c (asked for once per kernel and size).
+template <typename Kern>
+inline int cluster_slots(Kern kern, int c, unsigned threads, size_t smem, TileKernelState& state) {
+  int n = state.slots[c].load(std::memory_order_relaxed);
+  if (n == 0) {
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = (unsigned)c;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)c);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    int clusters = 0;
+    if (set_smem_once(kern, smem, state.smem_set_split) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&clusters, (const void*)kern, &cfg) != cudaSuccess) {
+      (void)cudaGetLastError();
+      clusters = 0;
+    }
+    n = clusters > 0 ? clusters * c : -1;
+    state.slots[c].store(n, std::memory_order_relaxed);
+  }
+  return n;
+}
+
+// Launch of a tensor-core kernel, one CTA per SM (more than half of an SM's shared memory is asked
+// for, so the 512-column tensor-memory allocation never waits for a co-resident CTA), with the split
+// its load asks for: `whole` where it is none, else `shared`.  A tile takes `tile_clocks`; other_clocks
+// is the same for the other side's kernel where that runs beside this one, else 0.
+template <typename... P>
+inline cudaError_t launch_tiles(void (*whole)(P...), void (*shared)(P...), const TmaMaps& maps, Geometry g, const Tensors& t,
+                                cudaStream_t s, bool col, unsigned threads, size_t smem_wanted, float tile_clocks, float other_clocks,
+                                TileKernelState& state) {
+  const long long units = (long long)g.BH * (((col ? g.N_kv : g.N_q) + BM - 1) / BM);
+  if (units <= 0) return cudaSuccess;
+  if (units * kMaxSplit > 0x7fffffffLL) return cudaErrorInvalidValue;
+  const size_t smem = smem_wanted < 122880u ? 122880u : smem_wanted;
+  g.split = 1;
+  // no split pays where half of the longest stream is cheaper than what a split costs
+  if (2 * units <= kSms && (col ? g.N_q : g.N_kv) * (0.5f / BN) * tile_clocks > split_clocks(g.D)) {
+    const SplitLoad w = stream_load(g, col, tile_clocks);
+    const bool paired = other_clocks > 0.f;
+    SplitLoad other = {0.f, 0.f, 0.f};
+    if (paired) other = stream_load(g, !col, other_clocks);
+    // of a pair, the kernel with the longer CTAs only: two kernels of clusters do not share the GPU well
+    if (w.longest * w.tile_clocks > other.longest * other.tile_clocks)
+      g.split = pick_split(w, paired ? &other : nullptr, g.D, [&](int c) { return cluster_slots(shared, c, threads, smem, state); });
+  }
+  auto kern = g.split > 1 ? shared : whole;
+  const cudaError_t e = set_smem_once(kern, smem, g.split > 1 ? state.smem_set_split : state.smem_set);
+  return e != cudaSuccess ? e : launch_pdl_cluster(kern, (unsigned)(units * g.split), threads, smem, (unsigned)g.split, s, maps, g, t);
+}
 
 // Control block of the single-tile self-test kernel (every attention kernel has its own).
 struct Control {
@@ -91,28 +271,6 @@ struct Control {
 
 // status codes: (kind + 1) << 8 | wait id
 __device__ __forceinline__ uint32_t wait_code(int kind, int id) { return ((uint32_t)(kind + 1) << 8) | (uint32_t)id; }
-
-template <typename T> struct Pack;
-template <> struct Pack<__nv_bfloat16> {
-  static constexpr int kIsBf16 = 1;
-  static __device__ __forceinline__ uint32_t pack(float lo, float hi) {
-    __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
-    return *reinterpret_cast<uint32_t*>(&v);
-  }
-  static __device__ __forceinline__ float2 unpack(uint32_t w) {
-    return __bfloat1622float2(*reinterpret_cast<__nv_bfloat162*>(&w));
-  }
-};
-template <> struct Pack<__half> {
-  static constexpr int kIsBf16 = 0;
-  static __device__ __forceinline__ uint32_t pack(float lo, float hi) {
-    __half2 v = __floats2half2_rn(lo, hi);
-    return *reinterpret_cast<uint32_t*>(&v);
-  }
-  static __device__ __forceinline__ float2 unpack(uint32_t w) {
-    return __half22float2(*reinterpret_cast<__half2*>(&w));
-  }
-};
 
 __device__ __forceinline__ float ex2(float x) {
   float y;

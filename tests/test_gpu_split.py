@@ -1,0 +1,44 @@
+"""Tensor-core kernels where few stationary tiles make the streamed tiles of one be shared by a cluster
+of CTAs: every cluster size, shares that are empty or begin inside a masked range, rows that see no key
+in some shares or in none, both tile widths and types; against the fp64 closed form."""
+import importlib
+
+import pytest
+import torch
+
+import attention_oracle as orc
+
+pytestmark = pytest.mark.gpu
+tcapi = importlib.import_module("610sample_b200.torch_capi")
+capi = importlib.import_module("610sample_b200.capi")
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("B,H,N_q,N_kv,D,window,chunk,mask", [
+    (1, 1, 128, 2048, 64, 2048, 15, 0),      # one query tile against 32 key tiles
+    (1, 1, 100, 1999, 128, 1999, 30, 0),     # ragged on both axes
+    (1, 2, 257, 900, 80, 300, 3, 0),         # window: the range of a tile starts inside a 64-row tile
+    (1, 1, 1500, 130, 128, 1500, 0, 1),      # the key side is the short one
+    (2, 3, 130, 1000, 96, 1000, 0, 0),       # most keys in front of the sequence
+    (1, 1, 64, 190, 64, 190, 9, 0),          # three tiles: fewer than the largest cluster
+    (1, 5, 640, 640, 64, 640, 0, 0),         # causal: shares of unequal tiles
+    (3, 16, 300, 1300, 128, 1000, 2, 0),     # enough CTAs for small clusters only
+    (1, 1, 70, 600, 16, 40, 0, 0),           # keys without a visible query in every share but one
+])
+def test_split_tiles_match_the_oracle(B, H, N_q, N_kv, D, window, chunk, mask, dtype):
+    inp = orc.make_inputs(B, H, N_q, N_kv, D, seed=N_q + N_kv, dtype=dtype)
+    ref = orc.closed_form_all(*(inp[n] for n in orc.INPUT_NAMES), window_size=window, chunk_id=chunk, mask_mode=mask)
+    g = {n: t.cuda() for n, t in inp.items()}
+    runs = []
+    for _ in range(2):
+        O, L = tcapi.forward(g["Q"], g["K"], g["V"], window, chunk, mask)
+        b = tcapi.backward(g["dO"], g["Q"], g["K"], g["V"], O, L, window, chunk, mask)
+        h = tcapi.double_backward(g["g_dQ"], g["g_dK"], g["g_dV"], g["dO"], g["Q"], g["K"], g["V"], O, L, window, chunk, mask)
+        runs.append((O,) + tuple(b) + tuple(h))
+    assert torch.allclose(L.cpu().double(), ref["L"].double(), rtol=1e-5, atol=1e-4)
+    for got, again, n in zip(*runs, ("O", "dQ", "dK", "dV", "g_dO", "g_Q", "g_K", "g_V")):
+        assert torch.equal(got, again), n
+        r = ref[n].double()
+        # the bound of the other parity tests: 2e-2 of the largest value (half-precision operands P and dS, rounded results)
+        assert float((got.double().cpu() - r).abs().max()) <= 2e-2 * max(1.0, float(r.abs().max())), n
+    assert capi.device_status() == 0
