@@ -37,8 +37,6 @@ namespace tc {
 
 enum FbKind { FB_BWD_ROW = 2, FB_BWD_COL = 3 };   // numbering of launch_fwd_bwd
 
-constexpr int kFbMmaWarp = 9;
-constexpr int kFbThreads = 352;    // 8 math warps, TMA producer, two MMA issuers
 constexpr int kFbMaxStages = 8;
 
 struct FbControl {
@@ -56,32 +54,41 @@ struct FbControl {
   volatile uint32_t abort_flag;
 };
 
-template <int KIND, int D>
+// DUAL: two CTAs per SM, each with one group of four math warps (D = 64; launch_fb)
+template <int KIND, int D, bool DUAL>
 struct FbCfg {
   static constexpr bool kCol = (KIND == FB_BWD_COL);
+  static constexpr bool kWholeRow = !kCol || DUAL;   // a math thread owns a whole row of a tile (else half of it)
+  static constexpr bool kStatTmem = !(kCol && DUAL); // the stationary operands move to tensor memory
+  static constexpr int kHalves = DUAL ? 1 : 2;       // math threads per stationary row
+  static constexpr int kMathWarps = 4 * kHalves, kMathThreads = 32 * kMathWarps;
+  static constexpr int kProducerWarp = kMathWarps, kMmaWarp = kMathWarps + 1;     // and a second MMA warp
+  static constexpr int kThreads = kMathThreads + 96;
+  static constexpr int kTmemCols = DUAL ? 256 : 512;
   static constexpr int kAtoms = D / 64;
   static constexpr int kNStat = 2;
   static constexpr int kNStream = 2;
-  static constexpr int kBufs = kCol ? 1 : 2;
+  static constexpr int kBufs = kCol || DUAL ? 1 : 2;
   static constexpr int kNOut = kCol ? 2 : 1;
   static constexpr uint32_t kStagingBytes = kNStat * kAtoms * kAtomBytesStat;
   static constexpr uint32_t kStageBytes = kNStream * kAtoms * kAtomBytesStrm;
   static constexpr uint32_t kAuxBytes = 512 + 2048;   // control; per-query scalars / L exchange
   // as many stream stages as fit (at most eight): a TMA load takes about 2 000 clocks from request
   // to arrival and a tile of these kernels much less, so the loads have to run several tiles ahead
-  static constexpr uint32_t kMaxSmem = 232448;
+  static constexpr uint32_t kMaxSmem = DUAL ? kHalfSmem : 232448;
   static constexpr int kFit = (int)((kMaxSmem - 1024 - kStagingBytes - kAuxBytes) / kStageBytes);
   static constexpr int kStages = kFit < kFbMaxStages ? kFit : kFbMaxStages;
   static_assert(kStages >= 3, "too few stream stages");
-  static_assert(kStages * kStageBytes >= kNOut * BM * D * 4, "the partial results of a split tile lie over the stages");
+  static_assert(DUAL || kStages * kStageBytes >= kNOut * BM * D * 4, "the partial results of a split tile lie over the stages");
   static constexpr uint32_t kContentBytes = kStagingBytes + kStages * kStageBytes + kAuxBytes;
   static constexpr uint32_t kSmemBytes = kContentBytes + 1024;
   // tensor-memory columns
   static constexpr int kRA = 0;
-  static constexpr int kRB = kCol ? 64 : 128;
-  static constexpr int kStat = kCol ? 128 : 384;      // stationary operand x at kStat + 64 x
-  static constexpr int kOut = 256;
-  static_assert(kOut + kNOut * D <= (kCol ? 512 : 384), "tensor memory over-subscribed");
+  static constexpr int kRB = 64 * kBufs;
+  static constexpr int kOut = DUAL ? 128 : 256;
+  static constexpr int kStatStride = DUAL ? D / 2 : 64;
+  static constexpr int kStat = DUAL ? kOut + kNOut * D : kCol ? 128 : 384;      // stationary operand x at kStat + kStatStride x
+  static_assert(DUAL ? kOut + kNOut * D + (kStatTmem ? D : 0) <= kTmemCols : kOut + kNOut * D <= (kCol ? 512 : 384), "tensor memory over-subscribed");
   __host__ __device__ static constexpr uint32_t stream_off(int slot, int atom) {
     return (uint32_t)(slot * kAtoms + atom) * kAtomBytesStrm;
   }
@@ -89,11 +96,13 @@ struct FbCfg {
   __host__ __device__ static constexpr int stream_tensor(int s) { return kCol ? (s == 0 ? T_Q : T_dO) : (s == 0 ? T_K : T_V); }
 };
 
-template <int KIND, int D, typename T, bool SPLIT>
-__global__ void __launch_bounds__(kFbThreads, 1)
+template <int KIND, int D, typename T, bool SPLIT, bool DUAL>
+__global__ void __launch_bounds__((FbCfg<KIND, D, DUAL>::kThreads), DUAL ? 2 : 1)
 fb_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Tensors t) {
-  using CF = FbCfg<KIND, D>;
-  constexpr int kAtoms = CF::kAtoms;
+  using CF = FbCfg<KIND, D, DUAL>;
+  constexpr int kAtoms = CF::kAtoms, kHalves = CF::kHalves;
+  constexpr int kMathWarps = CF::kMathWarps, kMathThreads = CF::kMathThreads, kProducerWarp = CF::kProducerWarp;
+  constexpr int kFbMmaWarp = CF::kMmaWarp, kTmemCols = CF::kTmemCols;
   constexpr int kBufs = CF::kBufs;
   constexpr int KCODE = 16 + KIND;     // kernel id inside device status codes
   constexpr uint32_t kIdesc64 = make_idesc(BM, 64, Pack<T>::kIsBf16, 0, 0);
@@ -173,9 +182,9 @@ fb_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Tensors 
     for (int b = 0; b < 2; ++b) {
       mbar_init(bar_ra_full(b), 1);
       mbar_init(bar_rb_full(b), 1);
-      // row kind: a tile belongs to one group of four math warps
-      mbar_init(bar_op_full(b), CF::kCol ? kMathWarps : kMathWarps / 2);
-      mbar_init(bar_ra_free(b), CF::kCol ? kMathWarps : kMathWarps / 2);
+      // whole rows: a tile belongs to one group of four math warps
+      mbar_init(bar_op_full(b), CF::kWholeRow ? 4 : kMathWarps);
+      mbar_init(bar_ra_free(b), CF::kWholeRow ? 4 : kMathWarps);
       mbar_init(smem_u32(&ctl->stats_ready[b]), kMathWarps);
     }
     mbar_init(bar_acc_done, 1);
@@ -240,7 +249,7 @@ fb_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Tensors 
   // =========================================================================
   else if (warp == kFbMmaWarp || warp == kFbMmaWarp + 1) {
     if (n_iter > 0) {
-      bool ok = mbar_wait(bar_stat_ready, 0, abort_flag, t.status, wait_code(KCODE, 2));
+      bool ok = mbar_wait(CF::kStatTmem ? bar_stat_ready : bar_staging_full, 0, abort_flag, t.status, wait_code(KCODE, 2));
       ok = __all_sync(0xffffffffu, ok);
       tc_fence_after_sync();
       // descriptor offsets (16-byte units) within a stage: K-major B, k-step ks of slot; MN-major B,
@@ -255,7 +264,13 @@ fb_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Tensors 
       // a head dimension below the tile width: skip the k-steps and output columns that are padding
       const int ks_n = g.D >> 4;
       const uint32_t idesc_out = make_idesc(BM, g.D, Pack<T>::kIsBf16, 0, 1);
-      const uint32_t stat0 = tmem_base + CF::kStat, stat1 = stat0 + 64;
+      const uint32_t stat0 = tmem_base + CF::kStat, stat1 = stat0 + CF::kStatStride;
+      const uint64_t stat_desc = smem_desc_sw128(staging, 16, 1024);
+      // score product: k-step ks of stationary operand x (tensor memory, or shared memory) with B
+      auto score_mma = [&](uint32_t acc, int x, int ks, uint64_t bd) {
+        if constexpr (CF::kStatTmem) mma_ts(acc, (x == 0 ? stat0 : stat1) + 8 * ks, bd, kIdesc64, ks > 0);
+        else mma_ss(acc, stat_desc + (uint64_t)((x * kAtoms * kAtomBytesStat + (ks >> 2) * kAtomBytesStat + (ks & 3) * 32) >> 4), bd, kIdesc64, ks > 0);
+      };
       const uint32_t out0 = tmem_base + CF::kOut, out1 = out0 + D;
       (void)stat1; (void)out1;
 
@@ -272,7 +287,7 @@ fb_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Tensors 
         const uint32_t acc = tmem_base + CF::kRA + 64 * b;
         if (elect_one()) {
           _Pragma("unroll") for (int ks = 0; ks < KS; ++ks)
-            if (ks < ks_n) mma_ts(acc, stat0 + 8 * ks, dk + koff(0, ks), kIdesc64, ks > 0);
+            if (ks < ks_n) score_mma(acc, 0, ks, dk + koff(0, ks));
           mma_commit(bar_ra_full(b));
         }
         __syncwarp();
@@ -283,7 +298,7 @@ fb_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Tensors 
         const uint32_t acc = tmem_base + CF::kRB + 64 * b;
         if (elect_one()) {
           _Pragma("unroll") for (int ks = 0; ks < KS; ++ks)
-            if (ks < ks_n) mma_ts(acc, stat1 + 8 * ks, dk + koff(1, ks), kIdesc64, ks > 0);
+            if (ks < ks_n) score_mma(acc, 1, ks, dk + koff(1, ks));
           mma_commit(bar_rb_full(b));
         }
         __syncwarp();
@@ -366,15 +381,15 @@ fb_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Tensors 
     // Shared-memory tile: per 64-column atom, row r at r*128 bytes, 16-byte chunks XOR-swizzled
     // by r % 8.  Tensor-memory A operand: lane = row, one 32-bit column per pair of K elements.
     bool ok = true;
-    if (n_iter > 0) {
+    if (CF::kStatTmem && n_iter > 0) {
       ok = mbar_wait(bar_staging_full, 0, abort_flag, t.status, wait_code(KCODE, 6));
       ok = __all_sync(0xffffffffu, ok);
       if (ok) {
-        constexpr int kChunksPerHalf = D / 16;
+        constexpr int kChunksPerHalf = D / 8 / kHalves;
 #pragma unroll
         for (int x = 0; x < CF::kNStat; ++x) {
           const uint32_t src = staging + x * kAtoms * kAtomBytesStat;
-          const uint32_t dst = lane_addr + CF::kStat + 64 * x;
+          const uint32_t dst = lane_addr + CF::kStat + CF::kStatStride * x;
 #pragma unroll
           for (int c = 0; c < kChunksPerHalf; c += 2) {
             uint32_t w[8];
@@ -429,18 +444,28 @@ fb_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Tensors 
     };
     if constexpr (CF::kCol) { if (n_iter > 0) publish_stat(0, fetch_stat(0)); }
 
-    if constexpr (!CF::kCol) {
+    if constexpr (CF::kWholeRow) {
       // ---- row kind: the eight math warps form two groups of four; group w takes the tiles of
       // parity w (= score buffer w), a thread its whole row of the tile (64 scores).  While one
-      // group waits for its products or for tensor-memory reads, the other one computes.
+      // group waits for its products or for tensor-memory reads, the other one computes.  With two
+      // CTAs per SM the other group is the other CTA's.
       const int grp = half;
-      for (int it = grp; it < n_iter && ok; it += 2) {
-        const int b = it & 1;
+      for (int it = grp; it < n_iter && ok; it += kBufs) {
+        const int b = it % kBufs;
+        const float* cs = aux_f + (it & 1) * 128;   // column kind: [-L*log2(e) | -Dv] x 64 queries
+        float next_stat = 0.f;
+        if constexpr (CF::kCol) {
+          // the scalars of tile it+1 are fetched now and published at the end of this tile
+          next_stat = fetch_stat(it + 1);
+          ok = mbar_wait(smem_u32(&ctl->stats_ready[it & 1]), (it >> 1) & 1, abort_flag, t.status, wait_code(KCODE, 9));
+          ok = __all_sync(0xffffffffu, ok);
+          if (!ok) break;
+        }
         const int j0 = (t_begin + it) * BN;
         const bool masked = !(j0 >= vlo && j0 + BN - 1 < vhi);
         const uint32_t ra = lane_addr + CF::kRA + 64 * b;
         const uint32_t rb = lane_addr + CF::kRB + 64 * b;
-        ok = mbar_wait(bar_ra_full(b), (it >> 1) & 1, abort_flag, t.status, wait_code(KCODE, 7));
+        ok = mbar_wait(bar_ra_full(b), (it / kBufs) & 1, abort_flag, t.status, wait_code(KCODE, 7));
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
         tc_fence_after_sync();
@@ -462,7 +487,9 @@ fb_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Tensors 
 #pragma unroll
             for (int e = 0; e < 16; e += 2) {
               const int cc = hh * 32 + ch * 16 + e;
-              const float2 x = __ffma2_rn(make_float2(__uint_as_float(s_[ch][e]), __uint_as_float(s_[ch][e + 1])), sl2, nL2);
+              float2 l2 = nL2;
+              if constexpr (CF::kCol) l2 = *reinterpret_cast<const float2*>(cs + cc);
+              const float2 x = __ffma2_rn(make_float2(__uint_as_float(s_[ch][e]), __uint_as_float(s_[ch][e + 1])), sl2, l2);
               float2 pp = make_float2(ex2(x.x), ex2(x.y));
               if (masked) {
                 pp.x = ((uint32_t)(j0 + cc - vlo) < vspan) ? pp.x : 0.f;
@@ -471,7 +498,7 @@ fb_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Tensors 
               pw[hh * 16 + ch * 8 + (e >> 1)] = pp;
             }
         }
-        ok = mbar_wait(bar_rb_full(b), (it >> 1) & 1, abort_flag, t.status, wait_code(KCODE, 8));
+        ok = mbar_wait(bar_rb_full(b), (it / kBufs) & 1, abort_flag, t.status, wait_code(KCODE, 8));
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
         tc_fence_after_sync();
@@ -487,19 +514,34 @@ fb_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Tensors 
           for (int ch = 0; ch < 2; ++ch)
 #pragma unroll
             for (int e = 0; e < 16; e += 2) {
-              const float2 dpd = __fadd2_rn(make_float2(__uint_as_float(d_[ch][e]), __uint_as_float(d_[ch][e + 1])), nDv);
+              float2 dv = nDv;
+              if constexpr (CF::kCol) dv = *reinterpret_cast<const float2*>(cs + 64 + hh * 32 + ch * 16 + e);
+              const float2 dpd = __fadd2_rn(make_float2(__uint_as_float(d_[ch][e]), __uint_as_float(d_[ch][e + 1])), dv);
               const float2 ds = __fmul2_rn(pw[hh * 16 + ch * 8 + (e >> 1)], dpd);
               kds[ch][e >> 1] = Pack<T>::pack(ds.x, ds.y);
             }
-          // dS over the dP columns this thread has just read (the layout the output product expects:
-          // 16 elements of k-step ks in 8 columns at 32 * (ks / 2) + 8 * (ks % 2))
-          tmem_st8(rb + hh * 32, kds[0]);
-          tmem_st8(rb + hh * 32 + 8, kds[1]);
+          // dS, in the column kind behind P, over the dP columns this thread has just read (the layout
+          // the output product expects: 16 elements of k-step ks in 8 columns at 32 * (ks / 2) + 8 * (ks % 2))
+          if constexpr (CF::kCol) {
+            uint32_t kp[2][8];
+#pragma unroll
+            for (int ch = 0; ch < 2; ++ch)
+#pragma unroll
+              for (int e = 0; e < 8; ++e) {
+                const float2 pp = pw[hh * 16 + ch * 8 + e];
+                kp[ch][e] = Pack<T>::pack(pp.x, pp.y);
+              }
+            tmem_st8(rb + hh * 32, kp[0]);
+            tmem_st8(rb + hh * 32 + 8, kp[1]);
+          }
+          tmem_st8(rb + hh * 32 + (CF::kCol ? 16 : 0), kds[0]);
+          tmem_st8(rb + hh * 32 + (CF::kCol ? 24 : 8), kds[1]);
         }
         tmem_st_wait();
         tc_fence_before_sync();
         __syncwarp();
         if (lane == 0) mbar_arrive(bar_op_full(b));
+        if constexpr (CF::kCol) { if (it + 1 < n_iter) publish_stat(it + 1, next_stat); }
       }
     } else
     for (int it = 0; it < n_iter && ok; ++it) {
@@ -599,7 +641,7 @@ fb_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Tensors 
       if (n_iter > 0 && ok) ok = mbar_wait(bar_acc_done, 0, abort_flag, t.status, wait_code(KCODE, 10));
       ok = __all_sync(0xffffffffu, ok);
       tc_fence_after_sync();
-      constexpr int kColsPerHalf = D / 2;
+      constexpr int kColsPerHalf = D / kHalves;
       constexpr int kChunks = kColsPerHalf / 16;
       // The result tiles go out through the staging buffer of the stationary operands (they
       // have been in tensor memory since the prologue).
@@ -642,7 +684,7 @@ fb_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Tensors 
         }
       }
       fence_proxy_async_smem();
-      named_barrier_sync(2, kMathWarps * 32);
+      named_barrier_sync(2, kMathThreads);
       if (!SPLIT && threadIdx.x == 0) {
         for (int o = 0; o < CF::kNOut; ++o) {
           const int id = (KIND == FB_BWD_ROW) ? TO_dQ : (o == 0 ? TO_dV : TO_dK);
@@ -677,13 +719,21 @@ fb_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Tensors 
 
 template <int KIND, int D, typename T>
 static cudaError_t launch_fb(const TmaMaps& maps, const Geometry& g_in, const Tensors& t, cudaStream_t s) {
-  using CF = FbCfg<KIND, D>;
+  constexpr bool kCol = KIND == FB_BWD_COL;
   Geometry g = g_in;
-  const long long ctas = (long long)g.BH * (((CF::kCol ? g.N_kv : g.N_q) + BM - 1) / BM);
-  g.head_group = pick_head_group(ctas, g.BH, 2ll * (CF::kCol ? g.N_q : g.N_kv) * g.D * 2);
+  const long long ctas = (long long)g.BH * (((kCol ? g.N_kv : g.N_q) + BM - 1) / BM);
+  g.head_group = pick_head_group(ctas, g.BH, 2ll * (kCol ? g.N_q : g.N_kv) * g.D * 2);
+  if constexpr (D == 64) {
+    if (two_per_sm_pays(g, kCol, kCol ? 1700.f : 1000.f, kCol ? 1200.f : 1000.f)) {
+      using CF = FbCfg<KIND, D, true>;
+      static std::atomic<unsigned long long> smem_set{0};
+      return launch_two_per_sm(fb_kernel<KIND, D, T, false, true>, maps, g, t, s, ctas, CF::kThreads, CF::kSmemBytes, smem_set);
+    }
+  }
+  using CF = FbCfg<KIND, D, false>;
   static TileKernelState state;
-  return launch_tiles(fb_kernel<KIND, D, T, false>, fb_kernel<KIND, D, T, true>, maps, g, t, s, CF::kCol, kFbThreads, CF::kSmemBytes,
-                      CF::kCol ? 1700.f : 1150.f, CF::kCol ? 1150.f : 1700.f, state);
+  return launch_tiles(fb_kernel<KIND, D, T, false, false>, fb_kernel<KIND, D, T, true, false>, maps, g, t, s, kCol, CF::kThreads,
+                      CF::kSmemBytes, kCol ? 1700.f : 1150.f, kCol ? 1150.f : 1700.f, state);
 }
 
 template <int D, typename T>

@@ -33,11 +33,8 @@
 namespace attn {
 namespace tc {
 
-constexpr int kFwdSWarp = 9;        // issues S = Q K^T
-constexpr int kFwdPvWarp = 10;      // issues O += P V
-constexpr int kFwdThreads = 352;    // 8 math warps, TMA producer, two MMA issuers
 constexpr int kFwdMaxStages = 8;
-constexpr int kFwdSBufs = 3;
+constexpr int kFwdMaxSBufs = 3;
 template <typename T> constexpr float kTau = Pack<T>::kIsBf16 ? 24.f : 15.f;     // log2 units
 constexpr int KFWD = 20;            // kernel id inside device status codes
 
@@ -46,9 +43,9 @@ struct FwdControl {
   uint64_t q_ready;                    // Q copied to tensor memory
   uint64_t stream_full[2][kFwdMaxStages];    // [0] K half, [1] V half
   uint64_t stream_empty[2][kFwdMaxStages];
-  uint64_t s_full[kFwdSBufs];          // score product complete
-  uint64_t p_full[kFwdSBufs];          // P written by the owning math group
-  uint64_t pv_done[kFwdSBufs];         // the P V product that read the buffer has completed
+  uint64_t s_full[kFwdMaxSBufs];       // score product complete
+  uint64_t p_full[kFwdMaxSBufs];       // P written by the owning math group
+  uint64_t pv_done[kFwdMaxSBufs];      // the P V product that read the buffer has completed
   uint64_t acc_done;
   uint32_t tmem_base;
   volatile uint32_t abort_flag;
@@ -56,31 +53,39 @@ struct FwdControl {
 
 static_assert(sizeof(FwdControl) <= 512, "control block larger than its slot");
 
-template <int D>
+// G: math groups of a CTA.  2, one CTA per SM; or 1, two CTAs per SM (launch_fwd_one).
+template <int D, int G>
 struct FwdCfg {
+  static constexpr int kMathWarps = 4 * G, kMathThreads = 128 * G;
+  static constexpr int kProducerWarp = kMathWarps, kSWarp = kMathWarps + 1, kPvWarp = kMathWarps + 2;   // S = Q K^T; O += P V
+  static constexpr int kThreads = kMathThreads + 96;
+  static constexpr int kSBufs = G == 2 ? 3 : 2;
+  static constexpr int kTmemCols = 256 * G;
   static constexpr int kAtoms = D / 64;
   static constexpr uint32_t kStagingBytes = kAtoms * kAtomBytesStat;        // Q, later the O tile
   static constexpr uint32_t kStageBytes = 2 * kAtoms * kAtomBytesStrm;      // K then V
   static constexpr uint32_t kAuxBytes = 512 + 2 * 2 * BM * 4;               // control; (m, l) of both groups
-  static constexpr uint32_t kMaxSmem = 232448;
+  static constexpr uint32_t kMaxSmem = G == 2 ? 232448 : kHalfSmem;
   static constexpr int kFit = (int)((kMaxSmem - 1024 - kStagingBytes - kAuxBytes) / kStageBytes);
   static constexpr int kStages = kFit < kFwdMaxStages ? kFit : kFwdMaxStages;
   static_assert(kStages >= 4, "too few stream stages");
   static_assert(kStages * kStageBytes >= BM * D * 4 && kStagingBytes >= (2 + kMaxSplit) * BM * 4, "room for a split tile's results");
   static constexpr uint32_t kContentBytes = kStagingBytes + kStages * kStageBytes + kAuxBytes;
   static constexpr uint32_t kSmemBytes = kContentBytes + 1024;
-  static constexpr int kS = 0, kQT = 192, kO = 256;       // O of group w at kO + w * D
-  static_assert(kQT + D / 2 <= kO && kO + 2 * D <= kTmemCols, "tensor memory over-subscribed");
+  static constexpr int kS = 0, kQT = 64 * kSBufs, kO = G == 2 ? 256 : kQT + D / 2;       // O of group w at kO + w * D
+  static_assert(kQT + D / 2 <= kO && kO + G * D <= kTmemCols, "tensor memory over-subscribed");
   __host__ __device__ static constexpr uint32_t stream_off(int slot, int atom) {   // slot 0 K, 1 V
     return (uint32_t)(slot * kAtoms + atom) * kAtomBytesStrm;
   }
 };
 
-template <int D, typename T, bool SPLIT>
-__global__ void __launch_bounds__(kFwdThreads, 1)
+template <int D, typename T, bool SPLIT, int G>
+__global__ void __launch_bounds__((FwdCfg<D, G>::kThreads), 3 - G)
 fwd_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Tensors t) {
-  using CF = FwdCfg<D>;
-  constexpr int kAtoms = CF::kAtoms;
+  using CF = FwdCfg<D, G>;
+  constexpr int kAtoms = CF::kAtoms, kFwdSBufs = CF::kSBufs;
+  constexpr int kMathWarps = CF::kMathWarps, kMathThreads = CF::kMathThreads, kProducerWarp = CF::kProducerWarp;
+  constexpr int kFwdSWarp = CF::kSWarp, kFwdPvWarp = CF::kPvWarp, kTmemCols = CF::kTmemCols;
   constexpr uint32_t kIdesc64 = make_idesc(BM, 64, Pack<T>::kIsBf16, 0, 0);
 
   extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -154,7 +159,7 @@ fwd_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Tensors
       }
     for (int b = 0; b < kFwdSBufs; ++b) {
       mbar_init(bar_s_full(b), 1);
-      mbar_init(bar_p_full(b), kMathWarps / 2);
+      mbar_init(bar_p_full(b), 4);
       mbar_init(bar_pv_done(b), 1);
     }
     mbar_init(bar_acc_done, 1);
@@ -262,7 +267,7 @@ fwd_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Tensors
         const uint32_t idesc_out = make_idesc(BM, g.D, Pack<T>::kIsBf16, 0, 1);
         auto moff = [](int ks) { return (uint64_t)((CF::stream_off(1, 0) + ks * 2048) >> 4); };
         for (int j = 0; j < n_iter && ok; ++j) {
-          const int b = j % kFwdSBufs, st = j % CF::kStages, w = j & 1;
+          const int b = j % kFwdSBufs, st = j % CF::kStages, w = j % G;
           ok = mbar_wait(bar_p_full(b), (j / kFwdSBufs) & 1, abort_flag, t.status, wait_code(KFWD, 5));
           ok = __all_sync(0xffffffffu, ok);
           if (ok) ok = wait_stream(1, j);
@@ -271,7 +276,7 @@ fwd_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Tensors
           const uint64_t dm = smem_desc_sw128(strm_base + st * CF::kStageBytes, kAtomBytesStrm, 1024);
           const uint32_t acc = tmem_base + CF::kO + (uint32_t)(w * D);
           const uint32_t pbuf = tmem_base + CF::kS + 64u * (uint32_t)b;
-          const bool first = j < 2;       // the first tile of either group overwrites its accumulator
+          const bool first = j < G;       // the first tile of either group overwrites its accumulator
           if (elect_one()) {
             _Pragma("unroll") for (int ks = 0; ks < KO; ++ks)
               mma_ts(acc, pbuf + 8 * ks, dm + moff(ks), idesc_out, !(first && ks == 0));
@@ -285,7 +290,7 @@ fwd_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Tensors
     }
   }
   // =========================================================================
-  // math warps: group w = warp / 4 takes the tiles of parity w, one thread per query row
+  // math warps: group w = warp / 4 takes every G-th tile from w, one thread per query row
   // =========================================================================
   else {
     const int quarter = warp & 3, grp = warp >> 2;
@@ -308,7 +313,7 @@ fwd_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Tensors
       ok = mbar_wait(bar_staging_full, 0, abort_flag, t.status, wait_code(KFWD, 6));
       ok = __all_sync(0xffffffffu, ok);
       if (ok) {
-        constexpr int kChunksPerHalf = D / 16;
+        constexpr int kChunksPerHalf = D / 8 / G;
 #pragma unroll
         for (int c = 0; c < kChunksPerHalf; c += 2) {
           uint32_t w[8];
@@ -331,7 +336,7 @@ fwd_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Tensors
 
     float m_ref = -INFINITY, l_sum = 0.f;     // this group's running maximum (log2 units) and sum for the row
     const uint32_t oacc = lane_addr + CF::kO + (uint32_t)(grp * D);
-    for (int it = grp; it < n_iter && ok; it += 2) {
+    for (int it = grp; it < n_iter && ok; it += G) {
       const int b = it % kFwdSBufs;
       const uint32_t sbuf = lane_addr + CF::kS + 64u * (uint32_t)b;
       const int j0 = (t_begin + it) * BN;
@@ -372,10 +377,10 @@ fwd_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Tensors
         const float f = (m_ref == -INFINITY) ? 0.f : ex2(m_ref - m_new);   // 1 for the rows that do not move
         l_sum *= f;
         m_ref = m_new;
-        if (it >= 2) {
+        if (it >= G) {
           // multiply this row of the group's O accumulator by f, once its previous P V product is complete
-          const int pb = (it - 2) % kFwdSBufs;
-          ok = mbar_wait(bar_pv_done(pb), ((it - 2) / kFwdSBufs) & 1, abort_flag, t.status, wait_code(KFWD, 8));
+          const int pb = (it - G) % kFwdSBufs;
+          ok = mbar_wait(bar_pv_done(pb), ((it - G) / kFwdSBufs) & 1, abort_flag, t.status, wait_code(KFWD, 8));
           ok = __all_sync(0xffffffffu, ok);
           if (!ok) break;
           tc_fence_after_sync();
@@ -422,11 +427,14 @@ fwd_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Tensors
     }
 
     // ---------------- merge of the two groups and output ------------------------------
-    float* mine = ml + grp * 2 * BM;
-    const float* other = ml + (grp ^ 1) * 2 * BM;
-    mine[row] = m_ref; mine[BM + row] = l_sum;
-    named_barrier_sync(1, kMathThreads);
-    const float m_o = other[row], l_o = other[BM + row];
+    float m_o = -INFINITY, l_o = 0.f;      // the other group's
+    if constexpr (G == 2) {
+      float* mine = ml + grp * 2 * BM;
+      const float* other = ml + (grp ^ 1) * 2 * BM;
+      mine[row] = m_ref; mine[BM + row] = l_sum;
+      named_barrier_sync(1, kMathThreads);
+      m_o = other[row]; l_o = other[BM + row];
+    }
     const float m_all = fmaxf(m_ref, m_o);
     float f_me = 0.f, f_ot = 0.f, l_all = 0.f;
     if (m_all > -INFINITY) {
@@ -443,10 +451,10 @@ fwd_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Tensors
     if (n_iter > 0 && ok) ok = mbar_wait(bar_acc_done, 0, abort_flag, t.status, wait_code(KFWD, 9));
     ok = __all_sync(0xffffffffu, ok);
     tc_fence_after_sync();
-    // this thread finishes column half `grp` of its row from both accumulators
+    // this thread finishes its group's share of the columns of its row from both accumulators
     const float f0 = (grp == 0 ? f_me : f_ot) * inv, f1 = (grp == 0 ? f_ot : f_me) * inv;
     const bool use0 = f0 > 0.f, use1 = f1 > 0.f && n_iter > 1;      // an accumulator nothing was added to is never read as a number
-    constexpr int kColsPerHalf = D / 2;
+    constexpr int kColsPerHalf = D / G;
 #pragma unroll
     for (int c = 0; c < kColsPerHalf / 16; ++c) {
       const int col = grp * kColsPerHalf + 16 * c;
@@ -454,9 +462,9 @@ fwd_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Tensors
       uint32_t a_[16], b_[16];
       if (n_iter > 0 && ok) {
         tmem_ld16(lane_addr + CF::kO + col, a_);
-        tmem_ld16(lane_addr + CF::kO + D + col, b_);
+        if constexpr (G == 2) tmem_ld16(lane_addr + CF::kO + D + col, b_);
         tmem_ld_wait(a_);
-        tmem_ld_wait(b_);
+        if constexpr (G == 2) tmem_ld_wait(b_);
       }
       uint32_t w[8];
       float f[16];
@@ -465,7 +473,7 @@ fwd_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Tensors
         float v0 = 0.f, v1 = 0.f;
         if (n_iter > 0 && ok) {
           if (use0) { v0 = __uint_as_float(a_[2 * e]) * f0; v1 = __uint_as_float(a_[2 * e + 1]) * f0; }
-          if (use1) { v0 = fmaf(__uint_as_float(b_[2 * e]), f1, v0); v1 = fmaf(__uint_as_float(b_[2 * e + 1]), f1, v1); }
+          if (G == 2 && use1) { v0 = fmaf(__uint_as_float(b_[2 * e]), f1, v0); v1 = fmaf(__uint_as_float(b_[2 * e + 1]), f1, v1); }
         }
         w[e] = Pack<T>::pack(v0, v1);
         f[2 * e] = v0; f[2 * e + 1] = v1;
@@ -474,7 +482,7 @@ fwd_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Tensors
       else if (gidx < g.N_q) store_op16(staging + (uint32_t)(col >> 6) * kAtomBytesStat, row, col & 63, w);
     }
     // the O tile leaves through the staging buffer (Q has been in tensor memory since the prologue)
-    store_tile_tma(&maps.out[TO_O], staging, g.D, r0, bh, !SPLIT && threadIdx.x == 0);
+    store_tile_tma(&maps.out[TO_O], staging, g.D, r0, bh, !SPLIT && threadIdx.x == 0, kMathThreads);
   }
 
   if constexpr (SPLIT) {
@@ -515,11 +523,19 @@ fwd_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Tensors
 
 template <int D, typename T>
 static cudaError_t launch_fwd_one(const TmaMaps& maps, const Geometry& g_in, const Tensors& t, cudaStream_t s) {
-  using CF = FwdCfg<D>;
   Geometry g = g_in;
-  g.head_group = pick_head_group((long long)g.BH * ((g.N_q + BM - 1) / BM), g.BH, 2ll * g.N_kv * g.D * 2);   // K, V
+  const long long ctas = (long long)g.BH * ((g.N_q + BM - 1) / BM);
+  g.head_group = pick_head_group(ctas, g.BH, 2ll * g.N_kv * g.D * 2);   // K, V
+  if constexpr (D == 64) {
+    if (two_per_sm_pays(g, false, 850.f, 850.f)) {
+      using CF = FwdCfg<D, 1>;
+      static std::atomic<unsigned long long> smem_set{0};
+      return launch_two_per_sm(fwd_kernel<D, T, false, 1>, maps, g, t, s, ctas, CF::kThreads, CF::kSmemBytes, smem_set);
+    }
+  }
+  using CF = FwdCfg<D, 2>;
   static TileKernelState state;
-  return launch_tiles(fwd_kernel<D, T, false>, fwd_kernel<D, T, true>, maps, g, t, s, false, kFwdThreads, CF::kSmemBytes, 850.f, 0.f, state);
+  return launch_tiles(fwd_kernel<D, T, false, 2>, fwd_kernel<D, T, true, 2>, maps, g, t, s, false, CF::kThreads, CF::kSmemBytes, 850.f, 0.f, state);
 }
 
 // forward: O and L in one launch

@@ -17,6 +17,7 @@ constexpr int kMathWarps = 8;
 constexpr int kMathThreads = kMathWarps * 32;
 constexpr int kProducerWarp = 8;   // the MMA-issuing warps follow it
 constexpr int kTmemCols = 512;
+constexpr uint32_t kHalfSmem = 233472 / 2 - 1024;   // dynamic shared memory of a CTA that shares its SM with another
 constexpr uint32_t kAtomBytesStat = BM * 128;   // [128 rows][64 halves], 16 KB
 constexpr uint32_t kAtomBytesStrm = BN * 128;   // [ 64 rows][64 halves],  8 KB
 
@@ -166,8 +167,8 @@ constexpr int kMaxSplit = 8;
 constexpr int kSms = 148;
 inline float split_clocks(int D) { return 3000.f + 45.f * D; }
 
-// a kernel's stationary tiles, the most streamed tiles one of them visits, clocks per tile
-struct SplitLoad { float units, longest, tile_clocks; };
+// a kernel's stationary tiles, the most and the mean streamed tiles one of them visits, clocks per tile
+struct SplitLoad { float units, longest, mean, tile_clocks; };
 
 template <typename Slots>
 inline int pick_split(const SplitLoad& w, const SplitLoad* other, int D, Slots slots) {
@@ -189,14 +190,16 @@ inline int pick_split(const SplitLoad& w, const SplitLoad* other, int D, Slots s
 inline SplitLoad stream_load(const Geometry& g, bool col, float tile_clocks) {
   const int n = col ? g.N_kv : g.N_q, tiles = (n + BM - 1) / BM;
   int most = 0;
+  long long sum = 0;
   for (int i = 0; i < tiles; ++i) {
     int lo, hi;
     if (col) query_range_for_keys(g, i * BM, (i + 1) * BM, lo, hi);
     else key_range_for_queries(g, i * BM, (i + 1) * BM, lo, hi);
     const int k = hi > lo ? (hi + BN - 1) / BN - lo / BN : 0;
     if (k > most) most = k;
+    sum += k;
   }
-  return {(float)g.BH * tiles, (float)most, tile_clocks};
+  return {(float)g.BH * tiles, (float)most, tiles > 0 ? (float)sum / tiles : 0.f, tile_clocks};
 }
 
 // What a kernel's launches keep: the devices its shared-memory opt-in has been made on, and the CTAs
@@ -250,7 +253,7 @@ inline cudaError_t launch_tiles(void (*whole)(P...), void (*shared)(P...), const
   if (2 * units <= kSms && (col ? g.N_q : g.N_kv) * (0.5f / BN) * tile_clocks > split_clocks(g.D)) {
     const SplitLoad w = stream_load(g, col, tile_clocks);
     const bool paired = other_clocks > 0.f;
-    SplitLoad other = {0.f, 0.f, 0.f};
+    SplitLoad other = {0.f, 0.f, 0.f, 0.f};
     if (paired) other = stream_load(g, !col, other_clocks);
     // of a pair, the kernel with the longer CTAs only: two kernels of clusters do not share the GPU well
     if (w.longest * w.tile_clocks > other.longest * other.tile_clocks)
@@ -259,6 +262,31 @@ inline cudaError_t launch_tiles(void (*whole)(P...), void (*shared)(P...), const
   auto kern = g.split > 1 ? shared : whole;
   const cudaError_t e = set_smem_once(kern, smem, g.split > 1 ? state.smem_set_split : state.smem_set);
   return e != cudaSuccess ? e : launch_pdl_cluster(kern, (unsigned)(units * g.split), threads, smem, (unsigned)g.split, s, maps, g, t);
+}
+
+// Two CTAs per SM, each with half of the tensor memory and one group of math warps (D = 64, where
+// that is enough): while one sets up, fills its pipeline or writes its result, the other computes.
+// A CTA costs kCtaClocks besides its tiles, a third of its time at 17 tiles of 64 keys; of that about
+// 4 thousand remain.  But a CTA then takes twice as long for a tile, so the longest one must not become
+// the bound: few CTAs stay one to an SM.  B8 H12 N2048 D64 causal: forward 117 -> 96 us, backward 324
+// -> 267; B2 H16 N8192: 406 -> 389 and 1251 -> 1157.
+inline bool two_per_sm_pays(const Geometry& g, bool col, float tile_clocks, float tile_clocks_two) {
+  const SplitLoad w = stream_load(g, col, tile_clocks);
+  if (w.units < kSms) return false;
+  auto larger = [](float x, float y) { return x > y ? x : y; };
+  const float one = larger(w.longest * tile_clocks + kCtaClocks, w.units / kSms * (w.mean * tile_clocks + kCtaClocks));
+  const float two = larger(2.f * w.longest * tile_clocks_two + kCtaClocks, w.units / kSms * (w.mean * tile_clocks_two + 4000.f));
+  return two < 0.95f * one;
+}
+
+template <typename... P>
+inline cudaError_t launch_two_per_sm(void (*kern)(P...), const TmaMaps& maps, const Geometry& g, const Tensors& t, cudaStream_t s,
+                                     long long ctas, unsigned threads, size_t smem_wanted, std::atomic<unsigned long long>& smem_set) {
+  if (ctas > 0x7fffffffLL) return cudaErrorInvalidValue;
+  // more than a third of an SM's shared memory: never a third CTA that would wait for tensor memory
+  const size_t smem = smem_wanted < 79872u ? 79872u : smem_wanted;
+  const cudaError_t e = set_smem_once(kern, smem, smem_set);
+  return e != cudaSuccess ? e : launch_pdl(kern, (unsigned)ctas, threads, smem, s, maps, g, t);
 }
 
 // Control block of the single-tile self-test kernel (every attention kernel has its own).
@@ -309,9 +337,9 @@ __device__ __forceinline__ void zero_rows(void* out, int plane, int row0, int n_
 // rows [row0, row0 + 128) of plane `plane` with one TMA store per atom (rows and columns beyond
 // the tensor are clipped by the map) and returns once shared memory has been read.
 __device__ __forceinline__ void store_tile_tma(const CUtensorMap* map, uint32_t tile, int cols, int row0, int plane,
-                                               bool leader) {
+                                               bool leader, int math_threads = kMathThreads) {
   fence_proxy_async_smem();
-  named_barrier_sync(2, kMathWarps * 32);
+  named_barrier_sync(2, (uint32_t)math_threads);
   if (leader) {
     for (int a = 0; a * 64 < cols; ++a) tma_store_3d(map, tile + (uint32_t)a * kAtomBytesStat, a * 64, row0, plane);
     bulk_commit_group();

@@ -1,6 +1,7 @@
-"""Tensor-core kernels where few stationary tiles make the streamed tiles of one be shared by a cluster
-of CTAs: every cluster size, shares that are empty or begin inside a masked range, rows that see no key
-in some shares or in none, both tile widths and types; against the fp64 closed form."""
+"""Tensor-core kernels at the ends of the range of stationary tiles, against the fp64 closed form.
+Few: the streamed tiles of one are shared by a cluster of CTAs (every cluster size, shares that are
+empty or begin inside a masked range, rows that see no key in some shares or in none, both tile widths
+and types).  Many, at D <= 64: two CTAs per SM."""
 import importlib
 
 import pytest
@@ -24,8 +25,11 @@ capi = importlib.import_module("610sample_b200.capi")
     (1, 5, 640, 640, 64, 640, 0, 0),         # causal: shares of unequal tiles
     (3, 16, 300, 1300, 128, 1000, 2, 0),     # enough CTAs for small clusters only
     (1, 1, 70, 600, 16, 40, 0, 0),           # keys without a visible query in every share but one
+    (8, 40, 129, 129, 64, 129, 0, 0),        # two CTAs per SM, one row in every second tile
+    (4, 50, 300, 520, 48, 200, 1, 0),        # the same with padding, a window and keys nobody sees
+    (6, 50, 60, 190, 64, 190, 0, 1),         # one tile per head
 ])
-def test_split_tiles_match_the_oracle(B, H, N_q, N_kv, D, window, chunk, mask, dtype):
+def test_few_and_many_tiles_match_the_oracle(B, H, N_q, N_kv, D, window, chunk, mask, dtype):
     inp = orc.make_inputs(B, H, N_q, N_kv, D, seed=N_q + N_kv, dtype=dtype)
     ref = orc.closed_form_all(*(inp[n] for n in orc.INPUT_NAMES), window_size=window, chunk_id=chunk, mask_mode=mask)
     g = {n: t.cuda() for n, t in inp.items()}
