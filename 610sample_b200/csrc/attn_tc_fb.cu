@@ -724,7 +724,7 @@ static cudaError_t launch_fb(const TmaMaps& maps, const Geometry& g_in, const Te
   const long long ctas = (long long)g.BH * (((kCol ? g.N_kv : g.N_q) + BM - 1) / BM);
   g.head_group = pick_head_group(ctas, g.BH, 2ll * (kCol ? g.N_q : g.N_kv) * g.D * 2);
   if constexpr (D == 64) {
-    if (two_per_sm_pays(g, kCol, kCol ? 1700.f : 1000.f, kCol ? 1200.f : 1000.f)) {
+    if (two_per_sm_pays(g, kCol, false, kCol ? 1700.f : 1000.f, kCol ? 1200.f : 1000.f)) {
       using CF = FbCfg<KIND, D, true>;
       static std::atomic<unsigned long long> smem_set{0};
       return launch_two_per_sm(fb_kernel<KIND, D, T, false, true>, maps, g, t, s, ctas, CF::kThreads, CF::kSmemBytes, smem_set);

@@ -5,25 +5,26 @@
 // A CTA owns 128 query rows (Q copied once into TENSOR MEMORY) and streams 64-row tiles of K and V
 // through a ring of TMA stages; the K half and the V half of a stage have their own barriers.
 // Per tile:   S = Q K^T  (N = 64)   ->   P = exp2(S * s * log2 e - m)   ->   O += P V.
-// Eight math warps form two groups of four; a thread owns one query row (= tensor-memory lane) and
-// all 64 scores of a tile.  Group 0 takes the even tiles, group 1 the odd ones, and each group has
-// its OWN running maximum m, running sum l and O accumulator, i.e. the keys are split in two
-// interleaved streams that never have to agree on a maximum while the loop runs; the epilogue
-// merges them: O = (O_0 2^(m_0 - m) + O_1 2^(m_1 - m)) / (l_0 2^(m_0 - m) + l_1 2^(m_1 - m)).
-// Rescaling is lazy: m only moves when a tile's maximum exceeds it by more than tau (in log2
-// units), so P <= 2^tau, and the O row is then multiplied in tensor memory by 2^(m_old - m_new)
-// (a read-modify-write of the row by its owner thread, after the group's previous P V product has
-// completed).  tau is as large as P's type allows: P has the same relative precision whatever its
-// exponent, in bf16 up to far beyond any sum that occurs, so 24 (O and l stay below 2^24 N |V|); in
-// f16 15, one below the largest exponent.  With peaked rows (scores of standard deviation 4) a
-// threshold of 8 made every row of a warp rescale once or twice at tiles of its own, each time
-// stalling the warp for about a tile: 2.20 against 1.85 ms at H32 N16384 D128, Q and K of twice unit
-// variance; 24 is beyond what a row's first tile leaves to come.
-// Tensor memory (512 columns): three score buffers S0, S1, S2 [0,192), Q [192,192+D/2),
-// O_0 [256,256+D), O_1 [256+D, 256+2D).  P is written (two halves per 32-bit column) over the
+// A thread owns one query row (= tensor-memory lane) and all 64 scores of a tile; four math warps form
+// a group.  Two CTAs of one group share an SM, or, where there are few tiles (launch_fwd_one), one CTA
+// has two: group 0 then takes the even tiles, group 1 the odd ones, and each group has its OWN reference
+// exponent m, running sum l and O accumulator, i.e. the keys are split in two interleaved streams that
+// never have to agree while the loop runs; the epilogue merges them:
+// O = (O_0 2^(m_0 - m) + O_1 2^(m_1 - m)) / (l_0 2^(m_0 - m) + l_1 2^(m_1 - m)).
+// Rescaling is lazy: m is a reference, not the maximum.  A row's first visible tile sets it to its
+// maximum; later tiles are exponentiated against it as it stands, and only where a row's sum over a
+// tile exceeds 2^tau does its warp take the maximum, multiply the O row in tensor memory by
+// 2^(m_old - m_new) (a read-modify-write by its owner thread, after the group's previous P V product
+// has completed) and do the tile again.  So no maximum is taken in nearly all tiles (D = 64: -4 to
+// -6 %).  tau is as large as P's type allows: P has the same relative precision whatever its exponent,
+// in bf16 up to far beyond any sum that occurs, so 24 (O and l stay below 2^24 N |V|); in f16 15, one
+// below the largest exponent.
+// Tensor memory, one CTA per SM (512 columns): three score buffers S0, S1, S2 [0,192), Q [192,192+D/2),
+// O_0 [256,256+D), O_1 [256+D, 256+2D); two per SM (256 columns): S0, S1 [0,128), Q behind them at
+// D = 64 (at D = 128 it stays in shared memory), O.  P is written (two halves per 32-bit column) over the
 // first 32 columns of the score buffer it was computed from and read from there as the A operand
 // of P V.  Two warps issue the MMAs, each batch by one elected lane inside a single branch: one
-// the score products (three tiles ahead: a buffer is free again once the P V product that read it
+// the score products (as many tiles ahead as there are buffers: a buffer is free again once the P V product that read it
 // has completed), the other the P V products.  Every wait is bounded.
 // The reference computes the same in two passes with the maximum and sum first
 // (csrc/flash_double_backward_v7.cu:380-530).
@@ -36,6 +37,7 @@ namespace tc {
 constexpr int kFwdMaxStages = 8;
 constexpr int kFwdMaxSBufs = 3;
 template <typename T> constexpr float kTau = Pack<T>::kIsBf16 ? 24.f : 15.f;     // log2 units
+template <typename T> constexpr float kMaxSum = Pack<T>::kIsBf16 ? 16777216.f : 32768.f;     // 2^tau
 constexpr int KFWD = 20;            // kernel id inside device status codes
 
 struct FwdControl {
@@ -61,6 +63,10 @@ struct FwdCfg {
   static constexpr int kThreads = kMathThreads + 96;
   static constexpr int kSBufs = G == 2 ? 3 : 2;
   static constexpr int kTmemCols = 256 * G;
+  // take the maximum of every tile instead of trying the reference as it stands (one CTA per SM at
+  // D = 128, where that is faster: 109 against 118 us at H32, 1024 queries, 9216 keys, D80)
+  static constexpr bool kTakeMax = G == 2 && D == 128;
+  static constexpr bool kQTmem = !(G == 1 && D == 128);     // Q moves to tensor memory where it has room
   static constexpr int kAtoms = D / 64;
   static constexpr uint32_t kStagingBytes = kAtoms * kAtomBytesStat;        // Q, later the O tile
   static constexpr uint32_t kStageBytes = 2 * kAtoms * kAtomBytesStrm;      // K then V
@@ -68,12 +74,12 @@ struct FwdCfg {
   static constexpr uint32_t kMaxSmem = G == 2 ? 232448 : kHalfSmem;
   static constexpr int kFit = (int)((kMaxSmem - 1024 - kStagingBytes - kAuxBytes) / kStageBytes);
   static constexpr int kStages = kFit < kFwdMaxStages ? kFit : kFwdMaxStages;
-  static_assert(kStages >= 4, "too few stream stages");
+  static_assert(kStages >= (kQTmem ? 4 : 2), "too few stream stages");
   static_assert(kStages * kStageBytes >= BM * D * 4 && kStagingBytes >= (2 + kMaxSplit) * BM * 4, "room for a split tile's results");
   static constexpr uint32_t kContentBytes = kStagingBytes + kStages * kStageBytes + kAuxBytes;
   static constexpr uint32_t kSmemBytes = kContentBytes + 1024;
-  static constexpr int kS = 0, kQT = 64 * kSBufs, kO = G == 2 ? 256 : kQT + D / 2;       // O of group w at kO + w * D
-  static_assert(kQT + D / 2 <= kO && kO + G * D <= kTmemCols, "tensor memory over-subscribed");
+  static constexpr int kS = 0, kQT = 64 * kSBufs, kO = G == 2 ? 256 : kQTmem ? kQT + D / 2 : kQT;       // O of group w at kO + w * D
+  static_assert(kQT + (kQTmem ? D / 2 : 0) <= kO && kO + G * D <= kTmemCols, "tensor memory over-subscribed");
   __host__ __device__ static constexpr uint32_t stream_off(int slot, int atom) {   // slot 0 K, 1 V
     return (uint32_t)(slot * kAtoms + atom) * kAtomBytesStrm;
   }
@@ -239,9 +245,10 @@ fwd_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Tensors
       };
       bool ok = true;
       if (warp == kFwdSWarp) {
-        ok = mbar_wait(bar_q_ready, 0, abort_flag, t.status, wait_code(KFWD, 2));
+        ok = mbar_wait(CF::kQTmem ? bar_q_ready : bar_staging_full, 0, abort_flag, t.status, wait_code(KFWD, 2));
         ok = __all_sync(0xffffffffu, ok);
         const uint32_t qt = tmem_base + CF::kQT;
+        const uint64_t qd = smem_desc_sw128(staging, 16, 1024);
         auto koff = [](int ks) { return (uint64_t)((CF::stream_off(0, ks >> 2) + (ks & 3) * 32) >> 4); };
         for (int j = 0; j < n_iter && ok; ++j) {
           const int b = j % kFwdSBufs, st = j % CF::kStages;
@@ -257,7 +264,10 @@ fwd_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Tensors
           const uint32_t sbuf = tmem_base + CF::kS + 64u * (uint32_t)b;
           if (elect_one()) {
             _Pragma("unroll") for (int ks = 0; ks < KS; ++ks)
-              if (ks < ks_n) mma_ts(sbuf, qt + 8 * ks, dk + koff(ks), kIdesc64, ks > 0);
+              if (ks < ks_n) {
+                if constexpr (CF::kQTmem) mma_ts(sbuf, qt + 8 * ks, dk + koff(ks), kIdesc64, ks > 0);
+                else mma_ss(sbuf, qd + (uint64_t)(((ks >> 2) * kAtomBytesStat + (ks & 3) * 32) >> 4), dk + koff(ks), kIdesc64, ks > 0);
+              }
             mma_commit(bar_s_full(b));
             mma_commit(bar_stream_empty(0, st));
           }
@@ -309,7 +319,7 @@ fwd_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Tensors
     // 16-byte chunks XOR-swizzled by r % 8; tensor-memory A operand: lane = row, one 32-bit
     // column per pair of K elements)
     bool ok = true;
-    if (n_iter > 0) {
+    if (CF::kQTmem && n_iter > 0) {
       ok = mbar_wait(bar_staging_full, 0, abort_flag, t.status, wait_code(KFWD, 6));
       ok = __all_sync(0xffffffffu, ok);
       if (ok) {
@@ -352,8 +362,6 @@ fwd_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Tensors
 #pragma unroll
       for (int c = 0; c < 4; ++c) tmem_ld_wait(s_[c]);
 
-      // maximum of the raw scores (-inf where masked) in eight independent chains; the scale
-      // (positive) is applied to the maximum here and to the scores inside the exponent's fma
       if (masked) {
 #pragma unroll
         for (int c = 0; c < 4; ++c)
@@ -361,65 +369,81 @@ fwd_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Tensors
           for (int e = 0; e < 16; ++e)
             if (!((uint32_t)(j0 + 16 * c + e - vlo) < vspan)) s_[c][e] = 0xff800000u;   // -inf
       }
-      float mx8[8];
+      float tile_sum = 0.f;
+      // P = 2^(s * scale - m), written over the score columns this thread has read, and its row sum; the
+      // scale sits in the exponent's fma
+      auto exponentials = [&](float nm) {
+        const float2 sc2 = make_float2(g.scale_log2e, g.scale_log2e), nm2 = make_float2(nm, nm);
+        float2 sum_a = make_float2(0.f, 0.f), sum_b = make_float2(0.f, 0.f);
 #pragma unroll
-      for (int e = 0; e < 8; ++e) mx8[e] = fmaxf(__uint_as_float(s_[0][e]), __uint_as_float(s_[0][8 + e]));
+        for (int c = 0; c < 4; ++c) {
+          uint32_t kp[8];
 #pragma unroll
-      for (int c = 1; c < 4; ++c)
+          for (int e = 0; e < 16; e += 4) {
+            const float2 xa = __ffma2_rn(make_float2(__uint_as_float(s_[c][e]), __uint_as_float(s_[c][e + 1])), sc2, nm2);
+            const float2 xb = __ffma2_rn(make_float2(__uint_as_float(s_[c][e + 2]), __uint_as_float(s_[c][e + 3])), sc2, nm2);
+            const float2 pa = make_float2(ex2(xa.x), ex2(xa.y)), pb = make_float2(ex2(xb.x), ex2(xb.y));
+            sum_a = __fadd2_rn(sum_a, pa);
+            sum_b = __fadd2_rn(sum_b, pb);
+            kp[e >> 1] = Pack<T>::pack(pa.x, pa.y);
+            kp[(e >> 1) + 1] = Pack<T>::pack(pb.x, pb.y);
+          }
+          tmem_st8(sbuf + 8 * c, kp);
+        }
+        tile_sum = (sum_a.x + sum_a.y) + (sum_b.x + sum_b.y);
+      };
+      // The reference is tried as it stands; only where the row sums show that it is too low (or a row
+      // has none yet) is the maximum taken and the tile done again.
+      bool redo = CF::kTakeMax || __any_sync(0xffffffffu, m_ref == -INFINITY);
+      if (!redo) {
+        exponentials(-m_ref);
+        redo = __any_sync(0xffffffffu, !(tile_sum <= kMaxSum<T>));
+      }
+      if (redo) {
+        // maximum of the raw scores (-inf where masked) in eight independent chains
+        float mx8[8];
 #pragma unroll
-        for (int e = 0; e < 8; ++e) mx8[e] = fmaxf(mx8[e], fmaxf(__uint_as_float(s_[c][e]), __uint_as_float(s_[c][8 + e])));
-      const float mx = fmaxf(fmaxf(fmaxf(mx8[0], mx8[1]), fmaxf(mx8[2], mx8[3])), fmaxf(fmaxf(mx8[4], mx8[5]), fmaxf(mx8[6], mx8[7]))) *
-                       g.scale_log2e;
-      // lazy rescale: the reference moves only when this tile exceeds it by more than kTau<T>
-      const bool grow = mx > m_ref + kTau<T> || (m_ref == -INFINITY && mx > -INFINITY);
-      if (__any_sync(0xffffffffu, grow)) {
-        const float m_new = grow ? mx : m_ref;
-        const float f = (m_ref == -INFINITY) ? 0.f : ex2(m_ref - m_new);   // 1 for the rows that do not move
-        l_sum *= f;
-        m_ref = m_new;
-        if (it >= G) {
-          // multiply this row of the group's O accumulator by f, once its previous P V product is complete
-          const int pb = (it - G) % kFwdSBufs;
-          ok = mbar_wait(bar_pv_done(pb), ((it - G) / kFwdSBufs) & 1, abort_flag, t.status, wait_code(KFWD, 8));
-          ok = __all_sync(0xffffffffu, ok);
-          if (!ok) break;
-          tc_fence_after_sync();
+        for (int e = 0; e < 8; ++e) mx8[e] = fmaxf(__uint_as_float(s_[0][e]), __uint_as_float(s_[0][8 + e]));
 #pragma unroll
-          for (int c = 0; c < D / 16; ++c) {
-            if (16 * c >= g.D) break;       // padding columns (uniform)
-            uint32_t o_[16];
-            tmem_ld16(oacc + 16 * c, o_);
-            tmem_ld_wait(o_);
-            uint32_t lo8[8], hi8[8];
+        for (int c = 1; c < 4; ++c)
 #pragma unroll
-            for (int e = 0; e < 8; ++e) {
-              lo8[e] = __float_as_uint(__uint_as_float(o_[e]) * f);
-              hi8[e] = __float_as_uint(__uint_as_float(o_[8 + e]) * f);
+          for (int e = 0; e < 8; ++e) mx8[e] = fmaxf(mx8[e], fmaxf(__uint_as_float(s_[c][e]), __uint_as_float(s_[c][8 + e])));
+        const float mx = fmaxf(fmaxf(fmaxf(mx8[0], mx8[1]), fmaxf(mx8[2], mx8[3])), fmaxf(fmaxf(mx8[4], mx8[5]), fmaxf(mx8[6], mx8[7]))) *
+                         g.scale_log2e;
+        // (a row above the limit has a score of at least m + tau - 6)
+        const bool grow = mx > m_ref + (CF::kTakeMax ? kTau<T> : 0.5f * kTau<T>) || (m_ref == -INFINITY && mx > -INFINITY);
+        if (__any_sync(0xffffffffu, grow)) {
+          const float m_new = grow ? mx : m_ref;
+          const float f = (m_ref == -INFINITY) ? 0.f : ex2(m_ref - m_new);   // 1 for the rows that do not move
+          l_sum *= f;
+          m_ref = m_new;
+          if (it >= G) {
+            // multiply this row of the group's O accumulator by f, once its previous P V product is complete
+            const int pb = (it - G) % kFwdSBufs;
+            ok = mbar_wait(bar_pv_done(pb), ((it - G) / kFwdSBufs) & 1, abort_flag, t.status, wait_code(KFWD, 8));
+            ok = __all_sync(0xffffffffu, ok);
+            if (!ok) break;
+            tc_fence_after_sync();
+#pragma unroll
+            for (int c = 0; c < D / 16; ++c) {
+              if (16 * c >= g.D) break;       // padding columns (uniform)
+              uint32_t o_[16];
+              tmem_ld16(oacc + 16 * c, o_);
+              tmem_ld_wait(o_);
+              uint32_t lo8[8], hi8[8];
+#pragma unroll
+              for (int e = 0; e < 8; ++e) {
+                lo8[e] = __float_as_uint(__uint_as_float(o_[e]) * f);
+                hi8[e] = __float_as_uint(__uint_as_float(o_[8 + e]) * f);
+              }
+              tmem_st8(oacc + 16 * c, lo8);
+              tmem_st8(oacc + 16 * c + 8, hi8);
             }
-            tmem_st8(oacc + 16 * c, lo8);
-            tmem_st8(oacc + 16 * c + 8, hi8);
           }
         }
+        exponentials((m_ref == -INFINITY) ? 0.f : -m_ref);    // no visible key yet: every score is -inf, every p 0
       }
-      const float nm = (m_ref == -INFINITY) ? 0.f : -m_ref;    // no visible key yet: every p below is masked to 0
-      const float2 sc2 = make_float2(g.scale_log2e, g.scale_log2e), nm2 = make_float2(nm, nm);
-      float2 sum_a = make_float2(0.f, 0.f), sum_b = make_float2(0.f, 0.f);
-#pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        uint32_t kp[8];
-#pragma unroll
-        for (int e = 0; e < 16; e += 4) {
-          const float2 xa = __ffma2_rn(make_float2(__uint_as_float(s_[c][e]), __uint_as_float(s_[c][e + 1])), sc2, nm2);
-          const float2 xb = __ffma2_rn(make_float2(__uint_as_float(s_[c][e + 2]), __uint_as_float(s_[c][e + 3])), sc2, nm2);
-          const float2 pa = make_float2(ex2(xa.x), ex2(xa.y)), pb = make_float2(ex2(xb.x), ex2(xb.y));
-          sum_a = __fadd2_rn(sum_a, pa);
-          sum_b = __fadd2_rn(sum_b, pb);
-          kp[e >> 1] = Pack<T>::pack(pa.x, pa.y);
-          kp[(e >> 1) + 1] = Pack<T>::pack(pb.x, pb.y);
-        }
-        tmem_st8(sbuf + 8 * c, kp);      // over score columns this thread has read
-      }
-      l_sum += (sum_a.x + sum_a.y) + (sum_b.x + sum_b.y);
+      l_sum += tile_sum;
       tmem_st_wait();
       tc_fence_before_sync();
       __syncwarp();
@@ -526,12 +550,10 @@ static cudaError_t launch_fwd_one(const TmaMaps& maps, const Geometry& g_in, con
   Geometry g = g_in;
   const long long ctas = (long long)g.BH * ((g.N_q + BM - 1) / BM);
   g.head_group = pick_head_group(ctas, g.BH, 2ll * g.N_kv * g.D * 2);   // K, V
-  if constexpr (D == 64) {
-    if (two_per_sm_pays(g, false, 850.f, 850.f)) {
-      using CF = FwdCfg<D, 1>;
-      static std::atomic<unsigned long long> smem_set{0};
-      return launch_two_per_sm(fwd_kernel<D, T, false, 1>, maps, g, t, s, ctas, CF::kThreads, CF::kSmemBytes, smem_set);
-    }
+  if (two_per_sm_pays(g, false, true, 850.f, 850.f)) {
+    using CF = FwdCfg<D, 1>;
+    static std::atomic<unsigned long long> smem_set{0};
+    return launch_two_per_sm(fwd_kernel<D, T, false, 1>, maps, g, t, s, ctas, CF::kThreads, CF::kSmemBytes, smem_set);
   }
   using CF = FwdCfg<D, 2>;
   static TileKernelState state;

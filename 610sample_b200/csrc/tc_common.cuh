@@ -264,18 +264,22 @@ inline cudaError_t launch_tiles(void (*whole)(P...), void (*shared)(P...), const
   return e != cudaSuccess ? e : launch_pdl_cluster(kern, (unsigned)(units * g.split), threads, smem, (unsigned)g.split, s, maps, g, t);
 }
 
-// Two CTAs per SM, each with half of the tensor memory and one group of math warps (D = 64, where
-// that is enough): while one sets up, fills its pipeline or writes its result, the other computes.
-// A CTA costs kCtaClocks besides its tiles, a third of its time at 17 tiles of 64 keys; of that about
-// 4 thousand remain.  But a CTA then takes twice as long for a tile, so the longest one must not become
-// the bound: few CTAs stay one to an SM.  B8 H12 N2048 D64 causal: forward 117 -> 96 us, backward 324
-// -> 267; B2 H16 N8192: 406 -> 389 and 1251 -> 1157.
-inline bool two_per_sm_pays(const Geometry& g, bool col, float tile_clocks, float tile_clocks_two) {
+// Two CTAs per SM, each with half of the tensor memory and one group of math warps (the forward, and
+// the first backward at D = 64, where that is enough): while one sets up, fills its pipeline or writes
+// its result, the other computes.  A CTA costs kCtaClocks besides its tiles, a third of its time at 17
+// tiles of 64 keys; of that about 4 thousand remain.  But a CTA then takes twice as long for a tile, so
+// the longest one must not become the bound: few CTAs stay one to an SM.  Equal CTAs, one to an SM and
+// with no other kernel to fill up with (`alone`), run in whole waves.
+// B8 H12 N2048 D64 causal: forward 117 -> 92 us, backward 324 -> 267; B4 H16 N1024 D128 forward 36 ->
+// 25; B4 H16 N4096 D128 280 -> 253; B2 H8 N2048 D128 without mask (256 CTAs) 40 -> 36.
+inline bool two_per_sm_pays(const Geometry& g, bool col, bool alone, float tile_clocks, float tile_clocks_two) {
   const SplitLoad w = stream_load(g, col, tile_clocks);
   if (w.units < kSms) return false;
   auto larger = [](float x, float y) { return x > y ? x : y; };
-  const float one = larger(w.longest * tile_clocks + kCtaClocks, w.units / kSms * (w.mean * tile_clocks + kCtaClocks));
-  const float two = larger(2.f * w.longest * tile_clocks_two + kCtaClocks, w.units / kSms * (w.mean * tile_clocks_two + 4000.f));
+  const float per_sm = w.units / kSms;
+  const float waves = alone && w.mean > 0.9f * w.longest ? (float)(int)(per_sm + 0.999f) : per_sm;
+  const float one = larger(w.longest * tile_clocks + kCtaClocks, waves * (w.mean * tile_clocks + kCtaClocks));
+  const float two = larger(2.f * w.longest * tile_clocks_two + kCtaClocks, per_sm * (w.mean * tile_clocks_two + 4000.f));
   return two < 0.95f * one;
 }
 

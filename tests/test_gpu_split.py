@@ -28,6 +28,8 @@ capi = importlib.import_module("610sample_b200.capi")
     (8, 40, 129, 129, 64, 129, 0, 0),        # two CTAs per SM, one row in every second tile
     (4, 50, 300, 520, 48, 200, 1, 0),        # the same with padding, a window and keys nobody sees
     (6, 50, 60, 190, 64, 190, 0, 1),         # one tile per head
+    (5, 40, 200, 200, 128, 200, 0, 0),       # two forward CTAs per SM, Q in shared memory
+    (4, 40, 190, 500, 80, 130, 1, 0),        # the same with padding and a window
 ])
 def test_few_and_many_tiles_match_the_oracle(B, H, N_q, N_kv, D, window, chunk, mask, dtype):
     inp = orc.make_inputs(B, H, N_q, N_kv, D, seed=N_q + N_kv, dtype=dtype)
@@ -46,3 +48,24 @@ def test_few_and_many_tiles_match_the_oracle(B, H, N_q, N_kv, D, window, chunk, 
         # the bound of the other parity tests: 2e-2 of the largest value (half-precision operands P and dS, rounded results)
         assert float((got.double().cpu() - r).abs().max()) <= 2e-2 * max(1.0, float(r.abs().max())), n
     assert capi.device_status() == 0
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("H,N,D", [(2, 700, 64), (2, 700, 128), (120, 513, 64), (100, 385, 128)])
+def test_forward_when_scores_grow_along_the_keys(H, N, D, dtype):
+    """Keys that grow with their position make the reference exponent of most rows too low again and
+    again (score maxima move by some 40 log2 units), in every variant of the forward."""
+    inp = orc.make_inputs(1, H, N, N, D, seed=H + D, dtype=torch.float32)
+    K = (inp["K"] * torch.linspace(0.1, 10.0, N).view(1, 1, N, 1)).to(dtype)
+    Q, V = inp["Q"].to(dtype), inp["V"].to(dtype)
+    for mask in (0, 1):
+        O, L = tcapi.forward(Q.cuda(), K.cuda(), V.cuda(), N, 0, mask)
+        S = torch.einsum("bhid,bhjd->bhij", Q.cuda().double(), K.cuda().double()) / D ** 0.5
+        if mask == 0:
+            S = S.masked_fill(torch.ones(N, N, device="cuda").triu(1).bool(), float("-inf"))
+        want_L = torch.logsumexp(S, -1)
+        want_O = torch.softmax(S, -1) @ V.cuda().double()
+        # L: fp32 sums; O: P rounded to the type (relative 2^-9 or 2^-12 of a convex combination of V) and the result
+        assert torch.allclose(L.double(), want_L, rtol=1e-5, atol=1e-4), mask
+        tol = {torch.bfloat16: 2 ** -7, torch.float16: 2 ** -10}[dtype]
+        assert float((O.double() - want_O).abs().max()) <= tol * float(V.double().abs().max()), mask
