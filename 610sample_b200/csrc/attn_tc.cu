@@ -240,8 +240,8 @@ static bool encode_map(CUtensorMap* map, const void* ptr, int is_bf16, long long
 
 // The maps an operation uses; the others are left alone.
 bool encode_maps(TmaMaps* maps, int op, const Geometry& g, const Tensors& t, int is_bf16, const char** err) {
-  const void* ins[T_COUNT] = {t.Q, t.K, t.V, t.dO, t.g_dQ, t.g_dK, t.g_dV};
-  const int in_rows[T_COUNT] = {g.N_q, g.N_kv, g.N_kv, g.N_q, g.N_q, g.N_kv, g.N_kv};
+  const void* ins[T_COUNT] = {t.Q, t.K, t.V, t.dO, t.g_dQ, t.g_dK, t.g_dV, t.O};
+  const int in_rows[T_COUNT] = {g.N_q, g.N_kv, g.N_kv, g.N_q, g.N_q, g.N_kv, g.N_kv, g.N_q};
   const int n_in = op == OP_FORWARD ? 3 : op == OP_BACKWARD ? 4 : T_COUNT;
   // outputs, stored by TMA in boxes of 64 columns x 128 rows
   void* outs[TO_COUNT] = {nullptr, nullptr, nullptr, nullptr};

@@ -145,10 +145,10 @@ fb_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Tensors 
     pdl_trigger();
     if (part == 0) {
       if constexpr (CF::kCol) {
-        zero_rows(t.out_dK, bh, r0, g.N_kv, g.D);
-        zero_rows(t.out_dV, bh, r0, g.N_kv, g.D);
+        zero_rows(t.out_dK, bh, r0, g.N_kv, g.D, blockDim.x);
+        zero_rows(t.out_dV, bh, r0, g.N_kv, g.D, blockDim.x);
       } else {
-        zero_rows(t.out_dQ, bh, r0, g.N_q, g.D);
+        zero_rows(t.out_dQ, bh, r0, g.N_q, g.D, blockDim.x);
       }
     }
     pdl_end(g);

@@ -133,7 +133,7 @@ fwd_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Tensors
     pdl_begin(g);
     pdl_trigger();
     if (part == 0) {
-      zero_rows(t.out_O, bh, r0, g.N_q, g.D);
+      zero_rows(t.out_O, bh, r0, g.N_q, g.D, blockDim.x);
       if (threadIdx.x < BM && r0 + threadIdx.x < g.N_q) t.out_L[(size_t)bh * g.N_q + r0 + threadIdx.x] = -INFINITY;
     }
     pdl_end(g);

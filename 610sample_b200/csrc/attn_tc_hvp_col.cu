@@ -127,8 +127,8 @@ hvp_col_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Ten
     pdl_begin(g);
     pdl_trigger();
     if (part == 0) {
-      zero_rows(t.out_g_K, bh, r0, g.N_kv, g.D);
-      zero_rows(t.out_g_V, bh, r0, g.N_kv, g.D);
+      zero_rows(t.out_g_K, bh, r0, g.N_kv, g.D, blockDim.x);
+      zero_rows(t.out_g_V, bh, r0, g.N_kv, g.D, blockDim.x);
     }
     pdl_end(g);
     return;

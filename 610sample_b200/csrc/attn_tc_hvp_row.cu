@@ -11,7 +11,7 @@
 //   ROW_Q      g_Q = s (dS g_dK + g_S K), given the scalars
 //
 // Both stream K, g_dK, V, g_dV in 64-row tiles (three TMA stages, six at D = 64) past 128 stationary
-// rows of Q, dO, g_dQ.  Q and dO are copied once into TENSOR MEMORY and used from there
+// rows of Q, dO, g_dQ.  Q and dO are copied into TENSOR MEMORY and used from there
 // as the A operand of their score products (an A operand in shared memory is re-read by
 // every MMA instruction: measured 48 instead of 32 clocks for an N = 64 product); g_dQ
 // stays in shared memory.
@@ -31,6 +31,11 @@
 // clocks even when satisfied) fell on an empty tensor pipe.  At D = 64 tensor memory has room for
 // a second RB region and the RB products run a tile ahead of the outputs.  The result tile leaves
 // through shared memory and a TMA store, which clips rows and columns beyond the tensor.
+// Where there are more tiles of queries than SMs the CTAs are persistent (tc_common.cuh) and the stages
+// a ring that runs on from one tile of queries to the next: its Q and dO tiles take an entry like a
+// streamed tile, and so does its result (the g_dO pass has O loaded there and subtracts in place).  What
+// remains of a CTA's fixed cost is the hand-over at the end of an item: B8 H12 N2048 D64 scalar pass 204 ->
+// 183 us, g_Q pass 198 -> 179; B4 H16 N1024 D128 87 -> 75 and 82 -> 78; N4096 755 -> 709 (g_Q unchanged).
 // Formulas: reference csrc/flash_double_backward_v7.cu:1257-1454.
 #include "attn_launch.h"
 #include "tc_common.cuh"
@@ -46,8 +51,9 @@ constexpr int kRowThreads = 352;    // 8 math warps, TMA producer, two MMA issue
 constexpr int kRowMaxStages = 6;
 
 struct RowControl {
+  WorkControl work;
   uint64_t stat_full;          // g_dQ tile in shared memory
-  uint64_t staging_full;       // Q and dO tiles in the staging buffer (the last stage)
+  uint64_t stat_empty;         // the RA products of an item's last tile have read it
   uint64_t stat_tmem_ready;    // Q and dO copied to tensor memory
   // a stage has two halves with their own barriers: [K, g_dK] (index 0) and [V, g_dV] (index 1)
   uint64_t stream_full[2][kRowMaxStages];
@@ -102,7 +108,7 @@ struct RowCfg {
   }
 };
 
-template <int MODE, int D, typename T, bool SPLIT>
+template <int MODE, int D, typename T, bool SPLIT, bool PERSIST>
 __global__ void __launch_bounds__(kRowThreads, 1)
 hvp_row_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Tensors t) {
   using CF = RowCfg<D>;
@@ -125,14 +131,11 @@ hvp_row_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Ten
   const uint32_t stat_base = smem_base;
   const uint32_t strm_base = stat_base + CF::kStatBytes;
   const uint32_t aux_off = CF::kStatBytes + CF::kStages * CF::kStageBytes;
-  const uint32_t staging = strm_base + (CF::kStages - 1) * CF::kStageBytes;   // Q then dO, before the last stage is used
   RowControl* ctl = reinterpret_cast<RowControl*>(smem_gen + aux_off);
-  // [2 halves][4][128] floats of row sums, exchanged after the last product has read the
-  // g_dQ tile: its shared memory is reused
-  float* row_sums = reinterpret_cast<float*>(smem_gen);
-  // a split tile: this part's four sums per row and the total dot2 behind them, its result tile over
+  // a split tile: over the g_dQ tile, which the last product has read, the row sums' exchange
+  // ([2 halves][4][128] floats), this part's four sums per row and the total dot2; its result tile over
   // the stream stages
-  float* part_sums = row_sums + 2 * 4 * BM;       // [4][128]
+  float* part_sums = reinterpret_cast<float*>(smem_gen) + 2 * 4 * BM;       // [4][128]
   float* part_dot2 = part_sums + 4 * BM;
   float* partial = reinterpret_cast<float*>(smem_gen + CF::kStatBytes);
 
@@ -140,35 +143,44 @@ hvp_row_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Ten
   const int tiles = (g.N_q + BM - 1) / BM;
   const unsigned split = SPLIT ? (unsigned)g.split : 1u;      // CTAs that share this tile: a cluster (tc_common.cuh)
   const int part = SPLIT ? (int)(blockIdx.x % split) : 0;
-  int bh, rank;
-  tile_to_head_and_rank(g, blockIdx.x / split, tiles, bh, rank);
-  const int tile = (g.mask_mode != 0) ? rank : (tiles - 1 - rank);   // heavy tiles first
-  const int r0 = tile * BM;
-
-  int lo, hi;
-  key_range_for_queries(g, r0, r0 + BM, lo, hi);
-  int t_begin = lo / BN;
-  int n_iter = (hi > lo) ? ((hi + BN - 1) / BN - t_begin) : 0;
-  if (n_iter == 0) {       // nothing to visit
-    pdl_begin(g);
-    pdl_trigger();
-    if (part == 0) {
-      zero_rows(MODE == ROW_PREDO ? t.out_g_dO : t.out_g_Q, bh, r0, g.N_q, g.D);
-      if constexpr (MODE == ROW_PREDO) {
-        const int r = r0 + threadIdx.x;
-        if (threadIdx.x < BM && r < g.N_q) {
-          const size_t at = (size_t)bh * g.N_q + r;
-          t.Dv[at] = t.dot2[at] = t.dot3[at] = 0.f;
-        }
+  struct Item { int bh, r0, t_begin, n_iter; };
+  auto item_of = [&](int unit) {
+    Item w;
+    int rank;
+    tile_to_head_and_rank(g, (unsigned)unit, tiles, w.bh, rank);
+    w.r0 = ((g.mask_mode != 0) ? rank : (tiles - 1 - rank)) * BM;   // heavy tiles first
+    int lo, hi;
+    key_range_for_queries(g, w.r0, w.r0 + BM, lo, hi);
+    w.t_begin = lo / BN;
+    w.n_iter = (hi > lo) ? ((hi + BN - 1) / BN - w.t_begin) : 0;
+    return w;
+  };
+  const int first_unit = (int)(blockIdx.x / split);
+  Item w = item_of(first_unit);
+  // rows that see nothing
+  auto write_zeros = [&](const Item& w, int threads) {
+    zero_rows(MODE == ROW_PREDO ? t.out_g_dO : t.out_g_Q, w.bh, w.r0, g.N_q, g.D, threads);
+    if constexpr (MODE == ROW_PREDO) {
+      const int r = w.r0 + threadIdx.x;
+      if (threadIdx.x < BM && r < g.N_q) {
+        const size_t at = (size_t)w.bh * g.N_q + r;
+        t.Dv[at] = t.dot2[at] = t.dot3[at] = 0.f;
       }
     }
-    pdl_end(g);
-    return;
+  };
+  if constexpr (SPLIT) {
+    if (w.n_iter == 0) {
+      pdl_begin(g);
+      pdl_trigger();
+      if (part == 0) write_zeros(w, kRowThreads);
+      pdl_end(g);
+      return;
+    }
+    take_share((int)split, part, w.t_begin, w.n_iter);      // may be none
   }
-  if constexpr (SPLIT) take_share((int)split, part, t_begin, n_iter);      // may be none
 
   const uint32_t bar_stat_full = smem_u32(&ctl->stat_full);
-  const uint32_t bar_staging_full = smem_u32(&ctl->staging_full);
+  const uint32_t bar_stat_empty = smem_u32(&ctl->stat_empty);
   const uint32_t bar_stat_tmem_ready = smem_u32(&ctl->stat_tmem_ready);
   const uint32_t bar_ra_full = smem_u32(&ctl->ra_full), bar_ra_free = smem_u32(&ctl->ra_free);
   auto bar_rb_full = [&](int b) { return smem_u32(&ctl->rb_full[b]); };
@@ -179,15 +191,52 @@ hvp_row_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Ten
   auto bar_stream_full = [&](int h, int s) { return smem_u32(&ctl->stream_full[h][s]); };
   auto bar_stream_empty = [&](int h, int s) { return smem_u32(&ctl->stream_empty[h][s]); };
 
+  // The ring of stages.  Every item takes an entry for its Q and dO tiles (halves 0 and 1, copied to
+  // tensor memory by the math warps and free again when they have said so), one for each of its tiles,
+  // and one through which its result leaves (half 0; the g_dO pass first receives O there).  Entries are
+  // numbered over all items of the CTA.
+  constexpr int S = CF::kStages;
+  auto slot_base = [&](int c) { return strm_base + (uint32_t)(c % S) * CF::kStageBytes; };
+  constexpr uint32_t kHalfBytes = CF::kStageBytes / 2;
+  auto entries = [](const Item& w) { return w.n_iter > 0 ? w.n_iter + (SPLIT ? 1 : 2) : 0; };
+  auto load_rows128 = [&](uint32_t dst, int tensor, const Item& w, uint32_t bar) {      // a [128][D] tile of the query side
+#pragma unroll
+    for (int a = 0; a < kAtoms; ++a)
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+        tma_load_3d(dst + a * kAtomBytesStat + h * kAtomBytesStrm, &maps.m[tensor], a * 64, w.r0 + h * 64, w.bh, bar);
+  };
+  auto load_stationary = [&](const Item& w, int c) {
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      mbar_arrive_expect_tx(bar_stream_full(h, c % S), kHalfBytes);
+      load_rows128(slot_base(c) + h * kHalfBytes, h == 0 ? T_Q : T_dO, w, bar_stream_full(h, c % S));
+    }
+  };
+  auto load_tile_half = [&](const Item& w, int it, int h, int c) {
+    mbar_arrive_expect_tx(bar_stream_full(h, c % S), kHalfBytes);
+#pragma unroll
+    for (int s2 = 0; s2 < 2; ++s2)
+#pragma unroll
+      for (int a = 0; a < kAtoms; ++a)
+        tma_load_3d(slot_base(c) + CF::stream_off(2 * h + s2, a), &maps.m[CF::stream_tensor(2 * h + s2)], a * 64, (w.t_begin + it) * BN,
+                    w.bh, bar_stream_full(h, c % S));
+  };
+  auto load_gdq = [&](const Item& w) {
+    mbar_arrive_expect_tx(bar_stat_full, CF::kStatBytes);
+    load_rows128(stat_base, T_gQ, w, bar_stat_full);
+  };
+
   // one barrier round of set-up: the producer initialises the mbarriers and, once the kernels this
   // one depends on are complete, requests the stationary tiles and the first streamed tile (their
   // latency is the longest item of the prologue); meanwhile an issuing warp allocates tensor memory
   if (warp == kProducerWarp && lane == 0) {
     for (int i = 0; i < T_COUNT; ++i) tma_prefetch_desc(&maps.m[i]);
+    work_init(&ctl->work);
     mbar_init(bar_stat_full, 1);
-    mbar_init(bar_staging_full, 1);
+    mbar_init(bar_stat_empty, 1);
     mbar_init(bar_stat_tmem_ready, kMathWarps);
-    for (int s = 0; s < CF::kStages; ++s) {
+    for (int s = 0; s < S; ++s) {
       for (int h = 0; h < 2; ++h) {
         mbar_init(bar_stream_full(h, s), 1);
         mbar_init(bar_stream_empty(h, s), 1);
@@ -208,32 +257,14 @@ hvp_row_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Ten
   }
   if (warp == kRowMmaWarp) tmem_alloc(smem_u32(&ctl->tmem_base), kTmemCols);
   pdl_begin(g);
-  if (warp == kProducerWarp && lane == 0) pdl_trigger();
-  if (warp == kProducerWarp && lane == 0 && n_iter > 0) {
-    mbar_arrive_expect_tx(bar_staging_full, CF::kStageBytes);
-#pragma unroll
-    for (int x = 0; x < 2; ++x)       // Q then dO: they are copied to tensor memory first
-#pragma unroll
-      for (int a = 0; a < kAtoms; ++a)
-#pragma unroll
-        for (int h = 0; h < 2; ++h)
-          tma_load_3d(staging + (x * kAtoms + a) * kAtomBytesStat + h * kAtomBytesStrm, &maps.m[x == 0 ? T_Q : T_dO],
-                      a * 64, r0 + h * 64, bh, bar_staging_full);
-    mbar_arrive_expect_tx(bar_stream_full(0, 0), CF::kStageBytes / 2);
-    mbar_arrive_expect_tx(bar_stream_full(1, 0), CF::kStageBytes / 2);
-#pragma unroll
-    for (int sl = 0; sl < CF::kNStream; ++sl)
-#pragma unroll
-      for (int a = 0; a < kAtoms; ++a)
-        tma_load_3d(strm_base + CF::stream_off(sl, a), &maps.m[CF::stream_tensor(sl)], a * 64, t_begin * BN, bh,
-                    bar_stream_full(sl >> 1, 0));
-    mbar_arrive_expect_tx(bar_stat_full, CF::kStatBytes);
-#pragma unroll
-    for (int a = 0; a < kAtoms; ++a)
-#pragma unroll
-      for (int h = 0; h < 2; ++h)
-        tma_load_3d(stat_base + a * kAtomBytesStat + h * kAtomBytesStrm, &maps.m[T_gQ], a * 64, r0 + h * 64, bh,
-                    bar_stat_full);
+  if (warp == kProducerWarp && lane == 0) {
+    pdl_trigger();
+    if (w.n_iter > 0) {
+      load_stationary(w, 0);
+      load_tile_half(w, 0, 0, 1);
+      load_tile_half(w, 0, 1, 1);
+      load_gdq(w);
+    }
   }
   tc_fence_before_sync();
   __syncthreads();
@@ -245,31 +276,60 @@ hvp_row_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Ten
   // TMA producer
   // =========================================================================
   if (warp == kProducerWarp) {
-    if (lane == 0 && n_iter > 0) {
+    if (lane == 0) {
       bool ok = true;
-      // The two halves of a stage are released at different times: [K, g_dK] is last read by the
-      // RA products in the scalar pass (long before the outputs of the tile), [V, g_dV] by the RB
-      // products in the g_Q pass.  Each half is requested as soon as its own buffer is free, so the
-      // loads the first issuing warp waits for leave a tile earlier than a whole-stage release would
-      // allow (a load takes about as long as a tile).
-      for (int it = 1; it < n_iter; ++it) {     // tile 0 was requested above
-        const int st = it % CF::kStages;
-        const uint32_t stage = strm_base + st * CF::kStageBytes;
+      int c0 = 0, items = 0;        // ring entries and items with tiles before this item
+      auto wait_half = [&](int h, int c) {
+        return mbar_wait(bar_stream_empty(h, c % S), ((c / S) & 1) ^ 1, abort_flag, t.status, wait_code(KIND, 1));
+      };
+      for (int k = 0; ok; ++k) {
+        int asked = 0;
+        if (w.n_iter > 0) {
+          if (k > 0) {
+            ok = wait_half(0, c0) && wait_half(1, c0);
+            if (!ok) break;
+            load_stationary(w, c0);
+          }
+          // The two halves of an entry are released at different times: [K, g_dK] is last read by the RA
+          // products in the scalar pass (long before the outputs of the tile), [V, g_dV] by the RB
+          // products in the g_Q pass.  Each half is requested as soon as its own buffer is free, so the
+          // loads the first issuing warp waits for leave a tile earlier than a whole-stage release would
+          // allow (a load takes about as long as a tile).
+          for (int it = k > 0 ? 0 : 1; it < w.n_iter && ok; ++it) {     // the first item's first tile was requested above
+            const int c = c0 + 1 + it;
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          ok = mbar_wait(bar_stream_empty(h, st), ((it / CF::kStages) & 1) ^ 1, abort_flag, t.status, wait_code(KIND, 1));
-          // the last stage doubles as the staging buffer of Q and dO until they are in tensor memory
-          if (ok && it == CF::kStages - 1) ok = mbar_wait(bar_stat_tmem_ready, 0, abort_flag, t.status, wait_code(KIND, 10));
+            for (int h = 0; h < 2; ++h) {
+              if (ok) ok = wait_half(h, c);
+              if (ok) load_tile_half(w, it, h, c);
+            }
+            if (ok && it == 0) {
+              ok = mbar_wait(bar_stat_empty, (items & 1) ^ 1, abort_flag, t.status, wait_code(KIND, 1));
+              if (ok) load_gdq(w);
+            }
+            if (PERSIST && asked == 0 && it + 3 >= w.n_iter) { work_request(&ctl->work); asked = 1; }
+          }
+          if (!SPLIT && ok) {       // the entry of the result
+            const int c = c0 + 1 + w.n_iter;
+            ok = wait_half(0, c) && wait_half(1, c);
+            if (!ok) break;
+            if constexpr (MODE == ROW_PREDO) {
+              mbar_arrive_expect_tx(bar_stream_full(0, c % S), kHalfBytes);
+              load_rows128(slot_base(c), T_O, w, bar_stream_full(0, c % S));
+            } else {
+              mbar_arrive(bar_stream_full(0, c % S));
+            }
+            mbar_arrive(bar_stream_full(1, c % S));
+          }
           if (!ok) break;
-          mbar_arrive_expect_tx(bar_stream_full(h, st), CF::kStageBytes / 2);
-#pragma unroll
-          for (int s2 = 0; s2 < 2; ++s2)
-#pragma unroll
-            for (int a = 0; a < kAtoms; ++a)
-              tma_load_3d(stage + CF::stream_off(2 * h + s2, a), &maps.m[CF::stream_tensor(2 * h + s2)], a * 64,
-                          (t_begin + it) * BN, bh, bar_stream_full(h, st));
+          ++items;
         }
-        if (!ok) break;
+        if (!PERSIST) break;
+        if (asked == 0) work_request(&ctl->work);
+        int unit;
+        c0 += entries(w);
+        ok = work_announce(&ctl->work, k, &unit, abort_flag, t.status, wait_code(KIND, 10));
+        if (!ok || unit < 0) break;
+        w = item_of(unit);
       }
       if (!ok) {   // give copies already in flight a bounded chance to land before the CTA exits
         const long long t0 = clock64();
@@ -281,11 +341,8 @@ hvp_row_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Ten
   // MMA issuers (converged warps, one elected lane issues)
   // =========================================================================
   else if (warp == kRowMmaWarp || warp == kRowMmaWarp + 1) {
-    if (n_iter > 0) {
-      bool ok = mbar_wait(bar_stat_full, 0, abort_flag, t.status, wait_code(KIND, 2));
-      if (ok) ok = mbar_wait(bar_stat_tmem_ready, 0, abort_flag, t.status, wait_code(KIND, 11));
-      ok = __all_sync(0xffffffffu, ok);
-      tc_fence_after_sync();
+    {
+      bool ok = true;
       const uint64_t d_stat = smem_desc_sw128(stat_base, 16, 1024);
       auto gq_desc = [&](int ks) {   // K-major A from shared memory: the g_dQ tile
         return d_stat + (uint64_t)(((ks >> 2) * kAtomBytesStat + (ks & 3) * 32) >> 4);
@@ -355,56 +412,86 @@ hvp_row_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Ten
       // other are queued.  The tensor pipe needs no order between the two streams: RA(j+1) only
       // waits for RA(j) to have been read, and RB(j+1) follows OUT(j), which reads RB, in the
       // second warp's own order.
-      auto wait_stream = [&](int h, int tile) {   // half h of the stage of `tile` has landed
-        return mbar_wait(bar_stream_full(h, tile % CF::kStages), (tile / CF::kStages) & 1, abort_flag, t.status, wait_code(KIND, 3));
+      auto wait_entry = [&](int h, int c) {   // half h of ring entry c has landed
+        return mbar_wait(bar_stream_full(h, c % S), (c / S) & 1, abort_flag, t.status, wait_code(KIND, 3));
       };
       // which issuing warp releases which half: the one whose products read it last
       constexpr bool kRaReleasesKG = (MODE == ROW_PREDO);   // scalar pass: the outputs read V, g_dV only
+      // Either warp's walk over the items: body(tiles, ring entry of the first tile, number of the first tile)
+      auto walk = [&](auto role, auto&& body) {
+        constexpr int kRole = decltype(role)::value;
+        int c0 = 0, g0 = 0, items = 0;      // ring entries, tiles and items with tiles before this item
+        for (int k = 0; ok; ++k) {
+          if (w.n_iter > 0) {
+            ok = mbar_wait(bar_stat_tmem_ready, items & 1, abort_flag, t.status, wait_code(KIND, 11));
+            if (ok && kRole == 0) ok = mbar_wait(bar_stat_full, items & 1, abort_flag, t.status, wait_code(KIND, 2));
+            ok = __all_sync(0xffffffffu, ok);
+            if (!ok) break;
+            tc_fence_after_sync();
+            if (lane == 0) mbar_arrive(bar_stream_empty(kRole, c0 % S));     // Q (first warp) and dO (second) are in tensor memory
+            body(w.n_iter, c0 + 1, g0);
+            g0 += w.n_iter;
+            ++items;
+          }
+          if (!PERSIST || !ok) break;
+          c0 += entries(w);
+          int unit;
+          ok = work_next(&ctl->work, k, &unit, abort_flag, t.status, wait_code(KIND, 14));
+          if (!ok || unit < 0) break;
+          w = item_of(unit);
+        }
+      };
       if (warp == kRowMmaWarp) {
         // ---- first warp: the RA products of every tile
-        for (int j = 0; j < n_iter && ok; ++j) {
-          ok = wait_stream(0, j);
-          if (ok && j > 0) ok = mbar_wait(bar_ra_free, (j - 1) & 1, abort_flag, t.status, wait_code(KIND, 4));
-          // ROW_Q keeps the pipe's order OUT(j-2), RB(j-1), RA(j): its second half-step is the long
-          // one, and RA(j) queued any earlier delays the outputs that half-step waits behind.  The
-          // scalar pass is faster with the two streams left to run freely (both measured).
-          if (MODE == ROW_Q && LA == 1 && ok && j > 0) ok = mbar_wait(bar_rb_issued(j - 1), ((j - 1) >> 1) & 1, abort_flag, t.status, wait_code(KIND, 13));
-          ok = __all_sync(0xffffffffu, ok);
-          if (!ok) break;
-          tc_fence_after_sync();
-          const uint32_t stage = strm_base + (j % CF::kStages) * CF::kStageBytes;
-          issue_ra(stage);
-          if (kRaReleasesKG) commit(bar_stream_empty(0, j % CF::kStages));
-        }
+        walk(Int<0>{}, [&](int n, int c1, int g0) {
+          for (int j = 0; j < n && ok; ++j) {
+            const int gj = g0 + j, c = c1 + j;
+            ok = wait_entry(0, c);
+            if (ok && gj > 0) ok = mbar_wait(bar_ra_free, (gj - 1) & 1, abort_flag, t.status, wait_code(KIND, 4));
+            // ROW_Q keeps the pipe's order OUT(j-2), RB(j-1), RA(j): its second half-step is the long
+            // one, and RA(j) queued any earlier delays the outputs that half-step waits behind.  The
+            // scalar pass is faster with the two streams left to run freely (both measured).
+            if (MODE == ROW_Q && LA == 1 && ok && gj > 0) ok = mbar_wait(bar_rb_issued(gj - 1), ((gj - 1) >> 1) & 1, abort_flag, t.status, wait_code(KIND, 13));
+            ok = __all_sync(0xffffffffu, ok);
+            if (!ok) break;
+            tc_fence_after_sync();
+            issue_ra(slot_base(c));
+            if (kRaReleasesKG) commit(bar_stream_empty(0, c % S));
+          }
+          if (ok) commit(bar_stat_empty);
+        });
       } else {
         // ---- second warp: RB products (LA tiles ahead) and outputs
-        for (int i = 0; i < LA && i < n_iter && ok; ++i) {
-          ok = wait_stream(1, i);
-          ok = __all_sync(0xffffffffu, ok);
-          if (!ok) break;
-          tc_fence_after_sync();
-          issue_rb(strm_base + (i % CF::kStages) * CF::kStageBytes, i % LA);
-          if (!kRaReleasesKG) commit(bar_stream_empty(1, i % CF::kStages));
-          if (LA == 1 && lane == 0) mbar_arrive(bar_rb_issued(i));
-        }
-        for (int j = 0; j < n_iter && ok; ++j) {
-          const int st = j % CF::kStages, b = j % LA;
-          const int nj = j + LA;
-          ok = mbar_wait(bar_op_full(b), (j / LA) & 1, abort_flag, t.status, wait_code(KIND, 6));
-          if (ok && nj < n_iter) ok = wait_stream(1, nj);
-          ok = __all_sync(0xffffffffu, ok);
-          if (!ok) break;
-          tc_fence_after_sync();
-          issue_out(strm_base + st * CF::kStageBytes, j == 0, b);
-          commit(bar_stream_empty(kRaReleasesKG ? 1 : 0, st));   // the half the outputs read
-          if (nj < n_iter) {
-            // buffer b again: after the outputs that read it, in this warp's own order
-            issue_rb(strm_base + (nj % CF::kStages) * CF::kStageBytes, b);
-            if (!kRaReleasesKG) commit(bar_stream_empty(1, nj % CF::kStages));
-            if (LA == 1 && lane == 0) mbar_arrive(bar_rb_issued(nj));
+        walk(Int<1>{}, [&](int n, int c1, int g0) {
+          for (int i = 0; i < LA && i < n && ok; ++i) {
+            const int c = c1 + i;
+            ok = wait_entry(1, c);
+            ok = __all_sync(0xffffffffu, ok);
+            if (!ok) break;
+            tc_fence_after_sync();
+            issue_rb(slot_base(c), (g0 + i) % LA);
+            if (!kRaReleasesKG) commit(bar_stream_empty(1, c % S));
+            if (LA == 1 && lane == 0) mbar_arrive(bar_rb_issued(g0 + i));
           }
-        }
-        if (ok) commit(bar_acc_done);
+          for (int j = 0; j < n && ok; ++j) {
+            const int gj = g0 + j, b = gj % LA, c = c1 + j, nc = c + LA;
+            const bool more = j + LA < n;
+            ok = mbar_wait(bar_op_full(b), (gj / LA) & 1, abort_flag, t.status, wait_code(KIND, 6));
+            if (ok && more) ok = wait_entry(1, nc);
+            ok = __all_sync(0xffffffffu, ok);
+            if (!ok) break;
+            tc_fence_after_sync();
+            issue_out(slot_base(c), j == 0, b);
+            commit(bar_stream_empty(kRaReleasesKG ? 1 : 0, c % S));   // the half the outputs read
+            if (more) {
+              // buffer b again: after the outputs that read it, in this warp's own order
+              issue_rb(slot_base(nc), b);
+              if (!kRaReleasesKG) commit(bar_stream_empty(1, nc % S));
+              if (LA == 1 && lane == 0) mbar_arrive(bar_rb_issued(gj + LA));
+            }
+          }
+          if (ok) commit(bar_acc_done);
+        });
       }
     }
   }
@@ -414,9 +501,22 @@ hvp_row_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Ten
   else {
     const int quarter = warp & 3, half = warp >> 2;
     const int row = quarter * 32 + lane;
-    const int gidx = r0 + row;
     const uint32_t lane_addr = tmem_base + ((uint32_t)(quarter * 32) << 16);
+    bool ok = true;
+    int c0 = 0, g0 = 0, items = 0;      // ring entries, tiles and items with tiles before this item
+    for (int k = 0; ok; ++k) {
+    const int n_iter = w.n_iter, t_begin = w.t_begin, bh = w.bh, r0 = w.r0;
+    if (!SPLIT && n_iter == 0) {
+      write_zeros(w, kMathThreads);
+    } else {
+    const int gidx = r0 + row;
     const size_t row_off = (size_t)bh * g.N_q;
+    // where the result leaves: its ring entry (a split tile has no such entry and does not use it)
+    const int c_out = c0 + 1 + n_iter;
+    const uint32_t out_tile = slot_base(c_out);
+    float* row_sums = SPLIT ? reinterpret_cast<float*>(smem_gen)
+                            : reinterpret_cast<float*>(smem_gen + (out_tile - smem_base) + kHalfBytes);    // the entry's other half
+    (void)row_sums; (void)out_tile;
 
     int vlo, vhi;
     key_range_for_queries(g, gidx, gidx + 1, vlo, vhi);
@@ -439,19 +539,21 @@ hvp_row_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Ten
     const float2 sc2 = make_float2(g.scale, g.scale);
     const float2 zero2 = make_float2(0.f, 0.f);
 
-    // ---- one-time copy of the stationary Q and dO rows from the staging buffer to tensor memory.
+    // ---- copy of the stationary Q and dO rows from their ring entry to tensor memory.
     // Tile layout in shared memory: per 64-column atom, row r at r*128 bytes with its 16-byte
     // chunks XOR-swizzled by r % 8.  Tensor-memory layout of an A operand: lane = row, one
     // 32-bit column per pair of consecutive K elements.  This thread moves its row's half.
-    bool ok = true;
     if (n_iter > 0) {
-      ok = mbar_wait(bar_staging_full, 0, abort_flag, t.status, wait_code(KIND, 12));
+      const uint32_t staging = slot_base(c0);
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+        if (ok) ok = mbar_wait(bar_stream_full(h, c0 % S), (c0 / S) & 1, abort_flag, t.status, wait_code(KIND, 12));
       ok = __all_sync(0xffffffffu, ok);
       if (ok) {
         constexpr int kChunksPerHalf = D / 16;    // 16-byte chunks (8 halves) of this thread's half row
 #pragma unroll
         for (int x = 0; x < 2; ++x) {             // 0: Q, 1: dO
-          const uint32_t src = staging + x * kAtoms * kAtomBytesStat;
+          const uint32_t src = staging + x * kHalfBytes;
           const uint32_t dst = lane_addr + (x == 0 ? CF::kQT : CF::kDOT);
 #pragma unroll
           for (int c = 0; c < kChunksPerHalf; c += 2) {
@@ -478,13 +580,14 @@ hvp_row_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Ten
     float2 acc_D = zero2, acc_2 = zero2, acc_A = zero2, acc_E = zero2;   // ROW_PREDO row sums
     const uint32_t ra = lane_addr + CF::kRA;
     for (int it = 0; it < n_iter && ok; ++it) {
-      const uint32_t rb = lane_addr + CF::kRB + 128u * (uint32_t)(it % LA);
+      const int gi = g0 + it;
+      const uint32_t rb = lane_addr + CF::kRB + 128u * (uint32_t)(gi % LA);
       const int j0 = (t_begin + it) * BN;
       const int first = j0 + half * 32;
       const bool masked = !(first >= vlo && first + 31 < vhi);
 
       // ---------------- half-step 1: RA ------------------------------------------
-      ok = mbar_wait(bar_ra_full, it & 1, abort_flag, t.status, wait_code(KIND, 7));
+      ok = mbar_wait(bar_ra_full, gi & 1, abort_flag, t.status, wait_code(KIND, 7));
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
       tc_fence_after_sync();
@@ -527,7 +630,7 @@ hvp_row_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Ten
       }
 
       // ---------------- half-step 2: RB ------------------------------------------
-      ok = mbar_wait(bar_rb_full(it % LA), (it / LA) & 1, abort_flag, t.status, wait_code(KIND, 8));
+      ok = mbar_wait(bar_rb_full(gi % LA), (gi / LA) & 1, abort_flag, t.status, wait_code(KIND, 8));
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
       tc_fence_after_sync();
@@ -566,11 +669,15 @@ hvp_row_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Ten
       tmem_st_wait();
       tc_fence_before_sync();
       __syncwarp();
-      if (lane == 0) mbar_arrive(bar_op_full(it % LA));
+      if (lane == 0) mbar_arrive(bar_op_full(gi % LA));
     }
 
     // ---------------- results ------------------------------------------------------
     float dot2_row = 0.f;
+    if constexpr (!SPLIT) {       // the ring entry of the result is free, in the g_dO pass with O in it
+      if (ok) ok = mbar_wait(bar_stream_full(0, c_out % S), (c_out / S) & 1, abort_flag, t.status, wait_code(KIND, 12));
+      ok = __all_sync(0xffffffffu, ok);
+    }
     if constexpr (MODE == ROW_PREDO) {
       // each row is summed by two threads (column halves): exchange through shared memory
       float* mine = row_sums + half * 512;
@@ -592,21 +699,7 @@ hvp_row_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Ten
     constexpr int kColsPerHalf = D / 2;
     constexpr int kChunks = kColsPerHalf / 16;
     const float mul = (MODE == ROW_PREDO) ? 1.f : g.scale;
-    // D is the padded head dimension of the tiles; the tensors in global memory have g.D columns
-    const size_t elem0 = ((size_t)bh * g.N_q + gidx) * g.D + half * kColsPerHalf;
-    // g_dO = g_dO' - dot2 * O: this thread's part of the O row is fetched while the last
-    // products are still running
-    uint4 o_[MODE == ROW_PREDO ? 2 * kChunks : 1];
-    if constexpr (MODE == ROW_PREDO) {
-#pragma unroll
-      for (int ch = 0; ch < kChunks; ++ch) {
-        const bool in = !SPLIT && gidx < g.N_q && half * kColsPerHalf + ch * 16 < g.D;
-        const uint4* orow = reinterpret_cast<const uint4*>((const T*)t.O + elem0 + ch * 16);
-        o_[2 * ch] = in ? __ldg(orow) : make_uint4(0u, 0u, 0u, 0u);
-        o_[2 * ch + 1] = in ? __ldg(orow + 1) : make_uint4(0u, 0u, 0u, 0u);
-      }
-    }
-    if (n_iter > 0 && ok) ok = mbar_wait(bar_acc_done, 0, abort_flag, t.status, wait_code(KIND, 9));
+    if (n_iter > 0 && ok) ok = mbar_wait(bar_acc_done, items & 1, abort_flag, t.status, wait_code(KIND, 9));
     ok = __all_sync(0xffffffffu, ok);
     tc_fence_after_sync();
     // all accumulator columns of this thread first, then the arithmetic and the stores
@@ -631,29 +724,45 @@ hvp_row_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Ten
         float f[16];
 #pragma unroll
         for (int e = 0; e < 16; ++e) f[e] = __uint_as_float(v[ch][e]) * mul;
-        if constexpr (MODE == ROW_PREDO) {
-          const uint4 o0 = o_[2 * ch], o1 = o_[2 * ch + 1];
-          const uint32_t ow[8] = {o0.x, o0.y, o0.z, o0.w, o1.x, o1.y, o1.z, o1.w};
-#pragma unroll
-          for (int e = 0; e < 8; ++e) {
-            const float2 of = Pack<T>::unpack(ow[e]);
-            f[2 * e] = fmaf(-dot2_row, of.x, f[2 * e]);
-            f[2 * e + 1] = fmaf(-dot2_row, of.y, f[2 * e + 1]);
-          }
-        }
         const int col = half * kColsPerHalf + ch * 16;
-        if constexpr (SPLIT) {      // O was not fetched: dot2 is not known yet
+        if constexpr (SPLIT) {      // dot2 is not known yet
           store_partial16<D>(partial, row, col, f);
         } else {
+          const uint32_t tile = out_tile + (uint32_t)(col >> 6) * kAtomBytesStat;
+          if constexpr (MODE == ROW_PREDO) {      // g_dO = g_dO' - dot2 * O, whose element is where the result goes
+            uint32_t ow[8];
+            load_op16(tile, row, col & 63, ow);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+              const float2 of = Pack<T>::unpack(ow[e]);
+              f[2 * e] = fmaf(-dot2_row, of.x, f[2 * e]);
+              f[2 * e + 1] = fmaf(-dot2_row, of.y, f[2 * e + 1]);
+            }
+          }
           uint32_t w[8];
 #pragma unroll
           for (int e = 0; e < 8; ++e) w[e] = Pack<T>::pack(f[2 * e], f[2 * e + 1]);
-          store_op16(strm_base + (uint32_t)(col >> 6) * kAtomBytesStat, row, col & 63, w);
+          store_op16(tile, row, col & 63, w);
         }
       }
     }
-    // the result tile goes out through the first stream stage (every product has completed)
-    store_tile_tma(&maps.out[MODE == ROW_PREDO ? TO_gdO : TO_gQ], strm_base, g.D, r0, bh, !SPLIT && threadIdx.x == 0);
+    if constexpr (!SPLIT) {
+      store_tile_tma(&maps.out[MODE == ROW_PREDO ? TO_gdO : TO_gQ], out_tile, g.D, r0, bh, threadIdx.x == 0);
+      if (threadIdx.x == 0) {
+        mbar_arrive(bar_stream_empty(0, c_out % S));
+        mbar_arrive(bar_stream_empty(1, c_out % S));
+      }
+    }
+    g0 += n_iter;
+    ++items;
+    }
+    if (!PERSIST || !ok) break;
+    c0 += entries(w);
+    int unit;
+    ok = work_next(&ctl->work, k, &unit, abort_flag, t.status, wait_code(KIND, 14));
+    if (!ok || unit < 0) break;
+    w = item_of(unit);
+    }
   }
 
   if constexpr (SPLIT) {
@@ -669,8 +778,8 @@ hvp_row_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Ten
             for (int i = 0; i < 4; ++i) sum[i] += theirs[i * BM + threadIdx.x];
           }
           part_dot2[threadIdx.x] = sum[1];
-          if (part == 0 && r0 + threadIdx.x < g.N_q) {
-            const size_t at = (size_t)bh * g.N_q + r0 + threadIdx.x;
+          if (part == 0 && w.r0 + threadIdx.x < g.N_q) {
+            const size_t at = (size_t)w.bh * g.N_q + w.r0 + threadIdx.x;
             t.Dv[at] = sum[0];
             t.dot2[at] = sum[1];
             t.dot3[at] = sum[2] - 2.f * sum[0] * sum[1] + sum[3];
@@ -678,9 +787,9 @@ hvp_row_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Ten
         }
         named_barrier_sync(1, kMathThreads);
       }
-      const size_t at = ((size_t)bh * g.N_q + r0) * g.D;
+      const size_t at = ((size_t)w.bh * g.N_q + w.r0) * g.D;
       const T* O_rows = (const T*)t.O + at;
-      reduce_parts<D, T>(partial, (int)split, part, (T*)(MODE == ROW_PREDO ? t.out_g_dO : t.out_g_Q) + at, min(BM, g.N_q - r0), g.D,
+      reduce_parts<D, T>(partial, (int)split, part, (T*)(MODE == ROW_PREDO ? t.out_g_dO : t.out_g_Q) + at, min(BM, g.N_q - w.r0), g.D,
                          [](int, int) { return 1.f; },
                          [&](int row, int col, float4& v) {
                            if constexpr (MODE == ROW_PREDO) {
@@ -700,16 +809,21 @@ hvp_row_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Ten
     tc_fence_after_sync();
     tmem_dealloc(tmem_base, kTmemCols);
   }
-  pdl_end(g);
+  if constexpr (PERSIST) pdl_end_persistent(g);
+  else pdl_end(g);
 }
 
 template <int MODE, int D, typename T>
 static cudaError_t launch_row(const TmaMaps& maps, const Geometry& g_in, const Tensors& t, cudaStream_t s) {
   using CF = RowCfg<D>;
   Geometry g = g_in;
-  g.head_group = pick_head_group((long long)g.BH * ((g.N_q + BM - 1) / BM), g.BH, 4ll * g.N_kv * g.D * 2);   // K, g_dK, V, g_dV
-  static TileKernelState state;
-  return launch_tiles(hvp_row_kernel<MODE, D, T, false>, hvp_row_kernel<MODE, D, T, true>, maps, g, t, s, false, kRowThreads, CF::kSmemBytes,
+  const long long units = (long long)g.BH * ((g.N_q + BM - 1) / BM);
+  g.head_group = pick_head_group(units, g.BH, 4ll * g.N_kv * g.D * 2);   // K, g_dK, V, g_dV
+  // persistent where a CTA has more than one tile's worth of work to take over
+  static TileKernelState states[2];
+  TileKernelState& state = states[units > kSms];
+  const auto whole = units > kSms ? hvp_row_kernel<MODE, D, T, false, true> : hvp_row_kernel<MODE, D, T, false, false>;
+  return launch_tiles(whole, hvp_row_kernel<MODE, D, T, true, false>, maps, g, t, s, false, kRowThreads, CF::kSmemBytes,
                       2000.f, MODE == ROW_Q ? 2700.f : 0.f, state);
 }
 

@@ -24,13 +24,15 @@ constexpr uint32_t kAtomBytesStrm = BN * 128;   // [ 64 rows][64 halves],  8 KB
 // Kernel ids inside device status codes (the backward kernels use 18 and 19, the forward kernel
 // 20, the self-test 0x6f); the values are documented with the C ABI and do not change.
 enum Kind { HVP_PRE = 4, HVP_ROW = 5, HVP_COL = 6 };
-enum TensorId { T_Q = 0, T_K, T_V, T_dO, T_gQ, T_gK, T_gV, T_COUNT };
+enum TensorId { T_Q = 0, T_K, T_V, T_dO, T_gQ, T_gK, T_gV, T_O, T_COUNT };
 
 // Output tensors by operation: forward {O}; backward {dQ, dK, dV}; double backward
 // {g_dO, g_Q, g_K, g_V}.  Output maps have a box of 64 columns x 128 rows.
 enum OutId { TO_O = 0, TO_dQ = 0, TO_dK = 1, TO_dV = 2, TO_gdO = 0, TO_gQ = 1, TO_gK = 2, TO_gV = 3, TO_COUNT = 4 };
 
 struct TmaMaps { CUtensorMap m[T_COUNT]; CUtensorMap out[TO_COUNT]; };
+
+template <int V> struct Int { static constexpr int value = V; };
 
 template <typename T> struct Pack;
 template <> struct Pack<__nv_bfloat16> {
@@ -65,6 +67,10 @@ template <> struct Pack<__half> {
 // and whatever follows in the stream may rely on both.  A second stream with an event fork and join does the same for 4 us more
 // of host time and a launch latency on either side, and cannot be used under stream capture.
 __device__ __forceinline__ void pdl_begin(const Geometry& g) { if (!g.beside) pdl_wait(); }
+// A persistent kernel's last CTA may have been taken over by another one, so there every CTA waits.
+__device__ __forceinline__ void pdl_end_persistent(const Geometry& g) {
+  if (g.beside && threadIdx.x == 0) pdl_wait();
+}
 __device__ __forceinline__ void pdl_end(const Geometry& g) {
   if (g.beside && blockIdx.x + 1 == gridDim.x && threadIdx.x == 0) pdl_wait();
 }
@@ -264,6 +270,54 @@ inline cudaError_t launch_tiles(void (*whole)(P...), void (*shared)(P...), const
   return e != cudaSuccess ? e : launch_pdl_cluster(kern, (unsigned)(units * g.split), threads, smem, (unsigned)g.split, s, maps, g, t);
 }
 
+// ---- Persistent CTAs -------------------------------------------------------------------------
+// The double-backward kernels fill an SM's shared and tensor memory, so a second CTA cannot hide what a
+// CTA costs besides its tiles.  There a running CTA takes over CTAs that have not been launched yet
+// (cluster launch control): the producer asks for the next one while the last tiles of the current one are
+// under way, announces it to the other warps, and its loads go straight on in the same ring of
+// stages.  Heavy tiles come first in the grid's order, as without it.
+struct WorkControl {
+  alignas(16) uint32_t answer[4];
+  uint64_t answered;
+  uint64_t full[2], empty[2];        // two announcements, used in turn
+  int unit[2];
+};
+constexpr int kWorkReaders = kMathWarps + 2;
+
+__device__ __forceinline__ void work_init(WorkControl* w) {
+  mbar_init(smem_u32(&w->answered), 1);
+  for (int i = 0; i < 2; ++i) {
+    mbar_init(smem_u32(&w->full[i]), 1);
+    mbar_init(smem_u32(&w->empty[i]), kWorkReaders);
+  }
+}
+// producer thread, once per item
+__device__ __forceinline__ void work_request(WorkControl* w) {
+  fence_proxy_async_smem();          // the previous answer has been read
+  mbar_arrive_expect_tx(smem_u32(&w->answered), 16);
+  clc_request(smem_u32(w->answer), smem_u32(&w->answered));
+}
+// producer thread: announcement number n, from 0; the unit, or -1 at the end
+__device__ __forceinline__ bool work_announce(WorkControl* w, int n, int* unit, volatile uint32_t* abort_flag, unsigned int* status,
+                                              uint32_t code) {
+  if (!mbar_wait(smem_u32(&w->answered), n & 1, abort_flag, status, code)) return false;
+  *unit = clc_answer(smem_u32(w->answer));
+  if (!mbar_wait(smem_u32(&w->empty[n & 1]), ((n >> 1) & 1) ^ 1, abort_flag, status, code)) return false;
+  w->unit[n & 1] = *unit;
+  mbar_arrive(smem_u32(&w->full[n & 1]));
+  return true;
+}
+// a whole warp of the other roles
+__device__ __forceinline__ bool work_next(WorkControl* w, int n, int* unit, volatile uint32_t* abort_flag, unsigned int* status,
+                                          uint32_t code) {
+  const bool ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&w->full[n & 1]), (n >> 1) & 1, abort_flag, status, code));
+  // the shuffle tells the compiler that the value, and every loop bound that follows from it, is uniform
+  *unit = __shfl_sync(0xffffffffu, *reinterpret_cast<volatile int*>(&w->unit[n & 1]), 0);
+  __syncwarp();
+  if ((threadIdx.x & 31) == 0) mbar_arrive(smem_u32(&w->empty[n & 1]));
+  return ok;
+}
+
 // Two CTAs per SM, each with half of the tensor memory and one group of math warps (the forward, and
 // the first backward at D = 64, where that is enough): while one sets up, fills its pipeline or writes
 // its result, the other computes.  A CTA costs kCtaClocks besides its tiles, a third of its time at 17
@@ -323,16 +377,24 @@ __device__ __forceinline__ void store_op16(uint32_t tile, int row, int col0, con
                : "memory");
 }
 
+__device__ __forceinline__ void load_op16(uint32_t tile, int row, int col0, uint32_t (&v)[8]) {
+#pragma unroll
+  for (int q = 0; q < 2; ++q)
+    asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(v[4 * q]), "=r"(v[4 * q + 1]), "=r"(v[4 * q + 2]), "=r"(v[4 * q + 3])
+                 : "r"(tile + sw128_offset(row, col0 + 8 * q))
+                 : "memory");
+}
 
 // Zeros in rows [row0, row0 + BM) of plane `plane` of a [planes][n_rows][D] half-precision tensor: the
 // result of a CTA that has no tile to visit (keys in front of the sequence in a chunk's window,
 // queries without a visible key).  It needs no barriers, tensor memory or loads.  At H12, the fourth
 // chunk of 1024 queries, 9216 keys, D64, 480 of 864 column CTAs are of this kind: backward 85 -> 78,
 // double backward 171 -> 165 us.
-__device__ __forceinline__ void zero_rows(void* out, int plane, int row0, int n_rows, int D) {
+__device__ __forceinline__ void zero_rows(void* out, int plane, int row0, int n_rows, int D, int threads) {
   const int rows = min(BM, n_rows - row0);
   uint4* p = reinterpret_cast<uint4*>(static_cast<uint16_t*>(out) + ((size_t)plane * n_rows + row0) * D);
-  for (int i = threadIdx.x; i < rows * D / 8; i += blockDim.x) p[i] = make_uint4(0u, 0u, 0u, 0u);
+  for (int i = threadIdx.x; i < rows * D / 8; i += threads) p[i] = make_uint4(0u, 0u, 0u, 0u);
 }
 
 // Epilogue of the tensor-core kernels.  The 256 math threads have written a [128 rows][cols]

@@ -108,6 +108,27 @@ __device__ __forceinline__ void named_barrier_sync(uint32_t id, uint32_t threads
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
+// Cluster launch control: a running CTA takes over a CTA of its grid that has not been launched yet.
+// The 16-byte answer is written to shared memory (completes 16 bytes on `bar`); clc_answer reads it:
+// the x index of the CTA taken over, or -1 when none was left (after which no further request is made).
+__device__ __forceinline__ void clc_request(uint32_t answer, uint32_t bar) {
+  asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];" ::"r"(answer), "r"(bar)
+               : "memory");
+}
+__device__ __forceinline__ int clc_answer(uint32_t answer) {
+  int x;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t.reg .b128 a;\n\t"
+      "ld.shared.b128 a, [%1];\n\t"
+      "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, a;\n\t"
+      "mov.s32 %0, -1;\n\t"
+      "@p clusterlaunchcontrol.query_cancel.get_first_ctaid::x.b32.b128 %0, a;\n\t}"
+      : "=r"(x)
+      : "r"(answer)
+      : "memory");
+  return x;
+}
+
 // ---------------------------------------------------------------------------
 // TMA: 3-D tiled load, global -> shared, completion on an mbarrier.
 // The innermost coordinate x is always a multiple of 64 half-precision elements

@@ -30,6 +30,8 @@ capi = importlib.import_module("610sample_b200.capi")
     (6, 50, 60, 190, 64, 190, 0, 1),         # one tile per head
     (5, 40, 200, 200, 128, 200, 0, 0),       # two forward CTAs per SM, Q in shared memory
     (4, 40, 190, 500, 80, 130, 1, 0),        # the same with padding and a window
+    (2, 200, 130, 70, 64, 20, 0, 0),         # persistent CTAs: items of one or two tiles
+    (2, 80, 300, 900, 128, 100, 0, 0),       # the same, and items without a tile in between
 ])
 def test_few_and_many_tiles_match_the_oracle(B, H, N_q, N_kv, D, window, chunk, mask, dtype):
     inp = orc.make_inputs(B, H, N_q, N_kv, D, seed=N_q + N_kv, dtype=dtype)
