@@ -366,9 +366,11 @@ hvp_row_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Ten
       // Every batch of products is issued by the elected lane inside one branch, with the
       // descriptor of the stage built once: the instruction stream between two MMAs is an add.
       // The RA batch goes out in two elected branches, the last kTail k-steps and the commit in the
-      // second: measured, the scalar pass loses 10 % when the whole batch is issued in one branch
-      // (the short gap lets the other issuing warp's products into the queue in between).
-      constexpr int kTail = (D == 128) ? 2 : 0;
+      // second: the short gap lets the other issuing warp's products into the queue in between.  The
+      // scalar pass takes 20 % more cycles when the whole batch is issued in one branch, 35 % more when it
+      // waits in the gap for the other warp's, and 5 % more at D = 80 and 96 with kTail = 2, where the
+      // second branch is left with padding steps only.
+      constexpr int kTail = (D == 128) ? (MODE == ROW_PREDO ? 5 : 2) : 0;
       auto issue_ra = [&](uint32_t stage) {           // ends with the commit of the batch
         const uint64_t dk = smem_desc_sw128(stage, 16, 1024);
         if (elect_one()) {
