@@ -48,7 +48,7 @@ COL_KERNEL_GEMMS = 8
 # dram__bytes_read.sum + dram__bytes_write.sum per launch of each kernel, from an `ncu --set full`
 # capture of this bench at 16 (batch, head) slices; traffic grows in proportion to the number of
 # slices, so the bench scales it by BH / 16.  To be refreshed whenever a kernel changes.
-NCU_TRAFFIC_BYTES_16_SLICES = {"pre": 193.3e6, "row": 173.6e6, "col": 137.3e6}
+NCU_TRAFFIC_BYTES_16_SLICES = {"pre": 193.0e6, "row": 171.0e6, "col": 136.9e6}
 # the same for one launch of the fused norm + rotary kernel (part of the output is still in L2 when it ends)
 NCU_PREP_TRAFFIC_BYTES = {"16384x32x128": 232.2e6}
 
