@@ -16,7 +16,8 @@ order is not supported.
 ``flash_attention_v7`` itself runs the same two functions from their C++ form in the
 extension (``attention_cuda.flash_attention``), which the autograd engine executes
 without the interpreter; the Python classes are the reference-facing surface for
-code that applies them directly.
+code that applies them directly, and serve calls under ``torch.jit.trace``, which
+records them, and calls with forward-mode tangents, which they refuse.
 
 Additive extension: ``mask_mode`` (0 = reference mask, 1 = no mask) as a trailing
 keyword of ``flash_attention_v7``.
@@ -97,6 +98,8 @@ def flash_attention_v7(Q, K, V, window_size, chunk_id, mask_mode=0):
     """
     fused = getattr(_attention_cuda, "flash_attention", None)
     if fused is not None:
-        return fused(Q, K, V, window_size, chunk_id, mask_mode)
-    # a module with the reference's three functions only (an older build, a test's stand-in)
+        O = fused(Q, K, V, window_size, chunk_id, mask_mode)
+        if O is not None:
+            return O
+    # traced or with a tangent; or a module with the reference's three functions only (a test's stand-in)
     return FlashAttentionV7.apply(Q, K, V, window_size, chunk_id, mask_mode)

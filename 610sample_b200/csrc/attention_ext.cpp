@@ -11,15 +11,19 @@
 // `flash_attention` is the twice-differentiable call of attention.py with its two chained autograd
 // functions written in C++: the autograd engine then runs both backward passes on its own thread
 // without taking the interpreter lock.  A Python autograd function costs 25-30 us per use on the
-// host (four of them in a second-order step) against about 5 us here.
+// host (four of them in a second-order step) against about 5 us here.  Calls that a Python
+// autograd function handles better (tracers, forward-mode tangents) are left to it.
 #include <torch/extension.h>
 #include <torch/csrc/autograd/custom_function.h>
+#include <torch/csrc/jit/frontend/tracer.h>
+#include <ATen/FuncTorchTLS.h>
 #include <ATen/cuda/CUDAContext.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAGuard.h>
 
 #include <atomic>
 #include <cstdio>
+#include <initializer_list>
 #include <mutex>
 #include <vector>
 
@@ -45,8 +49,10 @@ torch::Tensor dense(const torch::Tensor& t) {
 }
 
 // New tensors of a contiguous shape on t's device, straight from the caching allocator: the
-// dispatcher's factory functions take twice as long, and a call makes three to five tensors.
+// dispatcher's factory functions take twice as long, and a call makes three to five tensors.  A tracer
+// has to see where its tensors come from.
 torch::Tensor fresh(at::IntArrayRef sizes, at::ScalarType type, const torch::Tensor& t) {
+  if (torch::jit::tracer::isTracing()) return torch::empty(sizes, t.options().dtype(type));
   return at::detail::empty_cuda(sizes, type, t.device(), c10::nullopt);
 }
 torch::Tensor fresh_like(const torch::Tensor& t) { return fresh(t.sizes(), t.scalar_type(), t); }
@@ -199,6 +205,20 @@ namespace {
 using torch::autograd::AutogradContext;
 using torch::autograd::variable_list;
 
+bool has_tangent(std::initializer_list<const torch::Tensor*> inputs) {
+  for (const torch::Tensor* t : inputs)
+    if (t->defined() && t->_fw_grad(/*level=*/0).defined()) return true;
+  return false;
+}
+
+// A call for the Python autograd functions: torch.jit.trace records them, and they refuse a tangent,
+// which kernels called directly would drop.  Under a functorch transform neither kind of function has
+// a rule: refused here, whether or not gradients are asked for.
+bool leave_to_python(std::initializer_list<const torch::Tensor*> inputs) {
+  if (const auto& functorch = at::functorch::functorchTLSAccessor()) functorch->checkSupportsCppAutogradFunction();
+  return torch::jit::tracer::isTracing() || has_tangent(inputs);
+}
+
 struct MaskArgs { int window_size, chunk_id, mask_mode; };
 
 void save_mask(AutogradContext* ctx, int64_t window_size, int64_t chunk_id, int64_t mask_mode) {
@@ -253,8 +273,8 @@ struct Attention : public torch::autograd::Function<Attention> {
     if (!g[0].defined()) return out;
     const variable_list s = ctx->get_saved_variables();
     const MaskArgs m = saved_mask(ctx);
-    // without create_graph nothing will ask for the derivative of this backward
-    variable_list r = at::GradMode::is_enabled()
+    // without create_graph nothing will ask for the derivative of this backward (but a tangent has to be refused)
+    variable_list r = at::GradMode::is_enabled() || has_tangent({&g[0], &s[0], &s[1], &s[2]})
                           ? AttentionBackward::apply(g[0], s[0], s[1], s[2], s[3].detach(), s[4], (int64_t)m.window_size,
                                                      (int64_t)m.chunk_id, (int64_t)m.mask_mode)
                           : v7_backward_cuda(g[0], s[0], s[1], s[2], s[3], s[4], m.window_size, m.chunk_id, m.mask_mode, 0);
@@ -265,8 +285,10 @@ struct Attention : public torch::autograd::Function<Attention> {
 
 }  // namespace
 
-torch::Tensor flash_attention(const torch::Tensor& Q, const torch::Tensor& K, const torch::Tensor& V, int window_size,
-                              int chunk_id, int mask_mode) {
+// Nothing: a call for the Python function (attention.py).
+c10::optional<torch::Tensor> flash_attention(const torch::Tensor& Q, const torch::Tensor& K, const torch::Tensor& V, int window_size,
+                                             int chunk_id, int mask_mode) {
+  if (leave_to_python({&Q, &K, &V})) return c10::nullopt;
   const bool graph = at::GradMode::is_enabled() && (Q.requires_grad() || K.requires_grad() || V.requires_grad());
   if (!graph) return v7_forward_cuda(Q, K, V, window_size, chunk_id, mask_mode, 0)[0];
   return Attention::apply(Q, K, V, (int64_t)window_size, (int64_t)chunk_id, (int64_t)mask_mode);
@@ -444,7 +466,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("qk_norm_rope_diff", &qk_norm_rope_diff, "qk_norm_rope, twice differentiable",
         py::arg("x"), py::arg("weight"), py::arg("freqs"), py::arg("pos0") = 0, py::arg("eps") = 1e-6, py::arg("norm_from") = 0,
         py::call_guard<py::gil_scoped_release>());
-  m.def("flash_attention", &flash_attention, "Rectangular sliding-window flash attention, twice differentiable -> O",
+  m.def("flash_attention", &flash_attention, "Rectangular sliding-window flash attention, twice differentiable -> O (None: a call for the Python function)",
         py::arg("Q"), py::arg("K"), py::arg("V"), py::arg("window_size"), py::arg("chunk_id"), py::arg("mask_mode") = 0,
         py::call_guard<py::gil_scoped_release>());
   m.def("v7_forward", &v7_forward_cuda, "Rectangular sliding-window flash attention forward -> [O, L]",

@@ -259,3 +259,31 @@ def test_two_host_threads_on_their_own_streams():
         for a, b in zip(cases[i][3], results[i]):
             assert torch.equal(a, b)
     assert capi.device_status() == 0
+
+
+def test_transforms_and_tracing_are_those_of_the_python_functions(mods):
+    """Forward-mode tangents and functorch transforms have no rule and are refused, with and without
+    gradients, in the call and in its backward (a kernel called directly would drop the tangent);
+    torch.jit.trace records the call."""
+    import torch.autograd.forward_ad as fwad
+    _, flash = mods
+    q, k, v = (torch.randn(1, 2, 64, 64, device=DEV).to(torch.bfloat16) for _ in range(3))
+    call = lambda a: flash(a, k, v, 64, 0)
+    for grad in (False, True):
+        a = q.clone().requires_grad_(grad)
+        with fwad.dual_level(), pytest.raises(RuntimeError):
+            call(fwad.make_dual(a, torch.ones_like(a)))
+    for keep in (False, True):
+        a = q.clone().requires_grad_(True)
+        o = call(a)
+        with fwad.dual_level(), pytest.raises(RuntimeError):
+            torch.autograd.grad(o, [a], fwad.make_dual(torch.ones_like(o), torch.ones_like(o)), create_graph=keep)
+    for transformed in (lambda: torch.func.jvp(call, (q,), (q,)), lambda: torch.func.grad(lambda a: call(a).float().sum())(q),
+                        lambda: torch.func.vmap(call)(torch.stack([q, q]))):
+        with pytest.raises(RuntimeError, match="functorch transforms"):
+            transformed()
+    for grad in (False, True):
+        a = q.clone().requires_grad_(grad)
+        traced = torch.jit.trace(call, (a,), check_trace=False)
+        got, want = traced(a * 2), call(a * 2)
+        assert torch.equal(got, want) and got.requires_grad == grad
