@@ -442,6 +442,17 @@ struct QKNormRope : public torch::autograd::Function<QKNormRope> {
     if (!g[0].defined()) return out;
     const variable_list s = ctx->get_saved_variables();
     const PrepArgs a = saved_prep(ctx);
+    if (has_tangent({&g[0], &s[0], &s[1]})) {      // forward mode over this backward: the formulas have the rules
+      const bool keep_graph = at::GradMode::is_enabled();
+      at::AutoGradMode on(true);
+      auto leaf = [](const torch::Tensor& t) { return t.requires_grad() ? t : t.detach().requires_grad_(true); };
+      variable_list wrt{leaf(s[0])};
+      if (s[1].numel() > 0) wrt.push_back(leaf(s[1]));
+      const torch::Tensor y = qk_norm_rope_formula(wrt[0], wrt.size() > 1 ? wrt[1] : torch::Tensor(), s[2], a);
+      const variable_list r = torch::autograd::grad({y}, wrt, {g[0]}, c10::nullopt, keep_graph, true);
+      for (size_t i = 0; i < r.size(); ++i) out[i] = r[i];
+      return out;
+    }
     variable_list r = at::GradMode::is_enabled()
                           ? QKNormRopeBackward::apply(g[0], s[0], s[1], s[2], (int64_t)a.pos0, a.eps, (int64_t)a.norm_from)
                           : qk_norm_rope_backward(g[0], s[0], weight_or_none(s[1]), s[2], a, ctx->needs_input_grad(1));
@@ -452,9 +463,11 @@ struct QKNormRope : public torch::autograd::Function<QKNormRope> {
 
 }  // namespace
 
-torch::Tensor qk_norm_rope_diff(const torch::Tensor& x, c10::optional<torch::Tensor> weight, const torch::Tensor& freqs, int pos0,
-                                double eps, int norm_from) {
+// Nothing: a call for the Python function (qk_prep.py).
+c10::optional<torch::Tensor> qk_norm_rope_diff(const torch::Tensor& x, c10::optional<torch::Tensor> weight, const torch::Tensor& freqs,
+                                               int pos0, double eps, int norm_from) {
   const bool has_weight = weight.has_value() && weight->defined();
+  if (leave_to_python({&x, has_weight ? &*weight : &x, &freqs})) return c10::nullopt;
   if (!at::GradMode::is_enabled() || !(x.requires_grad() || (has_weight && weight->requires_grad())))
     return qk_norm_rope_cuda(x, weight, freqs, pos0, eps, norm_from);
   return QKNormRope::apply(x, has_weight ? *weight : fresh({0}, x.scalar_type(), x), freqs, (int64_t)pos0, eps, (int64_t)norm_from);
@@ -463,7 +476,7 @@ torch::Tensor qk_norm_rope_diff(const torch::Tensor& x, c10::optional<torch::Ten
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("qk_norm_rope", &qk_norm_rope_cuda, "fused RMS norm + rotary embedding + [n_tok,H,d] -> [1,H,n_tok,d]",
         py::arg("x"), py::arg("weight"), py::arg("freqs"), py::arg("pos0") = 0, py::arg("eps") = 1e-6, py::arg("norm_from") = 0);
-  m.def("qk_norm_rope_diff", &qk_norm_rope_diff, "qk_norm_rope, twice differentiable",
+  m.def("qk_norm_rope_diff", &qk_norm_rope_diff, "qk_norm_rope, twice differentiable (None: a call for the Python function)",
         py::arg("x"), py::arg("weight"), py::arg("freqs"), py::arg("pos0") = 0, py::arg("eps") = 1e-6, py::arg("norm_from") = 0,
         py::call_guard<py::gil_scoped_release>());
   m.def("flash_attention", &flash_attention, "Rectangular sliding-window flash attention, twice differentiable -> O (None: a call for the Python function)",

@@ -9,7 +9,9 @@ additive entry point: the reference surface (`attention.py`) does not depend on 
 
 `qk_norm_rope` is differentiable to second order, as test-time training needs
 (`attention_cuda.qk_norm_rope_diff`): the forward and the first backward run fused kernels; the
-second backward differentiates the same formulas written as ordinary operations.
+second backward differentiates the same formulas written as ordinary operations.  Calls under
+`torch.jit.trace`, which records Python autograd functions only, and calls with forward-mode
+tangents, which that function refuses, go through `_QKNormRope`.
 """
 import torch
 
@@ -47,8 +49,27 @@ def qk_norm_rope_torch(x, weight, freqs, pos0=0, eps=1e-6, norm_from=0):
     return out.permute(1, 0, 2).unsqueeze(0)
 
 
+class _QKNormRope(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, x, weight, freqs, pos0, eps, norm_from):
+        ctx.save_for_backward(x, weight if weight is not None else x.new_empty(0), freqs)
+        ctx.has_weight = weight is not None
+        ctx.args = (pos0, eps, norm_from)
+        return _attention_cuda.qk_norm_rope(x, weight, freqs, pos0, eps, norm_from)
+
+    @staticmethod
+    def backward(ctx, g):
+        x, weight, freqs = ctx.saved_tensors
+        with torch.enable_grad():
+            wrt = [t if t.requires_grad else t.detach().requires_grad_(True) for t in ([x, weight] if ctx.has_weight else [x])]
+            y = qk_norm_rope_torch(wrt[0], wrt[1] if ctx.has_weight else None, freqs, *ctx.args)
+        gx, gw = (*torch.autograd.grad(y, wrt, g, create_graph=torch.is_grad_enabled(), allow_unused=True), None)[:2]
+        return gx, gw, None, None, None, None
+
+
 def qk_norm_rope(x, weight, freqs, pos0=0, eps=1e-6, norm_from=0):
     """x: [n_tok, H, d] (fp16 / bf16 / fp32, CUDA); weight: [d] or None; freqs: `rope_table(...)`.
     Rows below `norm_from` are only rotated (keys taken from a cache are stored normalised).
     Returns [1, H, n_tok, d], ready for `flash_attention_v7`."""
-    return _attention_cuda.qk_norm_rope_diff(x, weight, freqs, pos0, eps, norm_from)
+    y = _attention_cuda.qk_norm_rope_diff(x, weight, freqs, pos0, eps, norm_from)
+    return y if y is not None else _QKNormRope.apply(x, weight, freqs, pos0, eps, norm_from)

@@ -156,3 +156,35 @@ def test_backward_kernel_matches_autograd_of_the_formulas(prep, n, H, D, norm_fr
         assert a.dtype == dtype and a.shape == c.shape
         assert torch.equal(a, b.detach())
         assert float((a.double() - c).abs().max()) <= tol * float(c.abs().max()), (n, H, D)
+
+
+@pytest.mark.gpu
+def test_transforms_and_tracing_are_those_of_the_python_function(prep):
+    """Forward mode and functorch transforms are refused by the call (a kernel called directly would drop
+    the tangent); forward mode over its backward follows the formulas; torch.jit.trace records the call."""
+    import torch.autograd.forward_ad as fwad
+    torch.manual_seed(11)
+    x, w = torch.randn(70, 3, 64, device="cuda"), 1 + 0.1 * torch.randn(64, device="cuda")
+    table = prep.rope_table(64, 70, device="cuda")
+    call = lambda a: prep.qk_norm_rope(a, w, table)
+    for grad in (False, True):
+        a = x.clone().requires_grad_(grad)
+        with fwad.dual_level(), pytest.raises(RuntimeError):
+            call(fwad.make_dual(a, torch.ones_like(a)))
+    for transformed in (lambda: torch.func.jvp(call, (x,), (x,)), lambda: torch.func.vmap(call)(torch.stack([x, x]))):
+        with pytest.raises(RuntimeError, match="functorch transforms"):
+            transformed()
+    u, du = torch.randn(1, 3, 70, 64, device="cuda"), torch.randn(1, 3, 70, 64, device="cuda")
+    for keep in (False, True):
+        a, b = (x.clone().requires_grad_(True) for _ in range(2))
+        y = call(a)
+        with fwad.dual_level():
+            g, = torch.autograd.grad(y, [a], fwad.make_dual(u, du), create_graph=keep)
+            got = fwad.unpack_dual(g).tangent
+        want, = torch.autograd.grad(prep.qk_norm_rope_torch(b, w, table), [b], du)      # the backward is linear in g
+        assert got is not None and torch.allclose(got, want, rtol=1e-4, atol=1e-5)
+    for grad in (False, True):
+        a = x.clone().requires_grad_(grad)
+        traced = torch.jit.trace(call, (a,), check_trace=False)
+        got, want = traced(a * 2), call(a * 2)
+        assert torch.equal(got, want) and got.requires_grad == grad
