@@ -468,7 +468,8 @@ c10::optional<torch::Tensor> qk_norm_rope_diff(const torch::Tensor& x, c10::opti
                                                int pos0, double eps, int norm_from) {
   const bool has_weight = weight.has_value() && weight->defined();
   if (leave_to_python({&x, has_weight ? &*weight : &x, &freqs})) return c10::nullopt;
-  if (!at::GradMode::is_enabled() || !(x.requires_grad() || (has_weight && weight->requires_grad())))
+  // the table has no gradient, but a table that asks for one makes the output part of the graph
+  if (!at::GradMode::is_enabled() || !(x.requires_grad() || freqs.requires_grad() || (has_weight && weight->requires_grad())))
     return qk_norm_rope_cuda(x, weight, freqs, pos0, eps, norm_from);
   return QKNormRope::apply(x, has_weight ? *weight : fresh({0}, x.scalar_type(), x), freqs, (int64_t)pos0, eps, (int64_t)norm_from);
 }

@@ -188,3 +188,11 @@ def test_transforms_and_tracing_are_those_of_the_python_function(prep):
         traced = torch.jit.trace(call, (a,), check_trace=False)
         got, want = traced(a * 2), call(a * 2)
         assert torch.equal(got, want) and got.requires_grad == grad
+
+
+@pytest.mark.gpu
+def test_a_table_that_asks_for_gradients_is_accepted_and_gets_none(prep):
+    table = prep.rope_table(64, 20, device="cuda").requires_grad_(True)
+    y = prep.qk_norm_rope(torch.randn(20, 2, 64, device="cuda"), torch.ones(64, device="cuda"), table)
+    y.sum().backward()
+    assert y.requires_grad and table.grad is None
