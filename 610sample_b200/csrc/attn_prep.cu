@@ -313,7 +313,8 @@ qk_norm_rope_bwd_kernel(const T* __restrict__ x, const T* __restrict__ weight, c
           dot += __shfl_xor_sync(0xffffffffu, dot, o);
         }
       }
-      if (norm) {
+      // a head or token that is not there has x = 0, and with eps = 0 its r is infinite: no part of the weight's gradient
+      if (norm && active && h0 + i < H) {
         const float r = rsqrtf(ss * inv_d + eps);
         const float k = r * r * r * inv_d * dot;
 #pragma unroll

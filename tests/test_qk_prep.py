@@ -196,3 +196,16 @@ def test_a_table_that_asks_for_gradients_is_accepted_and_gets_none(prep):
     y = prep.qk_norm_rope(torch.randn(20, 2, 64, device="cuda"), torch.ones(64, device="cuda"), table)
     y.sum().backward()
     assert y.requires_grad and table.grad is None
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,H", [(70, 4), (64, 3), (70, 3)])      # tokens or heads that do not fill a CTA's tile
+def test_backward_without_epsilon_is_finite(prep, n, H):
+    torch.manual_seed(2)
+    x = torch.randn(n, H, 64, device="cuda").requires_grad_(True)
+    w = (1 + 0.1 * torch.randn(64, device="cuda")).requires_grad_(True)
+    g, table = torch.randn(1, H, n, 64, device="cuda"), prep.rope_table(64, n, device="cuda")
+    got = torch.autograd.grad(prep.qk_norm_rope(x, w, table, eps=0.0), [x, w], g)
+    want = torch.autograd.grad(prep.qk_norm_rope_torch(x, w, table, eps=0.0), [x, w], g)
+    for a, b in zip(got, want):      # fp32 on both sides
+        assert torch.allclose(a, b, rtol=1e-4, atol=1e-5 * float(b.abs().max()))
