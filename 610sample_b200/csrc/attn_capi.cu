@@ -133,14 +133,10 @@ int run(int op, const attn_shape_t* s, attn::Tensors& t, void* stream, int phase
   // driver call and fails with "invalid context" on a thread that has made no runtime
   // call yet (e.g. a freshly started autograd worker thread).  cudaSetDevice on the current
   // device does that and, unlike a null cudaFree, is legal while a stream is being captured.
-  // Once per thread and device.
-  static thread_local int bound_device = -1;
+  // On every call: a host program may have made another context current, or none, since the last one.
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
-  if (e == cudaSuccess && dev != bound_device) {
-    e = cudaSetDevice(dev);
-    if (e == cudaSuccess) bound_device = dev;
-  }
+  if (e == cudaSuccess) e = cudaSetDevice(dev);
   if (e != cudaSuccess) return fail(ATTN_ECUDA, "binding the device context: %s", cudaGetErrorString(e));
   int rc = status_pointer(dev, &t.status);
   if (rc != ATTN_OK) return rc;

@@ -9,11 +9,13 @@
 * guard bands: every output, L and the scratch are carved out of NaN-filled buffers at ragged
   shapes; after the calls the bands are untouched (plain stores and TMA stores alike);
 * the phase masks of the double backward reproduce the one-call result bit for bit;
+* a call on a thread whose current context was taken away since its last call binds the device again;
 * a call captured into a CUDA graph on one host thread while another thread calls eagerly;
 * a thousand back-to-back calls of the three operations at shapes with many CTAs per SM: no
   wait runs out and every result is bit-identical to the first (the hand-offs between the issuing
   warps and the math groups are the kind of protocol whose faults show once in 10^5 CTAs).
 """
+import ctypes
 import importlib
 import os
 import sys
@@ -94,6 +96,24 @@ def test_selftest_gemm_against_matmul(N, K, flags, dtype):
     ref = A.float() @ Bnk.float().t()
     assert float((C - ref).abs().max()) <= 1e-3 * max(1.0, float(ref.abs().max()))
     assert capi.device_status() == 0
+
+
+def test_call_without_a_current_context_binds_the_device_again():
+    q = torch.randn(1, 2, 64, 64, device=DEV).to(torch.bfloat16)
+    want, _ = tcapi.forward(q, q, q, 64, 0)
+    O, L = torch.zeros_like(q), torch.empty(1, 2, 64, device=DEV)
+    s, stream = tcapi._shape(q, q, 64, 0, 0, 0), torch.cuda.current_stream().cuda_stream
+    torch.cuda.synchronize()
+    driver = ctypes.CDLL("libcuda.so.1")
+    context = ctypes.c_void_p()
+    assert driver.cuCtxGetCurrent(ctypes.byref(context)) == 0 and driver.cuCtxSetCurrent(None) == 0
+    try:
+        rc = capi.lib().attn_b200_forward(s, q.data_ptr(), q.data_ptr(), q.data_ptr(), O.data_ptr(), L.data_ptr(), stream)
+    finally:
+        assert driver.cuCtxSetCurrent(context) == 0
+    assert rc == 0, capi.lib().attn_b200_last_error()
+    torch.cuda.synchronize()
+    assert torch.equal(O, want)
 
 
 GUARD = 256    # elements of guard band on either side (multiples of 16 bytes for every dtype)
