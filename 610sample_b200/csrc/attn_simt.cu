@@ -362,7 +362,8 @@ __global__ void __launch_bounds__(threads_of(DC), DC == 1 ? 2 : 1) attn_simt_ker
           for (int h = 0; h < 2; ++h) out[0][a][c][h] = make_float2(out[0][a][c][h].x * f, out[0][a][c][h].y * f);
 #pragma unroll
         for (int b = 0; b < CB; ++b) {
-          const float pr = m_new == -INFINITY ? 0.f : exp2f(s[0][a][b] - m_new);
+          // a score that is not a number goes on to the result, also where it is all that a row sees (m_new = -inf)
+          const float pr = s[0][a][b] == -INFINITY ? 0.f : exp2f(s[0][a][b] - m_new);
           l_run[a] += pr;
           op[0][op_at(row0 + 4 * a, col0 + 8 * b)] = pr;
         }

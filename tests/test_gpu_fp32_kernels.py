@@ -37,3 +37,16 @@ def test_fp32_kernels_match_the_oracle(B, H, N_q, N_kv, D, window, chunk, mask):
         r = ref[n].double()
         # the family's stated tolerance: 1e-4 of the largest value (fp32 sums of at most N * D terms)
         assert float((got.double().cpu() - r).abs().max()) <= 1e-4 * max(1.0, float(r.abs().max())), n
+
+
+@pytest.mark.parametrize("B,H,N,D,impl,dtype", [(1, 4, 256, 64, 0, torch.float32), (2, 16, 500, 80, 0, torch.float32),
+                                                (1, 2, 200, 128, 1, torch.bfloat16)])
+def test_a_query_that_is_not_a_number_gives_a_row_that_is_not(B, H, N, D, impl, dtype):
+    inp = orc.make_inputs(B, H, N, N, D, seed=5, dtype=dtype)
+    Q, K, V = (inp[n].cuda() for n in ("Q", "K", "V"))
+    want, _ = tcapi.forward(Q, K, V, N, 0, 0, impl)
+    Q[:, 0, 7, 3] = float("nan")
+    O, _ = tcapi.forward(Q, K, V, N, 0, 0, impl)
+    assert bool(torch.isnan(O[:, 0, 7]).all())
+    O[:, 0, 7] = want[:, 0, 7]
+    assert torch.equal(O, want)
