@@ -212,6 +212,11 @@ template <int KIND, int DC, typename T>
 __global__ void __launch_bounds__(threads_of(DC), DC == 1 ? 2 : 1) attn_simt_kernel(const Geometry g, const Tensors t, const int split) {
   using SP = Spec<KIND>;
   constexpr int RA = rows_of(DC), NT = threads_of(DC);
+  // g_dO = P g_dV + (P o gdS) V - dot2 o (P V).  In fp32 P V is the O of the call; an O of half precision has
+  // been rounded, so there the kernel sums its own (bf16, g_dK offset by one: relative error 1.66e-3
+  // instead of 1.92e-3; 1.66e-3 is the rounding of the result).
+  constexpr bool kOwnPV = KIND == K_HVP_PRE && sizeof(T) == 2;
+  constexpr int kNSums = SP::kNOut + (kOwnPV ? 1 : 0);
   extern __shared__ __align__(16) float smem[];
   const int D = g.D;
   const Layout lay(D);
@@ -287,9 +292,9 @@ __global__ void __launch_bounds__(threads_of(DC), DC == 1 ? 2 : 1) attn_simt_ker
   float aD[RA] = {}, a2[RA] = {}, aA[RA] = {}, aE[RA] = {};   // HVP_PRE
 #pragma unroll
   for (int a = 0; a < RA; ++a) m_run[a] = -INFINITY;
-  float2 out[SP::kNOut][RA][DC][2];
+  float2 out[kNSums][RA][DC][2];
 #pragma unroll
-  for (int o = 0; o < SP::kNOut; ++o)
+  for (int o = 0; o < kNSums; ++o)
 #pragma unroll
     for (int a = 0; a < RA; ++a)
 #pragma unroll
@@ -404,7 +409,10 @@ __global__ void __launch_bounds__(threads_of(DC), DC == 1 ? 2 : 1) attn_simt_ker
     if constexpr (KIND == K_FWD) add(0, 0, 1);                                   // O += P V
     else if constexpr (KIND == K_BWD_ROW) add(0, 0, 0);                          // dQ += dS K
     else if constexpr (KIND == K_BWD_COL) { add(0, 0, 1); add(1, 1, 0); }        // dV += P^T dO; dK += dS^T Q
-    else if constexpr (KIND == K_HVP_PRE) { add(0, 0, 3); add(0, 1, 1); }        // g_dO' += P g_dV + (P o gdS) V
+    else if constexpr (KIND == K_HVP_PRE) {                                      // g_dO' += P g_dV + (P o gdS) V
+      add(0, 0, 3); add(0, 1, 1);
+      if constexpr (kOwnPV) add(1, 0, 1);                                        // P V
+    }
     else if constexpr (KIND == K_HVP_ROW) { add(0, 0, 2); add(0, 1, 0); }        // g_Q += dS g_dK + g_S K
     else { add(0, 0, 2); add(0, 1, 0); add(1, 2, 1); }                           // g_K += dS^T g_dQ + g_S^T Q; g_V += g_dp^T dO
   }
@@ -414,7 +422,7 @@ __global__ void __launch_bounds__(threads_of(DC), DC == 1 ? 2 : 1) attn_simt_ker
   // ---- results.  Row scalars of the two column halves (and of the other CTAs of the cluster) and
   // the output tiles are combined in the order of the halves and ranks.
   cg::cluster_group cluster = cg::this_cluster();
-  float* const partial = strm_base;                   // [kNOut][TS][D] of this CTA, when the cluster has several
+  float* const partial = strm_base;                   // [kNSums][TS][D] of this CTA, when the cluster has several
   float* const sums = op[0];                          // [2 halves][4][TS] row sums
   if constexpr (KIND == K_FWD || KIND == K_HVP_PRE) {
 #pragma unroll
@@ -430,7 +438,7 @@ __global__ void __launch_bounds__(threads_of(DC), DC == 1 ? 2 : 1) attn_simt_ker
   }
   if (split > 1) {
 #pragma unroll
-    for (int o = 0; o < SP::kNOut; ++o)
+    for (int o = 0; o < kNSums; ++o)
 #pragma unroll
       for (int a = 0; a < RA; ++a)
 #pragma unroll
@@ -474,8 +482,8 @@ __global__ void __launch_bounds__(threads_of(DC), DC == 1 ? 2 : 1) attn_simt_ker
       t.dot3[row_off + r0 + tid] = A - 2.f * D_ * d2_ + E;
     }
   }
-  // one float4 of output o, row r (within the tile), given its sum over the parts
-  auto finish = [&](int o, int r, int chunk, float4 v) {
+  // one float4 of output o, row r (within the tile), given its sum over the parts (and that of P V)
+  auto finish = [&](int o, int r, int chunk, float4 v, float4 pv) {
     if (r0 + r >= n_stat) return;
     const size_t at = (size_t)(r0 + r) * D + 4 * chunk;
     float mul = 1.f;
@@ -490,7 +498,7 @@ __global__ void __launch_bounds__(threads_of(DC), DC == 1 ? 2 : 1) attn_simt_ker
     }
     v = make_float4(v.x * mul, v.y * mul, v.z * mul, v.w * mul);
     if constexpr (KIND == K_HVP_PRE) {
-      const float4 of = load4(O + at);
+      const float4 of = kOwnPV ? pv : load4(O + at);
       const float dd = row_total(1, r);
       v.x = fmaf(-dd, of.x, v.x); v.y = fmaf(-dd, of.y, v.y); v.z = fmaf(-dd, of.z, v.z); v.w = fmaf(-dd, of.w, v.w);
     }
@@ -508,15 +516,19 @@ __global__ void __launch_bounds__(threads_of(DC), DC == 1 ? 2 : 1) attn_simt_ker
     const int total = SP::kNOut * TS * chunks;
     for (int i = part * NT + tid; i < total; i += split * NT) {
       const int row = i / chunks, chunk = i - row * chunks, r = row % TS;
-      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+      float4 v = make_float4(0.f, 0.f, 0.f, 0.f), pv = v;
       float m = 0.f;
       if constexpr (KIND == K_FWD) m = fwd_max(r);
       for (int q = 0; q < split; ++q) {
+        if constexpr (kOwnPV) {
+          const float4 y = reinterpret_cast<const float4*>(cluster.map_shared_rank(partial, q))[i + TS * chunks];
+          pv.x += y.x; pv.y += y.y; pv.z += y.z; pv.w += y.w;
+        }
         const float4 x = reinterpret_cast<const float4*>(cluster.map_shared_rank(partial, q))[i];
         const float f = KIND == K_FWD ? factor(q, r, m) : 1.f;
         v.x = fmaf(x.x, f, v.x); v.y = fmaf(x.y, f, v.y); v.z = fmaf(x.z, f, v.z); v.w = fmaf(x.w, f, v.w);
       }
-      finish(row / TS, r, chunk, v);
+      finish(row / TS, r, chunk, v, pv);
     }
     cluster.sync();                                   // nobody leaves while its shared memory is being read
   } else {
@@ -526,9 +538,10 @@ __global__ void __launch_bounds__(threads_of(DC), DC == 1 ? 2 : 1) attn_simt_ker
       for (int a = 0; a < RA; ++a)
 #pragma unroll
         for (int c = 0; c < DC; ++c)
-          if (chunk0 + 16 * c < chunks)
-            finish(o, row0 + 4 * a, chunk0 + 16 * c,
-                   make_float4(out[o][a][c][0].x, out[o][a][c][0].y, out[o][a][c][1].x, out[o][a][c][1].y));
+          if (chunk0 + 16 * c < chunks) {
+            auto sum = [&](int i) { return make_float4(out[i][a][c][0].x, out[i][a][c][0].y, out[i][a][c][1].x, out[i][a][c][1].y); };
+            finish(o, row0 + 4 * a, chunk0 + 16 * c, sum(o), sum(kNSums - 1));
+          }
   }
   tc::pdl_end(g);
 }

@@ -50,3 +50,21 @@ def test_a_query_that_is_not_a_number_gives_a_row_that_is_not(B, H, N, D, impl, 
     assert bool(torch.isnan(O[:, 0, 7]).all())
     O[:, 0, 7] = want[:, 0, 7]
     assert torch.equal(O, want)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("B,H,N_q,N_kv,D", [(1, 4, 300, 400, 64), (4, 24, 256, 320, 80)])      # a cluster per tile, none
+def test_half_inputs_give_the_rounded_exact_result(B, H, N_q, N_kv, D, dtype):
+    """The arithmetic is fp32, so the double backward is the exact one but for the rounding of its results
+    (g_dK has a mean, so that dot2 O is as large as the sum it is taken from)."""
+    inp = orc.make_inputs(B, H, N_q, N_kv, D, seed=3, dtype=torch.float32)
+    inp["g_dK"] = inp["g_dK"] + 1.0
+    inp = {n: t.to(dtype) for n, t in inp.items()}
+    ref = orc.closed_form_all(*(inp[n] for n in orc.INPUT_NAMES), window_size=N_kv, chunk_id=2, device="cuda")
+    g = {n: t.cuda() for n, t in inp.items()}
+    O, L = tcapi.forward(g["Q"], g["K"], g["V"], N_kv, 2, 0, 1)
+    h = tcapi.double_backward(g["g_dQ"], g["g_dK"], g["g_dV"], g["dO"], g["Q"], g["K"], g["V"], O, L, N_kv, 2, 0, 1)
+    # sums of 400 terms in fp32 are off by some 1e-6 of the sum's terms, a 2^10-th (f16) of the step from one result to the
+    # next: few results are rounded to the other side
+    for got, n in zip(h, ("g_dO", "g_Q", "g_K", "g_V")):
+        assert float((got.cpu() != ref[n].to(dtype)).float().mean()) <= 0.02, n
