@@ -400,6 +400,8 @@ fwd_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Tensors
         redo = __any_sync(0xffffffffu, !(tile_sum <= kMaxSum<T>));
       }
       if (redo) {
+        // the first attempt's P is on its way to the columns the second one goes to: stores are asynchronous
+        if (!CF::kTakeMax) tmem_st_wait();
         // maximum of the raw scores (-inf where masked) in eight independent chains
         float mx8[8];
 #pragma unroll

@@ -71,3 +71,23 @@ def test_forward_when_scores_grow_along_the_keys(H, N, D, dtype):
         assert torch.allclose(L.double(), want_L, rtol=1e-5, atol=1e-4), mask
         tol = {torch.bfloat16: 2 ** -7, torch.float16: 2 ** -10}[dtype]
         assert float((O.double() - want_O).abs().max()) <= tol * float(V.double().abs().max()), mask
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("H,N,D", [(8, 768, 64), (160, 512, 64), (100, 384, 128)])      # one and two CTAs per SM
+def test_tiles_done_again_keep_their_second_result(H, N, D, dtype):
+    """Every tile of 64 keys is far above the one before it, so that the forward does every tile of a
+    row twice: what stays must be the second P, bit for bit the same in every run."""
+    inp = orc.make_inputs(1, H, N, N, D, seed=7, dtype=torch.float32)
+    Q = torch.full((1, H, N, D), 0.25) + 0.01 * inp["Q"]
+    K = ((torch.arange(N) // 64).view(1, 1, N, 1) * (80.0 / D ** 0.5) + 0.01 * inp["K"]).to(dtype)      # 28 log2 units a tile
+    Q, V = Q.to(dtype), inp["V"].to(dtype)
+    q, k, v = Q.cuda(), K.cuda(), V.cuda()
+    first, L = tcapi.forward(q, k, v, N, 0, 1)
+    S = torch.einsum("bhid,bhjd->bhij", q.double(), k.double()) / D ** 0.5
+    want = torch.softmax(S, -1) @ v.double()
+    assert torch.allclose(L.double(), torch.logsumexp(S, -1), rtol=1e-5, atol=1e-4)
+    tol = {torch.bfloat16: 2 ** -7, torch.float16: 2 ** -10}[dtype]      # as above
+    assert float((first.double() - want).abs().max()) <= tol * float(v.double().abs().max())
+    for _ in range(50):
+        assert torch.equal(tcapi.forward(q, k, v, N, 0, 1)[0], first)
