@@ -1,4 +1,4 @@
-// Forward attention (O, L) on sm_100a in ONE pass: online softmax with the running maximum kept
+// Forward attention (O, L) on sm_100a in ONE pass: online softmax with the reference exponent kept
 // per row, O accumulated in tensor memory and rescaled there only when the maximum has grown by
 // more than a threshold (f16/bf16, D a multiple of 16 up to 128).
 //
@@ -12,13 +12,18 @@
 // never have to agree while the loop runs; the epilogue merges them:
 // O = (O_0 2^(m_0 - m) + O_1 2^(m_1 - m)) / (l_0 2^(m_0 - m) + l_1 2^(m_1 - m)).
 // Rescaling is lazy: m is a reference, not the maximum.  A row's first visible tile sets it to its
-// maximum; later tiles are exponentiated against it as it stands, and only where a row's sum over a
-// tile exceeds 2^tau does its warp take the maximum, multiply the O row in tensor memory by
-// 2^(m_old - m_new) (a read-modify-write by its owner thread, after the group's previous P V product
-// has completed) and do the tile again.  So no maximum is taken in nearly all tiles (D = 64: -4 to
-// -6 %).  tau is as large as P's type allows: P has the same relative precision whatever its exponent,
-// in bf16 up to far beyond any sum that occurs, so 24 (O and l stay below 2^24 N |V|); in f16 15, one
-// below the largest exponent.
+// maximum; a later tile moves it, to that tile's maximum, only where that is more than tau above it, and
+// then the O row in tensor memory is multiplied by 2^(m_old - m_new) (a read-modify-write by its owner
+// thread, after the group's previous P V product has completed).  A tile is exponentiated against m as
+// it stands, and its maximum taken only where a row's sum exceeds 2^tau, without which no score can be
+// more than tau above m.  So no maximum is taken in nearly all tiles (D = 64: -4 to -6 %).
+// tau is a question of precision: the largest P of a row whose m is its maximum is 1, which the half
+// types hold exactly, and a peaked row is little else than that P.  With 8 for two groups (each has a maximum of its own) and 6 for
+// one, whose streams of up to six tiles follow their maximum exactly, O is as close to the exact one as
+// taking every maximum with a threshold of 8 in two groups was: relative error 2.02e-3 at H32 N16384 D128, Q
+// and K of twice unit variance, where 24 gave 2.32e-3 and a rounded result alone is 1.66e-3.  The price, for
+// peaked rows: 2.34 instead of 1.83 ms there, 126 instead of 91 us at B8 H12 N2048 D64; for short streams 26
+// instead of 24 us at B4 H16 N1024 D128; inputs of unit variance stay at 91 us at B8 H12 N2048 D64.
 // Tensor memory, one CTA per SM (512 columns): three score buffers S0, S1, S2 [0,192), Q [192,192+D/2),
 // O_0 [256,256+D), O_1 [256+D, 256+2D); two per SM (256 columns): S0, S1 [0,128), Q behind them at
 // D = 64 (at D = 128 it stays in shared memory), O.  P is written (two halves per 32-bit column) over the
@@ -36,8 +41,6 @@ namespace tc {
 
 constexpr int kFwdMaxStages = 8;
 constexpr int kFwdMaxSBufs = 3;
-template <typename T> constexpr float kTau = Pack<T>::kIsBf16 ? 24.f : 15.f;     // log2 units
-template <typename T> constexpr float kMaxSum = Pack<T>::kIsBf16 ? 16777216.f : 32768.f;     // 2^tau
 constexpr int KFWD = 20;            // kernel id inside device status codes
 
 struct FwdControl {
@@ -66,6 +69,10 @@ struct FwdCfg {
   // take the maximum of every tile instead of trying the reference as it stands (one CTA per SM at
   // D = 128, where that is faster: 109 against 118 us at H32, 1024 queries, 9216 keys, D80)
   static constexpr bool kTakeMax = G == 2 && D == 128;
+  // how far (log2 units) a score may be above a row's reference exponent; 2^kTau; and the longest stream
+  // whose reference follows the maximum from tile to tile
+  static constexpr float kTau = G == 2 ? 8.f : 6.f, kMaxSum = G == 2 ? 256.f : 64.f;
+  static constexpr int kExactTiles = G == 2 ? 0 : 6;
   static constexpr bool kQTmem = !(G == 1 && D == 128);     // Q moves to tensor memory where it has room
   static constexpr int kAtoms = D / 64;
   static constexpr uint32_t kStagingBytes = kAtoms * kAtomBytesStat;        // Q, later the O tile
@@ -344,7 +351,10 @@ fwd_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Tensors
       if (lane == 0) mbar_arrive(bar_q_ready);
     }
 
-    float m_ref = -INFINITY, l_sum = 0.f;     // this group's running maximum (log2 units) and sum for the row
+    float m_ref = -INFINITY, l_sum = 0.f;     // this group's reference exponent (log2 units) and sum for the row
+    const bool exact = n_iter <= CF::kExactTiles;
+    const float tau = exact ? 0.f : CF::kTau;
+    bool need_max = true;      // a row of the warp has no reference yet, or moved its own in the last tile and is likely to again
     const uint32_t oacc = lane_addr + CF::kO + (uint32_t)(grp * D);
     for (int it = grp; it < n_iter && ok; it += G) {
       const int b = it % kFwdSBufs;
@@ -392,16 +402,14 @@ fwd_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Tensors
         }
         tile_sum = (sum_a.x + sum_a.y) + (sum_b.x + sum_b.y);
       };
-      // The reference is tried as it stands; only where the row sums show that it is too low (or a row
-      // has none yet) is the maximum taken and the tile done again.
-      bool redo = CF::kTakeMax || __any_sync(0xffffffffu, m_ref == -INFINITY);
-      if (!redo) {
+      // The reference is tried as it stands, unless the maximum is likely to be needed.
+      const bool attempt = !CF::kTakeMax && !exact && !need_max;
+      bool take_max = true;
+      if (attempt) {
         exponentials(-m_ref);
-        redo = __any_sync(0xffffffffu, !(tile_sum <= kMaxSum<T>));
+        take_max = __any_sync(0xffffffffu, !(tile_sum <= CF::kMaxSum));
       }
-      if (redo) {
-        // the first attempt's P is on its way to the columns the second one goes to: stores are asynchronous
-        if (!CF::kTakeMax) tmem_st_wait();
+      if (take_max) {
         // maximum of the raw scores (-inf where masked) in eight independent chains
         float mx8[8];
 #pragma unroll
@@ -412,9 +420,11 @@ fwd_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Tensors
           for (int e = 0; e < 8; ++e) mx8[e] = fmaxf(mx8[e], fmaxf(__uint_as_float(s_[c][e]), __uint_as_float(s_[c][8 + e])));
         const float mx = fmaxf(fmaxf(fmaxf(mx8[0], mx8[1]), fmaxf(mx8[2], mx8[3])), fmaxf(fmaxf(mx8[4], mx8[5]), fmaxf(mx8[6], mx8[7]))) *
                          g.scale_log2e;
-        // (a row above the limit has a score of at least m + tau - 6)
-        const bool grow = mx > m_ref + (CF::kTakeMax ? kTau<T> : 0.5f * kTau<T>) || (m_ref == -INFINITY && mx > -INFINITY);
-        if (__any_sync(0xffffffffu, grow)) {
+        // a row's own scores alone decide whether its reference moves
+        const bool grow = mx > m_ref + tau || (m_ref == -INFINITY && mx > -INFINITY);
+        const bool any_grow = __any_sync(0xffffffffu, grow);
+        need_max = __any_sync(0xffffffffu, grow == (m_ref > -INFINITY));      // moved, or still without one
+        if (any_grow) {
           const float m_new = grow ? mx : m_ref;
           const float f = (m_ref == -INFINITY) ? 0.f : ex2(m_ref - m_new);   // 1 for the rows that do not move
           l_sum *= f;
@@ -443,7 +453,11 @@ fwd_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Tensors
             }
           }
         }
-        exponentials((m_ref == -INFINITY) ? 0.f : -m_ref);    // no visible key yet: every score is -inf, every p 0
+        // (an attempt that no row moves after stands)
+        if (!attempt || any_grow) {
+          if (attempt) tmem_st_wait();      // its P is on its way to the same columns: stores are asynchronous
+          exponentials((m_ref == -INFINITY) ? 0.f : -m_ref);    // no visible key yet: every score is -inf, every p 0
+        }
       }
       l_sum += tile_sum;
       tmem_st_wait();
