@@ -150,8 +150,9 @@ __device__ __forceinline__ void reduce_parts(float* partial, int split, int part
     const int row = i / chunks, chunk = i - row * chunks;
     float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
     for (int q = 0; q < split; ++q) {
-      const float4 x = *reinterpret_cast<const float4*>(cluster.map_shared_rank(partial, q) + partial_at<DT>(row, chunk));
       const float w = weight(q, row);
+      if (!(w > 0.f)) continue;      // a part without weight is never read as a number, as in the epilogue of an unsplit tile
+      const float4 x = *reinterpret_cast<const float4*>(cluster.map_shared_rank(partial, q) + partial_at<DT>(row, chunk));
       v.x = fmaf(x.x, w, v.x); v.y = fmaf(x.y, w, v.y); v.z = fmaf(x.z, w, v.z); v.w = fmaf(x.w, w, v.w);
     }
     post(row, 4 * chunk, v);

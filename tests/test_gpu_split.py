@@ -110,3 +110,20 @@ def test_forward_of_peaked_rows_is_as_exact_as_its_type(B, H, N, D, dtype, bound
         err += float((O[b, h].double() - want).pow(2).sum())
         norm += float(want.pow(2).sum())
     assert (err / norm) ** 0.5 <= bound
+
+
+def test_split_rows_without_a_sum_are_those_of_the_unsplit_kernel():
+    """One key with an infinite element: rows whose score with it is +inf have no sum (L = -inf) and get
+    zeros, split or not; rows whose score is -inf do not see the key."""
+    N, D = 2048, 64
+    inp = orc.make_inputs(1, 1, 128, N, D, seed=9, dtype=torch.bfloat16)
+    Q, K, V = (inp[n].cuda() for n in ("Q", "K", "V"))
+    K[0, 0, 70, 3] = float("inf")
+    many = [t.expand(1, 160, -1, -1).contiguous() for t in (Q, K, V)]
+    for q, k, v in ((Q, K, V), many):
+        O, L = tcapi.forward(q, k, v, N, 15, 1)
+        lost = Q[0, 0, :, 3] > 0
+        assert bool(torch.isneginf(L[0, 0, lost]).all()) and float(O[0, 0, lost].float().abs().max()) == 0.0
+        S = (Q[0, 0].double() @ K[0, 0].double().T / D ** 0.5)[~lost]
+        want = torch.softmax(S, -1) @ V[0, 0].double()
+        assert float((O[0, 0, ~lost].double() - want).abs().max()) <= 2 ** -7 * float(V.double().abs().max())
