@@ -94,7 +94,7 @@ template <typename T> struct Pairs;
 template <> struct Pairs<float> {
   using P = float2;
   static __device__ __forceinline__ void load(const float* p, P (&v)[4]) {
-    const float4 a = __ldg(reinterpret_cast<const float4*>(p)), b = __ldg(reinterpret_cast<const float4*>(p) + 1);
+    const float4 a = reinterpret_cast<const float4*>(p)[0], b = reinterpret_cast<const float4*>(p)[1];
     v[0] = make_float2(a.x, a.y); v[1] = make_float2(a.z, a.w); v[2] = make_float2(b.x, b.y); v[3] = make_float2(b.z, b.w);
   }
   static __device__ __forceinline__ void store(float* p, const P (&v)[4]) {
@@ -109,7 +109,7 @@ template <> struct Pairs<float> {
 template <> struct Pairs<__half> {
   using P = __half2;
   static __device__ __forceinline__ void load(const __half* p, P (&v)[4]) {
-    const uint4 q = __ldg(reinterpret_cast<const uint4*>(p));
+    const uint4 q = *reinterpret_cast<const uint4*>(p);
     v[0] = *reinterpret_cast<const P*>(&q.x); v[1] = *reinterpret_cast<const P*>(&q.y);
     v[2] = *reinterpret_cast<const P*>(&q.z); v[3] = *reinterpret_cast<const P*>(&q.w);
   }
@@ -125,7 +125,7 @@ template <> struct Pairs<__half> {
 template <> struct Pairs<__nv_bfloat16> {
   using P = __nv_bfloat162;
   static __device__ __forceinline__ void load(const __nv_bfloat16* p, P (&v)[4]) {
-    const uint4 q = __ldg(reinterpret_cast<const uint4*>(p));
+    const uint4 q = *reinterpret_cast<const uint4*>(p);
     v[0] = *reinterpret_cast<const P*>(&q.x); v[1] = *reinterpret_cast<const P*>(&q.y);
     v[2] = *reinterpret_cast<const P*>(&q.z); v[3] = *reinterpret_cast<const P*>(&q.w);
   }
@@ -153,8 +153,7 @@ constexpr int kPrepHeads = 4;      // heads a lane group walks over for its toke
 // into are then compiled out (they were a third of the instructions of an issue-bound kernel).
 template <typename T, int G, bool kFast>
 __global__ void __launch_bounds__(kPrepThreads)
-qk_norm_rope_vec8_kernel(const T* __restrict__ x, const T* __restrict__ weight, const float* __restrict__ freqs,
-                         T* __restrict__ out, int n_tok, int H, int d, int pos0, int norm_from, float eps) {
+qk_norm_rope_vec8_kernel(const T* x, const T* weight, const float* freqs, T* out, int n_tok, int H, int d, int pos0, int norm_from, float eps) {
   using PR = Pairs<T>;
   using P = typename PR::P;
   tc::pdl_wait();
@@ -182,7 +181,7 @@ qk_norm_rope_vec8_kernel(const T* __restrict__ x, const T* __restrict__ weight, 
   P w[4];                     // its eight weights
   if (active) {
     const float4* f = reinterpret_cast<const float4*>(freqs + ((size_t)(pos0 + tok) * (d >> 1) + sub * 4) * 2);
-    const float4 f0 = __ldg(f), f1 = __ldg(f + 1);
+    const float4 f0 = f[0], f1 = f[1];
     cs[0] = f0.x; cs[1] = f0.y; cs[2] = f0.z; cs[3] = f0.w; cs[4] = f1.x; cs[5] = f1.y; cs[6] = f1.z; cs[7] = f1.w;
     if (norm) PR::load(weight + sub * 8, w);
   }
@@ -247,8 +246,7 @@ constexpr int kPrepMaxCtas = 592;      // four CTAs on each of 148 SMs: rows of 
 
 template <typename T, int G>
 __global__ void __launch_bounds__(kPrepThreads)
-qk_norm_rope_bwd_kernel(const T* __restrict__ x, const T* __restrict__ weight, const float* __restrict__ freqs,
-                        const T* __restrict__ g, T* __restrict__ gx, float* __restrict__ partial, int n_tok, int H, int d,
+qk_norm_rope_bwd_kernel(const T* x, const T* weight, const float* freqs, const T* g, T* gx, float* partial, int n_tok, int H, int d,
                         int pos0, int norm_from, float eps) {
   using PR = Pairs<T>;
   using P = typename PR::P;
@@ -290,7 +288,7 @@ qk_norm_rope_bwd_kernel(const T* __restrict__ x, const T* __restrict__ weight, c
     float cs[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     if (active) {
       const float4* f = reinterpret_cast<const float4*>(freqs + ((size_t)(pos0 + tok) * (d >> 1) + sub * 4) * 2);
-      const float4 f0 = __ldg(f), f1 = __ldg(f + 1);
+      const float4 f0 = f[0], f1 = f[1];
       cs[0] = f0.x; cs[1] = f0.y; cs[2] = f0.z; cs[3] = f0.w; cs[4] = f1.x; cs[5] = f1.y; cs[6] = f1.z; cs[7] = f1.w;
     }
 #pragma unroll
@@ -351,7 +349,7 @@ qk_norm_rope_bwd_kernel(const T* __restrict__ x, const T* __restrict__ weight, c
 // gw[c] = sum of the `rows` rows of `partial`: 32 columns per CTA, 32 interleaved row sums per column
 template <typename T>
 __global__ void __launch_bounds__(1024)
-qk_weight_grad_kernel(const float* __restrict__ partial, T* __restrict__ gw, int rows, int d) {
+qk_weight_grad_kernel(const float* partial, T* gw, int rows, int d) {
   __shared__ float sums[32][33];
   tc::pdl_wait();
   tc::pdl_trigger();

@@ -31,7 +31,7 @@ template <> __device__ __forceinline__ float2 widen_pair<__half>(uint32_t w) {
 
 template <typename T, int G>
 __global__ void __launch_bounds__(256)
-rowdot_kernel(const T* __restrict__ a, const T* __restrict__ b, float* __restrict__ out, long long rows, int D) {
+rowdot_kernel(const T* a, const T* b, float* out, long long rows, int D) {
   pdl_wait();
   pdl_trigger();
   const int sub = threadIdx.x % G;
@@ -42,8 +42,8 @@ rowdot_kernel(const T* __restrict__ a, const T* __restrict__ b, float* __restric
   for (int i = 0; i < kRowdotRows; ++i) {
     va[i] = vb[i] = make_uint4(0u, 0u, 0u, 0u);
     if (lane_on && r0 + i < rows) {
-      va[i] = __ldg(reinterpret_cast<const uint4*>(a + (r0 + i) * D + sub * 8));
-      vb[i] = __ldg(reinterpret_cast<const uint4*>(b + (r0 + i) * D + sub * 8));
+      va[i] = *reinterpret_cast<const uint4*>(a + (r0 + i) * D + sub * 8);
+      vb[i] = *reinterpret_cast<const uint4*>(b + (r0 + i) * D + sub * 8);
     }
   }
 #pragma unroll

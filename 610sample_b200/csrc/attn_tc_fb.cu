@@ -432,7 +432,7 @@ fb_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Tensors 
       const int qi = (t_begin + tile_it) * BN + c;
       float raw = (which == 0) ? INFINITY : 0.f;      // beyond N_q: L = +inf (p = 0), Dv = 0
       if (CF::kCol && threadIdx.x < 128 && tile_it < n_iter && qi < g.N_q)
-        raw = (which == 0) ? __ldg(t.L + row_off + qi) : __ldg(t.Dv + row_off + qi);
+        raw = (which == 0) ? t.L[row_off + qi] : t.Dv[row_off + qi];
       return raw;
     };
     auto publish_stat = [&](int tile_it, float raw) {

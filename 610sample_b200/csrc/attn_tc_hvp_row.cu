@@ -795,7 +795,7 @@ hvp_row_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Ten
                          [](int, int) { return 1.f; },
                          [&](int row, int col, float4& v) {
                            if constexpr (MODE == ROW_PREDO) {
-                             const uint2 w = __ldg(reinterpret_cast<const uint2*>(O_rows + (size_t)row * g.D + col));
+                             const uint2 w = *reinterpret_cast<const uint2*>(O_rows + (size_t)row * g.D + col);
                              const float2 a = Pack<T>::unpack(w.x), b = Pack<T>::unpack(w.y);
                              const float d = -part_dot2[row];
                              v.x = fmaf(d, a.x, v.x); v.y = fmaf(d, a.y, v.y); v.z = fmaf(d, b.x, v.z); v.w = fmaf(d, b.y, v.w);

@@ -59,7 +59,9 @@ template <> struct Pack<__half> {
 // Launches and the order between them.  Every tensor-core kernel is launched with programmatic
 // stream serialization: its CTAs may become resident while the predecessor in the stream still
 // runs, set up their barriers and tensor memory, and wait (pdl_wait) before the first access to
-// global memory.  Each CTA triggers its successor right after that wait.  A kernel that only has to
+// global memory.  What they read may therefore be written while they are already running: it goes through
+// ordinary loads, never through the read-only path (__ldg, const __restrict__), which a compiler may
+// move above the wait.  Each CTA triggers its successor right after that wait.  A kernel that only has to
 // come after the predecessor of its predecessor (Geometry::beside) skips the wait at its start: it
 // is launched when every CTA of the predecessor has passed ITS wait, so everything before the
 // predecessor is complete, and its CTAs take the SMs the predecessor's last CTAs leave idle.  Its

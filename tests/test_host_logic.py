@@ -132,3 +132,16 @@ def test_two_rank_gloo_sharding():
         assert p.exitcode == 0
     same, slow = out.get()
     assert same and slow == 2.0
+
+
+def test_kernels_that_start_early_do_not_use_the_read_only_path():
+    """Kernels launched with programmatic stream serialization run while their inputs may still be written,
+    so those inputs are not read-only for their lifetime.  The two kernels launched the ordinary way
+    may use the read-only path."""
+    import re
+    csrc = os.path.join(os.path.dirname(os.path.abspath(att.__file__)), "csrc")
+    for name in sorted(os.listdir(csrc)):
+        with open(os.path.join(csrc, name)) as f:
+            code = re.sub(r"//[^\n]*", "", f.read())
+        code = re.sub(r"(qk_norm_rope_kernel|selftest_gemm_kernel)\(.*?\)\s*\{", "", code, flags=re.S)
+        assert not re.search(r"__ldg\(|__restrict__|ld\.global\.nc", code), name
