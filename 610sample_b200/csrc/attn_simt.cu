@@ -79,7 +79,7 @@ __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wai
 
 // Four consecutive elements of a half-precision row, widened.
 template <typename T> __device__ __forceinline__ float4 widen4(const T* p) {
-  const uint2 w = *reinterpret_cast<const uint2*>(p);
+  const uint2 w = tc::from_l2(reinterpret_cast<const uint2*>(p));
   const float2 a = tc::Pack<T>::unpack(w.x), b = tc::Pack<T>::unpack(w.y);
   return make_float4(a.x, a.y, b.x, b.y);
 }
@@ -198,7 +198,7 @@ template <typename T> __device__ __forceinline__ void store4(T* p, const float4&
 }
 template <> __device__ __forceinline__ void store4<float>(float* p, const float4& v) { *reinterpret_cast<float4*>(p) = v; }
 template <typename T> __device__ __forceinline__ float4 load4(const T* p) { return widen4<T>(p); }
-template <> __device__ __forceinline__ float4 load4<float>(const float* p) { return *reinterpret_cast<const float4*>(p); }
+template <> __device__ __forceinline__ float4 load4<float>(const float* p) { return tc::from_l2(reinterpret_cast<const float4*>(p)); }
 
 // shared memory in floats
 template <int KIND>
@@ -273,9 +273,9 @@ __global__ void __launch_bounds__(threads_of(DC), DC == 1 ? 2 : 1) attn_simt_ker
     for (int a = 0; a < RA; ++a) {
       const int r = r0 + row0 + 4 * a;
       const bool in = r < g.N_q;
-      L2[a] = in ? t.L[row_off + r] * kLog2e : INFINITY;
+      L2[a] = in ? tc::from_l2(t.L + row_off + r) * kLog2e : INFINITY;
       if constexpr (KIND == K_HVP_ROW) {
-        if (in) { Dv[a] = t.Dv[row_off + r]; d2[a] = t.dot2[row_off + r]; d3[a] = t.dot3[row_off + r]; }
+        if (in) { Dv[a] = tc::from_l2(t.Dv + row_off + r); d2[a] = tc::from_l2(t.dot2 + row_off + r); d3[a] = tc::from_l2(t.dot3 + row_off + r); }
       }
       if constexpr (KIND == K_BWD_ROW) {      // D_i = sum_d dO * O from the stored (rounded) O
         float s = 0.f;
@@ -311,7 +311,7 @@ __global__ void __launch_bounds__(threads_of(DC), DC == 1 ? 2 : 1) attn_simt_ker
         for (int i = tid; i < 4 * TT; i += NT) {
           const int r = s0 + (i & 63), which = i >> 6;
           const float* src = which == 0 ? t.L : which == 1 ? t.Dv : which == 2 ? t.dot2 : t.dot3;
-          const float v = r < g.N_q ? src[row_off + r] : 0.f;
+          const float v = r < g.N_q ? tc::from_l2(src + row_off + r) : 0.f;
           aux[i] = which == 0 ? (r < g.N_q ? v * kLog2e : INFINITY) : v;
         }
       } else {
@@ -326,7 +326,7 @@ __global__ void __launch_bounds__(threads_of(DC), DC == 1 ? 2 : 1) attn_simt_ker
 #pragma unroll
         for (int o = TQ / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
         if (tid % TQ == 0) {
-          aux[tid / TQ] = r < g.N_q ? t.L[row_off + r] * kLog2e : INFINITY;
+          aux[tid / TQ] = r < g.N_q ? tc::from_l2(t.L + row_off + r) * kLog2e : INFINITY;
           aux[TT + tid / TQ] = s;
         }
       }

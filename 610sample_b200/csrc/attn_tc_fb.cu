@@ -415,7 +415,7 @@ fb_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Tensors 
     float2 nL2 = make_float2(-INFINITY, -INFINITY), nDv = make_float2(0.f, 0.f);
     if constexpr (KIND == FB_BWD_ROW) {
       if (gidx < g.N_q) {
-        const float L2 = t.L[row_off + gidx] * kLog2e, Dv = t.Dv[row_off + gidx];
+        const float L2 = from_l2(t.L + row_off + gidx) * kLog2e, Dv = from_l2(t.Dv + row_off + gidx);
         nL2 = make_float2(-L2, -L2);
         nDv = make_float2(-Dv, -Dv);
       }
@@ -432,7 +432,7 @@ fb_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Tensors 
       const int qi = (t_begin + tile_it) * BN + c;
       float raw = (which == 0) ? INFINITY : 0.f;      // beyond N_q: L = +inf (p = 0), Dv = 0
       if (CF::kCol && threadIdx.x < 128 && tile_it < n_iter && qi < g.N_q)
-        raw = (which == 0) ? t.L[row_off + qi] : t.Dv[row_off + qi];
+        raw = from_l2((which == 0 ? t.L : t.Dv) + row_off + qi);
       return raw;
     };
     auto publish_stat = [&](int tile_it, float raw) {

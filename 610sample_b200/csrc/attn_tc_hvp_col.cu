@@ -398,10 +398,10 @@ hvp_col_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Ten
       const int qi = (t_begin + tile_it) * BN + qc;
       float3 raw = make_float3((which == 0) ? INFINITY : 0.f, 0.f, 0.f);   // beyond N_q: L = +inf (p = 0), the rest 0
       if (tile_it < n_iter && qi < g.N_q) {
-        if (which == 0) raw.x = t.L[row_off + qi];
-        else if (which == 1) raw.x = t.dot2[row_off + qi];
-        else if (which == 2) raw.x = t.Dv[row_off + qi];
-        else { raw.x = t.dot2[row_off + qi]; raw.y = t.Dv[row_off + qi]; raw.z = t.dot3[row_off + qi]; }
+        if (which == 0) raw.x = from_l2(t.L + row_off + qi);
+        else if (which == 1) raw.x = from_l2(t.dot2 + row_off + qi);
+        else if (which == 2) raw.x = from_l2(t.Dv + row_off + qi);
+        else { raw.x = from_l2(t.dot2 + row_off + qi); raw.y = from_l2(t.Dv + row_off + qi); raw.z = from_l2(t.dot3 + row_off + qi); }
       }
       return raw;
     };

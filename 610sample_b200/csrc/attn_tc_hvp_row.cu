@@ -529,11 +529,11 @@ hvp_row_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Ten
     float2 nL2 = make_float2(-INFINITY, -INFINITY), nDv = make_float2(0.f, 0.f);
     float2 nD2 = make_float2(0.f, 0.f), nC3 = make_float2(0.f, 0.f);
     if (gidx < g.N_q) {
-      const float L2 = t.L[row_off + gidx] * kLog2e;
+      const float L2 = from_l2(t.L + row_off + gidx) * kLog2e;
       nL2 = make_float2(-L2, -L2);
       if constexpr (MODE == ROW_Q) {
-        const float Dv = t.Dv[row_off + gidx], d2 = t.dot2[row_off + gidx];
-        const float c3 = fmaf(d2, Dv, t.dot3[row_off + gidx]);
+        const float Dv = from_l2(t.Dv + row_off + gidx), d2 = from_l2(t.dot2 + row_off + gidx);
+        const float c3 = fmaf(d2, Dv, from_l2(t.dot3 + row_off + gidx));
         nDv = make_float2(-Dv, -Dv); nD2 = make_float2(-d2, -d2); nC3 = make_float2(-c3, -c3);
       }
     }

@@ -66,7 +66,9 @@ template <> struct Pack<__half> {
 // is launched when every CTA of the predecessor has passed ITS wait, so everything before the
 // predecessor is complete, and its CTAs take the SMs the predecessor's last CTAs leave idle.  Its
 // last CTA waits at its end instead, so that this kernel never completes before its predecessor
-// and whatever follows in the stream may rely on both.  A second stream with an event fork and join does the same for 4 us more
+// and whatever follows in the stream may rely on both.  Without the wait at its start nothing is promised
+// about what an SM's L1 holds, so such a kernel reads global memory through L2 only, where every write of
+// a completed kernel is: TMA, cp.async.cg, and from_l2 for the rest.  A second stream with an event fork and join does the same for 4 us more
 // of host time and a launch latency on either side, and cannot be used under stream capture.
 __device__ __forceinline__ void pdl_begin(const Geometry& g) { if (!g.beside) pdl_wait(); }
 // A persistent kernel's last CTA may have been taken over by another one, so there every CTA waits.
@@ -76,6 +78,8 @@ __device__ __forceinline__ void pdl_end_persistent(const Geometry& g) {
 __device__ __forceinline__ void pdl_end(const Geometry& g) {
   if (g.beside && blockIdx.x + 1 == gridDim.x && threadIdx.x == 0) pdl_wait();
 }
+
+template <typename V> __device__ __forceinline__ V from_l2(const V* p) { return __ldcg(p); }
 
 // Opt-in to `smem` bytes of dynamic shared memory, once per kernel and device (`done`: one bit per device).
 template <typename Kern>

@@ -9,6 +9,7 @@
 * guard bands: every output, L and the scratch are carved out of NaN-filled buffers at ragged
   shapes; after the calls the bands are untouched (plain stores and TMA stores alike);
 * the phase masks of the double backward reproduce the one-call result bit for bit;
+* calls with two sets of inputs in turn over one scratch, without a synchronisation in between;
 * a call on a thread whose current context was taken away since its last call binds the device again;
 * a call captured into a CUDA graph on one host thread while another thread calls eagerly;
 * a thousand back-to-back calls of the three operations at shapes with many CTAs per SM: no
@@ -257,3 +258,40 @@ def test_repeated_calls_stay_bit_identical_and_never_time_out(shape):
         assert capi.device_status() == 0
         for a, b in zip(outs, first):
             assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("BH,N_q,N_kv,D,ws,cid,dtype", [
+    (96, 512, 512, 64, 512, 0, torch.bfloat16),       # two CTAs per SM, column kernels first
+    (24, 640, 640, 128, 640, 0, torch.float16),       # few tiles, D = 128
+    (24, 1024, 1024, 128, 1024, 0, torch.float16),    # persistent query-side kernels
+    (8, 256, 2304, 64, 2048, 9, torch.bfloat16),      # chunk: row kernels first, split over clusters
+    (12, 200, 200, 64, 200, 0, torch.float32),        # the CUDA-core family
+])
+def test_inputs_in_turn_over_one_scratch(BH, N_q, N_kv, D, ws, cid, dtype):
+    """The second of two kernels that run side by side starts without waiting for the first, and reads
+    row scalars that a kernel before both has just written over those of the call before.  Two sets of
+    inputs in turn, all calls queued at once: a scalar of the other set would show."""
+    sets = []
+    for seed in (61, 62):
+        inp = orc.make_inputs(1, BH, N_q, N_kv, D, seed=seed, dtype=dtype)
+        sets.append({n: t.to(DEV) * (1 if seed == 61 else 2) for n, t in inp.items()})
+    O_L = [tcapi.forward(g["Q"], g["K"], g["V"], ws, cid) for g in sets]
+    s = tcapi._shape(sets[0]["Q"], sets[0]["K"], ws, cid, 0, 0)
+    scratch = torch.empty(capi.lib().attn_b200_double_backward_scratch_bytes(s) // 4 + 4, dtype=torch.float32, device=DEV)
+
+    def once(i, scratch):
+        g, (O, L) = sets[i], O_L[i]
+        b = tcapi.backward(g["dO"], g["Q"], g["K"], g["V"], O, L, ws, cid, scratch=scratch)
+        h = tcapi.double_backward(g["g_dQ"], g["g_dK"], g["g_dV"], g["dO"], g["Q"], g["K"], g["V"], O, L, ws, cid, scratch=scratch)
+        return tuple(b) + tuple(h)
+
+    want = []
+    for i in range(2):
+        want.append(once(i, torch.full_like(scratch, float("nan"))))
+        torch.cuda.synchronize()
+    for _ in range(10):
+        got = [once(i % 2, scratch) for i in range(20)]
+        for i, outs in enumerate(got):
+            for a, b in zip(outs, want[i % 2]):
+                assert torch.equal(a, b), i
+    assert capi.device_status() == 0
