@@ -215,17 +215,20 @@ inline SplitLoad stream_load(const Geometry& g, bool col, float tile_clocks) {
   return {(float)g.BH * tiles, (float)most, tiles > 0 ? (float)sum / tiles : 0.f, tile_clocks};
 }
 
-// What a kernel's launches keep: the devices its shared-memory opt-in has been made on, and the CTAs
-// that run at a time in clusters of each size.
+// What a kernel's launches keep: the devices its shared-memory opt-in has been made on, and by device
+// the CTAs that run at a time in clusters of each size (0: not asked for yet).
 struct TileKernelState {
   std::atomic<unsigned long long> smem_set{0}, smem_set_split{0};
-  std::atomic<int> slots[kMaxSplit + 1] = {};
+  std::atomic<int> slots[64][kMaxSplit + 1] = {};
 };
 
-// CTAs of `kern` that run at a time in clusters of c (asked for once per kernel and size).
+// CTAs of `kern` that run at a time in clusters of c on the current device; 0 where that cannot be told.
 template <typename Kern>
 inline int cluster_slots(Kern kern, int c, unsigned threads, size_t smem, TileKernelState& state) {
-  int n = state.slots[c].load(std::memory_order_relaxed);
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return 0;
+  std::atomic<int>& known = state.slots[dev & 63][c];
+  int n = known.load(std::memory_order_relaxed);
   if (n == 0) {
     cudaLaunchAttribute attr;
     attr.id = cudaLaunchAttributeClusterDimension;
@@ -241,10 +244,10 @@ inline int cluster_slots(Kern kern, int c, unsigned threads, size_t smem, TileKe
     if (set_smem_once(kern, smem, state.smem_set_split) != cudaSuccess ||
         cudaOccupancyMaxActiveClusters(&clusters, (const void*)kern, &cfg) != cudaSuccess) {
       (void)cudaGetLastError();
-      clusters = 0;
+      return 0;      // asked again by the next call
     }
     n = clusters > 0 ? clusters * c : -1;
-    state.slots[c].store(n, std::memory_order_relaxed);
+    known.store(n, std::memory_order_relaxed);
   }
   return n;
 }
