@@ -11,6 +11,7 @@ int failures = 0;
 void check(bool ok, const char* what) { if (!ok) { printf("failed: %s\n", what); ++failures; } }
 }  // namespace
 
+#ifndef __CUDA_ARCH__      // the device pass has its own
 extern "C" {
 cudaError_t CUDARTAPI cudaGetDevice(int* d) { *d = device; return cudaSuccess; }
 cudaError_t CUDARTAPI cudaFuncSetAttribute(const void*, cudaFuncAttribute, int) { return cudaSuccess; }
@@ -22,6 +23,7 @@ cudaError_t CUDARTAPI cudaOccupancyMaxActiveClusters(int* n, const void*, const 
 }
 cudaError_t CUDARTAPI cudaGetLastError(void) { return cudaSuccess; }
 }
+#endif
 
 using namespace attn;
 using namespace attn::tc;
