@@ -200,11 +200,16 @@ inline int pick_split(const SplitLoad& w, const SplitLoad* other, int D, Slots s
   return best;
 }
 
+// From every tile where there are up to 1024 (131072 rows), from that many evenly spaced ones above: every
+// launch pays for this on the host, some 10 ns a tile.
+constexpr int kLoadSamples = 1024;
 inline SplitLoad stream_load(const Geometry& g, bool col, float tile_clocks) {
   const int n = col ? g.N_kv : g.N_q, tiles = (n + BM - 1) / BM;
+  const int samples = tiles < kLoadSamples ? tiles : kLoadSamples;
   int most = 0;
   long long sum = 0;
-  for (int i = 0; i < tiles; ++i) {
+  for (int s = 0; s < samples; ++s) {
+    const int i = samples == tiles ? s : (int)((long long)s * (tiles - 1) / (samples - 1));
     int lo, hi;
     if (col) query_range_for_keys(g, i * BM, (i + 1) * BM, lo, hi);
     else key_range_for_queries(g, i * BM, (i + 1) * BM, lo, hi);
@@ -212,7 +217,7 @@ inline SplitLoad stream_load(const Geometry& g, bool col, float tile_clocks) {
     if (k > most) most = k;
     sum += k;
   }
-  return {(float)g.BH * tiles, (float)most, tiles > 0 ? (float)sum / tiles : 0.f, tile_clocks};
+  return {(float)g.BH * tiles, (float)most, samples > 0 ? (float)sum / samples : 0.f, tile_clocks};
 }
 
 // What a kernel's launches keep: the devices its shared-memory opt-in has been made on, and by device
@@ -337,8 +342,8 @@ __device__ __forceinline__ bool work_next(WorkControl* w, int n, int* unit, vola
 // B8 H12 N2048 D64 causal: forward 117 -> 92 us, backward 324 -> 267; B4 H16 N1024 D128 forward 36 ->
 // 25; B4 H16 N4096 D128 280 -> 253; B2 H8 N2048 D128 without mask (256 CTAs) 40 -> 36.
 inline bool two_per_sm_pays(const Geometry& g, bool col, bool alone, float tile_clocks, float tile_clocks_two) {
+  if ((long long)g.BH * (((col ? g.N_kv : g.N_q) + BM - 1) / BM) < kSms) return false;
   const SplitLoad w = stream_load(g, col, tile_clocks);
-  if (w.units < kSms) return false;
   auto larger = [](float x, float y) { return x > y ? x : y; };
   const float per_sm = w.units / kSms;
   const float waves = alone && w.mean > 0.9f * w.longest ? (float)(int)(per_sm + 0.999f) : per_sm;

@@ -2,6 +2,7 @@
 // defined here, ahead of the runtime library's.  Prints one line per check that fails.
 #include "tc_common.cuh"
 
+#include <chrono>
 #include <cstdio>
 
 namespace {
@@ -44,7 +45,41 @@ static void cluster_queries() {
   check(slots() == 40 && queries == before, "a known number is not asked for again");
 }
 
+static Geometry geometry(int BH, int N_q, int N_kv, int window, int mask_mode) {
+  Geometry g = {};
+  g.BH = BH; g.N_q = N_q; g.N_kv = N_kv; g.D = 64; g.ki_base = N_q - N_kv; g.window = window; g.mask_mode = mask_mode;
+  return g;
+}
+
+static void load_of_a_problem() {
+  const Geometry g = geometry(3, 1000, 1700, 600, 0);
+  for (int col = 0; col < 2; ++col) {
+    const SplitLoad w = stream_load(g, col != 0, 1.f);
+    const int n = col ? g.N_kv : g.N_q, tiles = (n + 127) / 128;
+    int most = 0, sum = 0;
+    for (int t = 0; t < tiles; ++t) {
+      int first = 1 << 30, last = -1;      // streamed tiles with a visible pair, one pair at a time
+      for (int a = t * 128; a < t * 128 + 128 && a < n; ++a)
+        for (int b = 0; b < (col ? g.N_q : g.N_kv); ++b)
+          if (col ? visible(g, b, a) : visible(g, a, b)) { first = b / 64 < first ? b / 64 : first; last = b / 64 > last ? b / 64 : last; }
+      const int k = last < 0 ? 0 : last - first + 1;
+      most = k > most ? k : most;
+      sum += k;
+    }
+    check(w.units == 3.f * tiles && w.longest == most && w.mean == (float)sum / tiles, "load of a small problem, tile by tile");
+  }
+  // A billion rows cost no more on the host than 131072, and the load is still that of the problem
+  const auto start = std::chrono::steady_clock::now();
+  const Geometry huge = geometry(1, 1 << 30, 1 << 30, 1 << 30, 0), narrow = geometry(1, 1 << 30, 1 << 30, 256, 0);
+  const SplitLoad w = stream_load(huge, false, 1.f), v = stream_load(narrow, true, 1.f);
+  check(!two_per_sm_pays(geometry(1, 1 << 12, 1 << 30, 1 << 30, 1), false, true, 850.f, 850.f), "few tiles: one CTA per SM");
+  check(std::chrono::steady_clock::now() - start < std::chrono::milliseconds(5), "host time of a long sequence");
+  check(w.longest == (float)(1 << 24) && w.mean > 0.99f * (1 << 23) && w.mean < 1.01f * (1 << 23), "load of a long sequence");
+  check(v.longest == 6.f && v.mean > 5.9f && v.mean <= 6.f, "load of a long sequence with a window");
+}
+
 int main() {
   cluster_queries();
+  load_of_a_problem();
   return failures;
 }
