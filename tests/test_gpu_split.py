@@ -1,7 +1,7 @@
 """Tensor-core kernels at the ends of the range of stationary tiles, against the fp64 closed form.
-Few: the streamed tiles of one are shared by a cluster of CTAs (every cluster size, shares that are
-empty or begin inside a masked range, rows that see no key in some shares or in none, both tile widths
-and types).  Many, at D <= 64: two CTAs per SM."""
+Few: the streamed tiles of one are shared by a cluster of CTAs (the cluster sizes that the rule takes,
+read from captured launches; shares without a tile or without a visible key; both tile widths and types).
+Many: two CTAs per SM, and persistent CTAs."""
 import importlib
 
 import pytest
@@ -13,18 +13,120 @@ pytestmark = pytest.mark.gpu
 tcapi = importlib.import_module("610sample_b200.torch_capi")
 capi = importlib.import_module("610sample_b200.capi")
 
+OUTPUTS = ("O", "dQ", "dK", "dV", "g_dO", "g_Q", "g_K", "g_V")
+# Operands P and dS and the results are rounded to the type, each to u = 2^-9 (bf16) or 2^-12 (f16) of itself: 4 u of
+# an output's norm, 8 u of its largest value for a single element.  A lost tile of 64 keys in 4096 is 12 % of the norm.
+UNIT = {torch.bfloat16: 2.0 ** -9, torch.float16: 2.0 ** -12}
+
+
+def _three_operations(g, window, chunk, mask):
+    O, L = tcapi.forward(g["Q"], g["K"], g["V"], window, chunk, mask)
+    b = tcapi.backward(g["dO"], g["Q"], g["K"], g["V"], O, L, window, chunk, mask)
+    h = tcapi.double_backward(g["g_dQ"], g["g_dK"], g["g_dV"], g["dO"], g["Q"], g["K"], g["V"], O, L, window, chunk, mask)
+    return L, (O,) + tuple(b) + tuple(h)
+
+
+def _check_against_the_oracle(B, H, N_q, N_kv, D, window, chunk, mask, dtype):
+    inp = orc.make_inputs(B, H, N_q, N_kv, D, seed=N_q + N_kv, dtype=dtype)
+    ref = orc.closed_form_all(*(inp[n] for n in orc.INPUT_NAMES), window_size=window, chunk_id=chunk, mask_mode=mask, device="cuda")
+    g = {n: t.cuda() for n, t in inp.items()}
+    L, first = _three_operations(g, window, chunk, mask)
+    _, second = _three_operations(g, window, chunk, mask)
+    assert torch.allclose(L.cpu().double(), ref["L"].double(), rtol=1e-5, atol=1e-4)
+    for got, again, n in zip(first, second, OUTPUTS):
+        assert torch.equal(got, again), n
+        r = ref[n].double()
+        diff = got.double().cpu() - r
+        assert float(diff.norm()) <= 4 * UNIT[dtype] * float(r.norm()), n
+        assert float(diff.abs().max()) <= 8 * UNIT[dtype] * float(r.abs().max()), n
+    assert capi.device_status() == 0
+    return g
+
+
+def _clusters(g, window, chunk, mask):
+    """{kernel: CTAs per cluster} of the three operations, from a captured graph."""
+    drv = pytest.importorskip("cuda.bindings.driver")
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph, stream=torch.cuda.Stream()):
+        keep = _three_operations(g, window, chunk, mask)
+    raw = drv.CUgraph(graph.raw_cuda_graph())
+    _, _, n = drv.cuGraphGetNodes(raw, 0)
+    _, nodes, _ = drv.cuGraphGetNodes(raw, n)
+    found = {}
+    for node in nodes:
+        if drv.cuGraphNodeGetType(node)[1] != drv.CUgraphNodeType.CU_GRAPH_NODE_TYPE_KERNEL:
+            continue
+        p = drv.cuGraphKernelNodeGetParams(node)[1]
+        name = (drv.cuFuncGetName(p.func) if int(p.func) else drv.cuKernelGetName(p.kern))[1].decode()
+        attr = drv.cuGraphKernelNodeGetAttribute(node, drv.CUkernelNodeAttrID.CU_LAUNCH_ATTRIBUTE_CLUSTER_DIMENSION)[1]
+        for part, kernel in (("fwd_kernel", "O"), ("fb_kernelILi2E", "dQ"), ("fb_kernelILi3E", "dK"), ("hvp_row_kernelILi0E", "g_dO"),
+                             ("hvp_row_kernelILi1E", "g_Q"), ("hvp_col_kernel", "g_K")):
+            if part in name:
+                found[kernel] = max(1, attr.clusterDim.x)
+    del keep
+    return found
+
+
+# (heads, queries, keys, D, window, chunk, mask): kernels whose tiles are shared there
+SPLIT = [
+    ((1, 128, 4096, 64, 4096, 0, 1), "O dQ g_dO g_Q"),            # one tile of queries against 64 of keys
+    ((1, 100, 1999, 128, 1999, 30, 0), "O dQ g_dO g_Q"),          # ragged on both axes
+    ((1, 128, 2048, 64, 700, 15, 0), "O dQ g_dO g_Q"),            # window: shares that half of the rows do not see
+    ((1, 128, 2048, 128, 1500, 15, 0), "O dQ g_dO g_Q"),
+    ((1, 2048, 2048, 64, 2048, 0, 0), "O g_dO dK"),               # causal: tiles of 2 to 32, shares without any
+    ((1, 2048, 2048, 128, 2048, 0, 0), "O g_dO dK"),
+    ((1, 4096, 128, 64, 4096, 0, 1), "dK g_K"),                   # the key side is the short one
+    ((1, 4000, 100, 128, 4096, 0, 1), "dK g_K"),
+    ((7, 4096, 128, 128, 4096, 0, 1), "dK g_K"),
+    ((8, 4096, 128, 64, 4096, 0, 1), "dK g_K"),
+    ((11, 4096, 128, 64, 4096, 0, 1), "dK g_K"),
+    ((14, 4000, 100, 80, 4096, 0, 1), "dK g_K"),
+    ((16, 4096, 128, 64, 4096, 0, 1), "dK g_K"),
+    ((7, 128, 4096, 64, 4096, 0, 1), "O dQ g_dO g_Q"),
+    ((8, 100, 4000, 80, 4096, 0, 1), "O dQ g_dO g_Q"),
+    ((9, 128, 4096, 128, 4096, 0, 1), "O dQ g_dO g_Q"),
+    ((12, 128, 4096, 64, 4096, 0, 1), "O dQ g_dO g_Q"),
+    ((20, 128, 4096, 128, 4096, 0, 1), "O g_dO g_Q"),
+    ((24, 128, 4096, 64, 4096, 0, 1), "O g_dO"),
+    ((30, 100, 4000, 96, 4096, 0, 1), "O g_dO"),
+    ((36, 128, 4096, 64, 4096, 0, 1), "O g_dO"),
+    ((60, 128, 4096, 128, 4096, 0, 1), "O g_dO"),
+]
+SIZES = {}
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("shape,kernels", SPLIT)
+def test_shared_tiles_match_the_oracle(shape, kernels, dtype):
+    H, N_q, N_kv, D, window, chunk, mask = shape
+    g = _check_against_the_oracle(1, H, N_q, N_kv, D, window, chunk, mask, dtype)
+    found = _clusters(g, window, chunk, mask)
+    assert len(found) == 6
+    for k in kernels.split():
+        assert found[k] > 1, (k, found)
+    for k, c in found.items():
+        SIZES.setdefault((k, D > 64), set()).add(c)
+
+
+def test_shared_tiles_cover_the_range_of_sizes():
+    """What the cases above have launched: at least four sizes of every kernel, pairs and eights among
+    them, in either tile width."""
+    if len(SIZES) < 12:
+        pytest.skip("needs the cases above")
+    for k in ("O", "dQ", "dK", "g_dO", "g_Q", "g_K"):
+        narrow, wide = SIZES[k, False] - {1}, SIZES[k, True] - {1}
+        assert 8 in narrow and 8 in wide and len(narrow | wide) >= 4 and min(narrow | wide) <= 3, (k, narrow, wide)
+
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("B,H,N_q,N_kv,D,window,chunk,mask", [
-    (1, 1, 128, 2048, 64, 2048, 15, 0),      # one query tile against 32 key tiles
-    (1, 1, 100, 1999, 128, 1999, 30, 0),     # ragged on both axes
     (1, 2, 257, 900, 80, 300, 3, 0),         # window: the range of a tile starts inside a 64-row tile
-    (1, 1, 1500, 130, 128, 1500, 0, 1),      # the key side is the short one
     (2, 3, 130, 1000, 96, 1000, 0, 0),       # most keys in front of the sequence
-    (1, 1, 64, 190, 64, 190, 9, 0),          # three tiles: fewer than the largest cluster
-    (1, 5, 640, 640, 64, 640, 0, 0),         # causal: shares of unequal tiles
-    (3, 16, 300, 1300, 128, 1000, 2, 0),     # enough CTAs for small clusters only
-    (1, 1, 70, 600, 16, 40, 0, 0),           # keys without a visible query in every share but one
+    (1, 1, 64, 190, 64, 190, 9, 0),          # three tiles
+    (1, 1, 1500, 130, 128, 1500, 0, 1),      # the key side is the short one
+    (1, 5, 640, 640, 64, 640, 0, 0),         # causal: tiles of 2 to 10
+    (3, 16, 300, 1300, 128, 1000, 2, 0),     # 144 tiles: no cluster
+    (1, 1, 70, 600, 16, 40, 0, 0),           # keys without a visible query
     (8, 40, 129, 129, 64, 129, 0, 0),        # two CTAs per SM, one row in every second tile
     (4, 50, 300, 520, 48, 200, 1, 0),        # the same with padding, a window and keys nobody sees
     (6, 50, 60, 190, 64, 190, 0, 1),         # one tile per head
@@ -34,22 +136,7 @@ capi = importlib.import_module("610sample_b200.capi")
     (2, 80, 300, 900, 128, 100, 0, 0),       # the same, and items without a tile in between
 ])
 def test_few_and_many_tiles_match_the_oracle(B, H, N_q, N_kv, D, window, chunk, mask, dtype):
-    inp = orc.make_inputs(B, H, N_q, N_kv, D, seed=N_q + N_kv, dtype=dtype)
-    ref = orc.closed_form_all(*(inp[n] for n in orc.INPUT_NAMES), window_size=window, chunk_id=chunk, mask_mode=mask)
-    g = {n: t.cuda() for n, t in inp.items()}
-    runs = []
-    for _ in range(2):
-        O, L = tcapi.forward(g["Q"], g["K"], g["V"], window, chunk, mask)
-        b = tcapi.backward(g["dO"], g["Q"], g["K"], g["V"], O, L, window, chunk, mask)
-        h = tcapi.double_backward(g["g_dQ"], g["g_dK"], g["g_dV"], g["dO"], g["Q"], g["K"], g["V"], O, L, window, chunk, mask)
-        runs.append((O,) + tuple(b) + tuple(h))
-    assert torch.allclose(L.cpu().double(), ref["L"].double(), rtol=1e-5, atol=1e-4)
-    for got, again, n in zip(*runs, ("O", "dQ", "dK", "dV", "g_dO", "g_Q", "g_K", "g_V")):
-        assert torch.equal(got, again), n
-        r = ref[n].double()
-        # the bound of the other parity tests: 2e-2 of the largest value (half-precision operands P and dS, rounded results)
-        assert float((got.double().cpu() - r).abs().max()) <= 2e-2 * max(1.0, float(r.abs().max())), n
-    assert capi.device_status() == 0
+    _check_against_the_oracle(B, H, N_q, N_kv, D, window, chunk, mask, dtype)
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
