@@ -589,8 +589,9 @@ static cudaError_t dispatch(int op, const Geometry& g, const Tensors& t, cudaStr
     if (e == cudaSuccess) e = launch_one<K_BWD_ROW, T>(beside, t, s);
     *n = 2;
   } else {
-    const bool row = (phases & HVP_PHASE_ROW) != 0, col = (phases & HVP_PHASE_COL) != 0;
-    if (phases & HVP_PHASE_PRE) { e = launch_one<K_HVP_PRE, T>(g, t, s); ++*n; }
+    // the scalars and both row-side outputs belong to either of their masks, as the C ABI documents it
+    const bool row = (phases & (HVP_PHASE_PRE | HVP_PHASE_ROW)) != 0, col = (phases & HVP_PHASE_COL) != 0;
+    if (row) { e = launch_one<K_HVP_PRE, T>(g, t, s); ++*n; }
     if (e == cudaSuccess && col) { e = launch_one<K_HVP_COL, T>(g, t, s); ++*n; }
     if (e == cudaSuccess && row) { e = launch_one<K_HVP_ROW, T>(col ? beside : g, t, s); ++*n; }
   }

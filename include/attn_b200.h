@@ -101,8 +101,8 @@ int attn_b200_double_backward(const attn_shape_t* shape, const void* g_dQ, const
  * kernel at a time: `phases` is a bit mask of 1 (per-row scalars Dv, dot2, dot3
  * into scratch, and g_dO), 2 (g_Q; needs the scalars in scratch) and 4 (g_K and
  * g_V; needs the scalars too).  7 is attn_b200_double_backward.  In the fp32 CUDA-core
- * family the scalars and both row-side outputs come from ONE kernel, so there masks 1
- * and 2 each run that kernel whole (scalars, g_dO and g_Q are all written).  The reference
+ * family the scalars and both row-side outputs are one phase: masks 1 and 2 each run
+ * it whole (scalars, g_dO and g_Q are all written).  The reference
  * splits its double backward the same way into kernel A (rows, two passes) and
  * kernel B (columns), csrc/flash_double_backward_v7.cu:1778-1807. */
 int attn_b200_double_backward_phases(const attn_shape_t* shape, const void* g_dQ, const void* g_dK,

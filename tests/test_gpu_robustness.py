@@ -190,6 +190,18 @@ def test_phase_masks_reproduce_the_single_call(impl, D, dtype):
     assert capi.device_status() == 0
 
 
+@pytest.mark.parametrize("phase", [1, 2])
+def test_row_side_of_the_fp32_family_is_one_phase(phase):
+    args = _hvp_case(seed=44, B=1, H=3, N=320, D=64, dtype=torch.float32)
+    want = tcapi.double_backward(*args)
+    s = tcapi._shape(args[4], args[5], 320, 0, 0, 0)
+    scratch = torch.full((capi.lib().attn_b200_double_backward_scratch_bytes(s) // 4 + 4,), float("nan"), device=DEV)
+    out = tuple(torch.full_like(t, float("nan")) for t in want)
+    tcapi.double_backward_phases(*args, scratch=scratch, out=out, phases=phase)
+    assert torch.equal(out[0], want[0]) and torch.equal(out[1], want[1])
+    assert bool(torch.isfinite(scratch[:3 * 3 * 320]).all())
+
+
 def test_capture_on_one_thread_while_another_calls_eagerly():
     """The shared helper stream is not used under capture, so a capture in progress on one host
     thread and eager calls of another thread cannot touch each other."""
