@@ -19,6 +19,7 @@
 
 namespace attn {
 
+constexpr int kSms = 148;      // SMs of a B200
 constexpr float kLog2e = 1.4426950408889634f;
 constexpr float kLn2 = 0.6931471805599453f;
 
@@ -149,7 +150,7 @@ __device__ __forceinline__ void tile_to_head_and_rank(const Geometry& g, unsigne
 // heads per group: as many as keep `streamed_bytes_per_head` of every head of the group within
 // about 16 MB of L2, all heads when the grid is small anyway
 inline int pick_head_group(long long ctas, int BH, long long streamed_bytes_per_head) {
-  if (ctas < 8 * 148) return BH > 0 ? BH : 1;
+  if (ctas < 8 * kSms) return BH > 0 ? BH : 1;
   long long n = (16ll << 20) / (streamed_bytes_per_head > 0 ? streamed_bytes_per_head : 1);
   if (n < 1) n = 1;
   if (n > BH) n = BH;

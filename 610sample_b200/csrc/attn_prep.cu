@@ -242,7 +242,7 @@ static cudaError_t launch_vec8(const void* x, const void* weight, const float* f
 // is reproducible.  2048 x 12 x 64 in bf16: 6 us for both launches; the same gradient out of
 // PyTorch operations is about thirty launches and 190 us.
 // ---------------------------------------------------------------------------
-constexpr int kPrepMaxCtas = 592;      // four CTAs on each of 148 SMs: rows of `partial`
+constexpr int kPrepMaxCtas = 4 * kSms;      // four CTAs on each SM: rows of `partial`
 
 template <typename T, int G>
 __global__ void __launch_bounds__(kPrepThreads)

@@ -11,7 +11,7 @@
 //   FWD       Q                 K, V              O, L (online softmax)
 //   BWD_ROW   Q, dO             K, V              dQ = s dS K
 //   BWD_COL   K, V              Q, dO             dV = P^T dO, dK = s dS^T Q
-//   HVP_PRE   Q, dO, g_dQ       K, V, g_dK, g_dV  Dv, dot2, dot3;  g_dO = P g_dV + (P o gdS) V - dot2 o O
+//   HVP_PRE   Q, dO, g_dQ       K, V, g_dK, g_dV  Dv, dot2, dot3;  g_dO = P g_dV + (P o gdS) V - dot2 o (P V)
 //   HVP_ROW   Q, dO, g_dQ       K, V, g_dK, g_dV  g_Q = s (dS g_dK + g_S K)
 //   HVP_COL   K, V, g_dK, g_dV  Q, dO, g_dQ       g_K = s (dS^T g_dQ + g_S^T Q), g_V = g_dp^T dO
 //
@@ -105,7 +105,7 @@ __device__ __forceinline__ void mac(float2& acc, const float4& x, const float4& 
   acc = __ffma2_rn(make_float2(x.z, x.w), make_float2(y.z, y.w), acc);
 }
 
-// The raw score matrices of a kind for this thread's 2 x 4 elements.
+// The raw score matrices of a kind for this thread's RA x 4 elements.
 template <int KIND, int RA>
 __device__ __forceinline__ void scores(float* const (&stat)[4], float* const (&strm)[4], const Layout& lay, int D,
                                        int row0, int col0, float (&out)[Spec<KIND>::kNAcc][RA][CB]) {
@@ -546,12 +546,12 @@ __global__ void __launch_bounds__(threads_of(DC), DC == 1 ? 2 : 1) attn_simt_ker
   tc::pdl_end(g);
 }
 
-// CTAs per stationary tile: enough for two CTAs on each of 148 SMs, but no more than there are
+// CTAs per stationary tile: enough for two CTAs on each SM, but no more than there are
 // streamed tiles for a stationary one.
 static int split_for(const Geometry& g, long long units, int n_strm) {
   const int most = g.mask_mode == 0 && g.window < n_strm ? g.window + TS : n_strm;
   int c = 1;
-  while (c < kMaxSplit && units * c * 2 <= 2 * 148 && 2 * c <= (most + TT - 1) / TT) c *= 2;
+  while (c < kMaxSplit && units * c * 2 <= 2 * kSms && 2 * c <= (most + TT - 1) / TT) c *= 2;
   return c;
 }
 

@@ -643,8 +643,9 @@ fb_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Tensors 
       tc_fence_after_sync();
       constexpr int kColsPerHalf = D / kHalves;
       constexpr int kChunks = kColsPerHalf / 16;
-      // The result tiles go out through the staging buffer of the stationary operands (they
-      // have been in tensor memory since the prologue).
+      // The result tiles go out through the staging buffer of the stationary operands.  They have been in
+      // tensor memory since the prologue, or, where the products read them from here, every product has
+      // completed: S products before their scores were read, the rest with acc_done.
 #pragma unroll
       for (int o = 0; o < CF::kNOut; ++o) {
         float mul = 1.f;

@@ -18,12 +18,14 @@
 // it stands, and its maximum taken only where a row's sum exceeds 2^tau, without which no score can be
 // more than tau above m.  So no maximum is taken in nearly all tiles (D = 64: -4 to -6 %).
 // tau is a question of precision: the largest P of a row whose m is its maximum is 1, which the half
-// types hold exactly, and a peaked row is little else than that P.  With 8 for two groups (each has a maximum of its own) and 6 for
-// one, whose streams of up to six tiles follow their maximum exactly, O is as close to the exact one as
-// taking every maximum with a threshold of 8 in two groups was: relative error 2.02e-3 at H32 N16384 D128, Q
-// and K of twice unit variance, where 24 gave 2.32e-3 and a rounded result alone is 1.66e-3.  The price, for
-// peaked rows: 2.34 instead of 1.83 ms there, 126 instead of 91 us at B8 H12 N2048 D64; for short streams 26
-// instead of 24 us at B4 H16 N1024 D128; inputs of unit variance stay at 91 us at B8 H12 N2048 D64.
+// types hold exactly, and a peaked row is little else than that P.  With 8 for two groups (each has a
+// maximum of its own) and 6 for one, whose streams of up to six tiles follow their maximum exactly, O is as
+// close to the exact one as with every maximum taken and 8 in two groups: relative error 2.02e-3 at H32
+// N16384 D128, Q and K of twice unit variance (24 gave 2.32e-3; a rounded result alone is 1.66e-3).  The
+// price, for peaked rows: 2.34 instead of 1.83 ms there, 126 instead of 91 us at B8 H12 N2048 D64; for
+// short streams 26 instead of 24 us at B4 H16 N1024 D128; inputs of unit variance stay at 91 us at B8 H12
+// N2048 D64.  5 for one group would have tiles of nearly equal scores, whose sums are 36 to 64, take the
+// maximum for nothing: 99 -> 115 us at B4 H16 N2048 D64 without a mask.
 // Tensor memory, one CTA per SM (512 columns): three score buffers S0, S1, S2 [0,192), Q [192,192+D/2),
 // O_0 [256,256+D), O_1 [256+D, 256+2D); two per SM (256 columns): S0, S1 [0,128), Q behind them at
 // D = 64 (at D = 128 it stays in shared memory), O.  P is written (two halves per 32-bit column) over the
@@ -221,7 +223,7 @@ fwd_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Tensors
         if (it < CF::kStages) return true;
         return mbar_wait(bar_stream_empty(h, it % CF::kStages), ((it / CF::kStages) & 1) ^ 1, abort_flag, t.status, wait_code(KFWD, 1));
       };
-      // K runs ahead of V by the three tiles the score products run ahead of the P V products
+      // K runs ahead of V by the tiles the score products run ahead of the P V products
       for (int u = 1; u < kFwdSBufs && u < n_iter; ++u) request_half(u, 0);
       for (int u = 0; u < n_iter && ok; ++u) {
         ok = wait_free(u, 1);
@@ -260,7 +262,7 @@ fwd_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Tensors
         for (int j = 0; j < n_iter && ok; ++j) {
           const int b = j % kFwdSBufs, st = j % CF::kStages;
           ok = wait_stream(0, j);
-          // the buffer was read (as P) by the P V product of tile j - 3
+          // the buffer was read (as P) by the P V product of tile j - kFwdSBufs
           if (ok && j >= kFwdSBufs) {
             ok = mbar_wait(bar_pv_done(b), ((j / kFwdSBufs) & 1) ^ 1, abort_flag, t.status, wait_code(KFWD, 4));
             ok = __all_sync(0xffffffffu, ok);
@@ -521,7 +523,8 @@ fwd_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Tensors
       if constexpr (SPLIT) store_partial16<D>(partial, row, col, f);
       else if (gidx < g.N_q) store_op16(staging + (uint32_t)(col >> 6) * kAtomBytesStat, row, col & 63, w);
     }
-    // the O tile leaves through the staging buffer (Q has been in tensor memory since the prologue)
+    // The O tile leaves through the staging buffer: Q has been in tensor memory since the prologue, or, where it is
+    // read from here, every score product was complete before its scores were read.
     store_tile_tma(&maps.out[TO_O], staging, g.D, r0, bh, !SPLIT && threadIdx.x == 0, kMathThreads);
   }
 

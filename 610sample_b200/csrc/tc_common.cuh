@@ -177,7 +177,6 @@ __device__ __forceinline__ void reduce_parts(float* partial, int split, int part
 // 10.5 us, with two 10.4.
 constexpr float kCtaClocks = 12000.f;
 constexpr int kMaxSplit = 8;
-constexpr int kSms = 148;
 inline float split_clocks(int D) { return 3000.f + 45.f * D; }
 
 // a kernel's stationary tiles, the most and the mean streamed tiles one of them visits, clocks per tile

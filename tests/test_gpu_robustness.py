@@ -203,8 +203,8 @@ def test_row_side_of_the_fp32_family_is_one_phase(phase):
 
 
 def test_capture_on_one_thread_while_another_calls_eagerly():
-    """The shared helper stream is not used under capture, so a capture in progress on one host
-    thread and eager calls of another thread cannot touch each other."""
+    """The library keeps every launch on the caller's stream and holds no stream of its own, so a capture
+    in progress on one host thread and eager calls of another thread cannot touch each other."""
     a_args, b_args = _hvp_case(seed=51, H=4, N=512), _hvp_case(seed=52, H=4, N=512)
     want_a, want_b = tcapi.double_backward(*a_args), tcapi.double_backward(*b_args)
     s = tcapi._shape(a_args[4], a_args[5], 512, 0, 0, 0)

@@ -185,9 +185,8 @@ def test_empty_inputs(mods):
 
 
 def test_double_backward_under_cuda_graph_capture():
-    """The call is capturable: under capture every launch stays on the capturing stream (the
-    library's helper stream is used by eager calls only), tensor maps travel as kernel parameters,
-    nothing is allocated by the library.  The replayed graph must reproduce the eager results bit
+    """The call is capturable: every launch stays on the caller's stream, tensor maps travel as kernel
+    parameters, nothing is allocated by the library.  The replayed graph must reproduce the eager results bit
     for bit."""
     tcapi = importlib.import_module("610sample_b200.torch_capi")
     capi = importlib.import_module("610sample_b200.capi")
@@ -221,8 +220,7 @@ def test_double_backward_under_cuda_graph_capture():
 
 def test_two_host_threads_on_their_own_streams():
     """Two host threads call the C ABI at the same time on different streams (ctypes drops the
-    GIL).  They share the device's helper stream and its fork / join events; each must still get
-    exactly the results of a serial call."""
+    GIL); each must get exactly the results of a serial call."""
     import threading
     tcapi = importlib.import_module("610sample_b200.torch_capi")
     capi = importlib.import_module("610sample_b200.capi")
