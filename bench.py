@@ -45,10 +45,10 @@ HVP_GEMMS = 12          # algorithmic contractions of the double backward
 ROW_KERNEL_GEMMS = 7    # contractions the g_Q kernel executes (5 score + 2 output)
 PRE_KERNEL_GEMMS = 7    # scalars + g_dO kernel (5 score + 2 output)
 COL_KERNEL_GEMMS = 8
-# dram__bytes_read.sum + dram__bytes_write.sum per launch of each kernel, from an `ncu --set full`
-# capture of this bench at 16 (batch, head) slices; traffic grows in proportion to the number of
-# slices, so the bench scales it by BH / 16.  To be refreshed whenever a kernel changes.
-NCU_TRAFFIC_BYTES_16_SLICES = {"pre": 193.0e6, "row": 171.0e6, "col": 136.9e6}
+# dram__bytes_read.sum + dram__bytes_write.sum per launch of each kernel, from an `ncu --metrics`
+# capture of one double backward at 16 (batch, head) slices of this workload; traffic grows in proportion
+# to the number of slices, so the bench scales it by BH / 16.  To be refreshed whenever a kernel changes.
+NCU_TRAFFIC_BYTES_16_SLICES = {"pre": 188.2e6, "row": 167.1e6, "col": 133.3e6}
 # the same for one launch of the fused norm + rotary kernel (part of the output is still in L2 when it ends)
 NCU_PREP_TRAFFIC_BYTES = {"16384x32x128": 232.2e6}
 
