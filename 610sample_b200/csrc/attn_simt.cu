@@ -15,21 +15,23 @@
 //   HVP_ROW   Q, dO, g_dQ       K, V, g_dK, g_dV  g_Q = s (dS g_dK + g_S K)
 //   HVP_COL   K, V, g_dK, g_dV  Q, dO, g_dQ       g_K = s (dS^T g_dQ + g_S^T Q), g_V = g_dp^T dO
 //
-// Bound by shared-memory reads: a float4 read of a warp takes four clocks of the SM's 128 bytes per
-// clock whether its lanes broadcast or not, so a thread has to do 16 multiply-adds per float4 before
-// the FMA pipe is the limit.  A warp is 4 x 8 threads and, at D <= 64, a thread holds 4 x 4 scores
-// of every score matrix of the kind, so that each float4 it reads serves several products (HVP: 28
-// reads for 320 multiply-adds).  Above, where one CTA fills the shared memory of an SM, a thread
-// holds 2 x 4 (22 for 160; 45 % of the FMA rate with the read path at 80 %): twice the warps hide
-// the latencies that eat what 4 x 4 saves (2.60 against 3.37 ms at B2 H8 N1024 D128).  The packed
-// f32x2 multiply-adds run along the head dimension without a move.  Rows are stored without padding
-// where D is a multiple of 32, their 16-byte chunks XOR-swizzled by the row, which lets two CTAs of
-// every kind share an SM at D <= 64: one computes while the other loads.
-// Small problems: with fewer than two CTAs per SM the streamed tiles of a stationary tile are dealt
-// out to a CLUSTER of 2 to 8 CTAs (split_for), whose partial sums are added through distributed
-// shared memory in a fixed order; results are bitwise reproducible either way.
-// B2 H4 N256 D64 causal, forward + backward + double backward on an idle B200: 447 us with 32 x 32
-// tiles, 2 x 2 scores per thread and no split (64 CTAs).
+// Bound by the FMA pipe and shared-memory reads together.  A float4 read of a warp takes four clocks of
+// the SM's 128 bytes per clock, or two where no quad of lanes reads more than two different float4s
+// (measured: 4.0 and 2.1 with 8 of 32 lanes' values different, depending on which lanes share).  So a warp is
+// 4 x 8 threads with 2 x 2 of them in every quad, which halves the reads of the streamed side; rows by
+// lane / 8 and columns by lane % 8 took, at D = 128, 10 to 17 % more time (B2 H8 N1024 forward 220 -> 180,
+// backward 690 -> 573, double backward 1 685 -> 1 509 us), at D = 64 1 to 5 %.  A thread holds 2 x 4 scores of every
+// score matrix of its kind; in the double backward at D <= 64, where four matrices share the operands it has
+// read, 4 x 4 (N1024 800 against 837 us, and the smaller backward the other way round: B2 H5 N479 62
+// against 65).  At D > 64 one CTA fills the shared memory of an SM, and twice the warps hide the latencies.
+// The packed f32x2 multiply-adds run along the head dimension without a move; as scalar ones they
+// have a higher rate with one or two warps per scheduler, but the issue slots they take cost 4 to 70 %.
+// Rows are stored without padding where D is a multiple of 32, their 16-byte chunks XOR-swizzled by the
+// row, which lets two CTAs of every kind share an SM at D <= 64: one computes while the other loads.
+// Loading the next tile behind the output products instead gave nothing (forward -1 to -3 %, backward +4 %).
+// Small problems: the streamed tiles of a stationary tile are dealt out to a CLUSTER of 2 to 8 CTAs
+// (split_for), whose partial sums are added through distributed shared memory in a fixed order; results are
+// bitwise reproducible either way.
 #include "attn_common.cuh"
 #include "attn_launch.h"
 #include "tc_common.cuh"
@@ -44,13 +46,14 @@ namespace cg = cooperative_groups;
 constexpr int TS = 32;        // stationary rows per CTA
 constexpr int TT = 64;        // streamed rows per iteration
 constexpr int CB = 4;         // score columns per thread, 8 apart
-// By tile width (DC = 1: D <= 64, 2: D <= 128): score rows per thread, 4 apart, and threads per CTA,
-// (8 / RA) x 2 warps over the 32 x 64 score tile.
-__host__ __device__ constexpr int rows_of(int DC) { return DC == 1 ? 4 : 2; }
-__host__ __device__ constexpr int threads_of(int DC) { return DC == 1 ? 128 : 256; }
 constexpr int kMaxSplit = 8;  // CTAs per cluster (the portable maximum)
 
 enum Kind { K_FWD = 0, K_BWD_ROW, K_BWD_COL, K_HVP_PRE, K_HVP_ROW, K_HVP_COL };
+
+// By kind and tile width (DC = 1: D <= 64, 2: D <= 128): score rows per thread, 4 apart, and threads per
+// CTA, (8 / RA) x 2 warps over the 32 x 64 score tile.
+__host__ __device__ constexpr int rows_of(int kind, int DC) { return DC == 1 && kind >= K_HVP_PRE ? 4 : 2; }
+__host__ __device__ constexpr int threads_of(int kind, int DC) { return 512 / rows_of(kind, DC); }
 
 template <int KIND> struct Spec {
   static constexpr bool kCol = KIND == K_BWD_COL || KIND == K_HVP_COL;
@@ -84,11 +87,11 @@ template <typename T> __device__ __forceinline__ float4 widen4(const T* p) {
   return make_float4(a.x, a.y, b.x, b.y);
 }
 
-// Stage `rows` rows from row0 of a [n_rows, D] matrix as fp32, zero beyond n_rows.  DC * 16 threads
+// Stage `rows` rows from row0 of a [n_rows, D] matrix as fp32, zero beyond n_rows.  DC * 16 of the NT threads
 // share a row.  float goes by cp.async (complete after cp_async_wait_all and a barrier).
-template <int DC, typename T>
+template <int DC, int NT, typename T>
 __device__ __forceinline__ void stage_tile(float* dst, const Layout& lay, const T* src, int row0, int rows, int n_rows, int D) {
-  constexpr int kLanes = 16 * DC, NT = threads_of(DC);
+  constexpr int kLanes = 16 * DC;
   const int chunk = threadIdx.x % kLanes;
   if (chunk * 4 >= D) return;
   for (int r = threadIdx.x / kLanes; r < rows; r += NT / kLanes) {
@@ -118,7 +121,7 @@ __device__ __forceinline__ void scores(float* const (&stat)[4], float* const (&s
     for (int a = 0; a < RA; ++a)
 #pragma unroll
       for (int b = 0; b < CB; ++b) acc[m][a][b] = make_float2(0.f, 0.f);
-#pragma unroll 2
+#pragma unroll (RA == 4 ? 2 : 4)
   for (int k = 0; k < (D >> 2); ++k) {
     float4 x[SP::kNStat][RA];
 #pragma unroll
@@ -156,7 +159,7 @@ __device__ __forceinline__ void scores(float* const (&stat)[4], float* const (&s
 template <int DC, int RA>
 __device__ __forceinline__ void out_fma(const float* op, const float* Z, const Layout& lay, int row0, int chunk0, int chunks,
                                         float2 (&out)[RA][DC][2]) {
-#pragma unroll 2
+#pragma unroll (RA == 4 ? 2 : 4)
   for (int j = 0; j < TT; j += 4) {
     float o[RA][4];
 #pragma unroll
@@ -184,12 +187,12 @@ __device__ __forceinline__ void out_fma(const float* op, const float* Z, const L
 // sum over the eight threads of a warp that share a row
 __device__ __forceinline__ float row_sum(float v) {
 #pragma unroll
-  for (int o = 4; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  for (int o = 8; o > 1; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
 }
 __device__ __forceinline__ float row_max(float v) {
 #pragma unroll
-  for (int o = 4; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
+  for (int o = 8; o > 1; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
   return v;
 }
 
@@ -209,9 +212,9 @@ __host__ __device__ constexpr int smem_floats(int D) {
 
 // DC: 1 for D <= 64, 2 up to 128.
 template <int KIND, int DC, typename T>
-__global__ void __launch_bounds__(threads_of(DC), DC == 1 ? 2 : 1) attn_simt_kernel(const Geometry g, const Tensors t, const int split) {
+__global__ void __launch_bounds__(threads_of(KIND, DC), DC == 1 ? 2 : 1) attn_simt_kernel(const Geometry g, const Tensors t, const int split) {
   using SP = Spec<KIND>;
-  constexpr int RA = rows_of(DC), NT = threads_of(DC);
+  constexpr int RA = rows_of(KIND, DC), NT = threads_of(KIND, DC);
   // g_dO = P g_dV + (P o gdS) V - dot2 o (P V).  In fp32 P V is the O of the call; an O of half precision has
   // been rounded, so there the kernel sums its own (bf16, g_dK offset by one: relative error 1.66e-3
   // instead of 1.92e-3; 1.66e-3 is the rounding of the result).
@@ -227,7 +230,7 @@ __global__ void __launch_bounds__(threads_of(DC), DC == 1 ? 2 : 1) attn_simt_ker
   const int tile = (SP::kCol || g.mask_mode != 0) ? rank : tiles - 1 - rank;     // heavy tiles first
   const int r0 = tile * TS;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int ty = lane >> 3, tx = lane & 7, wcol = warp & 1;
+  const int ty = (lane & 1) | ((lane >> 4) << 1), tx = (lane >> 1) & 7, wcol = warp & 1;      // 2 x 2 in every quad of lanes
   const int row0 = (warp >> 1) * 4 * RA + ty;         // this thread's rows: row0 + 4 a
   const int col0 = wcol * 32 + tx;                    // its score columns: col0 + 8 b
   const int chunk0 = wcol * 8 + tx, chunks = D >> 2;  // its output float4s: chunk0 + 16 c
@@ -264,7 +267,7 @@ __global__ void __launch_bounds__(threads_of(DC), DC == 1 ? 2 : 1) attn_simt_ker
   tc::pdl_trigger();
 
 #pragma unroll
-  for (int i = 0; i < SP::kNStat; ++i) stage_tile<DC, T>(stat[i], lay, stat_src[i], r0, TS, n_stat, D);
+  for (int i = 0; i < SP::kNStat; ++i) stage_tile<DC, NT, T>(stat[i], lay, stat_src[i], r0, TS, n_stat, D);
 
   // ---- scalars of this thread's rows (row kinds)
   float L2[RA] = {}, Dv[RA] = {}, d2[RA] = {}, d3[RA] = {};
@@ -304,7 +307,7 @@ __global__ void __launch_bounds__(threads_of(DC), DC == 1 ? 2 : 1) attn_simt_ker
     const int s0 = tt * TT;
     __syncthreads();                                  // the previous tile has been used
 #pragma unroll
-    for (int i = 0; i < SP::kNStream; ++i) stage_tile<DC, T>(strm[i], lay, strm_src[i], s0, TT, n_strm, D);
+    for (int i = 0; i < SP::kNStream; ++i) stage_tile<DC, NT, T>(strm[i], lay, strm_src[i], s0, TT, n_strm, D);
     if constexpr (SP::kCol) {                         // [L2 | Dv | dot2 | dot3] of the streamed queries
       if constexpr (SP::kHvp) {
 #pragma unroll
@@ -546,13 +549,39 @@ __global__ void __launch_bounds__(threads_of(DC), DC == 1 ? 2 : 1) attn_simt_ker
   tc::pdl_end(g);
 }
 
-// CTAs per stationary tile: enough for two CTAs on each SM, but no more than there are
-// streamed tiles for a stationary one.
-static int split_for(const Geometry& g, long long units, int n_strm) {
-  const int most = g.mask_mode == 0 && g.window < n_strm ? g.window + TS : n_strm;
-  int c = 1;
-  while (c < kMaxSplit && units * c * 2 <= 2 * kSms && 2 * c <= (most + TT - 1) / TT) c *= 2;
-  return c;
+// CTAs per stationary tile.  In units of the time a CTA that has its SM to itself takes for a streamed tile: a
+// CTA costs about one besides its tiles, 1.6 to 1.9 in a cluster (two barriers, the sum; where two share an SM
+// the other one hides some of it).  Bounds are the longest CTA, whose tiles take 1.5 where two share an SM
+// (D <= 64), and the whole load over the SMs, with that of the kernel beside it (`paired`).
+// B2 H5 N479 D64 (150 tiles of up to 8): forward 50 -> 31, backward 85 -> 62, double backward 258 -> 172 us
+// in pairs, where all that filled a CTA per SM used to go unsplit; B1 H3 N150 D128 (15 tiles of up to 3) in fours
+// 17 -> 10.5, 26 -> 15.5, 84 -> 50; B2 H7 N293 D80 (140 tiles of up to 5), which used to go in pairs, unsplit
+// 31 -> 28, 73 -> 54, 172 -> 156.
+static int split_for(const Geometry& g, long long units, bool col, bool narrow, bool paired) {
+  if (units > 2 * kSms) return 1;
+  const int n = col ? g.N_kv : g.N_q, tiles = (n + TS - 1) / TS;      // at most as many as there are units
+  int longest = 0;
+  long long per_head = 0;
+  for (int i = 0; i < tiles; ++i) {
+    int lo, hi;
+    if (col) query_range_for_keys(g, i * TS, (i + 1) * TS, lo, hi);
+    else key_range_for_queries(g, i * TS, (i + 1) * TS, lo, hi);
+    const int k = hi > lo ? (hi + TT - 1) / TT - lo / TT : 0;
+    if (k > longest) longest = k;
+    per_head += k;
+  }
+  const float total = (float)per_head * g.BH, shared = narrow ? 1.5f : 1.f;
+  const int slots = narrow ? 2 * kSms : kSms;
+  int best = 1;
+  float least = 0.f;
+  for (int c = 1; c <= kMaxSplit && c < 2 * longest; c *= 2) {
+    const float cta = c == 1 ? (narrow ? 1.f : 1.2f) : narrow ? 1.6f : 1.9f;
+    const float one = (float)((longest + c - 1) / c) * (units * c > kSms ? shared : 1.f) + cta;
+    const float all = (units * c * (narrow && c > 1 ? 1.32f : cta) + total) * shared / slots * (paired ? 2.f : 1.f);
+    const float t = one > all ? one : all;
+    if (c == 1 || t < 0.97f * least) { best = c; least = t; }
+  }
+  return best;
 }
 
 template <int KIND, int DC, typename T>
@@ -561,14 +590,15 @@ static cudaError_t launch_dc(const Geometry& g, const Tensors& t, cudaStream_t s
   const long long units = (long long)g.BH * ((n_stat + TS - 1) / TS);
   if (units <= 0) return cudaSuccess;
   if (units * kMaxSplit > 0x7fffffffLL) return cudaErrorInvalidValue;
-  const int split = split_for(g, units, Spec<KIND>::kCol ? g.N_q : g.N_kv);
+  const bool paired = KIND != K_FWD && KIND != K_HVP_PRE;
+  const int split = split_for(g, units, Spec<KIND>::kCol, DC == 1, paired);
   const size_t smem = sizeof(float) * smem_floats<KIND>(g.D);
   auto kern = attn_simt_kernel<KIND, DC, T>;
   static std::atomic<unsigned long long> smem_set{0};
   // the size at the variant's largest D, so that one setting serves every call
   const cudaError_t e = tc::set_smem_once(kern, sizeof(float) * smem_floats<KIND>(64 * DC), smem_set);
   if (e != cudaSuccess) return e;
-  return tc::launch_pdl_cluster(kern, (unsigned)(units * split), threads_of(DC), smem, (unsigned)split, stream, g, t, split);
+  return tc::launch_pdl_cluster(kern, (unsigned)(units * split), threads_of(KIND, DC), smem, (unsigned)split, stream, g, t, split);
 }
 
 template <int KIND, typename T>

@@ -68,3 +68,14 @@ def test_half_inputs_give_the_rounded_exact_result(B, H, N_q, N_kv, D, dtype):
     # next: few results are rounded to the other side
     for got, n in zip(h, ("g_dO", "g_Q", "g_K", "g_V")):
         assert float((got.cpu() != ref[n].to(dtype)).float().mean()) <= 0.02, n
+
+
+@pytest.mark.parametrize("B,H,N_q,N_kv,D,window,chunk,mask", [
+    (2, 5, 479, 479, 64, 479, 0, 0),     # 150 tiles of up to 8: pairs, parts without a tile
+    (1, 3, 150, 150, 128, 150, 0, 0),    # three tiles for a cluster of four
+    (2, 7, 160, 293, 80, 293, 1, 0),     # 70 and 140 tiles: a split on one side of a pair of kernels only
+    (1, 9, 1023, 65, 64, 1023, 0, 1),    # 288 tiles of two; 27 of 16
+    (1, 10, 961, 33, 96, 40, 0, 0),      # 310 tiles, most of which see nothing
+])
+def test_fp32_splits_match_the_oracle(B, H, N_q, N_kv, D, window, chunk, mask):
+    test_fp32_kernels_match_the_oracle(B, H, N_q, N_kv, D, window, chunk, mask)
