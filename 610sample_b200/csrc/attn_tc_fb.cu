@@ -260,9 +260,11 @@ fb_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Tensors 
       // 8 columns at col0 + 32*(ks/2) + 8*(ks%2) (owner half, then chunk)
       auto op_tmem = [&](int col0, int ks) { return tmem_base + (uint32_t)(col0 + 32 * (ks >> 1) + 8 * (ks & 1)); };
       auto commit = [&](uint32_t bar) { if (elect_one()) mma_commit(bar); };
-      constexpr int KS = D / 16, KO = BN / 16;
+      constexpr int KO = BN / 16;
+      with_k_steps<D>(g.D, [&](auto k_steps) {
+      constexpr int kSteps = decltype(k_steps)::value, KS = kSteps > 0 ? kSteps : D / 16;
       // a head dimension below the tile width: skip the k-steps and output columns that are padding
-      const int ks_n = g.D >> 4;
+      const int ks_n = kSteps > 0 ? KS : g.D >> 4;
       const uint32_t idesc_out = make_idesc(BM, g.D, Pack<T>::kIsBf16, 0, 1);
       const uint32_t stat0 = tmem_base + CF::kStat, stat1 = stat0 + CF::kStatStride;
       const uint64_t stat_desc = smem_desc_sw128(staging, 16, 1024);
@@ -305,6 +307,7 @@ fb_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Tensors 
       };
       auto issue_out = [&](int j) {
         const int b = j % kBufs;
+        (void)b;
         const uint64_t dm = smem_desc_sw128(stage_of(j), kAtomBytesStrm, 1024);
         const bool first = (j == 0);
         if (elect_one()) {
@@ -359,6 +362,7 @@ fb_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Tensors 
         }
         if (ok) commit(bar_acc_done);
       }
+      });
     }
   }
   // =========================================================================

@@ -34,6 +34,21 @@ struct TmaMaps { CUtensorMap m[T_COUNT]; CUtensorMap out[TO_COUNT]; };
 
 template <int V> struct Int { static constexpr int value = V; };
 
+// The issuing warps' loops with the k-steps of a head dimension: role(Int<steps>), a constant for the usual
+// ones, 0 (the tile width's steps, each compared with g.D / 16) for the others.  A comparison costs the issuing
+// thread about as much as the step it skips: a score batch of the forward took 335 clocks to issue at D = 96 as
+// at D = 128.  B4 H8, 1189 queries, 3531 keys, D80: forward 70.0 -> 68.5 us, backward 161 -> 158; B2 H8 N2648 D96 forward
+// 36.5 -> 35.2; H12, 1024 queries, 9216 keys, D64 forward 27.0 -> 26.1, backward 65.8 -> 65.0.  The double
+// backward keeps the comparisons: with two long batches in flight the gaps let the other issuing
+// warp's products in (85 us with, 90 without at B2 H16 N844 D128; D = 64 even).
+template <int D, typename Role>
+__device__ __forceinline__ void with_k_steps(int head_dim, Role&& role) {
+  if (head_dim == D) role(Int<D / 16>{});
+  else if (D == 128 && head_dim == 96) role(Int<6>{});
+  else if (D == 128 && head_dim == 80) role(Int<5>{});
+  else role(Int<0>{});
+}
+
 template <typename T> struct Pack;
 template <> struct Pack<__nv_bfloat16> {
   static constexpr int kIsBf16 = 1;
