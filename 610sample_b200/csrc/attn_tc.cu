@@ -269,11 +269,11 @@ cudaError_t launch_hvp_col(int D, int is_bf16, const TmaMaps& maps, const Geomet
 cudaError_t launch_hvp_row(int mode, int D, int is_bf16, const TmaMaps& maps, const Geometry& g,
                            const Tensors& t, cudaStream_t s);
 
-cudaError_t launch_fwd_bwd(int kind, int D, int is_bf16, const TmaMaps& maps, const Geometry& g, const Tensors& t,
-                           cudaStream_t s);
+cudaError_t launch_bwd(int D, int is_bf16, const TmaMaps& maps, const Geometry& g, const Tensors& t, cudaStream_t s, bool row_first,
+                       int* launches);
 cudaError_t launch_fwd(int D, int is_bf16, const TmaMaps& maps, const Geometry& g, const Tensors& t, cudaStream_t s);
 
-// dQ beside dK/dV and g_Q beside g_K/g_V: one kernel first, the other one on the SMs its last CTAs
+// dQ beside dK/dV and g_Q beside g_K/g_V: the CTAs of one first, the other's on the SMs its last CTAs
 // leave idle (tc_common.cuh).  The kernel with the longer CTAs goes first, so that the tail is made
 // of short ones: the row kernel where a query sees more keys than a key is seen by queries (chunks of
 // 1024 queries against a window of 8192: 128 tiles per row CTA, 16 per column CTA; backward 410 ->
@@ -309,10 +309,8 @@ static cudaError_t launch_op(int op, const TmaMaps& maps, const Geometry& g, con
     if (rows > 0) {
       e = launch_rowdot<T>((const T*)t.dO, (const T*)t.O, t.Dv, rows, g.D, s);
     }
-    if (e == cudaSuccess)
-      e = side_by_side(g, [&](const Geometry& q) { return launch_fwd_bwd(2, D, bf, maps, q, t, s); },      // dQ
-                       [&](const Geometry& q) { return launch_fwd_bwd(3, D, bf, maps, q, t, s); });       // dK, dV
-    *n = 3;
+    *n = 1;
+    if (e == cudaSuccess) e = launch_bwd(D, bf, maps, g, t, s, row_side_first(g), n);                     // dQ; dK, dV
   } else {
     if (phases & HVP_PHASE_PRE) { e = launch_hvp_row(0, D, bf, maps, g, t, s); ++*n; }                        // scalars + g_dO
     const bool row = (phases & HVP_PHASE_ROW) != 0, col = (phases & HVP_PHASE_COL) != 0;

@@ -35,7 +35,7 @@
 namespace attn {
 namespace tc {
 
-enum FbKind { FB_BWD_ROW = 2, FB_BWD_COL = 3 };   // numbering of launch_fwd_bwd
+enum FbKind { FB_BWD_ROW = 2, FB_BWD_COL = 3 };   // as in the device status codes
 
 constexpr int kFbMaxStages = 8;
 
@@ -97,9 +97,15 @@ struct FbCfg {
 };
 
 template <int KIND, int D, typename T, bool SPLIT, bool DUAL>
-__global__ void __launch_bounds__((FbCfg<KIND, D, DUAL>::kThreads), DUAL ? 2 : 1)
-fb_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Tensors t) {
+struct fb_kernel {
   using CF = FbCfg<KIND, D, DUAL>;
+  static constexpr int kThreads = CF::kThreads, kPerSm = DUAL ? 2 : 1;
+  static __device__ __forceinline__ void run(const TmaMaps& maps, const Geometry& g, const Tensors& t, unsigned block);
+};
+
+template <int KIND, int D, typename T, bool SPLIT, bool DUAL>
+__device__ __forceinline__ void fb_kernel<KIND, D, T, SPLIT, DUAL>::run(const TmaMaps& maps, const Geometry& g, const Tensors& t,
+                                                                        const unsigned block) {
   constexpr int kAtoms = CF::kAtoms, kHalves = CF::kHalves;
   constexpr int kMathWarps = CF::kMathWarps, kMathThreads = CF::kMathThreads, kProducerWarp = CF::kProducerWarp;
   constexpr int kFbMmaWarp = CF::kMmaWarp, kTmemCols = CF::kTmemCols;
@@ -129,9 +135,9 @@ fb_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Tensors 
   const int n_stat = CF::kCol ? g.N_kv : g.N_q;
   const int tiles = (n_stat + BM - 1) / BM;
   const unsigned split = SPLIT ? (unsigned)g.split : 1u;      // CTAs that share this tile: a cluster (tc_common.cuh)
-  const int part = SPLIT ? (int)(blockIdx.x % split) : 0;
+  const int part = SPLIT ? (int)(block % split) : 0;
   int bh, rank;
-  tile_to_head_and_rank(g, blockIdx.x / split, tiles, bh, rank);
+  tile_to_head_and_rank(g, block / split, tiles, bh, rank);
   const int tile = (CF::kCol || g.mask_mode != 0) ? rank : (tiles - 1 - rank);   // heavy tiles first
   const int r0 = tile * BM;
 
@@ -722,35 +728,87 @@ fb_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Tensors 
   pdl_end(g);
 }
 
+// How a kind is launched: two CTAs per SM, CTAs per tile.
+struct FbPlan { bool dual; int split; };
+
 template <int KIND, int D, typename T>
-static cudaError_t launch_fb(const TmaMaps& maps, const Geometry& g_in, const Tensors& t, cudaStream_t s) {
+static TileKernelState& fb_state() {
+  static TileKernelState state;
+  return state;
+}
+
+template <int KIND, int D, typename T>
+static FbPlan plan_fb(const Geometry& g) {
+  constexpr bool kCol = KIND == FB_BWD_COL;
+  if constexpr (D == 64) {
+    if (two_per_sm_pays(g, kCol, false, kCol ? 1700.f : 1000.f, kCol ? 1200.f : 1000.f)) return {true, 1};
+  }
+  using CF = FbCfg<KIND, D, false>;
+  return {false, choose_split(tile_kernel<fb_kernel<KIND, D, T, true, false>>, g, kCol, CF::kThreads, CF::kSmemBytes, kCol ? 1700.f : 1150.f,
+                              kCol ? 1150.f : 1700.f, fb_state<KIND, D, T>())};
+}
+
+template <int KIND, int D>
+static int fb_head_group(const Geometry& g) {
+  constexpr bool kCol = KIND == FB_BWD_COL;
+  return pick_head_group((long long)g.BH * (((kCol ? g.N_kv : g.N_q) + BM - 1) / BM), g.BH, 2ll * (kCol ? g.N_q : g.N_kv) * g.D * 2);
+}
+
+template <int KIND, int D, typename T>
+static cudaError_t launch_fb(const TmaMaps& maps, const Geometry& g_in, const Tensors& t, cudaStream_t s, const FbPlan& plan) {
   constexpr bool kCol = KIND == FB_BWD_COL;
   Geometry g = g_in;
-  const long long ctas = (long long)g.BH * (((kCol ? g.N_kv : g.N_q) + BM - 1) / BM);
-  g.head_group = pick_head_group(ctas, g.BH, 2ll * (kCol ? g.N_q : g.N_kv) * g.D * 2);
+  g.head_group = fb_head_group<KIND, D>(g);
   if constexpr (D == 64) {
-    if (two_per_sm_pays(g, kCol, false, kCol ? 1700.f : 1000.f, kCol ? 1200.f : 1000.f)) {
+    if (plan.dual) {
       using CF = FbCfg<KIND, D, true>;
       static std::atomic<unsigned long long> smem_set{0};
-      return launch_two_per_sm(fb_kernel<KIND, D, T, false, true>, maps, g, t, s, ctas, CF::kThreads, CF::kSmemBytes, smem_set);
+      return launch_two_per_sm(tile_kernel<fb_kernel<KIND, D, T, false, true>>, maps, g, t, s,
+                               (long long)g.BH * (((kCol ? g.N_kv : g.N_q) + BM - 1) / BM), CF::kThreads, CF::kSmemBytes, smem_set);
     }
   }
   using CF = FbCfg<KIND, D, false>;
-  static TileKernelState state;
-  return launch_tiles(fb_kernel<KIND, D, T, false, false>, fb_kernel<KIND, D, T, true, false>, maps, g, t, s, kCol, CF::kThreads,
-                      CF::kSmemBytes, kCol ? 1700.f : 1150.f, kCol ? 1150.f : 1700.f, state);
+  return launch_split(tile_kernel<fb_kernel<KIND, D, T, false, false>>, tile_kernel<fb_kernel<KIND, D, T, true, false>>, maps, g, t, s, kCol,
+                      CF::kThreads, CF::kSmemBytes, plan.split, fb_state<KIND, D, T>());
+}
+
+// Both kinds in one grid (pair_kernel)
+template <int D, typename T, bool DUAL>
+static cudaError_t launch_fb_pair(const TmaMaps& maps, const Geometry& g, const Tensors& t, cudaStream_t s, bool row_first) {
+  using Row = fb_kernel<FB_BWD_ROW, D, T, false, DUAL>;
+  using Col = fb_kernel<FB_BWD_COL, D, T, false, DUAL>;
+  constexpr uint32_t kWanted = Row::CF::kSmemBytes > Col::CF::kSmemBytes ? Row::CF::kSmemBytes : Col::CF::kSmemBytes;
+  static std::atomic<unsigned long long> smem_set[2];
+  const long long rows = (long long)g.BH * ((g.N_q + BM - 1) / BM), cols = (long long)g.BH * ((g.N_kv + BM - 1) / BM);
+  return row_first ? launch_pair<Row, Col>(maps, g, t, s, rows, fb_head_group<FB_BWD_ROW, D>(g), cols, fb_head_group<FB_BWD_COL, D>(g), kWanted, smem_set[0])
+                   : launch_pair<Col, Row>(maps, g, t, s, cols, fb_head_group<FB_BWD_COL, D>(g), rows, fb_head_group<FB_BWD_ROW, D>(g), kWanted, smem_set[1]);
 }
 
 template <int D, typename T>
-static cudaError_t launch_fb_kind(int kind, const TmaMaps& maps, const Geometry& g, const Tensors& t, cudaStream_t s) {
-  return kind == FB_BWD_ROW ? launch_fb<FB_BWD_ROW, D, T>(maps, g, t, s) : launch_fb<FB_BWD_COL, D, T>(maps, g, t, s);
+static cudaError_t launch_bwd_tiles(const TmaMaps& maps, const Geometry& g, const Tensors& t, cudaStream_t s, bool row_first, int* launches) {
+  const FbPlan row = plan_fb<FB_BWD_ROW, D, T>(g), col = plan_fb<FB_BWD_COL, D, T>(g);
+  // Streams of up to 32 tiles: above, the start of a second grid no longer shows (404 us before, 398 after, most
+  // of which is the k-steps', at H32, 1024 queries, 9216 keys, D80; 65.0 and 64.6 at H12 D64).
+  if (row.dual == col.dual && row.split == 1 && col.split == 1 && longest_stream(g) <= 32) {
+    *launches += 1;
+    if constexpr (D == 64) {
+      if (row.dual) return launch_fb_pair<D, T, true>(maps, g, t, s, row_first);
+    }
+    return launch_fb_pair<D, T, false>(maps, g, t, s, row_first);
+  }
+  *launches += 2;
+  Geometry second = g;
+  second.beside = 1;
+  const cudaError_t e = row_first ? launch_fb<FB_BWD_ROW, D, T>(maps, g, t, s, row) : launch_fb<FB_BWD_COL, D, T>(maps, g, t, s, col);
+  if (e != cudaSuccess) return e;
+  return row_first ? launch_fb<FB_BWD_COL, D, T>(maps, second, t, s, col) : launch_fb<FB_BWD_ROW, D, T>(maps, second, t, s, row);
 }
 
-// kind: 2 backward dQ, 3 backward dK and dV
-cudaError_t launch_fwd_bwd(int kind, int D, int is_bf16, const TmaMaps& maps, const Geometry& g, const Tensors& t,
-                           cudaStream_t s) {
-  if (D <= 64) return is_bf16 ? launch_fb_kind<64, __nv_bfloat16>(kind, maps, g, t, s) : launch_fb_kind<64, __half>(kind, maps, g, t, s);
-  return is_bf16 ? launch_fb_kind<128, __nv_bfloat16>(kind, maps, g, t, s) : launch_fb_kind<128, __half>(kind, maps, g, t, s);
+// dQ, dK and dV, given Dv; the kind with the longer CTAs first
+cudaError_t launch_bwd(int D, int is_bf16, const TmaMaps& maps, const Geometry& g, const Tensors& t, cudaStream_t s, bool row_first, int* launches) {
+  if (D <= 64)
+    return is_bf16 ? launch_bwd_tiles<64, __nv_bfloat16>(maps, g, t, s, row_first, launches) : launch_bwd_tiles<64, __half>(maps, g, t, s, row_first, launches);
+  return is_bf16 ? launch_bwd_tiles<128, __nv_bfloat16>(maps, g, t, s, row_first, launches) : launch_bwd_tiles<128, __half>(maps, g, t, s, row_first, launches);
 }
 
 }  // namespace tc

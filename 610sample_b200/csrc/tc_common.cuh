@@ -271,32 +271,80 @@ inline int cluster_slots(Kern kern, int c, unsigned threads, size_t smem, TileKe
   return n;
 }
 
-// Launch of a tensor-core kernel, one CTA per SM (more than half of an SM's shared memory is asked
-// for, so the 512-column tensor-memory allocation never waits for a co-resident CTA), with the split
-// its load asks for: `whole` where it is none, else `shared`.  A tile takes `tile_clocks`; other_clocks
-// is the same for the other side's kernel where that runs beside this one, else 0.
+// Shared memory of a CTA that has its SM to itself: more than half of it, so that the 512-column tensor-memory
+// allocation never waits for a co-resident CTA
+inline size_t whole_sm_smem(size_t wanted) { return wanted < 122880u ? 122880u : wanted; }
+
+// The split that a kernel's load asks for (`shared`: its form with a split).  A tile takes `tile_clocks`;
+// other_clocks is the same for the other side's kernel where that runs beside this one, else 0.
 template <typename... P>
-inline cudaError_t launch_tiles(void (*whole)(P...), void (*shared)(P...), const TmaMaps& maps, Geometry g, const Tensors& t,
-                                cudaStream_t s, bool col, unsigned threads, size_t smem_wanted, float tile_clocks, float other_clocks,
-                                TileKernelState& state) {
+inline int choose_split(void (*shared)(P...), const Geometry& g, bool col, unsigned threads, size_t smem_wanted, float tile_clocks, float other_clocks,
+                        TileKernelState& state) {
+  const long long units = (long long)g.BH * (((col ? g.N_kv : g.N_q) + BM - 1) / BM);
+  // no split pays where half of the longest stream is cheaper than what a split costs
+  if (2 * units > kSms || !((col ? g.N_q : g.N_kv) * (0.5f / BN) * tile_clocks > split_clocks(g.D))) return 1;
+  const SplitLoad w = stream_load(g, col, tile_clocks);
+  const bool paired = other_clocks > 0.f;
+  SplitLoad other = {0.f, 0.f, 0.f, 0.f};
+  if (paired) other = stream_load(g, !col, other_clocks);
+  // of a pair, the kernel with the longer CTAs only: two kernels of clusters do not share the GPU well
+  if (!(w.longest * w.tile_clocks > other.longest * other.tile_clocks)) return 1;
+  return pick_split(w, paired ? &other : nullptr, g.D, [&](int c) { return cluster_slots(shared, c, threads, whole_sm_smem(smem_wanted), state); });
+}
+
+// Launch of a tensor-core kernel, one CTA per SM, with `split` CTAs per tile: `whole` where that is one, else `shared`.
+template <typename... P>
+inline cudaError_t launch_split(void (*whole)(P...), void (*shared)(P...), const TmaMaps& maps, Geometry g, const Tensors& t,
+                                cudaStream_t s, bool col, unsigned threads, size_t smem_wanted, int split, TileKernelState& state) {
   const long long units = (long long)g.BH * (((col ? g.N_kv : g.N_q) + BM - 1) / BM);
   if (units <= 0) return cudaSuccess;
   if (units * kMaxSplit > 0x7fffffffLL) return cudaErrorInvalidValue;
-  const size_t smem = smem_wanted < 122880u ? 122880u : smem_wanted;
-  g.split = 1;
-  // no split pays where half of the longest stream is cheaper than what a split costs
-  if (2 * units <= kSms && (col ? g.N_q : g.N_kv) * (0.5f / BN) * tile_clocks > split_clocks(g.D)) {
-    const SplitLoad w = stream_load(g, col, tile_clocks);
-    const bool paired = other_clocks > 0.f;
-    SplitLoad other = {0.f, 0.f, 0.f, 0.f};
-    if (paired) other = stream_load(g, !col, other_clocks);
-    // of a pair, the kernel with the longer CTAs only: two kernels of clusters do not share the GPU well
-    if (w.longest * w.tile_clocks > other.longest * other.tile_clocks)
-      g.split = pick_split(w, paired ? &other : nullptr, g.D, [&](int c) { return cluster_slots(shared, c, threads, smem, state); });
-  }
+  const size_t smem = whole_sm_smem(smem_wanted);
+  g.split = split;
   auto kern = g.split > 1 ? shared : whole;
   const cudaError_t e = set_smem_once(kern, smem, g.split > 1 ? state.smem_set_split : state.smem_set);
   return e != cudaSuccess ? e : launch_pdl_cluster(kern, (unsigned)(units * g.split), threads, smem, (unsigned)g.split, s, maps, g, t);
+}
+
+template <typename... P>
+inline cudaError_t launch_tiles(void (*whole)(P...), void (*shared)(P...), const TmaMaps& maps, const Geometry& g, const Tensors& t,
+                                cudaStream_t s, bool col, unsigned threads, size_t smem_wanted, float tile_clocks, float other_clocks,
+                                TileKernelState& state) {
+  const int split = choose_split(shared, g, col, threads, smem_wanted, tile_clocks, other_clocks, state);
+  return launch_split(whole, shared, maps, g, t, s, col, threads, smem_wanted, split, state);
+}
+
+// Upper bound of the streamed tiles of any stationary tile, of either side.
+inline int longest_stream(const Geometry& g) {
+  const long long reach = g.mask_mode != 0 ? 1ll << 40 : (long long)g.window + BM;      // rows of one side that a tile of the other can see
+  const long long keys = reach < g.N_kv ? reach : g.N_kv, queries = reach < g.N_q ? reach : g.N_q, n = keys > queries ? keys : queries;
+  return (int)((n + BN - 1) / BN);
+}
+
+// ---- Two kernels in one grid ------------------------------------------------------------------
+// Two kernels of one operation that do not depend on each other, as one launch: a kernel is a type with `run`,
+// which does the work of CTA `block` of its own grid.  The CTAs of the first kind are in front, so those of
+// the second take the SMs that its last ones leave idle, without a launch of their own: one launch less on
+// the host (2 us), no start of a second grid to wait for, nothing to wait for at its end.  dQ with dK/dV: H4, 64 queries, 256
+// keys, D64 7.0 -> 5.9 us; B2 H8, 200 of 500, D96 11.0 -> 9.7; B2 H12, 777 of 1301, D80 42.2 -> 40.6; B4 H16
+// N1024 D128 96.9 -> 94.7.  Kernels in clusters and kernels that take over CTAs of their grid keep a launch
+// of their own, and so do long streams.
+template <typename Tile>
+__global__ void __launch_bounds__(Tile::kThreads, Tile::kPerSm)
+tile_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Tensors t) {
+  Tile::run(maps, g, t, blockIdx.x);
+}
+
+template <typename First, typename Second>
+__global__ void __launch_bounds__(First::kThreads, First::kPerSm)
+pair_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Tensors t, const unsigned first_ctas, const int second_head_group) {
+  if (blockIdx.x < first_ctas) {
+    First::run(maps, g, t, blockIdx.x);
+  } else {
+    Geometry q = g;
+    q.head_group = second_head_group;
+    Second::run(maps, q, t, blockIdx.x - first_ctas);
+  }
 }
 
 // ---- Persistent CTAs -------------------------------------------------------------------------
@@ -366,14 +414,29 @@ inline bool two_per_sm_pays(const Geometry& g, bool col, bool alone, float tile_
   return two < 0.95f * one;
 }
 
+// more than a third of an SM's shared memory: never a third CTA that would wait for tensor memory
+inline size_t half_sm_smem(size_t wanted) { return wanted < 79872u ? 79872u : wanted; }
+
 template <typename... P>
 inline cudaError_t launch_two_per_sm(void (*kern)(P...), const TmaMaps& maps, const Geometry& g, const Tensors& t, cudaStream_t s,
                                      long long ctas, unsigned threads, size_t smem_wanted, std::atomic<unsigned long long>& smem_set) {
   if (ctas > 0x7fffffffLL) return cudaErrorInvalidValue;
-  // more than a third of an SM's shared memory: never a third CTA that would wait for tensor memory
-  const size_t smem = smem_wanted < 79872u ? 79872u : smem_wanted;
+  const size_t smem = half_sm_smem(smem_wanted);
   const cudaError_t e = set_smem_once(kern, smem, smem_set);
   return e != cudaSuccess ? e : launch_pdl(kern, (unsigned)ctas, threads, smem, s, maps, g, t);
+}
+
+template <typename First, typename Second>
+inline cudaError_t launch_pair(const TmaMaps& maps, const Geometry& g_in, const Tensors& t, cudaStream_t s, long long first_ctas, int first_group,
+                               long long second_ctas, int second_group, size_t smem_wanted, std::atomic<unsigned long long>& smem_set) {
+  static_assert(First::kThreads == Second::kThreads && First::kPerSm == Second::kPerSm, "one launch configuration");
+  if (first_ctas + second_ctas > 0x7fffffffLL) return cudaErrorInvalidValue;
+  const size_t smem = First::kPerSm == 2 ? half_sm_smem(smem_wanted) : whole_sm_smem(smem_wanted);
+  Geometry g = g_in;
+  g.head_group = first_group;
+  const cudaError_t e = set_smem_once(pair_kernel<First, Second>, smem, smem_set);
+  return e != cudaSuccess ? e : launch_pdl(pair_kernel<First, Second>, (unsigned)(first_ctas + second_ctas), (unsigned)First::kThreads, smem, s, maps, g, t,
+                                           (unsigned)first_ctas, second_group);
 }
 
 // Control block of the single-tile self-test kernel (every attention kernel has its own).
