@@ -211,8 +211,9 @@ __host__ __device__ constexpr int smem_floats(int D) {
 }
 
 // DC: 1 for D <= 64, 2 up to 128.
+// The work of CTA `block` of a kind's grid.
 template <int KIND, int DC, typename T>
-__global__ void __launch_bounds__(threads_of(KIND, DC), DC == 1 ? 2 : 1) attn_simt_kernel(const Geometry g, const Tensors t, const int split) {
+__device__ __forceinline__ void simt_tile(const Geometry& g, const Tensors& t, const int split, const int block) {
   using SP = Spec<KIND>;
   constexpr int RA = rows_of(KIND, DC), NT = threads_of(KIND, DC);
   // g_dO = P g_dV + (P o gdS) V - dot2 o (P V).  In fp32 P V is the O of the call; an O of half precision has
@@ -225,7 +226,7 @@ __global__ void __launch_bounds__(threads_of(KIND, DC), DC == 1 ? 2 : 1) attn_si
   const Layout lay(D);
   const int n_stat = SP::kCol ? g.N_kv : g.N_q, n_strm = SP::kCol ? g.N_q : g.N_kv;
   const int tiles = (n_stat + TS - 1) / TS;
-  const int unit = blockIdx.x / split, part = blockIdx.x - unit * split;
+  const int unit = block / split, part = block - unit * split;
   const int bh = unit % g.BH, rank = unit / g.BH;
   const int tile = (SP::kCol || g.mask_mode != 0) ? rank : tiles - 1 - rank;     // heavy tiles first
   const int r0 = tile * TS;
@@ -549,6 +550,21 @@ __global__ void __launch_bounds__(threads_of(KIND, DC), DC == 1 ? 2 : 1) attn_si
   tc::pdl_end(g);
 }
 
+template <int KIND, int DC, typename T>
+__global__ void __launch_bounds__(threads_of(KIND, DC), DC == 1 ? 2 : 1) attn_simt_kernel(const Geometry g, const Tensors t, const int split) {
+  simt_tile<KIND, DC, T>(g, t, split, blockIdx.x);
+}
+
+// Two kinds of one operation that do not depend on each other in one grid, the CTAs of FIRST in front: one
+// launch less (a second-order step at B2 H4 N256 D64, which the host bounds, 6 % faster).
+template <int FIRST, int SECOND, int DC, typename T>
+__global__ void __launch_bounds__(threads_of(FIRST, DC), DC == 1 ? 2 : 1)
+attn_simt_pair_kernel(const Geometry g, const Tensors t, const int split, const int first_ctas) {
+  static_assert(threads_of(FIRST, DC) == threads_of(SECOND, DC), "one launch configuration");
+  if ((int)blockIdx.x < first_ctas) simt_tile<FIRST, DC, T>(g, t, split, blockIdx.x);
+  else simt_tile<SECOND, DC, T>(g, t, split, blockIdx.x - first_ctas);
+}
+
 // CTAs per stationary tile.  In units of the time a CTA that has its SM to itself takes for a streamed tile: a
 // CTA costs about one besides its tiles, 1.6 to 1.9 in a cluster (two barriers, the sum; where two share an SM
 // the other one hides some of it).  Bounds are the longest CTA, whose tiles take 1.5 where two share an SM
@@ -584,14 +600,19 @@ static int split_for(const Geometry& g, long long units, bool col, bool narrow, 
   return best;
 }
 
+template <int KIND>
+static long long units_of(const Geometry& g) { return (long long)g.BH * (((Spec<KIND>::kCol ? g.N_kv : g.N_q) + TS - 1) / TS); }
+
+template <int KIND>
+static int split_of(const Geometry& g) {
+  return split_for(g, units_of<KIND>(g), Spec<KIND>::kCol, g.D <= 64, KIND != K_FWD && KIND != K_HVP_PRE);
+}
+
 template <int KIND, int DC, typename T>
-static cudaError_t launch_dc(const Geometry& g, const Tensors& t, cudaStream_t stream) {
-  const int n_stat = Spec<KIND>::kCol ? g.N_kv : g.N_q;
-  const long long units = (long long)g.BH * ((n_stat + TS - 1) / TS);
+static cudaError_t launch_dc(const Geometry& g, const Tensors& t, cudaStream_t stream, int split) {
+  const long long units = units_of<KIND>(g);
   if (units <= 0) return cudaSuccess;
   if (units * kMaxSplit > 0x7fffffffLL) return cudaErrorInvalidValue;
-  const bool paired = KIND != K_FWD && KIND != K_HVP_PRE;
-  const int split = split_for(g, units, Spec<KIND>::kCol, DC == 1, paired);
   const size_t smem = sizeof(float) * smem_floats<KIND>(g.D);
   auto kern = attn_simt_kernel<KIND, DC, T>;
   static std::atomic<unsigned long long> smem_set{0};
@@ -602,28 +623,59 @@ static cudaError_t launch_dc(const Geometry& g, const Tensors& t, cudaStream_t s
 }
 
 template <int KIND, typename T>
-static cudaError_t launch_one(const Geometry& g, const Tensors& t, cudaStream_t stream) {
-  return g.D <= 64 ? launch_dc<KIND, 1, T>(g, t, stream) : launch_dc<KIND, 2, T>(g, t, stream);
+static cudaError_t launch_one(const Geometry& g, const Tensors& t, cudaStream_t stream, int split) {
+  return g.D <= 64 ? launch_dc<KIND, 1, T>(g, t, stream, split) : launch_dc<KIND, 2, T>(g, t, stream, split);
+}
+
+template <int FIRST, int SECOND, int DC, typename T>
+static cudaError_t launch_pair_dc(const Geometry& g, const Tensors& t, cudaStream_t stream, int split) {
+  constexpr auto bytes = [](int D) { return sizeof(float) * (smem_floats<FIRST>(D) > smem_floats<SECOND>(D) ? smem_floats<FIRST>(D) : smem_floats<SECOND>(D)); };
+  const long long first = units_of<FIRST>(g) * split, ctas = first + units_of<SECOND>(g) * split;
+  if (ctas > 0x7fffffffLL) return cudaErrorInvalidValue;
+  auto kern = attn_simt_pair_kernel<FIRST, SECOND, DC, T>;
+  static std::atomic<unsigned long long> smem_set{0};
+  const cudaError_t e = tc::set_smem_once(kern, bytes(64 * DC), smem_set);
+  if (e != cudaSuccess) return e;
+  return tc::launch_pdl_cluster(kern, (unsigned)ctas, threads_of(FIRST, DC), bytes(g.D), (unsigned)split, stream, g, t, split, (int)first);
+}
+
+// Both kinds: one grid where they ask for the same split, else SECOND behind FIRST without waiting for it.  At D <= 64
+// only where all CTAs run at once: larger ones lose in one grid what the launch gains (double backward 811 against 800 us
+// at B2 H8 N1024, backward 64.7 against 62.1 at B2 H5 N479; D = 128 1 503 against 1 509 and 568 against 573 at N1024).
+template <int FIRST, int SECOND, typename T>
+static cudaError_t launch_two(const Geometry& g, const Tensors& t, cudaStream_t stream, int* n) {
+  const int a = split_of<FIRST>(g), b = split_of<SECOND>(g);
+  if (a == b && (g.D > 64 || (units_of<FIRST>(g) + units_of<SECOND>(g)) * a <= 2 * kSms)) {
+    ++*n;
+    return g.D <= 64 ? launch_pair_dc<FIRST, SECOND, 1, T>(g, t, stream, a) : launch_pair_dc<FIRST, SECOND, 2, T>(g, t, stream, a);
+  }
+  *n += 2;
+  Geometry beside = g;
+  beside.beside = 1;
+  const cudaError_t e = launch_one<FIRST, T>(g, t, stream, a);
+  return e != cudaSuccess ? e : launch_one<SECOND, T>(beside, t, stream, b);
 }
 
 template <typename T>
 static cudaError_t dispatch(int op, const Geometry& g, const Tensors& t, cudaStream_t s, int* n, int phases) {
   cudaError_t e = cudaSuccess;
   *n = 0;
-  Geometry beside = g;      // behind the kernel in front of it in the stream, without waiting for it
-  beside.beside = 1;
+  auto one = [&](auto kind) {
+    constexpr int K = decltype(kind)::value;
+    ++*n;
+    return launch_one<K, T>(g, t, s, split_of<K>(g));
+  };
   if (op == OP_FORWARD) {
-    e = launch_one<K_FWD, T>(g, t, s); *n = 1;
+    e = one(tc::Int<K_FWD>{});
   } else if (op == OP_BACKWARD) {
-    e = launch_one<K_BWD_COL, T>(g, t, s);
-    if (e == cudaSuccess) e = launch_one<K_BWD_ROW, T>(beside, t, s);
-    *n = 2;
+    e = launch_two<K_BWD_COL, K_BWD_ROW, T>(g, t, s, n);
   } else {
     // the scalars and both row-side outputs belong to either of their masks, as the C ABI documents it
     const bool row = (phases & (HVP_PHASE_PRE | HVP_PHASE_ROW)) != 0, col = (phases & HVP_PHASE_COL) != 0;
-    if (row) { e = launch_one<K_HVP_PRE, T>(g, t, s); ++*n; }
-    if (e == cudaSuccess && col) { e = launch_one<K_HVP_COL, T>(g, t, s); ++*n; }
-    if (e == cudaSuccess && row) { e = launch_one<K_HVP_ROW, T>(col ? beside : g, t, s); ++*n; }
+    if (row) e = one(tc::Int<K_HVP_PRE>{});
+    if (e == cudaSuccess && row && col) e = launch_two<K_HVP_COL, K_HVP_ROW, T>(g, t, s, n);
+    else if (e == cudaSuccess && row) e = one(tc::Int<K_HVP_ROW>{});
+    else if (e == cudaSuccess && col) e = one(tc::Int<K_HVP_COL>{});
   }
   return e;
 }
