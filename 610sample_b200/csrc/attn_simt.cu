@@ -30,10 +30,11 @@
 // row, which lets two CTAs of every kind share an SM at D <= 64: one computes while the other loads.
 // Loading the next tile behind the output products instead gave nothing (forward -1 to -3 %, backward +4 %).
 // Small problems: the streamed tiles of a stationary tile are dealt out to a CLUSTER of 2 to 8 CTAs
-// (split_for), whose partial sums are added through distributed shared memory in a fixed order; results are
+// (simt_split.h), whose partial sums are added through distributed shared memory in a fixed order; results are
 // bitwise reproducible either way.
 #include "attn_common.cuh"
 #include "attn_launch.h"
+#include "simt_split.h"
 #include "tc_common.cuh"
 
 #include <cooperative_groups.h>
@@ -43,12 +44,7 @@ namespace simt {
 
 namespace cg = cooperative_groups;
 
-constexpr int TS = 32;        // stationary rows per CTA
-constexpr int TT = 64;        // streamed rows per iteration
 constexpr int CB = 4;         // score columns per thread, 8 apart
-constexpr int kMaxSplit = 8;  // CTAs per cluster (the portable maximum)
-
-enum Kind { K_FWD = 0, K_BWD_ROW, K_BWD_COL, K_HVP_PRE, K_HVP_ROW, K_HVP_COL };
 
 // By kind and tile width (DC = 1: D <= 64, 2: D <= 128): score rows per thread, 4 apart, and threads per
 // CTA, (8 / RA) x 2 warps over the 32 x 64 score tile.
@@ -565,66 +561,46 @@ attn_simt_pair_kernel(const Geometry g, const Tensors t, const int split, const 
   else simt_tile<SECOND, DC, T>(g, t, split, blockIdx.x - first_ctas);
 }
 
-// CTAs per stationary tile.  In units of the time a CTA that has its SM to itself takes for a streamed tile: a
-// CTA costs about one besides its tiles, 1.6 to 1.9 in a cluster (two barriers, the sum; where two share an SM
-// the other one hides some of it).  Bounds are the longest CTA, whose tiles take 1.5 where two share an SM
-// (D <= 64), and the whole load over the SMs, with that of the kernel beside it (`paired`).
-// B2 H5 N479 D64 (150 tiles of up to 8): forward 50 -> 31, backward 85 -> 62, double backward 258 -> 172 us
-// in pairs, where all that filled a CTA per SM used to go unsplit; B1 H3 N150 D128 (15 tiles of up to 3) in fours
-// 17 -> 10.5, 26 -> 15.5, 84 -> 50; B2 H7 N293 D80 (140 tiles of up to 5), which used to go in pairs, unsplit
-// 31 -> 28, 73 -> 54, 172 -> 156.
-static int split_for(const Geometry& g, long long units, bool col, bool narrow, bool paired) {
-  if (units > 2 * kSms) return 1;
-  const int n = col ? g.N_kv : g.N_q, tiles = (n + TS - 1) / TS;      // at most as many as there are units
-  int longest = 0;
-  long long per_head = 0;
-  for (int i = 0; i < tiles; ++i) {
-    int lo, hi;
-    if (col) query_range_for_keys(g, i * TS, (i + 1) * TS, lo, hi);
-    else key_range_for_queries(g, i * TS, (i + 1) * TS, lo, hi);
-    const int k = hi > lo ? (hi + TT - 1) / TT - lo / TT : 0;
-    if (k > longest) longest = k;
-    per_head += k;
-  }
-  const float total = (float)per_head * g.BH, shared = narrow ? 1.5f : 1.f;
-  const int slots = narrow ? 2 * kSms : kSms;
-  int best = 1;
-  float least = 0.f;
-  for (int c = 1; c <= kMaxSplit && c < 2 * longest; c *= 2) {
-    const float cta = c == 1 ? (narrow ? 1.f : 1.2f) : narrow ? 1.6f : 1.9f;
-    const float one = (float)((longest + c - 1) / c) * (units * c > kSms ? shared : 1.f) + cta;
-    const float all = (units * c * (narrow && c > 1 ? 1.32f : cta) + total) * shared / slots * (paired ? 2.f : 1.f);
-    const float t = one > all ? one : all;
-    if (c == 1 || t < 0.97f * least) { best = c; least = t; }
-  }
-  return best;
-}
-
 template <int KIND>
 static long long units_of(const Geometry& g) { return (long long)g.BH * (((Spec<KIND>::kCol ? g.N_kv : g.N_q) + TS - 1) / TS); }
 
-template <int KIND>
-static int split_of(const Geometry& g) {
-  return split_for(g, units_of<KIND>(g), Spec<KIND>::kCol, g.D <= 64, KIND != K_FWD && KIND != K_HVP_PRE);
+template <int KIND, int DC, typename T>
+static tc::TileKernelState& state_of() {
+  static tc::TileKernelState state;
+  return state;
+}
+
+// the shared memory of the variant's largest D, so that one setting serves every call
+template <int KIND, int DC> constexpr size_t kVariantSmem = sizeof(float) * smem_floats<KIND>(64 * DC);
+
+// CTAs that run at a time in clusters of c
+template <int KIND, int DC, typename T>
+static int slots_of(int c) {
+  if (c == 1) return DC == 1 ? 2 * kSms : kSms;
+  return tc::cluster_slots(attn_simt_kernel<KIND, DC, T>, c, threads_of(KIND, DC), kVariantSmem<KIND, DC>, state_of<KIND, DC, T>());
 }
 
 template <int KIND, int DC, typename T>
-static cudaError_t launch_dc(const Geometry& g, const Tensors& t, cudaStream_t stream, int split) {
+static cudaError_t launch_split(const Geometry& g, const Tensors& t, cudaStream_t stream, int split) {
   const long long units = units_of<KIND>(g);
   if (units <= 0) return cudaSuccess;
   if (units * kMaxSplit > 0x7fffffffLL) return cudaErrorInvalidValue;
-  const size_t smem = sizeof(float) * smem_floats<KIND>(g.D);
   auto kern = attn_simt_kernel<KIND, DC, T>;
-  static std::atomic<unsigned long long> smem_set{0};
-  // the size at the variant's largest D, so that one setting serves every call
-  const cudaError_t e = tc::set_smem_once(kern, sizeof(float) * smem_floats<KIND>(64 * DC), smem_set);
+  const cudaError_t e = tc::set_smem_once(kern, kVariantSmem<KIND, DC>, state_of<KIND, DC, T>().smem_set_split);
   if (e != cudaSuccess) return e;
-  return tc::launch_pdl_cluster(kern, (unsigned)(units * split), threads_of(KIND, DC), smem, (unsigned)split, stream, g, t, split);
+  return tc::launch_pdl_cluster(kern, (unsigned)(units * split), threads_of(KIND, DC), sizeof(float) * smem_floats<KIND>(g.D), (unsigned)split, stream,
+                                g, t, split);
+}
+
+template <int KIND, int DC, typename T>
+static cudaError_t launch_dc(const Geometry& g, const Tensors& t, cudaStream_t stream) {
+  const Splits s = pick_splits(work_of(g, (Kind)KIND, DC == 1), nullptr, shared_tile(DC == 1), slots_of<KIND, DC, T>, slots_of<KIND, DC, T>);
+  return launch_split<KIND, DC, T>(g, t, stream, s.a);
 }
 
 template <int KIND, typename T>
-static cudaError_t launch_one(const Geometry& g, const Tensors& t, cudaStream_t stream, int split) {
-  return g.D <= 64 ? launch_dc<KIND, 1, T>(g, t, stream, split) : launch_dc<KIND, 2, T>(g, t, stream, split);
+static cudaError_t launch_one(const Geometry& g, const Tensors& t, cudaStream_t stream) {
+  return g.D <= 64 ? launch_dc<KIND, 1, T>(g, t, stream) : launch_dc<KIND, 2, T>(g, t, stream);
 }
 
 template <int FIRST, int SECOND, int DC, typename T>
@@ -642,18 +618,24 @@ static cudaError_t launch_pair_dc(const Geometry& g, const Tensors& t, cudaStrea
 // Both kinds: one grid where they ask for the same split, else SECOND behind FIRST without waiting for it.  At D <= 64
 // only where all CTAs run at once: larger ones lose in one grid what the launch gains (double backward 811 against 800 us
 // at B2 H8 N1024, backward 64.7 against 62.1 at B2 H5 N479; D = 128 1 503 against 1 509 and 568 against 573 at N1024).
-template <int FIRST, int SECOND, typename T>
-static cudaError_t launch_two(const Geometry& g, const Tensors& t, cudaStream_t stream, int* n) {
-  const int a = split_of<FIRST>(g), b = split_of<SECOND>(g);
-  if (a == b && (g.D > 64 || (units_of<FIRST>(g) + units_of<SECOND>(g)) * a <= 2 * kSms)) {
+template <int FIRST, int SECOND, int DC, typename T>
+static cudaError_t launch_two_dc(const Geometry& g, const Tensors& t, cudaStream_t stream, int* n) {
+  const Work first = work_of(g, (Kind)FIRST, DC == 1), second = work_of(g, (Kind)SECOND, DC == 1);
+  const Splits s = pick_splits(first, &second, shared_tile(DC == 1), slots_of<FIRST, DC, T>, slots_of<SECOND, DC, T>);
+  if (s.a == s.b && (DC == 2 || (units_of<FIRST>(g) + units_of<SECOND>(g)) * s.a <= 2 * kSms)) {
     ++*n;
-    return g.D <= 64 ? launch_pair_dc<FIRST, SECOND, 1, T>(g, t, stream, a) : launch_pair_dc<FIRST, SECOND, 2, T>(g, t, stream, a);
+    return launch_pair_dc<FIRST, SECOND, DC, T>(g, t, stream, s.a);
   }
   *n += 2;
   Geometry beside = g;
   beside.beside = 1;
-  const cudaError_t e = launch_one<FIRST, T>(g, t, stream, a);
-  return e != cudaSuccess ? e : launch_one<SECOND, T>(beside, t, stream, b);
+  const cudaError_t e = launch_split<FIRST, DC, T>(g, t, stream, s.a);
+  return e != cudaSuccess ? e : launch_split<SECOND, DC, T>(beside, t, stream, s.b);
+}
+
+template <int FIRST, int SECOND, typename T>
+static cudaError_t launch_two(const Geometry& g, const Tensors& t, cudaStream_t stream, int* n) {
+  return g.D <= 64 ? launch_two_dc<FIRST, SECOND, 1, T>(g, t, stream, n) : launch_two_dc<FIRST, SECOND, 2, T>(g, t, stream, n);
 }
 
 template <typename T>
@@ -663,7 +645,7 @@ static cudaError_t dispatch(int op, const Geometry& g, const Tensors& t, cudaStr
   auto one = [&](auto kind) {
     constexpr int K = decltype(kind)::value;
     ++*n;
-    return launch_one<K, T>(g, t, s, split_of<K>(g));
+    return launch_one<K, T>(g, t, s);
   };
   if (op == OP_FORWARD) {
     e = one(tc::Int<K_FWD>{});
