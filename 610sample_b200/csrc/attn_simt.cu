@@ -615,14 +615,11 @@ static cudaError_t launch_pair_dc(const Geometry& g, const Tensors& t, cudaStrea
   return tc::launch_pdl_cluster(kern, (unsigned)ctas, threads_of(FIRST, DC), bytes(g.D), (unsigned)split, stream, g, t, split, (int)first);
 }
 
-// Both kinds: one grid where they ask for the same split, else SECOND behind FIRST without waiting for it.  At D <= 64
-// only where all CTAs run at once: larger ones lose in one grid what the launch gains (double backward 811 against 800 us
-// at B2 H8 N1024, backward 64.7 against 62.1 at B2 H5 N479; D = 128 1 503 against 1 509 and 568 against 573 at N1024).
 template <int FIRST, int SECOND, int DC, typename T>
 static cudaError_t launch_two_dc(const Geometry& g, const Tensors& t, cudaStream_t stream, int* n) {
   const Work first = work_of(g, (Kind)FIRST, DC == 1), second = work_of(g, (Kind)SECOND, DC == 1);
   const Splits s = pick_splits(first, &second, shared_tile(DC == 1), slots_of<FIRST, DC, T>, slots_of<SECOND, DC, T>);
-  if (s.a == s.b && (DC == 2 || (units_of<FIRST>(g) + units_of<SECOND>(g)) * s.a <= 2 * kSms)) {
+  if (one_grid(s, DC == 1, FIRST == K_HVP_COL, units_of<FIRST>(g) + units_of<SECOND>(g))) {
     ++*n;
     return launch_pair_dc<FIRST, SECOND, DC, T>(g, t, stream, s.a);
   }

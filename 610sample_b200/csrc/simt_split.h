@@ -133,5 +133,18 @@ inline Splits pick_splits(const Work& a, const Work* b, float shared, SlotsA slo
   return best;
 }
 
+// Both kernels in one grid, where they have the same split (`ctas` of both without it), or the second behind the first
+// without waiting for it.  At D > 64, one CTA per SM, one grid takes 1 to 3 % less time in the backward at any size, and in the
+// double backward up to one CTA per SM (above, 1 % less to 0.6 % more on average).  At D <= 64 a grid that wants more than an SM per
+// CTA puts the second kind's long CTAs beside the first's: backward 1.2 times the time at 148 to 296 CTAs (10 heads
+// N320 52 against 40 us) and up to 1.1 from 120 CTAs in clusters of four, but 2 to 4 % less where every CTA has an SM;
+// double backward the same without clusters, in clusters 1 to 5 % less up to two per SM.
+inline bool one_grid(const Splits& s, bool narrow, bool second_order, float ctas) {
+  if (s.a != s.b) return false;
+  if (!narrow) return true;
+  if (second_order && s.a > 1) return ctas * s.a <= 2 * kSms;
+  return s.a <= 2 && ctas * s.a <= kSms;
+}
+
 }  // namespace simt
 }  // namespace attn

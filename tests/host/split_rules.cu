@@ -70,6 +70,18 @@ void limits() {
     }
 }
 
+// Pairs of kernels measured in one grid and in two
+void grids() {
+  check(!one_grid({1, 1}, true, false, 200), "backward, 10 heads N320 D64: 52 us in one grid, 40 in two");
+  check(!one_grid({2, 2}, true, false, 98), "backward, 7 heads N200 D64: 27 us in one grid, 19 in two");
+  check(!one_grid({4, 4}, true, false, 32), "backward, 2 heads N256 D64: 12.2 us in one grid, 11.1 in two");
+  check(!one_grid({1, 1}, true, true, 160), "double backward, 16 heads N160 D64: 1.1 times the time in one grid");
+  check(one_grid({1, 1}, true, false, 128) && one_grid({2, 2}, true, false, 64), "an SM for every CTA: one grid");
+  check(one_grid({2, 2}, true, true, 98) && !one_grid({2, 2}, true, true, 149), "double backward in clusters: two CTAs per SM");
+  check(one_grid({1, 1}, false, false, 5000) && one_grid({8, 8}, false, true, 40), "D > 64: one grid");
+  check(!one_grid({2, 1}, false, false, 20), "different splits: two launches");
+}
+
 void long_sequences() {
   const int n = 0x7fffffff;
   const auto start = std::chrono::steady_clock::now();
@@ -85,6 +97,7 @@ void long_sequences() {
 int main() {
   measured_sizes();
   limits();
+  grids();
   long_sequences();
   return failures;
 }
