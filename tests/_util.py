@@ -4,6 +4,7 @@ import json
 import os
 
 import numpy as np
+import pytest
 import torch
 
 from attention_oracle import INPUT_NAMES, OUTPUT_NAMES
@@ -53,3 +54,25 @@ def record_errors(name, table):
     if path:
         with open(path, "a") as f:
             f.write(json.dumps({"case": name, "errors": table}) + "\n")
+
+
+def captured_kernels(call):
+    """[(mangled name, CTAs per cluster)] of the kernels that `call` launches on the current stream, in the
+    order of a captured graph."""
+    drv = pytest.importorskip("cuda.bindings.driver")
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph, stream=torch.cuda.Stream()):
+        keep = call()
+    raw = drv.CUgraph(graph.raw_cuda_graph())
+    _, _, n = drv.cuGraphGetNodes(raw, 0)
+    _, nodes, _ = drv.cuGraphGetNodes(raw, n)
+    found = []
+    for node in nodes:
+        if drv.cuGraphNodeGetType(node)[1] != drv.CUgraphNodeType.CU_GRAPH_NODE_TYPE_KERNEL:
+            continue
+        p = drv.cuGraphKernelNodeGetParams(node)[1]
+        name = (drv.cuFuncGetName(p.func) if int(p.func) else drv.cuKernelGetName(p.kern))[1].decode()
+        attr = drv.cuGraphKernelNodeGetAttribute(node, drv.CUkernelNodeAttrID.CU_LAUNCH_ATTRIBUTE_CLUSTER_DIMENSION)[1]
+        found.append((name, max(1, attr.clusterDim.x)))
+    del keep
+    return found
