@@ -615,24 +615,28 @@ static cudaError_t launch_pair_dc(const Geometry& g, const Tensors& t, cudaStrea
   return tc::launch_pdl_cluster(kern, (unsigned)ctas, threads_of(FIRST, DC), bytes(g.D), (unsigned)split, stream, g, t, split, (int)first);
 }
 
+// Both kinds, or one of them (`which`: 1 the first, 2 the second, 3 both).  The splits are those of both together in
+// either case, so that the phases of a double backward give the bits of a single call.
 template <int FIRST, int SECOND, int DC, typename T>
-static cudaError_t launch_two_dc(const Geometry& g, const Tensors& t, cudaStream_t stream, int* n) {
+static cudaError_t launch_two_dc(const Geometry& g, const Tensors& t, cudaStream_t stream, int* n, int which) {
   const Work first = work_of(g, (Kind)FIRST, DC == 1), second = work_of(g, (Kind)SECOND, DC == 1);
   const Splits s = pick_splits(first, &second, shared_tile(DC == 1), slots_of<FIRST, DC, T>, slots_of<SECOND, DC, T>);
-  if (one_grid(s, DC == 1, FIRST == K_HVP_COL, units_of<FIRST>(g) + units_of<SECOND>(g))) {
+  if (which == 3 && one_grid(s, DC == 1, FIRST == K_HVP_COL, units_of<FIRST>(g) + units_of<SECOND>(g))) {
     ++*n;
     return launch_pair_dc<FIRST, SECOND, DC, T>(g, t, stream, s.a);
   }
-  *n += 2;
-  Geometry beside = g;
-  beside.beside = 1;
-  const cudaError_t e = launch_split<FIRST, DC, T>(g, t, stream, s.a);
-  return e != cudaSuccess ? e : launch_split<SECOND, DC, T>(beside, t, stream, s.b);
+  cudaError_t e = cudaSuccess;
+  if (which & 1) { e = launch_split<FIRST, DC, T>(g, t, stream, s.a); ++*n; }
+  if (e != cudaSuccess || (which & 2) == 0) return e;
+  ++*n;
+  Geometry second_of = g;
+  second_of.beside = which == 3;
+  return launch_split<SECOND, DC, T>(second_of, t, stream, s.b);
 }
 
 template <int FIRST, int SECOND, typename T>
-static cudaError_t launch_two(const Geometry& g, const Tensors& t, cudaStream_t stream, int* n) {
-  return g.D <= 64 ? launch_two_dc<FIRST, SECOND, 1, T>(g, t, stream, n) : launch_two_dc<FIRST, SECOND, 2, T>(g, t, stream, n);
+static cudaError_t launch_two(const Geometry& g, const Tensors& t, cudaStream_t stream, int* n, int which = 3) {
+  return g.D <= 64 ? launch_two_dc<FIRST, SECOND, 1, T>(g, t, stream, n, which) : launch_two_dc<FIRST, SECOND, 2, T>(g, t, stream, n, which);
 }
 
 template <typename T>
@@ -652,9 +656,7 @@ static cudaError_t dispatch(int op, const Geometry& g, const Tensors& t, cudaStr
     // the scalars and both row-side outputs belong to either of their masks, as the C ABI documents it
     const bool row = (phases & (HVP_PHASE_PRE | HVP_PHASE_ROW)) != 0, col = (phases & HVP_PHASE_COL) != 0;
     if (row) e = one(tc::Int<K_HVP_PRE>{});
-    if (e == cudaSuccess && row && col) e = launch_two<K_HVP_COL, K_HVP_ROW, T>(g, t, s, n);
-    else if (e == cudaSuccess && row) e = one(tc::Int<K_HVP_ROW>{});
-    else if (e == cudaSuccess && col) e = one(tc::Int<K_HVP_COL>{});
+    if (e == cudaSuccess && (row || col)) e = launch_two<K_HVP_COL, K_HVP_ROW, T>(g, t, s, n, (col ? 1 : 0) | (row ? 2 : 0));
   }
   return e;
 }
