@@ -787,9 +787,10 @@ static cudaError_t launch_fb_pair(const TmaMaps& maps, const Geometry& g, const 
 template <int D, typename T>
 static cudaError_t launch_bwd_tiles(const TmaMaps& maps, const Geometry& g, const Tensors& t, cudaStream_t s, bool row_first, int* launches) {
   const FbPlan row = plan_fb<FB_BWD_ROW, D, T>(g), col = plan_fb<FB_BWD_COL, D, T>(g);
-  // Streams of up to 32 tiles: above, the start of a second grid no longer shows (404 us before, 398 after, most
-  // of which is the k-steps', at H32, 1024 queries, 9216 keys, D80; 65.0 and 64.6 at H12 D64).
-  if (row.dual == col.dual && row.split == 1 && col.split == 1 && longest_stream(g) <= 32) {
+  // One grid against two launches, 220 sizes (512 to 8192 rows; causal, in chunks against a window, without a mask; 8 to
+  // 96 heads): up to 33 tiles 0.983, 0.982, 0.983 and 0.985 of the time at D = 64, 80, 96 and 128, the more the shorter
+  // (0.93 to 1.009 each); 34 to 146 tiles 0.997, 0.992, 0.989 and 0.991 (0.95 to 1.013), so the limit is no crossing.
+  if (row.dual == col.dual && row.split == 1 && col.split == 1 && longest_stream(g) <= 33) {
     *launches += 1;
     if constexpr (D == 64) {
       if (row.dual) return launch_fb_pair<D, T, true>(maps, g, t, s, row_first);

@@ -316,9 +316,11 @@ inline cudaError_t launch_tiles(void (*whole)(P...), void (*shared)(P...), const
 
 // Upper bound of the streamed tiles of any stationary tile, of either side.
 inline int longest_stream(const Geometry& g) {
-  const long long reach = g.mask_mode != 0 ? 1ll << 40 : (long long)g.window + BM;      // rows of one side that a tile of the other can see
-  const long long keys = reach < g.N_kv ? reach : g.N_kv, queries = reach < g.N_q ? reach : g.N_q, n = keys > queries ? keys : queries;
-  return (int)((n + BN - 1) / BN);
+  const long long n = g.N_kv > g.N_q ? g.N_kv : g.N_q, all = (n + BN - 1) / BN;
+  if (g.mask_mode != 0) return (int)all;
+  const long long rows = (long long)g.window + BM - 1;              // of one side that a tile of the other can see, from any row on
+  const long long seen = (rows - 1 + BN - 1) / BN + 1;
+  return (int)(seen < all ? seen : all);
 }
 
 // ---- Two kernels in one grid ------------------------------------------------------------------

@@ -78,8 +78,26 @@ static void load_of_a_problem() {
   check(v.longest == 6.f && v.mean > 5.9f && v.mean <= 6.f, "load of a long sequence with a window");
 }
 
+static void bound_of_a_stream() {
+  unsigned seed = 1;
+  auto below = [&](int n) { seed = seed * 1664525u + 1013904223u; return (int)((seed >> 8) % (unsigned)n); };
+  for (int i = 0; i < 20000; ++i) {
+    Geometry g = geometry(1, 1 + below(4000), 1 + below(4000), 1 + below(4200), below(8) == 0);
+    const int chunk = below(9);
+    if (i == 0) g = geometry(1, 1024, 4000, 1920, 0);       // keys 1057 to 3103 of a tile of queries: 33 tiles
+    g.qi_base = (i == 0 ? 8 : chunk) * g.N_q;
+    g.ki_base = g.qi_base + g.N_q - g.N_kv;
+    const float row = stream_load(g, false, 1.f).longest, col = stream_load(g, true, 1.f).longest;
+    check((float)longest_stream(g) >= (row > col ? row : col), "bound of the streamed tiles");
+    if (failures > 3) return;
+  }
+  check(longest_stream(geometry(1, 2048, 2048, 2048, 0)) == 32 && longest_stream(geometry(1, 2048, 2048, 1, 1)) == 32, "whole sequences");
+  check(longest_stream(geometry(1, 9000, 9000, 64, 0)) == 4, "a window");
+}
+
 int main() {
   cluster_queries();
   load_of_a_problem();
+  bound_of_a_stream();
   return failures;
 }
