@@ -594,7 +594,7 @@ static cudaError_t launch_split(const Geometry& g, const Tensors& t, cudaStream_
 
 template <int KIND, int DC, typename T>
 static cudaError_t launch_dc(const Geometry& g, const Tensors& t, cudaStream_t stream) {
-  const Splits s = pick_splits(work_of(g, (Kind)KIND, DC == 1), nullptr, shared_tile(DC == 1), slots_of<KIND, DC, T>, slots_of<KIND, DC, T>);
+  const Splits s = pick_splits(work_of(g, (Kind)KIND, DC == 1), nullptr, DC == 1, false, slots_of<KIND, DC, T>);
   return launch_split<KIND, DC, T>(g, t, stream, s.a);
 }
 
@@ -620,8 +620,8 @@ static cudaError_t launch_pair_dc(const Geometry& g, const Tensors& t, cudaStrea
 template <int FIRST, int SECOND, int DC, typename T>
 static cudaError_t launch_two_dc(const Geometry& g, const Tensors& t, cudaStream_t stream, int* n, int which) {
   const Work first = work_of(g, (Kind)FIRST, DC == 1), second = work_of(g, (Kind)SECOND, DC == 1);
-  const Splits s = pick_splits(first, &second, shared_tile(DC == 1), slots_of<FIRST, DC, T>, slots_of<SECOND, DC, T>);
-  if (which == 3 && one_grid(s, DC == 1, FIRST == K_HVP_COL, units_of<FIRST>(g) + units_of<SECOND>(g))) {
+  const Splits s = pick_splits(first, &second, DC == 1, FIRST == K_HVP_COL, slots_of<FIRST, DC, T>);
+  if (which == 3 && s.together) {
     ++*n;
     return launch_pair_dc<FIRST, SECOND, DC, T>(g, t, stream, s.a);
   }

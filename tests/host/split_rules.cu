@@ -25,9 +25,9 @@ enum Op { FWD, BWD, HVP };
 Splits rule(Op op, const Geometry& g) {
   const bool narrow = g.D <= 64;
   auto s = [&](int c) { return slots(narrow, c); };
-  if (op == FWD) return pick_splits(work_of(g, K_FWD, narrow), nullptr, shared_tile(narrow), s, s);
+  if (op == FWD) return pick_splits(work_of(g, K_FWD, narrow), nullptr, narrow, false, s);
   const Work a = work_of(g, op == BWD ? K_BWD_COL : K_HVP_COL, narrow), b = work_of(g, op == BWD ? K_BWD_ROW : K_HVP_ROW, narrow);
-  return pick_splits(a, &b, shared_tile(narrow), s, s);
+  return pick_splits(a, &b, narrow, op == HVP, s);
 }
 
 // Sizes at which a split that a model without the second wave of clusters, or without the kernel beside, takes is
@@ -65,21 +65,22 @@ void limits() {
       const Geometry g = geometry(1, 576, 576, D, 576, 0, 0);
       const Work a = work_of(g, K_HVP_COL, D == 64), b = work_of(g, K_HVP_ROW, D == 64);
       auto pairs = [&](int c) { return c <= 2 ? slots(D == 64, c) : c == 4 ? 0 : -1; };
-      const Splits s = pick_splits(a, &b, shared_tile(D == 64), pairs, pairs);
+      const Splits s = pick_splits(a, &b, D == 64, true, pairs);
       check(s.a == 2 && s.b == 2, "clusters of two where larger ones do not run");
     }
 }
 
-// Pairs of kernels measured in one grid and in two
+// Pairs of kernels in one grid and in two
 void grids() {
-  check(!one_grid({1, 1}, true, false, 200), "backward, 10 heads N320 D64: 52 us in one grid, 40 in two");
-  check(!one_grid({2, 2}, true, false, 98), "backward, 7 heads N200 D64: 27 us in one grid, 19 in two");
-  check(!one_grid({4, 4}, true, false, 32), "backward, 2 heads N256 D64: 12.2 us in one grid, 11.1 in two");
-  check(!one_grid({1, 1}, true, true, 160), "double backward, 16 heads N160 D64: 1.1 times the time in one grid");
-  check(one_grid({1, 1}, true, false, 128) && one_grid({2, 2}, true, false, 64), "an SM for every CTA: one grid");
-  check(one_grid({2, 2}, true, true, 98) && !one_grid({2, 2}, true, true, 149), "double backward in clusters: two CTAs per SM");
-  check(one_grid({1, 1}, false, false, 5000) && one_grid({8, 8}, false, true, 40), "D > 64: one grid");
-  check(!one_grid({2, 1}, false, false, 20), "different splits: two launches");
+  auto together = [](Op op, const Geometry& g) { return rule(op, g).together; };
+  check(together(BWD, geometry(4, 128, 128, 64, 128, 0, 0)) && together(HVP, geometry(4, 100, 100, 48, 100, 0, 0)), "an SM for every CTA: one grid");
+  check(!together(BWD, geometry(10, 320, 320, 64, 320, 0, 0)), "backward, 10 heads N320 D64: 52 us in one grid, 35 in two");
+  check(!together(BWD, geometry(2, 383, 383, 64, 383, 0, 0)), "backward, 2 heads N383 D64: 24.7 us in one grid, 18.9 in two");
+  check(together(BWD, geometry(8, 256, 256, 64, 256, 0, 0)), "CTAs of two tiles: the launch counts");
+  check(!one_grid(1, 1, true, true, 160, 2) && one_grid(2, 2, true, true, 98, 2) && !one_grid(2, 2, true, true, 149, 2), "double backward: in clusters, up to two CTAs per SM");
+  check(together(BWD, geometry(16, 320, 320, 128, 320, 0, 0)) && one_grid(8, 8, false, true, 40, 4), "D > 64: one grid");
+  check(!one_grid(2, 1, false, false, 20, 4) && !one_grid(2, 1, true, true, 20, 1), "different splits: two launches");
+  check(!rule(FWD, geometry(1, 64, 64, 64, 64, 0, 0)).together, "one kernel");
 }
 
 void long_sequences() {

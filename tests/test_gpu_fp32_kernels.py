@@ -96,20 +96,22 @@ def _parsed(forms):
 # (B, H, N_q, N_kv, D, window, chunk, mask) and the forms that the rule takes there
 FORMS = [
     ((2, 5, 479, 479, 64, 479, 0, 0), "O 2 dQ 2 dK 2 g_dO 4 g_Q 4 g_K 2"),            # 150 tiles of up to 8: parts without a tile
+    ((4, 1, 383, 383, 48, 383, 0, 0), "O 4 dQ 4 dK 4 g_dO 4 g_Q 4 g_K 4"),
+    ((1, 1, 700, 700, 64, 700, 0, 0), "O 8 dQ 8 dK 8 g_dO 8 g_Q 8 g_K 8"),
     ((1, 3, 150, 150, 128, 150, 0, 0), "O 4 g_dO 4 dK+dQ 4 g_K+g_Q 4"),               # three streamed tiles for a cluster of four
-    ((2, 7, 160, 293, 80, 293, 1, 0), "O 2 dQ 2 dK 1 g_dO 2 g_Q 2 g_K 1"),            # 70 and 140 tiles: one side split
+    ((2, 7, 160, 293, 80, 293, 1, 0), "O 2 g_dO 2 dK+dQ 1 g_Q 2 g_K 1"),              # 140 and 70 tiles: one side split
     ((2, 5, 160, 293, 80, 293, 1, 0), "O 4 dQ 2 dK 1 g_dO 4 g_Q 2 g_K 1"),
     ((1, 9, 1023, 65, 64, 1023, 0, 1), "O 1 dQ 1 dK 8 g_dO 1 g_Q 1 g_K 8"),           # 288 tiles of two, 27 of 16
     ((1, 10, 961, 33, 96, 40, 0, 0), "O 1 dQ 1 dK 2 g_dO 1 g_Q 1 g_K 2"),             # 310 tiles, most of which see nothing
-    ((1, 1, 520, 520, 64, 520, 0, 0), "O 8 dQ 4 dK 4 g_dO 8 g_K+g_Q 8"),
-    ((1, 1, 400, 400, 64, 400, 0, 0), "O 8 dQ 8 dK 8 g_dO 8 g_K+g_Q 8"),
+    ((1, 1, 520, 520, 64, 520, 0, 0), "O 8 g_dO 8 dK+dQ 8 g_K+g_Q 8"),
+    ((1, 1, 400, 400, 64, 400, 0, 0), "O 8 g_dO 8 dK+dQ 8 g_K+g_Q 8"),
     ((1, 1, 520, 520, 128, 520, 0, 0), "O 8 g_dO 8 dK+dQ 4 g_K+g_Q 4"),
     ((1, 1, 300, 300, 80, 300, 0, 0), "O 8 dQ 4 dK 8 g_dO 8 g_Q 4 g_K 8"),
     ((1, 1, 33, 500, 96, 500, 0, 1), "O 8 dQ 8 dK 1 g_dO 8 g_Q 8 g_K 1"),
     ((1, 1, 500, 33, 112, 500, 0, 1), "O 1 dQ 1 dK 8 g_dO 1 g_Q 1 g_K 8"),
     ((1, 1, 95, 250, 80, 250, 2, 0), "O 4 dQ 4 dK 2 g_dO 4 g_Q 4 g_K 2"),
     ((1, 4, 100, 100, 64, 100, 0, 0), "O 2 g_dO 2 dK+dQ 2 g_K+g_Q 2"),
-    ((2, 2, 250, 250, 64, 250, 0, 0), "O 4 dQ 4 dK 4 g_dO 4 g_K+g_Q 4"),
+    ((2, 2, 250, 250, 64, 250, 0, 0), "O 4 g_dO 4 dK+dQ 4 g_K+g_Q 4"),
     ((1, 1, 32, 64, 64, 64, 0, 1), "O 1 g_dO 1 dK+dQ 1 g_K+g_Q 1"),                   # one tile: one grid without a cluster
     ((2, 8, 600, 600, 64, 600, 0, 0), "O 1 dQ 1 dK 1 g_dO 1 g_Q 1 g_K 1"),            # 304 tiles: no split
     ((1, 1, 264, 586, 80, 586, 0, 0), "O 8 g_dO 8 dK+dQ 4 g_K+g_Q 8"),                # keys without a visible query
@@ -136,5 +138,5 @@ def test_fp32_forms_cover_every_kernel():
     for wide in (False, True):
         for k in ("O", "dQ", "dK", "g_dO", "g_Q", "g_K"):
             assert seen[k, wide] == {1, 2, 4, 8}, (k, wide, seen[k, wide])
-    assert seen["dK+dQ", False] == {1, 2} and seen["g_K+g_Q", False] == {1, 2, 4, 8}
+    assert seen["dK+dQ", False] == {1, 2, 4, 8} and seen["g_K+g_Q", False] == {1, 2, 4, 8}
     assert {1, 4} <= seen["dK+dQ", True] and {4, 8} <= seen["g_K+g_Q", True]
