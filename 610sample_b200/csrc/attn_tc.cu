@@ -269,31 +269,8 @@ cudaError_t launch_hvp_col(int D, int is_bf16, const TmaMaps& maps, const Geomet
 cudaError_t launch_hvp_row(int mode, int D, int is_bf16, const TmaMaps& maps, const Geometry& g,
                            const Tensors& t, cudaStream_t s);
 
-cudaError_t launch_bwd(int D, int is_bf16, const TmaMaps& maps, const Geometry& g, const Tensors& t, cudaStream_t s, bool row_first,
-                       int* launches);
+cudaError_t launch_bwd(int D, int is_bf16, const TmaMaps& maps, const Geometry& g, const Tensors& t, cudaStream_t s, int* launches);
 cudaError_t launch_fwd(int D, int is_bf16, const TmaMaps& maps, const Geometry& g, const Tensors& t, cudaStream_t s);
-
-// dQ beside dK/dV and g_Q beside g_K/g_V: the CTAs of one first, the other's on the SMs its last CTAs
-// leave idle (tc_common.cuh).  The kernel with the longer CTAs goes first, so that the tail is made
-// of short ones: the row kernel where a query sees more keys than a key is seen by queries (chunks of
-// 1024 queries against a window of 8192: 128 tiles per row CTA, 16 per column CTA; backward 410 ->
-// 392 us at H32 D80), else the column kernel, whose tile costs more.
-static bool row_side_first(const Geometry& g) {
-  if (g.mask_mode != 0) return g.N_kv > g.N_q;
-  return (g.window < g.N_kv ? g.window : g.N_kv) > (g.window < g.N_q ? g.window : g.N_q);
-}
-
-template <typename Row, typename Col>
-static cudaError_t side_by_side(const Geometry& g, Row row, Col col) {
-  Geometry second = g;
-  second.beside = 1;
-  if (row_side_first(g)) {
-    const cudaError_t e = row(g);
-    return e == cudaSuccess ? col(second) : e;
-  }
-  const cudaError_t e = col(g);
-  return e == cudaSuccess ? row(second) : e;
-}
 
 template <typename T>
 static cudaError_t launch_op(int op, const TmaMaps& maps, const Geometry& g, const Tensors& t, cudaStream_t s,
@@ -310,7 +287,7 @@ static cudaError_t launch_op(int op, const TmaMaps& maps, const Geometry& g, con
       e = launch_rowdot<T>((const T*)t.dO, (const T*)t.O, t.Dv, rows, g.D, s);
     }
     *n = 1;
-    if (e == cudaSuccess) e = launch_bwd(D, bf, maps, g, t, s, row_side_first(g), n);                     // dQ; dK, dV
+    if (e == cudaSuccess) e = launch_bwd(D, bf, maps, g, t, s, n);                                       // dQ; dK, dV
   } else {
     if (phases & HVP_PHASE_PRE) { e = launch_hvp_row(0, D, bf, maps, g, t, s); ++*n; }                        // scalars + g_dO
     const bool row = (phases & HVP_PHASE_ROW) != 0, col = (phases & HVP_PHASE_COL) != 0;

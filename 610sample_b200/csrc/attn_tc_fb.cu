@@ -312,8 +312,7 @@ __device__ __forceinline__ void fb_kernel<KIND, D, T, SPLIT, DUAL>::run(const Tm
         __syncwarp();
       };
       auto issue_out = [&](int j) {
-        const int b = j % kBufs;
-        (void)b;
+        [[maybe_unused]] const int b = j % kBufs;
         const uint64_t dm = smem_desc_sw128(stage_of(j), kAtomBytesStrm, 1024);
         const bool first = (j == 0);
         if (elect_one()) {
@@ -774,18 +773,18 @@ static cudaError_t launch_fb(const TmaMaps& maps, const Geometry& g_in, const Te
 
 // Both kinds in one grid (pair_kernel)
 template <int D, typename T, bool DUAL>
-static cudaError_t launch_fb_pair(const TmaMaps& maps, const Geometry& g, const Tensors& t, cudaStream_t s, bool row_first) {
+static cudaError_t launch_fb_pair(const TmaMaps& maps, const Geometry& g, const Tensors& t, cudaStream_t s) {
   using Row = fb_kernel<FB_BWD_ROW, D, T, false, DUAL>;
   using Col = fb_kernel<FB_BWD_COL, D, T, false, DUAL>;
   constexpr uint32_t kWanted = Row::CF::kSmemBytes > Col::CF::kSmemBytes ? Row::CF::kSmemBytes : Col::CF::kSmemBytes;
   static std::atomic<unsigned long long> smem_set[2];
   const long long rows = (long long)g.BH * ((g.N_q + BM - 1) / BM), cols = (long long)g.BH * ((g.N_kv + BM - 1) / BM);
-  return row_first ? launch_pair<Row, Col>(maps, g, t, s, rows, fb_head_group<FB_BWD_ROW, D>(g), cols, fb_head_group<FB_BWD_COL, D>(g), kWanted, smem_set[0])
+  return row_side_first(g) ? launch_pair<Row, Col>(maps, g, t, s, rows, fb_head_group<FB_BWD_ROW, D>(g), cols, fb_head_group<FB_BWD_COL, D>(g), kWanted, smem_set[0])
                    : launch_pair<Col, Row>(maps, g, t, s, cols, fb_head_group<FB_BWD_COL, D>(g), rows, fb_head_group<FB_BWD_ROW, D>(g), kWanted, smem_set[1]);
 }
 
 template <int D, typename T>
-static cudaError_t launch_bwd_tiles(const TmaMaps& maps, const Geometry& g, const Tensors& t, cudaStream_t s, bool row_first, int* launches) {
+static cudaError_t launch_bwd_tiles(const TmaMaps& maps, const Geometry& g, const Tensors& t, cudaStream_t s, int* launches) {
   const FbPlan row = plan_fb<FB_BWD_ROW, D, T>(g), col = plan_fb<FB_BWD_COL, D, T>(g);
   // One grid against two launches, 220 sizes (512 to 8192 rows; causal, in chunks against a window, without a mask; 8 to
   // 96 heads): up to 33 tiles 0.983, 0.982, 0.983 and 0.985 of the time at D = 64, 80, 96 and 128, the more the shorter
@@ -793,23 +792,20 @@ static cudaError_t launch_bwd_tiles(const TmaMaps& maps, const Geometry& g, cons
   if (row.dual == col.dual && row.split == 1 && col.split == 1 && longest_stream(g) <= 33) {
     *launches += 1;
     if constexpr (D == 64) {
-      if (row.dual) return launch_fb_pair<D, T, true>(maps, g, t, s, row_first);
+      if (row.dual) return launch_fb_pair<D, T, true>(maps, g, t, s);
     }
-    return launch_fb_pair<D, T, false>(maps, g, t, s, row_first);
+    return launch_fb_pair<D, T, false>(maps, g, t, s);
   }
   *launches += 2;
-  Geometry second = g;
-  second.beside = 1;
-  const cudaError_t e = row_first ? launch_fb<FB_BWD_ROW, D, T>(maps, g, t, s, row) : launch_fb<FB_BWD_COL, D, T>(maps, g, t, s, col);
-  if (e != cudaSuccess) return e;
-  return row_first ? launch_fb<FB_BWD_COL, D, T>(maps, second, t, s, col) : launch_fb<FB_BWD_ROW, D, T>(maps, second, t, s, row);
+  return side_by_side(g, [&](const Geometry& q) { return launch_fb<FB_BWD_ROW, D, T>(maps, q, t, s, row); },
+                      [&](const Geometry& q) { return launch_fb<FB_BWD_COL, D, T>(maps, q, t, s, col); });
 }
 
-// dQ, dK and dV, given Dv; the kind with the longer CTAs first
-cudaError_t launch_bwd(int D, int is_bf16, const TmaMaps& maps, const Geometry& g, const Tensors& t, cudaStream_t s, bool row_first, int* launches) {
+// dQ, dK and dV, given Dv
+cudaError_t launch_bwd(int D, int is_bf16, const TmaMaps& maps, const Geometry& g, const Tensors& t, cudaStream_t s, int* launches) {
   if (D <= 64)
-    return is_bf16 ? launch_bwd_tiles<64, __nv_bfloat16>(maps, g, t, s, row_first, launches) : launch_bwd_tiles<64, __half>(maps, g, t, s, row_first, launches);
-  return is_bf16 ? launch_bwd_tiles<128, __nv_bfloat16>(maps, g, t, s, row_first, launches) : launch_bwd_tiles<128, __half>(maps, g, t, s, row_first, launches);
+    return is_bf16 ? launch_bwd_tiles<64, __nv_bfloat16>(maps, g, t, s, launches) : launch_bwd_tiles<64, __half>(maps, g, t, s, launches);
+  return is_bf16 ? launch_bwd_tiles<128, __nv_bfloat16>(maps, g, t, s, launches) : launch_bwd_tiles<128, __half>(maps, g, t, s, launches);
 }
 
 }  // namespace tc

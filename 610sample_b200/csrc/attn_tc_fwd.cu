@@ -259,8 +259,7 @@ fwd_kernel(const __grid_constant__ TmaMaps maps, const Geometry g, const Tensors
       if (warp == kFwdSWarp) {
         ok = mbar_wait(CF::kQTmem ? bar_q_ready : bar_staging_full, 0, abort_flag, t.status, wait_code(KFWD, 2));
         ok = __all_sync(0xffffffffu, ok);
-        const uint32_t qt = tmem_base + CF::kQT;
-        (void)qt;
+        [[maybe_unused]] const uint32_t qt = tmem_base + CF::kQT;
         const uint64_t qd = smem_desc_sw128(staging, 16, 1024);
         auto koff = [](int ks) { return (uint64_t)((CF::stream_off(0, ks >> 2) + (ks & 3) * 32) >> 4); };
         for (int j = 0; j < n_iter && ok; ++j) {

@@ -34,13 +34,17 @@ struct TmaMaps { CUtensorMap m[T_COUNT]; CUtensorMap out[TO_COUNT]; };
 
 template <int V> struct Int { static constexpr int value = V; };
 
-// The issuing warps' loops with the k-steps of a head dimension: role(Int<steps>), a constant for the usual
-// ones, 0 (the tile width's steps, each compared with g.D / 16) for the others.  A comparison costs the issuing
-// thread about as much as the step it skips: a score batch of the forward took 335 clocks to issue at D = 96 as
-// at D = 128.  B4 H8, 1189 queries, 3531 keys, D80: forward 70.0 -> 68.5 us, backward 161 -> 158; B2 H8 N2648 D96 forward
-// 36.5 -> 35.2; H12, 1024 queries, 9216 keys, D64 forward 27.0 -> 26.1, backward 65.8 -> 65.0.  The double
-// backward keeps the comparisons: with two long batches in flight the gaps let the other issuing
-// warp's products in (85 us with, 90 without at B2 H16 N844 D128; D = 64 even).
+// The issuing warps' loops with the k-steps of a head dimension: role(Int<steps>), a constant for the tile widths and the
+// head dimensions of models between them, 0 (the tile width's steps, each compared with g.D / 16) for 16, 32, 48
+// and 112, which would be four more copies of the loops.  A comparison costs the issuing thread about as much as the
+// step it skips: a score batch of the forward took 335 clocks to issue at D = 96 as at D = 128.  First backward, two
+// launches, 220 sizes of 512 to 8192 rows: 0.987, 0.979, 0.986 and 0.993 of the time at D = 64, 80, 96 and 128, where no
+// step is skipped but the gaps between the steps go (0.95 to 1.026 each).  Forward, 547 sizes of 32 to 5000 rows, with V
+// awaited ahead of P: 0.987, 0.994, 0.987 and 0.988 on average; at D = 80 below 8 us 1.006 (0.05 us: the loops of the third
+// head dimension in line lie apart from the code before), and single sizes that change between the two modes of the tile's
+// period take up to 1.065 of the time, others 0.93 (the same source compiled with the loops in another order
+// moves them as far).  The double backward keeps the comparisons: with two long batches in flight the gaps let the other
+// issuing warp's products in (85 us with, 90 without at B2 H16 N844 D128; D = 64 even).
 template <int D, typename Role>
 __device__ __forceinline__ void with_k_steps(int head_dim, Role&& role) {
   if (head_dim == D) role(Int<D / 16>{});
@@ -130,6 +134,30 @@ inline cudaError_t launch_pdl_cluster(void (*kern)(P...), unsigned ctas, unsigne
 template <typename... P, typename... A>
 inline cudaError_t launch_pdl(void (*kern)(P...), unsigned ctas, unsigned threads, size_t smem, cudaStream_t s, const A&... args) {
   return launch_pdl_cluster(kern, ctas, threads, smem, 1, s, args...);
+}
+
+// Two kernels of one operation that do not depend on each other, dQ and dK/dV or g_Q and g_K/g_V: the CTAs of one first,
+// the other's on the SMs its last CTAs leave idle.  The kernel with the longer CTAs goes first, so that the
+// tail is made of short ones: the row kernel where a query sees more keys than a key is seen by queries (chunks of
+// 1024 queries against a window of 8192: 128 tiles per row CTA, 16 per column CTA; backward 410 ->
+// 392 us at H32 D80), else the column kernel, whose tile costs more.
+inline bool row_side_first(const Geometry& g) {
+  if (g.mask_mode != 0) return g.N_kv > g.N_q;
+  return (g.window < g.N_kv ? g.window : g.N_kv) > (g.window < g.N_q ? g.window : g.N_q);
+}
+
+// As two launches, the second beside the first (always the double backward, the first backward where it is not one
+// grid): the second one relies on the first having been launched, so it is not launched where that failed.
+template <typename Row, typename Col>
+inline cudaError_t side_by_side(const Geometry& g, Row row, Col col) {
+  Geometry second = g;
+  second.beside = 1;
+  if (row_side_first(g)) {
+    const cudaError_t e = row(g);
+    return e == cudaSuccess ? col(second) : e;
+  }
+  const cudaError_t e = col(g);
+  return e == cudaSuccess ? row(second) : e;
 }
 
 // ---- Splitting the streamed tiles of a stationary tile over a cluster --------------------------
