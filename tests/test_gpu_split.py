@@ -8,6 +8,7 @@ import pytest
 import torch
 
 import attention_oracle as orc
+from _util import captured_kernels
 
 pytestmark = pytest.mark.gpu
 tcapi = importlib.import_module("610sample_b200.torch_capi")
@@ -214,3 +215,22 @@ def test_split_rows_without_a_sum_are_those_of_the_unsplit_kernel():
         S = (Q[0, 0].double() @ K[0, 0].double().T / D ** 0.5)[~lost]
         want = torch.softmax(S, -1) @ V[0, 0].double()
         assert float((O[0, 0, ~lost].double() - want).abs().max()) <= 2 ** -7 * float(V.double().abs().max())
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("H,D", [(10, 64), (60, 64), (10, 80), (10, 112), (10, 128)])      # one CTA per SM, two (60 heads)
+def test_first_backward_in_one_grid_and_in_two_gives_the_same_bits(H, D, dtype):
+    """1000 queries at the start of the sequence against 3048 keys, 2048 of them in front of it: no window from 1000 on
+    hides a key, but a wide one makes the bound of the streamed tiles 48 instead of 19, so dQ and dK/dV
+    get a launch each."""
+    inp = orc.make_inputs(1, H, 1000, 3048, D, seed=H + D, dtype=dtype)
+    g = {n: t.cuda() for n, t in inp.items()}
+    results = []
+    for window, launches in ((1000, ["pair"]), (8192, ["tile", "tile"])):
+        O, L = tcapi.forward(g["Q"], g["K"], g["V"], window, 0, 0)
+        call = lambda: tcapi.backward(g["dO"], g["Q"], g["K"], g["V"], O, L, window, 0, 0)
+        assert [n.split("_kernel")[0][-4:] for n, c in captured_kernels(call) if "fb_kernel" in n] == launches
+        results.append((O, L) + tuple(call()))
+    assert float(results[0][3][:, :, 2048:].float().norm()) > 0
+    for one, two, name in zip(*results, ("O", "L", "dQ", "dK", "dV")):
+        assert torch.equal(one, two), name
