@@ -573,12 +573,16 @@ static tc::TileKernelState& state_of() {
 // the shared memory of the variant's largest D, so that one setting serves every call
 template <int KIND, int DC> constexpr size_t kVariantSmem = sizeof(float) * smem_floats<KIND>(64 * DC);
 
-// CTAs that run at a time in clusters of c
+// CTAs of a kind that run at a time in clusters of c on the current device, asked for once
 template <int KIND, int DC, typename T>
-static int slots_of(int c) {
-  if (c == 1) return DC == 1 ? 2 * kSms : kSms;
-  return tc::cluster_slots(attn_simt_kernel<KIND, DC, T>, c, threads_of(KIND, DC), kVariantSmem<KIND, DC>, state_of<KIND, DC, T>());
-}
+struct Slots {
+  int dev = -1;
+  Slots() { if (cudaGetDevice(&dev) != cudaSuccess) dev = -1; }
+  int operator()(int c) const {
+    if (c == 1) return DC == 1 ? 2 * kSms : kSms;
+    return dev < 0 ? 0 : tc::cluster_slots_on(dev, attn_simt_kernel<KIND, DC, T>, c, threads_of(KIND, DC), kVariantSmem<KIND, DC>, state_of<KIND, DC, T>());
+  }
+};
 
 template <int KIND, int DC, typename T>
 static cudaError_t launch_split(const Geometry& g, const Tensors& t, cudaStream_t stream, int split) {
@@ -594,7 +598,7 @@ static cudaError_t launch_split(const Geometry& g, const Tensors& t, cudaStream_
 
 template <int KIND, int DC, typename T>
 static cudaError_t launch_dc(const Geometry& g, const Tensors& t, cudaStream_t stream) {
-  const Splits s = pick_splits(work_of(g, (Kind)KIND, DC == 1), nullptr, DC == 1, false, slots_of<KIND, DC, T>);
+  const Splits s = pick_splits(work_of(g, (Kind)KIND, DC == 1), nullptr, DC == 1, false, Slots<KIND, DC, T>());
   return launch_split<KIND, DC, T>(g, t, stream, s.a);
 }
 
@@ -620,7 +624,7 @@ static cudaError_t launch_pair_dc(const Geometry& g, const Tensors& t, cudaStrea
 template <int FIRST, int SECOND, int DC, typename T>
 static cudaError_t launch_two_dc(const Geometry& g, const Tensors& t, cudaStream_t stream, int* n, int which) {
   const Work first = work_of(g, (Kind)FIRST, DC == 1), second = work_of(g, (Kind)SECOND, DC == 1);
-  const Splits s = pick_splits(first, &second, DC == 1, FIRST == K_HVP_COL, slots_of<FIRST, DC, T>);
+  const Splits s = pick_splits(first, &second, DC == 1, FIRST == K_HVP_COL, Slots<FIRST, DC, T>());
   if (which == 3 && s.together) {
     ++*n;
     return launch_pair_dc<FIRST, SECOND, DC, T>(g, t, stream, s.a);

@@ -113,7 +113,7 @@ struct Part {
 // N320 D80 forward 19.7 -> 14.1 (8 -> 4).  Over 396 sizes the rule's choice takes 0.3 to 1.5 % more time than the best
 // one of each (the other rule 3 to 11 %), at worst a fifth, at tiles most of which have no work.
 template <typename Slots>
-inline Splits pick_splits(const Work& a, const Work* b, bool narrow, bool second_order, Slots slots) {
+inline Splits pick_splits(const Work& a, const Work* b, bool narrow, bool second_order, const Slots& slots) {
   // no split where there are more CTAs than two per SM, or shares without a tile would be the rule
   auto most = [](const Work& w) {
     int e = 0;

@@ -269,11 +269,9 @@ struct TileKernelState {
   std::atomic<int> slots[64][kMaxSplit + 1] = {};
 };
 
-// CTAs of `kern` that run at a time in clusters of c on the current device; 0 where that cannot be told.
+// CTAs of `kern` that run at a time in clusters of c on the current device `dev`; 0 where that cannot be told.
 template <typename Kern>
-inline int cluster_slots(Kern kern, int c, unsigned threads, size_t smem, TileKernelState& state) {
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess) return 0;
+inline int cluster_slots_on(int dev, Kern kern, int c, unsigned threads, size_t smem, TileKernelState& state) {
   std::atomic<int>& known = state.slots[dev & 63][c];
   int n = known.load(std::memory_order_relaxed);
   if (n == 0) {
@@ -297,6 +295,11 @@ inline int cluster_slots(Kern kern, int c, unsigned threads, size_t smem, TileKe
     known.store(n, std::memory_order_relaxed);
   }
   return n;
+}
+template <typename Kern>
+inline int cluster_slots(Kern kern, int c, unsigned threads, size_t smem, TileKernelState& state) {
+  int dev = 0;
+  return cudaGetDevice(&dev) == cudaSuccess ? cluster_slots_on(dev, kern, c, threads, smem, state) : 0;
 }
 
 // Shared memory of a CTA that has its SM to itself: more than half of it, so that the 512-column tensor-memory
