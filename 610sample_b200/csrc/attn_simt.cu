@@ -23,7 +23,10 @@
 // backward 690 -> 573, double backward 1 685 -> 1 509 us), at D = 64 1 to 5 %.  A thread holds 2 x 4 scores of every
 // score matrix of its kind; in the double backward at D <= 64, where four matrices share the operands it has
 // read, 4 x 4 (N1024 800 against 837 us, and the smaller backward the other way round: B2 H5 N479 62
-// against 65).  At D > 64 one CTA fills the shared memory of an SM, and twice the warps hide the latencies.
+// against 65).  At D > 64 a CTA has an SM to itself, by its registers (199 to 255 per thread, 256 threads) in the forward
+// and the first backward (89 to 113 KB of shared memory at D = 128), by its shared memory too in the double
+// backward (185 to 193 KB); twice the warps hide the latencies.  At D <= 64 two fit by both (124 to 128 registers
+// of 256 threads, 240 to 255 of 128; at most 105 KB).
 // The packed f32x2 multiply-adds run along the head dimension without a move; as scalar ones they
 // have a higher rate with one or two warps per scheduler, but the issue slots they take cost 4 to 70 %.
 // Rows are stored without padding where D is a multiple of 32, their 16-byte chunks XOR-swizzled by the
@@ -552,7 +555,7 @@ __global__ void __launch_bounds__(threads_of(KIND, DC), DC == 1 ? 2 : 1) attn_si
 }
 
 // Two kinds of one operation that do not depend on each other in one grid, the CTAs of FIRST in front: one
-// launch less (a second-order step at B2 H4 N256 D64, which the host bounds, 6 % faster).
+// launch less, 1.9 us of the host.
 template <int FIRST, int SECOND, int DC, typename T>
 __global__ void __launch_bounds__(threads_of(FIRST, DC), DC == 1 ? 2 : 1)
 attn_simt_pair_kernel(const Geometry g, const Tensors t, const int split, const int first_ctas) {
