@@ -91,7 +91,7 @@ void long_sequences() {
     check(rule(FWD, g).a == 1 && rule(BWD, g).a == 1, "a long sequence is not split");
   }
   check(rule(FWD, geometry(1, 64, n >> 1, 64, n >> 1, 0, 1)).a == 8, "two tiles of queries against many keys");
-  check(std::chrono::steady_clock::now() - start < std::chrono::milliseconds(1), "host time of a long sequence");
+  check(std::chrono::steady_clock::now() - start < std::chrono::milliseconds(5), "host time of a long sequence");
 }
 }  // namespace
 
