@@ -500,13 +500,18 @@ __device__ __forceinline__ void fb_kernel<KIND, D, T, SPLIT, DUAL>::run(const Tm
               if constexpr (CF::kCol) l2 = *reinterpret_cast<const float2*>(cs + cc);
               const float2 x = __ffma2_rn(make_float2(__uint_as_float(s_[ch][e]), __uint_as_float(s_[ch][e + 1])), sl2, l2);
               float2 pp = make_float2(ex2(x.x), ex2(x.y));
-              if (masked) {
+              if (!DUAL && masked) {
                 pp.x = ((uint32_t)(j0 + cc - vlo) < vspan) ? pp.x : 0.f;
                 pp.y = ((uint32_t)(j0 + cc + 1 - vlo) < vspan) ? pp.y : 0.f;
               }
               pw[hh * 16 + ch * 8 + (e >> 1)] = pp;
             }
         }
+        // With two CTAs per SM the schedulers are what is short (54 % of their slots used): B4 H16 N2048 D64 without mask 302 -> 278 us,
+        // B8 H12 N2048 D64 causal 261 -> 248, B4 H16 N512 D64 27.0 -> 26.3.  With one, where most tiles may have a mask's edge
+        // and a half-step's latency counts, the test stays in the loop (64 queries against 256 keys 5.9 us, 6.1 with a pass of
+        // its own; B2 H12, 777 of 1301, D80 40.6, 41.3).
+        if (DUAL && __any_sync(0xffffffffu, masked)) mask_pairs(pw, j0 - vlo, vspan);
         ok = mbar_wait(bar_rb_full(b), (it / kBufs) & 1, abort_flag, t.status, wait_code(KCODE, 8));
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;

@@ -489,6 +489,18 @@ __device__ __forceinline__ float ex2(float x) {
   return y;
 }
 
+// Scores of one row that are not visible, as zeros: element i is number `first` + i of the row's visible range [0, span).  A pass
+// of its own for the tiles that have such elements: within the loop of the exponentials its three instructions for an
+// element are executed in every tile.
+template <int N>
+__device__ __forceinline__ void mask_pairs(float2 (&p)[N], int first, uint32_t span) {
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    p[i].x = (uint32_t)(first + 2 * i) < span ? p[i].x : 0.f;
+    p[i].y = (uint32_t)(first + 2 * i + 1) < span ? p[i].y : 0.f;
+  }
+}
+
 // 16 packed halves (two 16-byte chunks) of operand-tile row `row`, columns
 // [col0, col0+16), into a 128-byte-swizzled [128][64] tile.
 __device__ __forceinline__ void store_op16(uint32_t tile, int row, int col0, const uint32_t (&v)[8]) {
