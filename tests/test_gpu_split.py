@@ -3,6 +3,7 @@ Few: the streamed tiles of one are shared by a cluster of CTAs (the cluster size
 read from captured launches; shares without a tile or without a visible key; both tile widths and types).
 Many: two CTAs per SM, and persistent CTAs."""
 import importlib
+import re
 
 import pytest
 import torch
@@ -234,3 +235,20 @@ def test_first_backward_in_one_grid_and_in_two_gives_the_same_bits(H, D, dtype):
     assert float(results[0][3][:, :, 2048:].float().norm()) > 0
     for one, two, name in zip(*results, ("O", "L", "dQ", "dK", "dV")):
         assert torch.equal(one, two), name
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("shape,two", [
+    ((24, 1000, 1000, 64, 1000, 0, 0), True),       # causal, ragged: 192 tiles of either side
+    ((32, 700, 1500, 48, 333, 2, 0), True),         # both edges of a window inside the tiles
+    ((48, 500, 450, 64, 500, 0, 1), True),          # no mask: equal CTAs of short streams, the ends of both axes
+    ((80, 250, 250, 64, 20, 0, 0), True),           # a narrow window: most scores of every tile masked
+    ((10, 2000, 2000, 64, 2000, 0, 0), False),      # few tiles, long streams: the longest CTA would be the bound
+])
+def test_first_backward_with_two_ctas_per_sm(shape, two, dtype):
+    H, N_q, N_kv, D, window, chunk, mask = shape
+    g = _check_against_the_oracle(1, *shape, dtype)
+    O, L = tcapi.forward(g["Q"], g["K"], g["V"], window, chunk, mask)
+    kernels = [n for n, _ in captured_kernels(lambda: tcapi.backward(g["dO"], g["Q"], g["K"], g["V"], O, L, window, chunk, mask)) if "fb_kernel" in n]
+    forms = [f for n in kernels for f in re.findall(r"fb_kernelILi\d+ELi64E.*?Lb[01]ELb([01])E", n)]
+    assert len(forms) >= 1 and set(forms) == {"1" if two else "0"}, kernels
