@@ -434,16 +434,21 @@ __device__ __forceinline__ bool work_next(WorkControl* w, int n, int* unit, vola
 // tiles of 64 keys; of that about 4 thousand remain.  But a CTA then takes twice as long for a tile, so
 // the longest one must not become the bound: few CTAs stay one to an SM.  Equal CTAs, one to an SM and
 // with no other kernel to fill up with (`alone`), run in whole waves.
-// B8 H12 N2048 D64 causal: forward 117 -> 92 us, backward 324 -> 267; B4 H16 N1024 D128 forward 36 ->
+// B8 H12 N2048 D64 causal: forward 117 -> 92 us; B4 H16 N1024 D128 forward 36 ->
 // 25; B4 H16 N4096 D128 280 -> 253; B2 H8 N2048 D128 without mask (256 CTAs) 40 -> 36.
+// Short unequal CTAs with nothing beside them: what the longest costs besides its tiles is no 12 thousand clocks there but 8,
+// its neighbour being done before it.  Forward, streams of up to 8 tiles, 148 to 296 tiles of queries: H96 N256 D64 9.9 -> 7.9 us, H96
+// N249 D80 11.7 -> 8.9, H80 N176 D128 11.7 -> 8.2, H64 N384 D64 10.3 -> 9.5.  With 8 thousand for longer ones too some gain
+// (H24 N2048 D128 35.3 -> 31.0) and some lose (H24 N1860 D80 30.1 -> 32.8, H40 N783 D80 16.4 -> 18.0).
 inline bool two_per_sm_pays(const Geometry& g, bool col, bool alone, float tile_clocks, float tile_clocks_two) {
   if ((long long)g.BH * (((col ? g.N_kv : g.N_q) + BM - 1) / BM) < kSms) return false;
   const SplitLoad w = stream_load(g, col, tile_clocks);
   auto larger = [](float x, float y) { return x > y ? x : y; };
   const float per_sm = w.units / kSms;
-  const float waves = alone && w.mean > 0.9f * w.longest ? (float)(int)(per_sm + 0.999f) : per_sm;
+  const bool equal = w.mean > 0.9f * w.longest;
+  const float waves = alone && equal ? (float)(int)(per_sm + 0.999f) : per_sm;
   const float one = larger(w.longest * tile_clocks + kCtaClocks, waves * (w.mean * tile_clocks + kCtaClocks));
-  const float two = larger(2.f * w.longest * tile_clocks_two + kCtaClocks, per_sm * (w.mean * tile_clocks_two + 4000.f));
+  const float two = larger(2.f * w.longest * tile_clocks_two + (alone && !equal && w.longest <= 8.f ? 8000.f : kCtaClocks), per_sm * (w.mean * tile_clocks_two + 4000.f));
   return two < 0.95f * one;
 }
 

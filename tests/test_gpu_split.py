@@ -252,3 +252,15 @@ def test_first_backward_with_two_ctas_per_sm(shape, two, dtype):
     kernels = [n for n, _ in captured_kernels(lambda: tcapi.backward(g["dO"], g["Q"], g["K"], g["V"], O, L, window, chunk, mask)) if "fb_kernel" in n]
     forms = [f for n in kernels for f in re.findall(r"fb_kernelILi\d+ELi64E.*?Lb[01]ELb([01])E", n)]
     assert len(forms) >= 1 and set(forms) == {"1" if two else "0"}, kernels
+
+
+@pytest.mark.parametrize("shape,two", [
+    ((96, 250, 250, 96, 250, 0, 0), True),          # short streams of unequal length
+    ((24, 1500, 1500, 64, 1500, 0, 0), False),
+])
+def test_forward_with_two_ctas_per_sm(shape, two):
+    H, N_q, N_kv, D, window, chunk, mask = shape
+    g = _check_against_the_oracle(1, *shape, torch.bfloat16)
+    kernels = [n for n, _ in captured_kernels(lambda: tcapi.forward(g["Q"], g["K"], g["V"], window, chunk, mask)) if "fwd_kernel" in n]
+    forms = [f for n in kernels for f in re.findall(r"fwd_kernelILi\d+E.*?Lb[01]ELi([12])E", n)]      # groups of math warps of a CTA
+    assert forms == ["1" if two else "2"], kernels
