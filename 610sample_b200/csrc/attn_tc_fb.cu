@@ -507,7 +507,7 @@ __device__ __forceinline__ void fb_kernel<KIND, D, T, SPLIT, DUAL>::run(const Tm
               pw[hh * 16 + ch * 8 + (e >> 1)] = pp;
             }
         }
-        // With two CTAs per SM the schedulers are what is short (54 % of their slots used): B4 H16 N2048 D64 without mask 302 -> 278 us,
+        // With two CTAs per SM the schedulers were what is short (54 % of their slots used, now 42): B4 H16 N2048 D64 without mask 302 -> 278 us,
         // B8 H12 N2048 D64 causal 261 -> 248, B4 H16 N512 D64 27.0 -> 26.3.  With one, where most tiles may have a mask's edge
         // and a half-step's latency counts, the test stays in the loop (64 queries against 256 keys 5.9 us, 6.1 with a pass of
         // its own; B2 H12, 777 of 1301, D80 40.6, 41.3).
