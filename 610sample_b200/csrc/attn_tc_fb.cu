@@ -741,26 +741,6 @@ static TileKernelState& fb_state() {
   return state;
 }
 
-// Two CTAs per SM for both kinds, which share the GPU.  A tile takes `one` clocks of an SM that one CTA has to itself, `two` where
-// two CTAs share it, a CTA 8 thousand besides, of which 4 remain with two.  Unequal CTAs fill the GPU up, so their sum is the
-// bound, or the longest CTA, which takes twice the clocks per tile with two on its SM.  Equal ones (no mask) run in waves,
-// of 148 or of 296: with less than about 1.5 of the latter two per SM pays for short streams only, whose CTAs cost most
-// besides their tiles.  Measured, 69 sizes of 160 to 768 tiles of either side, of the time with a rule for each kind by itself: 0.78 to 1.00,
-// 0.957 on average (H32 N1024 causal 36.8 -> 28.7 us, H20 N2048 67.0 -> 53.8, H24 N1536 50.0 -> 40.1, H16 N2048 without mask 85.2 -> 79.5);
-// two where this keeps one: H10 N2048 35.9 and 44.7, without mask 67.1 and 72.2; H12 N2048 69.4 and 76.3.
-static bool both_two_per_sm_pay(const Geometry& g) {
-  const long long rows = (long long)g.BH * ((g.N_q + BM - 1) / BM), cols = (long long)g.BH * ((g.N_kv + BM - 1) / BM);
-  if (rows < kSms || cols < kSms) return false;
-  const SplitLoad r = stream_load(g, false, 1.f), c = stream_load(g, true, 1.f);
-  if (r.mean > 0.9f * r.longest && c.mean > 0.9f * c.longest)
-    return r.units + c.units >= 3.1f * kSms || (r.units + c.units >= 2.5f * kSms && r.mean + c.mean <= 24.f);
-  auto larger = [](float x, float y) { return x > y ? x : y; };
-  auto sum = [&](float row, float col, float besides) { return (r.units * (r.mean * row + besides) + c.units * (c.mean * col + besides)) / kSms; };
-  const float one = larger(larger(r.longest * 1000.f, c.longest * 1700.f) + 8000.f, sum(1000.f, 1700.f, 8000.f));
-  const float two = larger(2.f * larger(r.longest * 930.f, c.longest * 1300.f) + 8000.f, sum(930.f, 1400.f, 4000.f));
-  return two < one;
-}
-
 template <int KIND, int D, typename T>
 static FbPlan plan_fb(const Geometry& g) {
   constexpr bool kCol = KIND == FB_BWD_COL;

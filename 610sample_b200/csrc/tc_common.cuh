@@ -222,8 +222,9 @@ constexpr float kCtaClocks = 12000.f;
 constexpr int kMaxSplit = 8;
 inline float split_clocks(int D) { return 3000.f + 45.f * D; }
 
-// a kernel's stationary tiles, the most and the mean streamed tiles one of them visits, clocks per tile
-struct SplitLoad { float units, longest, mean, tile_clocks; };
+// a kernel's stationary tiles, the most and the mean streamed tiles one of them visits, clocks per tile; how many of
+// the stationary tiles visit any (keys in front of the sequence or of its windows do not), and the mean of those
+struct SplitLoad { float units, longest, mean, tile_clocks, busy, busy_mean; };
 
 template <typename Slots>
 inline int pick_split(const SplitLoad& w, const SplitLoad* other, int D, Slots slots) {
@@ -248,7 +249,7 @@ constexpr int kLoadSamples = 1024;
 inline SplitLoad stream_load(const Geometry& g, bool col, float tile_clocks) {
   const int n = col ? g.N_kv : g.N_q, tiles = (n + BM - 1) / BM;
   const int samples = tiles < kLoadSamples ? tiles : kLoadSamples;
-  int most = 0;
+  int most = 0, busy = 0;
   long long sum = 0;
   for (int s = 0; s < samples; ++s) {
     const int i = samples == tiles ? s : (int)((long long)s * (tiles - 1) / (samples - 1));
@@ -258,8 +259,10 @@ inline SplitLoad stream_load(const Geometry& g, bool col, float tile_clocks) {
     const int k = hi > lo ? (hi + BN - 1) / BN - lo / BN : 0;
     if (k > most) most = k;
     sum += k;
+    busy += k > 0;
   }
-  return {(float)g.BH * tiles, (float)most, samples > 0 ? (float)sum / samples : 0.f, tile_clocks};
+  return {(float)g.BH * tiles, (float)most, samples > 0 ? (float)sum / samples : 0.f, tile_clocks,
+          samples > 0 ? (float)g.BH * tiles * busy / samples : 0.f, busy > 0 ? (float)sum / busy : 0.f};
 }
 
 // What a kernel's launches keep: the devices its shared-memory opt-in has been made on, and by device
@@ -316,7 +319,7 @@ inline int choose_split(void (*shared)(P...), const Geometry& g, bool col, unsig
   if (2 * units > kSms || !((col ? g.N_q : g.N_kv) * (0.5f / BN) * tile_clocks > split_clocks(g.D))) return 1;
   const SplitLoad w = stream_load(g, col, tile_clocks);
   const bool paired = other_clocks > 0.f;
-  SplitLoad other = {0.f, 0.f, 0.f, 0.f};
+  SplitLoad other = {};
   if (paired) other = stream_load(g, !col, other_clocks);
   // of a pair, the kernel with the longer CTAs only: two kernels of clusters do not share the GPU well
   if (!(w.longest * w.tile_clocks > other.longest * other.tile_clocks)) return 1;
@@ -440,18 +443,44 @@ __device__ __forceinline__ bool work_next(WorkControl* w, int n, int* unit, vola
 // its neighbour being done before it.  Forward, streams of up to 8 tiles, 148 to 296 tiles of queries: H96 N256 D64 9.9 -> 7.9 us, H96
 // N249 D80 11.7 -> 8.9, H80 N176 D128 11.7 -> 8.2, H64 N384 D64 10.3 -> 9.5.  With 8 thousand for longer ones too some gain
 // (H24 N2048 D128 35.3 -> 31.0) and some lose (H24 N1860 D80 30.1 -> 32.8, H40 N783 D80 16.4 -> 18.0).
+// Only tiles that visit any count, on either side of the rule: the first chunks of a sliding window have most of their
+// keys in front of the sequence, and a CTA without a tile costs next to nothing.  First backward with 148 tiles of keys
+// and fewer of queries, 320 sizes drawn after the constants were chosen: 100 go to the other form, which takes 0.932 of the
+// time (0.80 to 1.15; H20, 128 queries of 1374 keys, D64, 40 of 220 tiles of keys with a query: 10.5 -> 8.4 us).
 inline bool two_per_sm_pays(const Geometry& g, bool col, bool alone, float tile_clocks, float tile_clocks_two) {
   if ((long long)g.BH * (((col ? g.N_kv : g.N_q) + BM - 1) / BM) < kSms) return false;
   const SplitLoad w = stream_load(g, col, tile_clocks);
   auto larger = [](float x, float y) { return x > y ? x : y; };
-  const float per_sm = w.units / kSms;
-  const bool equal = w.mean > 0.9f * w.longest;
+  if (w.busy < kSms) return false;
+  const float per_sm = w.busy / kSms;
+  const bool equal = w.busy_mean > 0.9f * w.longest;
   const float waves = alone && equal ? (float)(int)(per_sm + 0.999f) : per_sm;
-  const float one = larger(w.longest * tile_clocks + kCtaClocks, waves * (w.mean * tile_clocks + kCtaClocks));
-  const float two = larger(2.f * w.longest * tile_clocks_two + (alone && !equal && w.longest <= 8.f ? 8000.f : kCtaClocks), per_sm * (w.mean * tile_clocks_two + 4000.f));
+  const float one = larger(w.longest * tile_clocks + kCtaClocks, waves * (w.busy_mean * tile_clocks + kCtaClocks));
+  const float besides = !alone ? 10000.f : !equal && w.longest <= 8.f ? 8000.f : kCtaClocks;
+  const float two = larger(2.f * w.longest * tile_clocks_two + besides, per_sm * (w.busy_mean * tile_clocks_two + 4000.f));
   return two < 0.95f * one;
 }
 
+// Two CTAs per SM for both kinds, which share the GPU.  A tile takes `one` clocks of an SM that one CTA has to itself, `two` where
+// two CTAs share it, a CTA 8 thousand besides, of which 4 remain with two.  Unequal CTAs fill the GPU up, so their sum is the
+// bound, or the longest CTA, which takes twice the clocks per tile with two on its SM.  Equal ones (no mask) run in waves,
+// of 148 or of 296: with less than about 1.5 of the latter two per SM pays for short streams only, whose CTAs cost most
+// besides their tiles.  Measured, 69 sizes of 160 to 768 tiles of either side, of the time with a rule for each kind by itself: 0.78 to 1.00,
+// 0.957 on average (H32 N1024 causal 36.8 -> 28.7 us, H20 N2048 67.0 -> 53.8, H24 N1536 50.0 -> 40.1, H16 N2048 without mask 85.2 -> 79.5);
+// two where this keeps one: H10 N2048 35.9 and 44.7, without mask 67.1 and 72.2; H12 N2048 69.4 and 76.3.
+inline bool both_two_per_sm_pay(const Geometry& g) {
+  const long long rows = (long long)g.BH * ((g.N_q + BM - 1) / BM), cols = (long long)g.BH * ((g.N_kv + BM - 1) / BM);
+  if (rows < kSms || cols < kSms) return false;
+  const SplitLoad r = stream_load(g, false, 1.f), c = stream_load(g, true, 1.f);
+  if (r.busy < kSms || c.busy < kSms) return false;
+  if (r.busy_mean > 0.9f * r.longest && c.busy_mean > 0.9f * c.longest)
+    return r.busy + c.busy >= 3.1f * kSms || (r.busy + c.busy >= 2.5f * kSms && r.busy_mean + c.busy_mean <= 24.f);
+  auto larger = [](float x, float y) { return x > y ? x : y; };
+  auto sum = [&](float row, float col, float besides) { return (r.busy * (r.busy_mean * row + besides) + c.busy * (c.busy_mean * col + besides)) / kSms; };
+  const float one = larger(larger(r.longest * 1000.f, c.longest * 1700.f) + 8000.f, sum(1000.f, 1700.f, 8000.f));
+  const float two = larger(2.f * larger(r.longest * 930.f, c.longest * 1300.f) + 8000.f, sum(930.f, 1400.f, 4000.f));
+  return two < one;
+}
 // more than a third of an SM's shared memory: never a third CTA that would wait for tensor memory
 inline size_t half_sm_smem(size_t wanted) { return wanted < 79872u ? 79872u : wanted; }
 

@@ -95,7 +95,25 @@ static void bound_of_a_stream() {
   check(longest_stream(geometry(1, 9000, 9000, 64, 0)) == 4, "a window");
 }
 
+// Keys in front of the sequence have no query: their tiles cost next to nothing, so they change no decision.
+static void keys_in_front() {
+  int paying = 0;
+  for (int BH = 4; BH <= 96; BH += 4)
+    for (int N = 128; N <= 2304; N += 160) {
+      const Geometry plain = geometry(BH, N, N, 8192, 0), front = geometry(BH, N, N + 8192, 8192, 0);
+      const bool both = both_two_per_sm_pay(plain), cols = two_per_sm_pays(plain, true, false, 1700.f, 1200.f);
+      check(both_two_per_sm_pay(front) == both, "keys in front of the sequence, both kinds");
+      check(two_per_sm_pays(front, true, false, 1700.f, 1200.f) == cols, "keys in front of the sequence, the key side");
+      paying += both + cols;
+      const SplitLoad w = stream_load(front, true, 1.f), v = stream_load(plain, true, 1.f);
+      check(w.busy == v.units && v.busy == v.units && w.busy_mean == v.mean && w.units == v.units + 64.f * BH, "tiles without a stream");
+      if (failures > 5) return;
+    }
+  check(paying > 100 && paying < 600, "either answer occurs");
+}
+
 int main() {
+  keys_in_front();
   cluster_queries();
   load_of_a_problem();
   bound_of_a_stream();
