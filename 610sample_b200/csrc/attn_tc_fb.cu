@@ -742,11 +742,9 @@ static TileKernelState& fb_state() {
 }
 
 template <int KIND, int D, typename T>
-static FbPlan plan_fb(const Geometry& g) {
+static FbPlan plan_fb(const Geometry& g, bool two_per_sm) {
   constexpr bool kCol = KIND == FB_BWD_COL;
-  if constexpr (D == 64) {
-    if (two_per_sm_pays(g, kCol, false, kCol ? 1700.f : 1000.f, kCol ? 1200.f : 1000.f)) return {true, 1};
-  }
+  if (two_per_sm) return {true, 1};
   using CF = FbCfg<KIND, D, false>;
   return {false, choose_split(tile_kernel<fb_kernel<KIND, D, T, true, false>>, g, kCol, CF::kThreads, CF::kSmemBytes, kCol ? 1700.f : 1150.f,
                               kCol ? 1150.f : 1700.f, fb_state<KIND, D, T>())};
@@ -790,8 +788,8 @@ static cudaError_t launch_fb_pair(const TmaMaps& maps, const Geometry& g, const 
 
 template <int D, typename T>
 static cudaError_t launch_bwd_tiles(const TmaMaps& maps, const Geometry& g, const Tensors& t, cudaStream_t s, int* launches) {
-  const bool both = D == 64 && both_two_per_sm_pay(g);
-  const FbPlan row = both ? FbPlan{true, 1} : plan_fb<FB_BWD_ROW, D, T>(g), col = both ? FbPlan{true, 1} : plan_fb<FB_BWD_COL, D, T>(g);
+  const TwoPerSm two = D == 64 ? backward_two_per_sm(g) : TwoPerSm{false, false};
+  const FbPlan row = plan_fb<FB_BWD_ROW, D, T>(g, two.row), col = plan_fb<FB_BWD_COL, D, T>(g, two.col);
   // One grid against two launches, 220 sizes (512 to 8192 rows; causal, in chunks against a window, without a mask; 8 to
   // 96 heads): up to 33 tiles 0.983, 0.982, 0.983 and 0.985 of the time at D = 64, 80, 96 and 128, the more the shorter
   // (0.93 to 1.009 each); 34 to 146 tiles 0.997, 0.992, 0.989 and 0.991 (0.95 to 1.013), so the limit is no crossing.

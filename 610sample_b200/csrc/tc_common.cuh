@@ -445,42 +445,57 @@ __device__ __forceinline__ bool work_next(WorkControl* w, int n, int* unit, vola
 // (H24 N2048 D128 35.3 -> 31.0) and some lose (H24 N1860 D80 30.1 -> 32.8, H40 N783 D80 16.4 -> 18.0).
 // Only tiles that visit any count, on either side of the rule: the first chunks of a sliding window have most of their
 // keys in front of the sequence, and a CTA without a tile costs next to nothing.  First backward with 148 tiles of keys
-// and fewer of queries, 320 sizes drawn after the constants were chosen: 100 go to the other form, which takes 0.932 of the
-// time (0.80 to 1.15; H20, 128 queries of 1374 keys, D64, 40 of 220 tiles of keys with a query: 10.5 -> 8.4 us).
-inline bool two_per_sm_pays(const Geometry& g, bool col, bool alone, float tile_clocks, float tile_clocks_two) {
-  if ((long long)g.BH * (((col ? g.N_kv : g.N_q) + BM - 1) / BM) < kSms) return false;
-  const SplitLoad w = stream_load(g, col, tile_clocks);
-  auto larger = [](float x, float y) { return x > y ? x : y; };
+// and fewer of queries, 640 drawn sizes: 191 go to the other form for it, which takes 0.938 of the time (0.81 to 1.17; H20, 128
+// queries of 1374 keys, D64, 40 of 220 tiles of keys with a query: 10.5 -> 8.4 us).
+inline bool two_per_sm_pays(const SplitLoad& w, bool alone, float tile_clocks_two) {
   if (w.busy < kSms) return false;
+  auto larger = [](float x, float y) { return x > y ? x : y; };
   const float per_sm = w.busy / kSms;
   const bool equal = w.busy_mean > 0.9f * w.longest;
   const float waves = alone && equal ? (float)(int)(per_sm + 0.999f) : per_sm;
-  const float one = larger(w.longest * tile_clocks + kCtaClocks, waves * (w.busy_mean * tile_clocks + kCtaClocks));
-  const float besides = !alone ? 10000.f : !equal && w.longest <= 8.f ? 8000.f : kCtaClocks;
+  const float one = larger(w.longest * w.tile_clocks + kCtaClocks, waves * (w.busy_mean * w.tile_clocks + kCtaClocks));
+  const float besides = !alone ? 9000.f : !equal && w.longest <= 8.f ? 8000.f : kCtaClocks;
   const float two = larger(2.f * w.longest * tile_clocks_two + besides, per_sm * (w.busy_mean * tile_clocks_two + 4000.f));
   return two < 0.95f * one;
 }
+inline bool two_per_sm_pays(const Geometry& g, bool col, bool alone, float tile_clocks, float tile_clocks_two) {
+  return (long long)g.BH * (((col ? g.N_kv : g.N_q) + BM - 1) / BM) >= kSms && two_per_sm_pays(stream_load(g, col, tile_clocks), alone, tile_clocks_two);
+}
 
-// Two CTAs per SM for both kinds, which share the GPU.  A tile takes `one` clocks of an SM that one CTA has to itself, `two` where
-// two CTAs share it, a CTA 8 thousand besides, of which 4 remain with two.  Unequal CTAs fill the GPU up, so their sum is the
-// bound, or the longest CTA, which takes twice the clocks per tile with two on its SM.  Equal ones (no mask) run in waves,
-// of 148 or of 296: with less than about 1.5 of the latter two per SM pays for short streams only, whose CTAs cost most
-// besides their tiles.  Measured, 69 sizes of 160 to 768 tiles of either side, of the time with a rule for each kind by itself: 0.78 to 1.00,
-// 0.957 on average (H32 N1024 causal 36.8 -> 28.7 us, H20 N2048 67.0 -> 53.8, H24 N1536 50.0 -> 40.1, H16 N2048 without mask 85.2 -> 79.5);
-// two where this keeps one: H10 N2048 35.9 and 44.7, without mask 67.1 and 72.2; H12 N2048 69.4 and 76.3.
-inline bool both_two_per_sm_pay(const Geometry& g) {
-  const long long rows = (long long)g.BH * ((g.N_q + BM - 1) / BM), cols = (long long)g.BH * ((g.N_kv + BM - 1) / BM);
-  if (rows < kSms || cols < kSms) return false;
-  const SplitLoad r = stream_load(g, false, 1.f), c = stream_load(g, true, 1.f);
-  if (r.busy < kSms || c.busy < kSms) return false;
+// First backward at D <= 64: clocks of a streamed tile of dQ and of dK/dV, with one and with two CTAs per SM
+constexpr float kRowClocks = 1000.f, kRowClocksTwo = 930.f, kColClocks = 1700.f, kColClocksTwo = 1250.f;
+
+// Both kinds, which share the GPU, with a full set of CTAs each: one answer for the two of them.  A CTA costs 8 thousand
+// clocks besides its tiles, of which 4 remain where two share an SM.  Unequal CTAs fill the GPU up, so the bound is the sum
+// of all, or the longest CTA, whose tiles take twice the clocks with two on its SM.  Equal CTAs (no mask) run in rounds: up
+// to three rounds of 148 one per SM is faster (two take 1.02 to 1.08 of the time at 2.8 to 3 rounds), unless streams are so short
+// (24 tiles of both kinds) that what a CTA costs besides them is the larger part.  A fourth round turns it: two per SM 0.955 of
+// the time at H16 N1700, 0.89 at H32 N866, 0.84 at H28, 778 of 1139.  One kind with two per SM and the other with one, in two
+// launches, is up to 13 % faster where the one round of the one leaves room for the other (H20, 1152 of 1408), as much slower
+// elsewhere, and 1 % slower on average over the 121 sizes where each kind asked by itself took it.
+inline bool both_two_per_sm_pay(const SplitLoad& r, const SplitLoad& c) {
   if (r.busy_mean > 0.9f * r.longest && c.busy_mean > 0.9f * c.longest)
-    return r.busy + c.busy >= 3.1f * kSms || (r.busy + c.busy >= 2.5f * kSms && r.busy_mean + c.busy_mean <= 24.f);
+    return r.busy + c.busy > 3 * kSms || (r.busy + c.busy >= 2.5f * kSms && r.busy_mean + c.busy_mean <= 24.f);
   auto larger = [](float x, float y) { return x > y ? x : y; };
   auto sum = [&](float row, float col, float besides) { return (r.busy * (r.busy_mean * row + besides) + c.busy * (c.busy_mean * col + besides)) / kSms; };
-  const float one = larger(larger(r.longest * 1000.f, c.longest * 1700.f) + 8000.f, sum(1000.f, 1700.f, 8000.f));
-  const float two = larger(2.f * larger(r.longest * 930.f, c.longest * 1300.f) + 8000.f, sum(930.f, 1400.f, 4000.f));
+  const float one = larger(larger(r.longest * kRowClocks, c.longest * kColClocks) + 8000.f, sum(kRowClocks, kColClocks, 8000.f));
+  const float two = larger(2.f * larger(r.longest * kRowClocksTwo, c.longest * kColClocksTwo) + 8000.f, sum(kRowClocksTwo, kColClocksTwo, 4000.f));
   return two < one;
 }
+
+// Whether dQ and dK/dV run two CTAs per SM at D <= 64.  With fewer CTAs than SMs on one side the other side decides by itself.
+struct TwoPerSm { bool row, col; };
+inline TwoPerSm backward_two_per_sm(const Geometry& g) {
+  const long long rows = (long long)g.BH * ((g.N_q + BM - 1) / BM), cols = (long long)g.BH * ((g.N_kv + BM - 1) / BM);
+  if (rows < kSms && cols < kSms) return {false, false};
+  const SplitLoad r = stream_load(g, false, kRowClocks), c = stream_load(g, true, kColClocks);
+  if (r.busy >= kSms && c.busy >= kSms) {
+    const bool both = both_two_per_sm_pay(r, c);
+    return {both, both};
+  }
+  return {two_per_sm_pays(r, false, kRowClocksTwo), two_per_sm_pays(c, false, kColClocksTwo)};
+}
+
 // more than a third of an SM's shared memory: never a third CTA that would wait for tensor memory
 inline size_t half_sm_smem(size_t wanted) { return wanted < 79872u ? 79872u : wanted; }
 

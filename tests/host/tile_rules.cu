@@ -101,10 +101,11 @@ static void keys_in_front() {
   for (int BH = 4; BH <= 96; BH += 4)
     for (int N = 128; N <= 2304; N += 160) {
       const Geometry plain = geometry(BH, N, N, 8192, 0), front = geometry(BH, N, N + 8192, 8192, 0);
-      const bool both = both_two_per_sm_pay(plain), cols = two_per_sm_pays(plain, true, false, 1700.f, 1200.f);
-      check(both_two_per_sm_pay(front) == both, "keys in front of the sequence, both kinds");
-      check(two_per_sm_pays(front, true, false, 1700.f, 1200.f) == cols, "keys in front of the sequence, the key side");
-      paying += both + cols;
+      const TwoPerSm alone = backward_two_per_sm(plain), with = backward_two_per_sm(front);
+      check(with.row == alone.row && with.col == alone.col, "keys in front of the sequence, both kinds");
+      const bool cols = two_per_sm_pays(plain, true, false, kColClocks, kColClocksTwo);
+      check(two_per_sm_pays(front, true, false, kColClocks, kColClocksTwo) == cols, "keys in front of the sequence, the key side");
+      paying += (alone.row && alone.col) + cols;
       const SplitLoad w = stream_load(front, true, 1.f), v = stream_load(plain, true, 1.f);
       check(w.busy == v.units && v.busy == v.units && w.busy_mean == v.mean && w.units == v.units + 64.f * BH, "tiles without a stream");
       if (failures > 5) return;
@@ -112,8 +113,34 @@ static void keys_in_front() {
   check(paying > 100 && paying < 600, "either answer occurs");
 }
 
+// Where both kinds have a CTA for every SM there is one answer for the two of them.  Without a mask it turns with the
+// fourth round of CTAs (444 of them), or with streams of 24 tiles in all; with few long streams the longest is the bound.
+static void one_answer_for_both_kinds() {
+  int twos = 0, ones = 0;
+  for (int BH = 4; BH <= 96; BH += 4)
+    for (int N = 200; N <= 4000; N += 119)
+      for (int other = 0; other < 4; ++other) {
+        const Geometry g = geometry(BH, N, other == 0 ? N : N * (3 + other) / 4 + 128 * other, 4096, other != 3);
+        const SplitLoad r = stream_load(g, false, 1.f), c = stream_load(g, true, 1.f);
+        const TwoPerSm two = backward_two_per_sm(g);
+        if (r.busy >= kSms && c.busy >= kSms) {
+          check(two.row == two.col, "one answer for both kinds");
+          ++(two.row ? twos : ones);
+        }
+        check((!two.row || r.busy >= kSms) && (!two.col || c.busy >= kSms), "two CTAs per SM need a CTA for every SM");
+        if (failures > 5) return;
+      }
+  check(twos > 100 && ones > 100, "either answer occurs");
+  auto both = [](int BH, int N_q, int N_kv, int mask_mode) { return backward_two_per_sm(geometry(BH, N_q, N_kv, N_kv, mask_mode)).row; };
+  check(!both(20, 1354, 1354, 1) && !both(24, 1110, 1110, 1), "without a mask, three rounds");
+  check(both(16, 1700, 1700, 1) && both(32, 866, 866, 1) && both(28, 778, 1139, 1), "without a mask, a fourth round");
+  check(both(36, 768, 768, 1) && !both(18, 1500, 1400, 1), "without a mask, short streams");
+  check(both(32, 1024, 1024, 0) && both(20, 2048, 2048, 0) && !both(12, 2048, 2048, 0) && !both(10, 2000, 2000, 0), "causal");
+}
+
 int main() {
   keys_in_front();
+  one_answer_for_both_kinds();
   cluster_queries();
   load_of_a_problem();
   bound_of_a_stream();

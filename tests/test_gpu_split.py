@@ -244,6 +244,8 @@ def test_first_backward_in_one_grid_and_in_two_gives_the_same_bits(H, D, dtype):
     ((48, 500, 450, 64, 500, 0, 1), True),          # no mask: equal CTAs of short streams, the ends of both axes
     ((80, 250, 250, 64, 20, 0, 0), True),           # a narrow window: most scores of every tile masked
     ((10, 2000, 2000, 64, 2000, 0, 0), False),      # few tiles, long streams: the longest CTA would be the bound
+    ((28, 778, 1139, 64, 778, 0, 1), True),         # no mask: more than three rounds of CTAs, both kinds together
+    ((24, 1060, 1060, 64, 1060, 0, 1), False),      # no mask: three rounds
     ((20, 128, 1374, 64, 1246, 0, 0), False),       # 220 tiles of keys, 180 of them in front of the sequence
 ])
 def test_first_backward_with_two_ctas_per_sm(shape, two, dtype):
