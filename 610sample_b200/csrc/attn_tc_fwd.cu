@@ -575,7 +575,7 @@ static cudaError_t launch_fwd_one(const TmaMaps& maps, const Geometry& g_in, con
   Geometry g = g_in;
   const long long ctas = (long long)g.BH * ((g.N_q + BM - 1) / BM);
   g.head_group = pick_head_group(ctas, g.BH, 2ll * g.N_kv * g.D * 2);   // K, V
-  if (two_per_sm_pays(g, false, true, 850.f, 850.f)) {
+  if (forward_two_per_sm(g)) {
     using CF = FwdCfg<D, 1>;
     static std::atomic<unsigned long long> smem_set{0};
     return launch_two_per_sm(fwd_kernel<D, T, false, 1>, maps, g, t, s, ctas, CF::kThreads, CF::kSmemBytes, smem_set);

@@ -431,18 +431,30 @@ __device__ __forceinline__ bool work_next(WorkControl* w, int n, int* unit, vola
   return ok;
 }
 
+// Equal CTAs with no other kernel to fill up with run in rounds: of 148 one to an SM, of 296 two to an SM, where a
+// last round of up to 148 takes 0.8 of a whole one, half of its CTAs having an SM to themselves.  The rounds come apart as there
+// are more of them.  Long streams, whose tiles take longer with two CTAs per SM, so want whole rounds: forward, D64, 24 heads
+// of 2048 queries against a window of 6090 (2.6 rounds) 122 us with one per SM, 164 with two; 16 heads N3000 without mask
+// 67 and 77; but 64 heads N2048 without mask (6.9 rounds) 107 and 99.  1539 drawn sizes of 90 to 16384 rows, masks and
+// no masks, both forms timed: the form taken is 0.3 % from the faster one on average, 1.4 % with 850 clocks per tile in either
+// form and no rounds of 296; the 252 that change form take 0.935 of the time (0.74 to 1.22, 30 of them more than 1.02).
+inline bool two_per_sm_pays_in_rounds(const SplitLoad& w, float tile_clocks_two) {
+  if (w.busy <= kSms) return false;      // one round: 74 heads N256 D64 without mask 5.7 us, 7.0 with a group of math warps for each
+  const long long n = (long long)w.busy, ones = (n - 1) / kSms, pairs = n / (2 * kSms), rest = n % (2 * kSms);
+  // rounds, the last one whole, and by how much the others' coming apart makes up for that
+  const float per_sm = w.busy / kSms, per_pair = per_sm / 2.f, last = rest == 0 ? 0.f : rest <= kSms ? 0.8f : 1.f;
+  const float rounds = per_sm + (ones + 1 - per_sm) / (1.f + 0.1f * ones);
+  const float rounds_two = per_pair + (pairs + last - per_pair) / (1.f + 0.5f * pairs);
+  return rounds_two * (2.f * w.busy_mean * tile_clocks_two + 8000.f) < rounds * (w.busy_mean * w.tile_clocks + 10000.f);
+}
+
 // Two CTAs per SM, each with half of the tensor memory and one group of math warps (the forward, and
 // the first backward at D = 64, where that is enough): while one sets up, fills its pipeline or writes
 // its result, the other computes.  A CTA costs kCtaClocks besides its tiles, a third of its time at 17
-// tiles of 64 keys; of that about 4 thousand remain.  But a CTA then takes twice as long for a tile, so
-// the longest one must not become the bound: few CTAs stay one to an SM.  Equal CTAs, one to an SM and
-// with no other kernel to fill up with (`alone`), run in whole waves.
+// tiles of 64 keys; of that 2 to 4 thousand remain.  But a CTA then takes twice as long for a tile, and a little
+// more, so the longest one must not become the bound: few CTAs stay one to an SM.
 // B8 H12 N2048 D64 causal: forward 117 -> 92 us; B4 H16 N1024 D128 forward 36 ->
 // 25; B4 H16 N4096 D128 280 -> 253; B2 H8 N2048 D128 without mask (256 CTAs) 40 -> 36.
-// Short unequal CTAs with nothing beside them: what the longest costs besides its tiles is no 12 thousand clocks there but 8,
-// its neighbour being done before it.  Forward, streams of up to 8 tiles, 148 to 296 tiles of queries: H96 N256 D64 9.9 -> 7.9 us, H96
-// N249 D80 11.7 -> 8.9, H80 N176 D128 11.7 -> 8.2, H64 N384 D64 10.3 -> 9.5.  With 8 thousand for longer ones too some gain
-// (H24 N2048 D128 35.3 -> 31.0) and some lose (H24 N1860 D80 30.1 -> 32.8, H40 N783 D80 16.4 -> 18.0).
 // Only tiles that visit any count, on either side of the rule: the first chunks of a sliding window have most of their
 // keys in front of the sequence, and a CTA without a tile costs next to nothing.  First backward with 148 tiles of keys
 // and fewer of queries, 640 drawn sizes: 191 go to the other form for it, which takes 0.938 of the time (0.81 to 1.17; H20, 128
@@ -450,16 +462,22 @@ __device__ __forceinline__ bool work_next(WorkControl* w, int n, int* unit, vola
 inline bool two_per_sm_pays(const SplitLoad& w, bool alone, float tile_clocks_two) {
   if (w.busy < kSms) return false;
   auto larger = [](float x, float y) { return x > y ? x : y; };
+  if (alone && w.busy_mean > 0.88f * w.longest) return two_per_sm_pays_in_rounds(w, tile_clocks_two);
   const float per_sm = w.busy / kSms;
-  const bool equal = w.busy_mean > 0.9f * w.longest;
-  const float waves = alone && equal ? (float)(int)(per_sm + 0.999f) : per_sm;
-  const float one = larger(w.longest * w.tile_clocks + kCtaClocks, waves * (w.busy_mean * w.tile_clocks + kCtaClocks));
-  const float besides = !alone ? 9000.f : !equal && w.longest <= 8.f ? 8000.f : kCtaClocks;
-  const float two = larger(2.f * w.longest * tile_clocks_two + besides, per_sm * (w.busy_mean * tile_clocks_two + 4000.f));
+  const float one = larger(w.longest * w.tile_clocks + kCtaClocks, per_sm * (w.busy_mean * w.tile_clocks + kCtaClocks));
+  // the longest CTA of a few short ones (up to 8 tiles) that have the GPU to themselves pays less, its neighbour being done before it
+  const float besides = !alone ? 9000.f : w.longest <= 8.f ? 4000.f : 10000.f;
+  const float two = larger(2.f * w.longest * tile_clocks_two + besides, per_sm * (w.busy_mean * tile_clocks_two + (alone ? 2000.f : 4000.f)));
   return two < 0.95f * one;
 }
 inline bool two_per_sm_pays(const Geometry& g, bool col, bool alone, float tile_clocks, float tile_clocks_two) {
   return (long long)g.BH * (((col ? g.N_kv : g.N_q) + BM - 1) / BM) >= kSms && two_per_sm_pays(stream_load(g, col, tile_clocks), alone, tile_clocks_two);
+}
+
+// Forward: a streamed tile takes 700 clocks with one CTA (of two groups of math warps) per SM, 850 per CTA with two, more above D = 64
+inline bool forward_two_per_sm(const Geometry& g) {
+  const float past = g.D > 64 ? g.D - 64.f : 0.f;
+  return two_per_sm_pays(g, false, true, 700.f + 3.f * past, 850.f + 2.f * past);
 }
 
 // First backward at D <= 64: clocks of a streamed tile of dQ and of dK/dV, with one and with two CTAs per SM

@@ -138,7 +138,26 @@ static void one_answer_for_both_kinds() {
   check(both(32, 1024, 1024, 0) && both(20, 2048, 2048, 0) && !both(12, 2048, 2048, 0) && !both(10, 2000, 2000, 0), "causal");
 }
 
+// Forward: equal tiles run in rounds of 148 or of 296, and long streams take longer with two CTAs per SM.
+static void forward_in_rounds() {
+  auto two = [](int BH, int N_q, int N_kv, int D, int window, int chunk, int mask_mode) {
+    Geometry g = geometry(BH, N_q, N_kv, window, mask_mode);
+    g.D = D; g.qi_base = chunk * N_q; g.ki_base = g.qi_base + N_q - N_kv;
+    return forward_two_per_sm(g);
+  };
+  check(!two(24, 2048, 8138, 64, 6090, 5, 0) && !two(28, 1825, 7146, 48, 5321, 5, 0) && !two(20, 2048, 6165, 64, 4117, 2, 0), "long windows");
+  check(!two(16, 3000, 3000, 64, 3000, 0, 1) && !two(16, 3000, 3000, 96, 3000, 0, 1) && !two(16, 3000, 3000, 128, 3000, 0, 1), "long, no mask");
+  check(!two(8, 5888, 5888, 96, 5888, 0, 1) && !two(36, 1487, 6545, 96, 5058, 5, 0), "two to three rounds");
+  check(!two(148, 128, 128, 64, 128, 0, 1) && !two(74, 256, 256, 64, 256, 0, 1) && two(76, 256, 256, 64, 256, 0, 1), "one round");
+  check(two(64, 2048, 2048, 64, 2048, 0, 1) && two(128, 1692, 1692, 128, 1692, 0, 1), "many rounds");
+  check(two(16, 2048, 2048, 128, 2048, 0, 1) && two(20, 2048, 2048, 48, 1024, 8, 0), "two rounds of short streams");
+  check(two(96, 2048, 2048, 64, 2048, 0, 0) && two(64, 1024, 1024, 128, 1024, 0, 0) && two(64, 4096, 4096, 128, 4096, 0, 0), "causal");
+  check(two(96, 256, 256, 64, 256, 0, 0) && two(80, 176, 176, 128, 176, 0, 0) && two(80, 174, 363, 96, 189, 5, 0), "causal, short");
+  check(!two(10, 7197, 7197, 64, 7197, 0, 0) && !two(16, 12708, 12708, 64, 12708, 0, 0) && !two(24, 1860, 1860, 80, 1860, 0, 0), "causal, the longest is the bound");
+}
+
 int main() {
+  forward_in_rounds();
   keys_in_front();
   one_answer_for_both_kinds();
   cluster_queries();

@@ -257,13 +257,17 @@ def test_first_backward_with_two_ctas_per_sm(shape, two, dtype):
     assert len(forms) >= 1 and set(forms) == {"1" if two else "0"}, kernels
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("shape,two", [
     ((96, 250, 250, 96, 250, 0, 0), True),          # short streams of unequal length
     ((24, 1500, 1500, 64, 1500, 0, 0), False),
+    ((20, 1000, 1100, 64, 1000, 0, 1), True),       # no mask: two rounds of 148 CTAs, short streams
+    ((22, 900, 3100, 80, 2200, 3, 0), False),       # a window: two rounds, long streams
+    ((148, 120, 200, 64, 200, 0, 1), False),        # one round
 ])
-def test_forward_with_two_ctas_per_sm(shape, two):
+def test_forward_with_two_ctas_per_sm(shape, two, dtype):
     H, N_q, N_kv, D, window, chunk, mask = shape
-    g = _check_against_the_oracle(1, *shape, torch.bfloat16)
+    g = _check_against_the_oracle(1, *shape, dtype)
     kernels = [n for n, _ in captured_kernels(lambda: tcapi.forward(g["Q"], g["K"], g["V"], window, chunk, mask)) if "fwd_kernel" in n]
     forms = [f for n in kernels for f in re.findall(r"fwd_kernelILi\d+E.*?Lb[01]ELi([12])E", n)]      # groups of math warps of a CTA
     assert forms == ["1" if two else "2"], kernels
