@@ -507,10 +507,10 @@ __device__ __forceinline__ void fb_kernel<KIND, D, T, SPLIT, DUAL>::run(const Tm
               pw[hh * 16 + ch * 8 + (e >> 1)] = pp;
             }
         }
-        // With two CTAs per SM the schedulers were what is short (54 % of their slots used, now 42): B4 H16 N2048 D64 without mask 302 -> 278 us,
-        // B8 H12 N2048 D64 causal 261 -> 248, B4 H16 N512 D64 27.0 -> 26.3.  With one, where most tiles may have a mask's edge
-        // and a half-step's latency counts, the test stays in the loop (64 queries against 256 keys 5.9 us, 6.1 with a pass of
-        // its own; B2 H12, 777 of 1301, D80 40.6, 41.3).
+        // With two CTAs per SM the visibility test is a pass of its own over the tiles that need it: in the loop above its three
+        // instructions for an element would run in every tile (B2 H32 N2048 D64 54 % of the issue slots and 317 k cycles; 42 % and 303 k
+        // as it is).  With one, where most tiles may have a mask's edge and a half-step's latency counts, the test stays in the loop (64
+        // queries against 256 keys 5.9 us, 6.1 with a pass of its own; B2 H12, 777 of 1301, D80 40.6, 41.3).
         if (DUAL && __any_sync(0xffffffffu, masked)) mask_pairs(pw, j0 - vlo, vspan);
         ok = mbar_wait(bar_rb_full(b), (it / kBufs) & 1, abort_flag, t.status, wait_code(KCODE, 8));
         ok = __all_sync(0xffffffffu, ok);
@@ -732,7 +732,7 @@ __device__ __forceinline__ void fb_kernel<KIND, D, T, SPLIT, DUAL>::run(const Tm
   pdl_end(g);
 }
 
-// How a kind is launched: two CTAs per SM, CTAs per tile.
+// How a kind is launched: two CTAs per SM (backward_two_per_sm), CTAs per tile.
 struct FbPlan { bool dual; int split; };
 
 template <int KIND, int D, typename T>

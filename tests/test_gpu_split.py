@@ -237,24 +237,46 @@ def test_first_backward_in_one_grid_and_in_two_gives_the_same_bits(H, D, dtype):
         assert torch.equal(one, two), name
 
 
+def _backward_forms(call):
+    """[two CTAs per SM] of each launch of the first backward's tiles (both kinds of a pair have the same form)."""
+    kernels = [n for n, _ in captured_kernels(call) if "fb_kernel" in n]
+    forms = [f for n in kernels for f in re.findall(r"fb_kernelILi\d+ELi64E.*?Lb[01]ELb([01])E", n)[:1]]
+    assert len(forms) == len(kernels), kernels
+    return [f == "1" for f in forms]
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
-@pytest.mark.parametrize("shape,two", [
-    ((24, 1000, 1000, 64, 1000, 0, 0), True),       # causal, ragged: 192 tiles of either side
-    ((32, 700, 1500, 48, 333, 2, 0), True),         # both edges of a window inside the tiles
-    ((48, 500, 450, 64, 500, 0, 1), True),          # no mask: equal CTAs of short streams, the ends of both axes
-    ((80, 250, 250, 64, 20, 0, 0), True),           # a narrow window: most scores of every tile masked
-    ((10, 2000, 2000, 64, 2000, 0, 0), False),      # few tiles, long streams: the longest CTA would be the bound
-    ((28, 778, 1139, 64, 778, 0, 1), True),         # no mask: more than three rounds of CTAs, both kinds together
-    ((24, 1060, 1060, 64, 1060, 0, 1), False),      # no mask: three rounds
-    ((20, 128, 1374, 64, 1246, 0, 0), False),       # 220 tiles of keys, 180 of them in front of the sequence
+@pytest.mark.parametrize("shape,forms", [
+    ((24, 1000, 1000, 64, 1000, 0, 0), [True]),         # causal, ragged: 192 tiles of either side
+    ((32, 700, 1500, 48, 333, 2, 0), [True]),           # both edges of a window inside the tiles
+    ((48, 500, 450, 64, 500, 0, 1), [True]),            # no mask: equal CTAs of short streams, the ends of both axes
+    ((80, 250, 250, 64, 20, 0, 0), [True]),             # a narrow window: most scores of every tile masked
+    ((10, 2000, 2000, 64, 2000, 0, 0), [False]),        # few tiles, long streams: the longest CTA would be the bound
+    ((28, 778, 1139, 64, 778, 0, 1), [True]),           # no mask: more than three rounds of CTAs, both kinds together
+    ((24, 1060, 1060, 64, 1060, 0, 1), [False]),        # no mask: three rounds
+    ((16, 1600, 2200, 64, 1600, 0, 1), [True, True]),   # streams of more than 33 tiles: a launch for each kind
+    ((20, 128, 1374, 64, 1246, 0, 0), [False]),         # 220 tiles of keys, 180 of them in front of the sequence
+    ((24, 187, 1440, 48, 1253, 5, 0), [False, True]),   # fewer tiles of queries than SMs: the keys' kind decides by itself
 ])
-def test_first_backward_with_two_ctas_per_sm(shape, two, dtype):
+def test_first_backward_with_two_ctas_per_sm(shape, forms, dtype):
     H, N_q, N_kv, D, window, chunk, mask = shape
     g = _check_against_the_oracle(1, *shape, dtype)
     O, L = tcapi.forward(g["Q"], g["K"], g["V"], window, chunk, mask)
-    kernels = [n for n, _ in captured_kernels(lambda: tcapi.backward(g["dO"], g["Q"], g["K"], g["V"], O, L, window, chunk, mask)) if "fb_kernel" in n]
-    forms = [f for n in kernels for f in re.findall(r"fb_kernelILi\d+ELi64E.*?Lb[01]ELb([01])E", n)]
-    assert len(forms) >= 1 and set(forms) == {"1" if two else "0"}, kernels
+    got = _backward_forms(lambda: tcapi.backward(g["dO"], g["Q"], g["K"], g["V"], O, L, window, chunk, mask))
+    assert sorted(got) == forms
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_first_backward_with_one_and_two_ctas_per_sm_gives_the_same_bits(dtype):
+    """24 heads have two CTAs per SM, the first 10 of them by themselves one; neither form shares a tile over a cluster."""
+    N = 1000
+    g = {n: t.cuda() for n, t in orc.make_inputs(1, 24, N, N, 64, seed=24, dtype=dtype).items()}
+    args = [g["dO"], g["Q"], g["K"], g["V"], *tcapi.forward(g["Q"], g["K"], g["V"], N, 0, 0)]
+    few = [t[:, :10].contiguous() for t in args]
+    calls = [lambda a=a: tcapi.backward(*a, N, 0, 0) for a in (args, few)]
+    assert [_backward_forms(c) for c in calls] == [[True], [False]]
+    for two, one, name in zip(calls[0](), calls[1](), ("dQ", "dK", "dV")):
+        assert torch.equal(two[:, :10], one), name
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
