@@ -435,17 +435,15 @@ __device__ __forceinline__ bool work_next(WorkControl* w, int n, int* unit, vola
 // last round of up to 148 takes 0.8 of a whole one, half of its CTAs having an SM to themselves.  The rounds come apart as there
 // are more of them.  Long streams, whose tiles take longer with two CTAs per SM, so want whole rounds: forward, D64, 24 heads
 // of 2048 queries against a window of 6090 (2.6 rounds) 122 us with one per SM, 164 with two; 16 heads N3000 without mask
-// 67 and 77; but 64 heads N2048 without mask (6.9 rounds) 107 and 99.  1539 drawn sizes of 90 to 16384 rows, masks and
-// no masks, both forms timed: the form taken is 0.3 % from the faster one on average, 1.4 % with 850 clocks per tile in either
-// form and no rounds of 296; the 252 that change form take 0.935 of the time (0.74 to 1.22, 30 of them more than 1.02).
+// 67 and 77; but 64 heads N2048 without mask (6.9 rounds) 107 and 99.
 inline bool two_per_sm_pays_in_rounds(const SplitLoad& w, float tile_clocks_two) {
   if (w.busy <= kSms) return false;      // one round: 74 heads N256 D64 without mask 5.7 us, 7.0 with a group of math warps for each
   const long long n = (long long)w.busy, ones = (n - 1) / kSms, pairs = n / (2 * kSms), rest = n % (2 * kSms);
   // rounds, the last one whole, and by how much the others' coming apart makes up for that
   const float per_sm = w.busy / kSms, per_pair = per_sm / 2.f, last = rest == 0 ? 0.f : rest <= kSms ? 0.8f : 1.f;
   const float rounds = per_sm + (ones + 1 - per_sm) / (1.f + 0.1f * ones);
-  const float rounds_two = per_pair + (pairs + last - per_pair) / (1.f + 0.5f * pairs);
-  return rounds_two * (2.f * w.busy_mean * tile_clocks_two + 8000.f) < rounds * (w.busy_mean * w.tile_clocks + 10000.f);
+  const float rounds_two = per_pair + (pairs + last - per_pair) / (1.f + 0.3f * pairs);
+  return rounds_two * (2.f * w.longest * tile_clocks_two + 8000.f) < rounds * (w.busy_mean * w.tile_clocks + 10000.f);
 }
 
 // Two CTAs per SM, each with half of the tensor memory and one group of math warps (the forward, and
@@ -462,22 +460,28 @@ inline bool two_per_sm_pays_in_rounds(const SplitLoad& w, float tile_clocks_two)
 inline bool two_per_sm_pays(const SplitLoad& w, bool alone, float tile_clocks_two) {
   if (w.busy < kSms) return false;
   auto larger = [](float x, float y) { return x > y ? x : y; };
-  if (alone && w.busy_mean > 0.88f * w.longest) return two_per_sm_pays_in_rounds(w, tile_clocks_two);
+  if (alone && w.busy_mean > 0.9f * w.longest) return two_per_sm_pays_in_rounds(w, tile_clocks_two);
   const float per_sm = w.busy / kSms;
   const float one = larger(w.longest * w.tile_clocks + kCtaClocks, per_sm * (w.busy_mean * w.tile_clocks + kCtaClocks));
   // the longest CTA of a few short ones (up to 8 tiles) that have the GPU to themselves pays less, its neighbour being done before it
-  const float besides = !alone ? 9000.f : w.longest <= 8.f ? 4000.f : 10000.f;
-  const float two = larger(2.f * w.longest * tile_clocks_two + besides, per_sm * (w.busy_mean * tile_clocks_two + (alone ? 2000.f : 4000.f)));
-  return two < 0.95f * one;
+  const float besides = !alone ? 9000.f : w.longest <= 8.f ? 5000.f : kCtaClocks;
+  const float two = larger(2.f * w.longest * tile_clocks_two + besides, per_sm * (w.busy_mean * tile_clocks_two + (alone ? 1000.f : 4000.f)));
+  return two < (alone ? 0.97f : 0.95f) * one;
 }
 inline bool two_per_sm_pays(const Geometry& g, bool col, bool alone, float tile_clocks, float tile_clocks_two) {
   return (long long)g.BH * (((col ? g.N_kv : g.N_q) + BM - 1) / BM) >= kSms && two_per_sm_pays(stream_load(g, col, tile_clocks), alone, tile_clocks_two);
 }
 
-// Forward: a streamed tile takes 700 clocks with one CTA (of two groups of math warps) per SM, 850 per CTA with two, more above D = 64
+// Forward: clocks of a streamed tile with one CTA (of two groups of math warps) per SM, and of each of two.  The time depends
+// on the data: where rows are peaked (Q and K of twice unit variance against once) a row's reference moves more often, and the time
+// with two per SM over that with one changes by 0.95 to 0.83 at D <= 64, the longer the streams the more, and by 1.04 to 1.11 at
+// D > 64 up to 40 tiles, 1.0 from 80 on.  The host does not see the data, so the clocks lie between those of either kind.
+// 1577 drawn sizes (90 to 16384 rows, causal, windows, no mask, D = 48 to 128), both forms timed: the form taken is 0.6 % from the faster
+// one on average, 0.5 % with peaked rows; 1.5 and 1.0 % with 850 clocks in either form and no rounds of 296.  The 156 that
+// change form take 0.915 and 0.949 of the time (0.74 to 1.16 and 0.72 to 1.13).
 inline bool forward_two_per_sm(const Geometry& g) {
   const float past = g.D > 64 ? g.D - 64.f : 0.f;
-  return two_per_sm_pays(g, false, true, 700.f + 3.f * past, 850.f + 2.f * past);
+  return two_per_sm_pays(g, false, true, 710.f + 3.2f * past, g.D > 64 ? 870.f + 1.5f * past : 770.f);
 }
 
 // First backward at D <= 64: clocks of a streamed tile of dQ and of dK/dV, with one and with two CTAs per SM

@@ -153,7 +153,8 @@ static void forward_in_rounds() {
   check(two(16, 2048, 2048, 128, 2048, 0, 1) && two(20, 2048, 2048, 48, 1024, 8, 0), "two rounds of short streams");
   check(two(96, 2048, 2048, 64, 2048, 0, 0) && two(64, 1024, 1024, 128, 1024, 0, 0) && two(64, 4096, 4096, 128, 4096, 0, 0), "causal");
   check(two(96, 256, 256, 64, 256, 0, 0) && two(80, 176, 176, 128, 176, 0, 0) && two(80, 174, 363, 96, 189, 5, 0), "causal, short");
-  check(!two(10, 7197, 7197, 64, 7197, 0, 0) && !two(16, 12708, 12708, 64, 12708, 0, 0) && !two(24, 1860, 1860, 80, 1860, 0, 0), "causal, the longest is the bound");
+  check(two(96, 12000, 12000, 64, 12000, 0, 0) && two(48, 9345, 9345, 64, 9345, 0, 0) && two(32, 16384, 16384, 128, 16384, 0, 0), "causal, many rounds");
+  check(!two(16, 12488, 12488, 80, 12488, 0, 0) && !two(24, 1860, 1860, 80, 1860, 0, 0) && !two(24, 1500, 1500, 64, 1500, 0, 0), "causal, one per SM");
 }
 
 int main() {
